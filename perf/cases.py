@@ -129,7 +129,8 @@ def _csc_matrix(c, seed):
         cap = max(20, n // 50)
         raw = np.minimum(np.random.default_rng(seed).zipf(1.2, size=d), cap).astype(np.float64)
         counts = np.round(raw * (c["per_col"] * d / raw.sum())).astype(np.int64)
-        counts = torch.from_numpy(np.clip(counts, 1, cap)).cuda()
+        # at least 8 entries: shorter columns coincide now and then, and x is then not unique
+        counts = torch.from_numpy(np.clip(counts, 8, cap)).cuda()
     else:
         counts = torch.full((d,), c["per_col"], dtype=torch.int64, device="cuda")
     cols = torch.repeat_interleave(torch.arange(d, device="cuda"), counts)
