@@ -17,7 +17,8 @@ constexpr int kGBM = 64, kGBN = 64, kGBK = 16;
 
 // TRI = 0: general.  TRI = 1: op(A) is upper triangular (terms with k < row
 // vanish).  TRI = 2: op(B) is upper triangular (terms with k > col vanish).
-// Tiles skip the K range that is structurally zero.
+// Tiles skip the K range that is structurally zero.  TRI = 3: only the tiles on
+// and above C's diagonal are formed (a symmetric product's upper half).
 // BAT: blockIdx.z indexes a batch of equally shaped products whose operands
 // sit bsa / bsb / bsc elements apart (no split-K).
 template <typename T, bool TA, bool TB, int TRI = 0, bool BAT = false>
@@ -32,6 +33,7 @@ k_gemm(int M, int N, int K, T alpha, const T* __restrict__ A, int64_t lda,
     const int tid = threadIdx.x;
     const int tx = tid & 15, ty = tid >> 4;     // 16 x 16 threads
     const int m0 = blockIdx.x * kGBM, n0 = blockIdx.y * kGBN;
+    if (TRI == 3 && n0 + kGBN <= m0) return;
     if (BAT) {
         A += blockIdx.z * bsa;
         B += blockIdx.z * bsb;
@@ -451,7 +453,7 @@ inline void gemm_launch_generic(bool ta, bool tb, int M, int N, int K, T alpha, 
                                 T* partial, int64_t partial_cap, int tri, cudaStream_t st)
 {
     if (M <= 0 || N <= 0) return;
-    int splits = (K > 0 && partial && tri == 0) ? gemm_splits(M, N, K) : 1;
+    int splits = (K > 0 && partial && (tri == 0 || tri == 3)) ? gemm_splits(M, N, K) : 1;
     while (splits > 1 && (int64_t)splits * M * N > partial_cap) splits >>= 1;
     int kchunk = K;
     if (splits > 1) {
@@ -465,6 +467,8 @@ inline void gemm_launch_generic(bool ta, bool tb, int M, int N, int K, T alpha, 
     if (tri == 1) launch_k(k_gemm<T, false, false, 1>, grid, 256, 0, st, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, kchunk, part,
                                   (int64_t)0, (int64_t)0, (int64_t)0);
     else if (tri == 2) launch_k(k_gemm<T, false, false, 2>, grid, 256, 0, st, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, kchunk, part,
+                                  (int64_t)0, (int64_t)0, (int64_t)0);
+    else if (tri == 3) launch_k(k_gemm<T, true, false, 3>, grid, 256, 0, st, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, kchunk, part,
                                   (int64_t)0, (int64_t)0, (int64_t)0);
     else if (!ta && !tb) launch_k(k_gemm<T, false, false>, grid, 256, 0, st, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, kchunk, part,
                                   (int64_t)0, (int64_t)0, (int64_t)0);
@@ -553,6 +557,16 @@ void trmm(int tri, int M, int N, int K, T alpha, const T* A, int64_t lda, const 
 {
     gemm_launch<T>(false, false, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, partial, partial_cap, tri,
                    st);
+}
+
+// C = alpha * A^T * B + beta * C on the 64 x 64 tiles on and above the diagonal
+// of C (the other tiles are not written, or hold nothing of use).
+template <typename T>
+void gemm_upper(int M, int N, int K, T alpha, const T* A, int64_t lda, const T* B, int64_t ldb, T beta,
+                T* C, int64_t ldc, T* partial, int64_t partial_cap, cudaStream_t st)
+{
+    gemm_launch_generic<T>(true, false, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, partial, partial_cap,
+                           3, st);
 }
 
 // batch products C_z = alpha op(A_z) op(B_z) + beta C_z, z = 0..batch-1, with

@@ -116,7 +116,7 @@ __global__ void k_inf_rowsum_max(const double* __restrict__ part, int nchunks, i
 }
 
 template <typename T>
-static void inf_norm_upper(const T* X, int64_t ld, int64_t r, double* part, double* out, cudaStream_t st)
+void inf_norm_upper(const T* X, int64_t ld, int64_t r, double* part, double* out, cudaStream_t st)
 {
     const int nchunks = (int)((r + kInfCols - 1) / kInfCols);
     dim3 g((unsigned)((r + kInfRows - 1) / kInfRows), nchunks);
@@ -215,6 +215,8 @@ int64_t count_rank(const T* R, int64_t ld, int64_t dmin, double abs_thresh, doub
     return *host_pinned;
 }
 
+template void inf_norm_upper<float>(const float*, int64_t, int64_t, double*, double*, cudaStream_t);
+template void inf_norm_upper<double>(const double*, int64_t, int64_t, double*, double*, cudaStream_t);
 template size_t trinv_workspace_bytes<float>(int64_t);
 template size_t trinv_workspace_bytes<double>(int64_t);
 template void trinv_upper<float>(const float*, int64_t, int64_t, double, float*, int64_t, double*,

@@ -312,7 +312,8 @@ static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, do
 
     // ---- workspace layout (sized once, then carved) ----
     const size_t qr_ws = cpqr_workspace_bytes<T>(m, d);
-    const size_t inv_ws = trinv_workspace_bytes<T>(d) + (size_t)d * d * sizeof(T);
+    const size_t inv_ws = std::max(trinv_workspace_bytes<T>(d) + (size_t)d * d * sizeof(T),
+                                   gram_enabled() && m >= d ? gram_workspace_bytes<T>(m, d) : 0);
     LsqrProblem Pq;
     Pq.n = n; Pq.d = d; Pq.nnz = nnz; Pq.r = d; Pq.precision = o.precision;
     const size_t lsqr_ws = lsqr_workspace_bytes(Pq);
@@ -329,6 +330,7 @@ static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, do
     S.add<char>((int64_t)std::max({qr_ws, inv_ws, lsqr_ws, csr_scr, bkt_scr}));
     S.add<float2>(d);
     S.add<double>(m);
+    S.add<int>(kGramDropMax);
     C.arena.reserve(S.bytes());
     C.arena.reset();
     Arena& Ar = C.arena;
@@ -359,6 +361,7 @@ static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, do
     double* scal = Ar.alloc<double>(8);
     void* work = Ar.take(std::max({qr_ws, inv_ws, lsqr_ws, csr_scr, bkt_scr}));
     float2* ysplit = Ar.alloc<float2>(d);
+    int* drop = Ar.alloc<int>(kGramDropMax);
     double* gm = Ar.alloc<double>(m);   // S r_s during the sketch-solution refinement
 
     cudaEvent_t* ev = C.ev;
@@ -420,7 +423,7 @@ static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, do
     }
     trace_phase(st, "sketch");
     SKL_CUDA(cudaEventRecord(ev[3], st));
-    // ---- randomized CPQR, c = Q^T S b ----
+    // ---- factorization of the sketch, c = coefficients of S b ----
     if (tuning && mixed) {
         // whole factorizations of a copy of the sketch at each panel width
         T* SAc = nullptr;
@@ -447,16 +450,7 @@ static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, do
         SKL_CUDA(cudaFreeAsync(cc, st));
         SKL_CUDA(cudaMemsetAsync(C.dev_status, 0, sizeof(unsigned), st));
     }
-    cpqr<T>(SA, m, d, ld, jpvt, tau, work, C.dev_status, st, cvec, 1,
-            o.profile ? info.qr_prof_ms : nullptr, tuned.nb);
-    {
-        const unsigned qs = read_status(C, st);
-        if (qs & kStatusTcTimeout) fail(SKL_ERR_TIMEOUT, "a kernel's bounded wait gave up (tensor-core product or sample QRP exchange)");
-        if (qs & kQrSelectBit) fail(SKL_ERR_NONFINITE, "non-finite values in the sketch factorization");
-    }
-    trace_phase(st, "cpqr");
-    SKL_CUDA(cudaEventRecord(ev[4], st));
-    // ---- rank, inverse, condition ----
+    // ---- the rank rule ----
     // FP64: SPQR's default tolerance 20 (m + d) eps relative to the largest
     // (equilibrated) column.  FP32: an exactly dependent column leaves |R_ii|
     // of up to ~sqrt(m) eps_32 |R_00| (measured: 1.6e-6 at m = 8,500), so the
@@ -471,24 +465,51 @@ static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, do
     if (!(rel > 0.0))
         rel = mixed ? 2.0 * std::sqrt((double)m) * 5.960464477539063e-08
                     : 20.0 * (double)(m + d) * 2.220446049250313e-16;
-    int64_t rank = count_rank<T>(SA, ld, mn, 0.0, rel, dint, (int*)C.host_pinned, st);
-    if (rank == 0) fail(SKL_ERR_RANK_ZERO, "SPQR Factorization fails");
-    info.rank = rank;
-    const int64_t rank_lsqr = carry_unresolved ? mn : rank;
-    info.unresolved_cols = rank_lsqr - rank;
-    const int64_t ldm = round_up(rank_lsqr, 4);   // 16-byte aligned rows/columns of M
-    trinv_upper<T>(SA, ld, rank, 0.0, Mc, ldm, norms, work, st);
-    SKL_CUDA(cudaMemcpyAsync(C.host_pinned, norms, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
-    SKL_CUDA(cudaStreamSynchronize(st));
-    double nr = ((double*)C.host_pinned)[0], nm = ((double*)C.host_pinned)[1];
-    double rcond = (nr > 0 && nm > 0) ? 1.0 / (nr * nm) : 0.0;
-    info.rcond_r11 = rcond;
-    info.success = rcond > o.rcond_threshold ? 1 : 0;
-    if (!info.success && o.perturb != 0.0) {
-        trinv_upper<T>(SA, ld, rank, o.perturb, Mc, ldm, norms, work, st);
+    int64_t rank = d, rank_lsqr = d;
+    int64_t ldm = round_up(d, 4);   // 16-byte aligned rows/columns of M
+    GramResult gres;
+    // a well-conditioned sketch (but for exactly dependent columns, carried below):
+    // Cholesky of its Gram matrix, the rank proven from M; any other one:
+    // randomized CPQR, rank by its diagonal
+    const bool gram = gram_enabled() && m >= d &&
+                      gram_precond<T>(SA, m, d, ld, cvec, jpvt, Mc, Mr, ldm, 0.0, rel, o.rcond_threshold, gres,
+                                      carry_unresolved ? drop : nullptr, work, C.dev_status, C.host_pinned, st);
+    if (gram) {
+        info.rank = d - gres.dropped;
+        info.unresolved_cols = gres.dropped;
+        info.rcond_r11 = 1.0 / (gres.norm_r * gres.norm_m);
+        info.success = 1;
+        SKL_CUDA(cudaEventRecord(ev[4], st));
+    } else {
+        cpqr<T>(SA, m, d, ld, jpvt, tau, work, C.dev_status, st, cvec, 1,
+                o.profile ? info.qr_prof_ms : nullptr, tuned.nb);
+        {
+            const unsigned qs = read_status(C, st);
+            if (qs & kStatusTcTimeout) fail(SKL_ERR_TIMEOUT, "a kernel's bounded wait gave up (tensor-core product or sample QRP exchange)");
+            if (qs & kQrSelectBit) fail(SKL_ERR_NONFINITE, "non-finite values in the sketch factorization");
+        }
+        trace_phase(st, "cpqr");
+        SKL_CUDA(cudaEventRecord(ev[4], st));
+        // ---- rank, inverse, condition ----
+        rank = count_rank<T>(SA, ld, mn, 0.0, rel, dint, (int*)C.host_pinned, st);
+        if (rank == 0) fail(SKL_ERR_RANK_ZERO, "SPQR Factorization fails");
+        info.rank = rank;
+        rank_lsqr = carry_unresolved ? mn : rank;
+        info.unresolved_cols = rank_lsqr - rank;
+        ldm = round_up(rank_lsqr, 4);   // 16-byte aligned rows/columns of M
+        trinv_upper<T>(SA, ld, rank, 0.0, Mc, ldm, norms, work, st);
+        SKL_CUDA(cudaMemcpyAsync(C.host_pinned, norms, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
+        SKL_CUDA(cudaStreamSynchronize(st));
+        double nr = ((double*)C.host_pinned)[0], nm = ((double*)C.host_pinned)[1];
+        double rcond = (nr > 0 && nm > 0) ? 1.0 / (nr * nm) : 0.0;
+        info.rcond_r11 = rcond;
+        info.success = rcond > o.rcond_threshold ? 1 : 0;
+        if (!info.success && o.perturb != 0.0) {
+            trinv_upper<T>(SA, ld, rank, o.perturb, Mc, ldm, norms, work, st);
+        }
+        extend_identity<T>(Mc, ldm, rank, rank_lsqr, st);
+        transpose_upper<T>(Mc, ldm, rank_lsqr, Mr, st);
     }
-    extend_identity<T>(Mc, ldm, rank, rank_lsqr, st);
-    transpose_upper<T>(Mc, ldm, rank_lsqr, Mr, st);
     trace_phase(st, "rank+inverse");
     LsqrProblem P;
     P.n = n; P.d = d; P.nnz = nnz;
@@ -584,6 +605,7 @@ static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, do
         // 120,000 x 5,000 workload that left ||b - A x|| 1.4e-3 relative above
         // the minimum and the backward error at 2.3e-3 instead of 3.4e-4).
         P.r = rank_lsqr;
+        gram_unit_dropped(drop, gres.dropped, Mc, Mr, ldm, st);
         int64_t total_it = 0;
         int flag = 1;
         int64_t restarts = 0;

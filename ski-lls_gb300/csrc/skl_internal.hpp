@@ -211,6 +211,42 @@ template <typename T>
 int64_t count_rank(const T* R, int64_t ld, int64_t dmin, double abs_thresh, double rel_thresh,
                    int* dev_out, int* host_pinned, cudaStream_t st);
 
+// *out = max(*out, ||upper triangle of X (r x r, ld)||_inf); part holds
+// ceil(r / 128) * r doubles.
+template <typename T>
+void inf_norm_upper(const T* X, int64_t ld, int64_t r, double* part, double* out, cudaStream_t st);
+
+// -------------------------------------------------------- k_gramchol.cu --
+// Preconditioner of a well-conditioned sketch SA (m x d, ld, m >= d) by Cholesky
+// of its Gram matrix.  Returns true when the sketch provably has full rank
+// under the rule |R_ii| > max(abs_thresh, rel_thresh |R_00|) for every column
+// order, is well conditioned enough for the Gram matrix, and
+// 1 / (||R||_inf ||M||_inf) > rcond_min: then Mc (column-major) and Mr (its
+// row-major copy, both ldm, a multiple of 4) hold M = R^{-1} in natural column
+// order (jpvt = 0..d-1) and c (m entries, S b on entry; may be null) the d
+// coefficients of the sketched least-squares solution x = M c.
+// With drop (device, kGramDropMax entries; FP32 only) up to d / 4 columns may
+// depend on the others at FP32 resolution (distance at most a quarter of the
+// rule's threshold): res.dropped of them are listed, their rows and columns of
+// M and entries of c are zero.
+// Otherwise false: SA and c are untouched, Mc and Mr undefined.
+constexpr int kGramDropMax = 512;
+struct GramResult {
+    double norm_r = 0.0, norm_m = 0.0;   // ||R||_inf, ||M||_inf of the kept columns
+    int64_t dropped = 0;
+};
+template <typename T>
+size_t gram_workspace_bytes(int64_t m, int64_t d);
+template <typename T>
+bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int* jpvt, T* Mc, T* Mr, int64_t ldm,
+                  double abs_thresh, double rel_thresh, double rcond_min, GramResult& res, int* drop, void* work,
+                  unsigned* status, void* host_pinned, cudaStream_t st);
+// M(j, j) = 1 for the k dropped columns (LSQR carries them unpreconditioned).
+void gram_unit_dropped(const int* drop, int64_t k, float* Mc, float* Mr, int64_t ldm, cudaStream_t st);
+void gram_unit_dropped(const int* drop, int64_t k, double* Mc, double* Mr, int64_t ldm, cudaStream_t st);
+// SKILLS_GRAM=0 always takes the pivoted (or blocked) QR, for comparison.
+bool gram_enabled();
+
 // ------------------------------------------------------------ k_lsqr.cu --
 struct LsqrProblem {
     int64_t n = 0, d = 0, nnz = 0;
