@@ -720,7 +720,7 @@ def run_batched(args, rank, world):
         "config": {"workload": "batched_sparse", "problems": total,
                    "problems_per_rank": len(probs),
                    "d_range": [50, 500], "n_rule": "n ~ U[2000, 50000], n >= 20 d",
-                   "streams": int(os.environ.get("SKILLS_BATCH_STREAMS", "8")), "gamma": 1.7,
+                   "streams": int(os.environ.get("SKILLS_BATCH_STREAMS", "16")), "gamma": 1.7,
                    "k": 2, "it_tol": IT_TOL, "backward_tol": BATCH_BACKWARD_TOL, "inputs": "host buffers (H2D inside the timing)"},
         "e2e": {"value": total / best, "unit": "problems/s",
                 "h2d_bytes_per_step": int(sum(16 * A.nnz + 8 * (A.shape[1] + 1) + 8 * A.shape[0]

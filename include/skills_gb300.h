@@ -185,7 +185,7 @@ skl_status skl_dense_solve(const double* A, int64_t lda, int64_t n, int64_t d,
  * of every problem is drawn in problem order exactly as a loop of
  * skl_sparse_solve calls with the same options would draw it, so each x[p] is
  * bit-identical to that loop's; the problems then run concurrently on worker
- * threads, each with its own stream (SKILLS_BATCH_STREAMS, default 8;
+ * threads, each with its own stream (SKILLS_BATCH_STREAMS, default 16;
  * opts->stream is not used).  info[p] and status[p] (both optional) per
  * problem; the return value is the first failing problem's status. */
 skl_status skl_batched_sparse_solve(int64_t nprob, const skl_csc* A, const double* const* b,

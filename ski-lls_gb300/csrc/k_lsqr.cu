@@ -35,6 +35,7 @@
 #include "skl_internal.hpp"
 #include "launch.cuh"
 #include "common.cuh"
+#include "lsqr_types.cuh"
 
 namespace skl {
 
@@ -130,50 +131,6 @@ SKL_DEV bool arrive_last(unsigned* counter)
     __syncthreads();
     return last;
 }
-
-template <bool MIXED>
-struct VecT {
-    using type = double;
-};
-template <>
-struct VecT<true> {
-    using type = float2;
-};
-
-template <bool MIXED>
-SKL_DEV typename VecT<MIXED>::type store_val(double x)
-{
-    if constexpr (MIXED) {
-        ff f = ff_from_double(x);
-        return make_float2(f.hi, f.lo);
-    } else {
-        return x;
-    }
-}
-
-template <bool MIXED>
-struct Acc {
-    ff a{0.f, 0.f};
-    SKL_DEV void fma_mv(float2 m, float2 x) { ff_fma(a, ff{m.x, m.y}, ff{x.x, x.y}); }
-    SKL_DEV void fma_f(float m, float2 x) { ff_fma_f(a, m, ff{x.x, x.y}); }
-    SKL_DEV void add(const Acc& o) { ff_add(a, o.a); }
-    SKL_DEV Acc shfl_xor(int o) const { Acc r; r.a = ff_shfl_xor(a, o); return r; }
-    SKL_DEV double value() const { return ff_to_double(a); }
-};
-template <>
-struct Acc<false> {
-    double a = 0.0;
-    SKL_DEV void fma_mv(double m, double x) { a = fma(m, x, a); }
-    SKL_DEV void fma_f(double m, double x) { a = fma(m, x, a); }
-    SKL_DEV void add(const Acc& o) { a += o.a; }
-    SKL_DEV Acc shfl_xor(int o) const { Acc r; r.a = __shfl_xor_sync(0xffffffffu, a, o); return r; }
-    SKL_DEV double value() const { return a; }
-};
-
-template <bool MIXED>
-using MatT = typename std::conditional<MIXED, float, double>::type;
-template <bool MIXED>
-using ValT = typename VecT<MIXED>::type;   // stored A values: float2 (hi,lo) or double
 
 // ------------------------------------------------------- triangular dots --
 // Partial dot of M[j0:j1] (contiguous) with v[j0:j1] for one thread of a block
@@ -940,6 +897,8 @@ size_t lsqr_workspace_bytes(const LsqrProblem& P)
     if (P.Ad) {
         const int c = dense_n_chunk(P);
         b += (size_t)((P.r + c - 1) / c) * P.n * sizeof(double) + 256;
+    } else {
+        b = std::max(b, lsqr_persist_workspace_bytes(P));
     }
     return b;
 }
@@ -1175,6 +1134,8 @@ LsqrResult lsqr_run(const LsqrProblem& P, const double* b, double tol, int64_t m
                     cudaStream_t capture_stream)
 {
     (void)status;
+    if (lsqr_persist_fits(P))
+        return lsqr_persist_run(P, b, tol, max_it, y, work, host_pinned, st, profile, capture_stream);
     if (P.precision == SKL_PREC_MIXED)
         return run_impl<true>(P, b, tol, max_it, y, work, host_pinned, st, profile, capture_stream);
     return run_impl<false>(P, b, tol, max_it, y, work, host_pinned, st, profile, capture_stream);

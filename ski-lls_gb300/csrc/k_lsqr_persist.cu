@@ -1,0 +1,1063 @@
+// k_lsqr_persist.cu -- the whole LSQR iteration in one persistent kernel
+// (sparse problems).
+//
+// The iteration of k_lsqr.cu (src/IterSolver.cpp:160-284) is five kernels of
+// 5-15 us that each do a few microseconds of work on problems up to a few
+// thousand columns: 30-40 us per iteration went into ramp-up, tails, the
+// launches between them and a host round trip per four iterations (20,000 x
+// 1,000: 36 us per iteration, here 22; 31,013 x 1,507: 40 -> 24; 2,000 x 60: 30 ->
+// 14; 1e6 x 1e4, which streams 0.6 GB: 288 -> 205).  Here the CTAs stay resident and the phases are separated by grid barriers:
+//   A  z = M v        rows of the triangle, v in shared memory
+//   B  u = A z - (alpha / beta) u,  partial ||u||^2      z in shared memory
+//   C  t = A^T u      column chunks
+//   D  v = M^T t / beta - (beta / alpha) v,  partial ||v||^2   t in shared memory
+// u and v stay unnormalised and every scale (1 / alpha, 1 / beta) is applied by
+// the phase after the one that would have waited for the norm, so an iteration
+// has four barriers; each CTA reduces the norms' partials itself, in the same
+// order, and runs the scalar recurrences redundantly.  Small problems run as
+// one 16-CTA cluster (hardware barrier, no co-residency to ask for, so several
+// of them share the GPU), larger ones as a cooperative grid of one CTA per SM.
+//
+// Work split: phases A and D deal the triangle's rows (columns) to the CTAs in
+// snake order, so that every CTA has long and short ones, and cut each into S
+// segments, one warp per segment; the segments' sums meet in shared memory and
+// one thread per row finishes it.  Phase C cuts columns into chunks of at most
+// kChunkSteps steps, so that a power-law column does not hang on one warp; the
+// last chunk of a column to finish adds the column's chunks up in order.
+// Every sum has a fixed order: results are bitwise reproducible.
+// FP64 is slow enough (see Sum) that the scalar recurrences of one lane take 2-5
+// us: a warp of their own runs them beside phases A (alpha) and C (beta), and
+// another one updates y and w of the previous iteration beside phase C.
+#include <algorithm>
+#include <chrono>
+#include <cmath>
+#include <cstdlib>
+#include <cstring>
+#include <vector>
+
+#include "skl_internal.hpp"
+#include "launch.cuh"
+#include "common.cuh"
+#include "lsqr_types.cuh"
+
+namespace skl {
+
+namespace {
+
+// Threads per CTA: 512 (two CTAs of different solves fit an SM, barriers and block
+// sums are cheaper), 1,024 for problems that stream from HBM.
+constexpr int kSmallCta = 512, kBigCta = 1024;
+constexpr int kCluster = 16;              // CTAs of the single-cluster variant
+constexpr int kIterPerGraph = 4;          // iterations per graph of phase kernels
+constexpr int kTU = 8;                    // entries per lane per step (columns)
+// Steps per column chunk (1e6 x 1e4, power-law columns, LSQR of 118 iterations: 24.8 ms
+// with 2, 25.3 with 4, 27.8 with 8, 29.3 with 16).
+constexpr int kChunkSteps = 2;
+constexpr unsigned kBarLimit = 1u << 23;  // polls before a grid barrier gives up
+constexpr int kItersPerLaunch = 256;
+
+// Scalars of the iteration: one copy per CTA in the persistent kernel, two
+// slots in memory otherwise (a phase kernel reads one and writes the other).
+struct PScal {
+    double alpha, beta, rhobar, phibar, nrm_a, nrm_ar;
+    double ia, ib, coef_n, coef_t;         // 1/alpha, 1/beta, alpha/beta, beta/alpha
+    double cs, sn, irho, t1, t2;
+    double y_t1, y_t2, y_ia;               // the outstanding update of y and w
+    long long it;
+    int done, flag;
+    int pend;              // a finished iteration's alpha scalars are outstanding
+    int ypend;             // its update of y and w is outstanding
+};
+
+struct PState {
+    PScal sc[2];
+    double tol;
+    long long max_it;
+    unsigned bar;          // grid barrier arrivals of this launch
+    int timeout;
+};
+
+template <bool MIXED>
+struct PArgs {
+    using V = ValT<MIXED>;
+    using MT = MatT<MIXED>;
+    int n, r, d, L_n, L_t, S_seg;
+    const int* rp; const int* ci; const V* cv;      // CSR
+    const int* cp; const int* ri; const V* rv;      // CSC
+    const int* cols; const double* opscale;
+    const int4* chunks;       // per chunk: CSC range, column slot, chunks of the column
+    const int* coff;          // first chunk of column slot i; coff[r] = all
+    unsigned* ccnt;           // finished chunks of a column with several
+    const MT* Mr; const MT* Mc; int64_t ldm;
+    const double* b;
+    V* us; V* vs; V* z; V* t; V* tpart;
+    double* w; double* y;
+    V* pa; V* pb;
+    PState* S;
+};
+
+// loads of what other CTAs wrote in this launch: from L2
+SKL_DEV float2 ld_cg(const float2* p) { return __ldcg(p); }
+SKL_DEV double ld_cg(const double* p) { return __ldcg(p); }
+
+template <bool CLUSTER>
+SKL_DEV bool bar_all(PState* S, unsigned& gen)
+{
+    if constexpr (CLUSTER) {
+        __syncthreads();
+        cluster_sync();
+        return true;
+    } else {
+        __shared__ int s_ok;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            gen += gridDim.x;
+            __threadfence();
+            atomicAdd(&S->bar, 1u);
+            unsigned v = 0, k = 0;
+            do {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&S->bar) : "memory");
+            } while (v < gen && ++k < kBarLimit);
+            s_ok = v >= gen;
+            __threadfence();
+        }
+        __syncthreads();
+        return s_ok != 0;
+    }
+}
+
+// Sums of squares: float-float on the mixed path.  GB300 issues two FP64 FMAs
+// per SM and cycle, so one FP64 instruction of a warp holds the pipe for 16
+// cycles whatever its active lanes: an epilogue of ten of them in each of 32
+// warps is 2.7 us, and the mixed path's vector updates and norms therefore run
+// in float-float too; FP64 is left to the scalars of one lane and to y and w.
+template <bool MIXED>
+struct Sum {
+    ff a{0.f, 0.f};
+    SKL_DEV void add_sq(ff x) { ff_fma(a, x, x); }
+    SKL_DEV float2 block(ff* red) const
+    {
+        const ff t = block_sum_ff(a, red);
+        return make_float2(t.hi, t.lo);
+    }
+};
+template <>
+struct Sum<false> {
+    double a = 0.0;
+    SKL_DEV void add_sq(double x) { a = fma(x, x, a); }
+    SKL_DEV double block(double* red) const { return block_sum(a, red); }
+};
+
+// Fixed-order sum of the CTAs' partials (one warp; every lane gets it).
+SKL_DEV double sum_partials(const float2* p, int np)
+{
+    ff s{0.f, 0.f};
+    for (int i = threadIdx.x & 31; i < np; i += 32) {
+        const float2 v = __ldcg(p + i);
+        ff_add(s, v.x, v.y);
+    }
+    return ff_to_double(warp_sum_ff(s));
+}
+SKL_DEV double sum_partials(const double* p, int np)
+{
+    double s = 0.0;
+    for (int i = threadIdx.x & 31; i < np; i += 32) s += __ldcg(p + i);
+    return warp_sum(s);
+}
+
+SKL_DEV float2 acc_store(const Acc<true>& a) { return make_float2(a.a.hi, a.a.lo); }
+SKL_DEV double acc_store(const Acc<false>& a) { return a.a; }
+SKL_DEV double val64(float2 v) { return (double)v.x + (double)v.y; }
+SKL_DEV double val64(double v) { return v; }
+SKL_DEV void acc_load(Acc<true>& a, float2 v) { a.a = ff{v.x, v.y}; }
+SKL_DEV void acc_load(Acc<false>& a, double v) { a.a = v; }
+
+// s * dot - c * old, with s and c as the caller split them once
+struct ScaleF {
+    ff s, c;
+    SKL_DEV ScaleF(double s64, double c64) : s(ff_from_double(s64)), c(ff_from_double(-c64)) {}
+    SKL_DEV ff operator()(const Acc<true>& dot, float2 old) const
+    {
+        ff v{0.f, 0.f};
+        ff_fma(v, s, dot.a);
+        ff_fma(v, c, ff{old.x, old.y});
+        return v;
+    }
+};
+struct ScaleD {
+    double s, c;
+    SKL_DEV ScaleD(double s64, double c64) : s(s64), c(c64) {}
+    SKL_DEV double operator()(const Acc<false>& dot, double old) const { return dot.a * s - c * old; }
+};
+template <bool MIXED> using Scale = typename std::conditional<MIXED, ScaleF, ScaleD>::type;
+template <bool MIXED> using RedT = typename std::conditional<MIXED, ff, double>::type;
+SKL_DEV float2 to_v(ff x) { return make_float2(x.hi, x.lo); }
+SKL_DEV double to_v(double x) { return x; }
+
+template <bool MIXED>
+SKL_DEV Acc<MIXED> warp_reduce(Acc<MIXED> a)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a.add(a.shfl_xor(o));
+    return a;
+}
+
+// Partial dot of x[lo..hi) (contiguous, x 4-element aligned at index 0) with
+// the staged vector sv, by `nl` lanes (lane index l): four elements per load.
+template <bool MIXED>
+SKL_DEV Acc<MIXED> dot_seg(const MatT<MIXED>* __restrict__ x, const ValT<MIXED>* sv, int lo, int hi, int l, int nl)
+{
+    Acc<MIXED> a0, a1;
+    const int c1 = hi >> 2;                  // whole chunks end here
+    int c = (lo >> 2) + l;
+    // the first chunk may start before lo, the last may be ragged
+    auto edge = [&](int cc) {
+        for (int k = 4 * cc; k < 4 * cc + 4; ++k)
+            if (k >= lo && k < hi) a0.fma_f(x[k], sv[k]);
+    };
+    if (l == 0 && (lo & 3)) {
+        edge(c);
+        c += nl;
+    }
+    if constexpr (MIXED) {
+        const float4* x4 = reinterpret_cast<const float4*>(x);
+        const float4* s4 = reinterpret_cast<const float4*>(sv);   // two entries each
+        for (; c + 3 * nl < c1; c += 4 * nl) {
+            float4 m[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) m[q] = __ldg(x4 + c + q * nl);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float4 u = s4[2 * (c + q * nl)], w = s4[2 * (c + q * nl) + 1];
+                a0.fma_f(m[q].x, make_float2(u.x, u.y));
+                a1.fma_f(m[q].y, make_float2(u.z, u.w));
+                a0.fma_f(m[q].z, make_float2(w.x, w.y));
+                a1.fma_f(m[q].w, make_float2(w.z, w.w));
+            }
+        }
+        for (; c < c1; c += nl) {
+            const float4 m = __ldg(x4 + c);
+            const float4 u = s4[2 * c], w = s4[2 * c + 1];
+            a0.fma_f(m.x, make_float2(u.x, u.y));
+            a1.fma_f(m.y, make_float2(u.z, u.w));
+            a0.fma_f(m.z, make_float2(w.x, w.y));
+            a1.fma_f(m.w, make_float2(w.z, w.w));
+        }
+    } else {
+        const double2* x2 = reinterpret_cast<const double2*>(x);
+        for (; c < c1; c += nl) {
+            const double2 m0 = __ldg(x2 + 2 * c), m1 = __ldg(x2 + 2 * c + 1);
+            a0.fma_f(m0.x, sv[4 * c]);
+            a1.fma_f(m0.y, sv[4 * c + 1]);
+            a0.fma_f(m1.x, sv[4 * c + 2]);
+            a1.fma_f(m1.y, sv[4 * c + 3]);
+        }
+    }
+    if (c == c1 && 4 * c1 < hi) edge(c1);
+    a0.add(a1);
+    return a0;
+}
+
+constexpr int kMaxUnits = 512;            // row segments of a CTA
+
+// What a CTA needs in every phase.
+template <bool MIXED, int NT>
+struct Cta {
+    using V = ValT<MIXED>;
+    static constexpr int kPT = NT, kPW = NT / 32;
+    static constexpr int kSWarp = kPW - 1;   // the scalars' warp in phases A and C
+    static constexpr int kYWarp = kPW - 2;   // the warp of y and w in phase C
+    const PArgs<MIXED>& g;
+    PScal& sc;              // shared memory
+    V* sv;                  // staged vector, max(r, d) entries
+    V* s_unit;              // kMaxUnits segment sums
+    RedT<MIXED>* red;
+    int tid, lane, warp, G, bid, nloc;
+
+    // Rows of the triangle this CTA owns, longest first: local row k is the q-th
+    // longest, q = k G + bid (k even) or (k + 1) G - 1 - bid (k odd).
+    SKL_DEV int tri_row(int k, bool rows) const
+    {
+        const int q = (k & 1) ? (k + 1) * G - 1 - bid : k * G + bid;
+        return q >= g.r ? -1 : rows ? q : g.r - 1 - q;
+    }
+    // Dots of the owned rows (columns) with the staged vector: segment sums to
+    // s_unit by the first nw warps.
+    SKL_DEV void tri_units(const MatT<MIXED>* M, bool rows, int nw) const
+    {
+        for (int u = warp; u < nloc * g.S_seg; u += nw) {
+            const int k = u / g.S_seg, s = u - k * g.S_seg;
+            const int i = tri_row(k, rows);
+            if (i < 0) continue;
+            const int lo = rows ? i : 0, hi = rows ? g.r : i + 1, base = lo & ~3;
+            const int len = ((hi - lo) / g.S_seg + 4) & ~3;
+            const int a0 = max(lo, base + s * len);
+            const int a1 = s == g.S_seg - 1 ? hi : min(hi, base + (s + 1) * len);
+            Acc<MIXED> a;
+            if (a0 < a1) a = dot_seg<MIXED>(M + (int64_t)i * g.ldm, sv, a0, a1, lane, 32);
+            a = warp_reduce<MIXED>(a);
+            if (lane == 0) s_unit[u] = acc_store(a);
+        }
+    }
+    SKL_DEV Acc<MIXED> tri_sum(int k) const
+    {
+        Acc<MIXED> a;
+        acc_load(a, s_unit[k * g.S_seg]);
+        for (int s = 1; s < g.S_seg; ++s) {
+            Acc<MIXED> o;
+            acc_load(o, s_unit[k * g.S_seg + s]);
+            a.add(o);
+        }
+        return a;
+    }
+
+    // u = b, partial ||b||^2
+    SKL_DEV void init_u() const
+    {
+        Sum<MIXED> ss;
+        for (int i = bid * kPT + tid; i < g.n; i += G * kPT) {
+            const V x = store_val<MIXED>(g.b[i]);
+            g.us[i] = x;
+            if constexpr (MIXED) ss.add_sq(ff{x.x, x.y});
+            else ss.add_sq(x);
+        }
+        const V tot = ss.block(red);
+        if (tid == 0) g.pb[bid] = tot;
+    }
+    // beta_1 (one warp)
+    SKL_DEV void init_beta() const
+    {
+        const double beta = sqrt(sum_partials(g.pb, G));
+        if (lane == 0) {
+            sc.beta = beta;
+            sc.ib = beta > 0.0 ? 1.0 / beta : 0.0;
+            sc.coef_t = 0.0;
+        }
+    }
+    // alpha_1 (one warp); w = v, y = 0 by the warp that updates them later
+    SKL_DEV void init_alpha() const
+    {
+        const double alpha = sqrt(sum_partials(g.pa, G));
+        if (lane == 0) {
+            sc.alpha = alpha;
+            sc.ia = alpha > 0.0 ? 1.0 / alpha : 0.0;
+            sc.coef_n = alpha * sc.ib;
+            sc.rhobar = alpha;
+            sc.phibar = sc.beta;
+            sc.nrm_a = sc.nrm_ar = 0.0;
+            sc.it = 0;
+            // the reference's loop ends at once on alpha beta = 0 (IterSolver.cpp:200)
+            sc.done = alpha * sc.beta == 0.0 ? 1 : 0;
+            sc.flag = sc.done ? 0 : 1;
+            sc.pend = sc.ypend = 0;
+        }
+    }
+    SKL_DEV void init_yw() const
+    {
+        for (int i = bid * 32 + lane; i < g.r; i += G * 32) {
+            g.w[i] = val64(ld_cg(g.vs + i)) * sc.ia;
+            g.y[i] = 0.0;
+        }
+    }
+    // y += t1 w, w = v + t2 w of this CTA's entries (one warp)
+    SKL_DEV void update_yw() const
+    {
+        const double t1 = sc.y_t1, t2 = sc.y_t2, ia = sc.y_ia;
+        for (int i = bid * 32 + lane; i < g.r; i += G * 32) {
+            const double v = ia != 0.0 ? val64(ld_cg(g.vs + i)) * ia : 0.0;
+            const double wi = g.w[i];
+            g.y[i] += t1 * wi;
+            g.w[i] = t2 * wi + v;
+        }
+    }
+
+    // ---- A: z = M v (unscaled); alpha, stop test (last warp).  Returns with
+    // sc.done decided; z is written unless it is set or `last`.
+    SKL_DEV void phase_a(bool last) const
+    {
+        for (int i = tid; i < g.r; i += kPT) sv[i] = ld_cg(g.vs + i);
+        __syncthreads();
+        if (warp < kSWarp) {
+            tri_units(g.Mr, true, kSWarp);
+        } else if (sc.pend) {
+            const double a = sqrt(sum_partials(g.pa, G));
+            if (lane == 0) {
+                // the reference skips the A^T u step when beta == 0 (IterSolver.cpp:242)
+                const double alpha = sc.beta > 0.0 ? a : sc.alpha;
+                sc.alpha = alpha;
+                sc.ia = alpha > 0.0 ? 1.0 / alpha : 0.0;
+                sc.coef_n = alpha * sc.ib;
+                sc.t2 = -sc.sn * alpha * sc.irho;
+                sc.rhobar = -sc.cs * alpha;
+                sc.it += 1;
+                sc.nrm_ar = sc.phibar * alpha * fabs(sc.cs);
+                if (sc.nrm_ar < g.S->tol * sc.nrm_a * sc.phibar) {
+                    sc.done = 1;
+                    sc.flag = 0;
+                } else if (sc.it >= g.S->max_it) {
+                    sc.done = 1;
+                    sc.flag = 1;
+                }
+                sc.y_t1 = sc.t1;
+                sc.y_t2 = sc.t2;
+                sc.y_ia = sc.beta > 0.0 ? sc.ia : 0.0;
+                sc.pend = 0;
+                sc.ypend = 1;
+            }
+        }
+        __syncthreads();
+        if (last || sc.done) return;
+        for (int k = tid; k < nloc; k += kPT) {
+            const int i = tri_row(k, true);
+            if (i < 0) continue;
+            const Acc<MIXED> a = tri_sum(k);
+            const int c = __ldg(g.cols + i);
+            g.z[c] = g.opscale ? store_val<MIXED>(a.value() * g.opscale[c]) : acc_store(a);
+        }
+    }
+
+    // ---- B: u = A z / alpha - (alpha / beta) u; partial ||u||^2
+    SKL_DEV void phase_b() const
+    {
+        const int L = g.L_n, l = lane & (L - 1), per = 32 / L, rstep = G * kPW * per;
+        for (int j = tid; j < g.d; j += kPT) sv[j] = ld_cg(g.z + j);
+        __syncthreads();
+        const Scale<MIXED> sc2(sc.ia, sc.coef_n);
+        Sum<MIXED> ss;
+        // the next row's entries and old u are loaded before this row's products
+        int cc[4], nc[4];
+        V aa[4], na[4], uo{}, nuo{};
+        auto load_row = [&](int i, int& p0, int& p1, int (&c)[4], V (&a)[4], V& u) {
+            p0 = p1 = 0;
+            if (i < g.n) {
+                p0 = __ldg(g.rp + i) + l;
+                p1 = __ldg(g.rp + i + 1);
+                if (l == 0) u = ld_cg(g.us + i);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const bool ok = p0 + k * L < p1;
+                c[k] = ok ? __ldg(g.ci + p0 + k * L) : 0;
+                if (ok) a[k] = __ldg(g.cv + p0 + k * L);
+                else a[k] = V{};
+            }
+        };
+        int base = (bid * kPW + warp) * per;
+        int i = base + lane / L, p0, p1, np0, np1;
+        load_row(i, p0, p1, cc, aa, uo);
+        for (; base < g.n; base += rstep) {
+            load_row(i + rstep, np0, np1, nc, na, nuo);
+            Acc<MIXED> acc, acc2;
+#pragma unroll
+            for (int k = 0; k < 4; k += 2) {
+                acc.fma_mv(aa[k], sv[cc[k]]);
+                acc2.fma_mv(aa[k + 1], sv[cc[k + 1]]);
+            }
+            for (int p = p0 + 4 * L; p < p1; p += 2 * L) {   // rows longer than 4 L
+                const int c0 = __ldg(g.ci + p);
+                acc.fma_mv(__ldg(g.cv + p), sv[c0]);
+                if (p + L < p1) {
+                    const int c1 = __ldg(g.ci + p + L);
+                    acc2.fma_mv(__ldg(g.cv + p + L), sv[c1]);
+                }
+            }
+            acc.add(acc2);
+            for (int o = L / 2; o > 0; o >>= 1) acc.add(acc.shfl_xor(o));
+            if (i < g.n && l == 0) {
+                const auto nv = sc2(acc, uo);
+                g.us[i] = to_v(nv);
+                ss.add_sq(nv);
+            }
+            i += rstep;
+            p0 = np0;
+            p1 = np1;
+            uo = nuo;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                cc[k] = nc[k];
+                aa[k] = na[k];
+            }
+        }
+        const V tot = ss.block(red);
+        if (tid == 0) g.pb[bid] = tot;
+    }
+
+    // beta and the Givens rotation (one warp, beside the chunks of phase C)
+    SKL_DEV void beta_scalars() const
+    {
+        const double beta = sqrt(sum_partials(g.pb, G));
+        if (lane == 0) {
+            sc.beta = beta;
+            sc.ib = beta > 0.0 ? 1.0 / beta : 0.0;
+            sc.coef_t = beta * sc.ia;
+            const double rho = sqrt(sc.rhobar * sc.rhobar + beta * beta);
+            sc.irho = 1.0 / rho;
+            sc.cs = sc.rhobar * sc.irho;
+            sc.sn = beta * sc.irho;
+            sc.t1 = sc.cs * sc.phibar * sc.irho;
+            if (beta > 0.0) sc.nrm_a = sqrt(sc.nrm_a * sc.nrm_a + sc.alpha * sc.alpha + beta * beta);
+            sc.phibar = sc.sn * sc.phibar;
+            sc.pend = 1;
+            sc.ypend = 0;
+        }
+    }
+
+    // ---- C: t(i) = A(:, c)^T u by chunks, on the first nw warps of each CTA
+    SKL_DEV void chunks(int nw) const
+    {
+        if (warp >= nw) return;
+        const int Lt = g.L_t, lt = lane & (Lt - 1), pert = 32 / Lt;
+        const int total = __ldg(g.coff + g.r);
+        for (int q0 = (bid * nw + warp) * pert; q0 < total; q0 += G * nw * pert) {
+            const int q = q0 + lane / Lt;
+            Acc<MIXED> acc, acc2;
+            int4 ch = make_int4(0, 0, 0, 0);
+            if (q < total) {
+                ch = __ldg(g.chunks + q);
+                for (int p = ch.x + lt; p < ch.y; p += kTU * Lt) {
+                    int rr[kTU];
+                    V aa[kTU], uu[kTU];
+#pragma unroll
+                    for (int k = 0; k < kTU; ++k) {
+                        const bool ok = p + k * Lt < ch.y;
+                        rr[k] = ok ? __ldg(g.ri + p + k * Lt) : -1;
+                        if (ok) aa[k] = __ldg(g.rv + p + k * Lt);
+                        else aa[k] = V{};
+                    }
+#pragma unroll
+                    for (int k = 0; k < kTU; ++k) {
+                        if (rr[k] >= 0) uu[k] = g.us[rr[k]];   // plain: the barrier's acquire dropped stale L1 lines
+                        else uu[k] = V{};
+                    }
+#pragma unroll
+                    for (int k = 0; k < kTU; k += 2) {
+                        acc.fma_mv(aa[k], uu[k]);
+                        acc2.fma_mv(aa[k + 1], uu[k + 1]);
+                    }
+                }
+            }
+            acc.add(acc2);
+            for (int o = Lt / 2; o > 0; o >>= 1) acc.add(acc.shfl_xor(o));
+            if (q < total && lt == 0) {
+                bool fin = true;
+                if (ch.w > 1) {
+                    g.tpart[q] = acc_store(acc);
+                    unsigned before;
+                    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;"
+                                 : "=r"(before)
+                                 : "l"(g.ccnt + ch.z)
+                                 : "memory");
+                    fin = before == (unsigned)ch.w - 1;
+                    if (fin) {
+                        g.ccnt[ch.z] = 0;
+                        const V* part = g.tpart + __ldg(g.coff + ch.z);
+                        acc = Acc<MIXED>();
+                        for (int k0 = 0; k0 < ch.w; k0 += 8) {
+                            V x[8];
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) {
+                                if (k0 + k < ch.w) x[k] = ld_cg(part + k0 + k);
+                                else x[k] = V{};
+                            }
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) {
+                                Acc<MIXED> o;
+                                acc_load(o, x[k]);
+                                acc.add(o);
+                            }
+                        }
+                    }
+                }
+                if (fin) g.t[ch.z] = g.opscale ? store_val<MIXED>(acc.value() * g.opscale[g.cols[ch.z]]) : acc_store(acc);
+            }
+        }
+    }
+    SKL_DEV void phase_c() const
+    {
+        const int yp = sc.ypend;
+        __syncthreads();   // beta_scalars clears the flag
+        if (warp == kSWarp) beta_scalars();
+        else if (warp == kYWarp && yp) update_yw();
+        chunks(kYWarp);
+    }
+
+    // ---- D: v = M^T t / beta - (beta / alpha) v; partial ||v||^2
+    SKL_DEV void phase_d() const
+    {
+        for (int i = tid; i < g.r; i += kPT) sv[i] = ld_cg(g.t + i);
+        __syncthreads();
+        tri_units(g.Mc, false, kPW);
+        __syncthreads();
+        Sum<MIXED> ss;
+        const double ib = sc.ib, coef_t = sc.coef_t;
+        const Scale<MIXED> sc2(ib, coef_t);
+        for (int k = tid; k < nloc; k += kPT) {
+            const int j = tri_row(k, false);
+            if (j < 0) continue;
+            const V old = coef_t != 0.0 ? g.vs[j] : V{};
+            const auto nv = sc2(tri_sum(k), old);
+            if (ib > 0.0) g.vs[j] = to_v(nv);   // v stays when beta = 0 (IterSolver.cpp:242)
+            ss.add_sq(nv);
+        }
+        const V tot = ss.block(red);
+        if (tid == 0) g.pa[bid] = tot;
+    }
+};
+
+#define SKL_CTA(MIXED, NT)                                                                                   \
+    extern __shared__ __align__(16) unsigned char smem_raw[];                                            \
+    __shared__ PScal sc;                                                                                 \
+    __shared__ ValT<MIXED> s_unit[kMaxUnits];                                                            \
+    __shared__ RedT<MIXED> red[NT / 32];                                                                 \
+    using C = Cta<MIXED, NT>;                                                                            \
+    const C c{g, sc, reinterpret_cast<ValT<MIXED>*>(smem_raw), s_unit, red, (int)threadIdx.x,   \
+                       (int)threadIdx.x & 31, (int)threadIdx.x >> 5, (int)gridDim.x, (int)blockIdx.x,    \
+                       (g.r + (int)gridDim.x - 1) / (int)gridDim.x}
+
+// The persistent iteration: up to `budget` iterations from the state in slot 0
+// (start != 0: from b), back to slot 0.
+template <bool MIXED, int NT, bool CLUSTER>
+__global__ void __launch_bounds__(NT, 1024 / NT) k_lsqr_persist(const PArgs<MIXED> g, int start, int budget)
+{
+    pdl_wait();
+    SKL_CTA(MIXED, NT);
+    PState* S = g.S;
+    unsigned gen = 0;
+    auto give_up = [&] {
+        if (c.tid == 0) S->timeout = 1;
+    };
+    if (start) {
+        c.init_u();
+        if (!bar_all<CLUSTER>(S, gen)) return give_up();
+        if (c.warp == C::kSWarp) c.init_beta();
+        c.chunks(C::kYWarp);
+        if (!bar_all<CLUSTER>(S, gen)) return give_up();
+        c.phase_d();
+        if (!bar_all<CLUSTER>(S, gen)) return give_up();
+        if (c.warp == C::kYWarp) c.init_alpha();
+        __syncthreads();
+        if (c.warp == C::kYWarp) c.init_yw();
+    } else {
+        if (c.tid == 0) sc = S->sc[0];
+    }
+    __syncthreads();
+    while (!sc.done) {
+        c.phase_a(budget <= 0);
+        if (sc.done || budget <= 0) break;
+        --budget;
+        if (!bar_all<CLUSTER>(S, gen)) return give_up();
+        c.phase_b();
+        if (!bar_all<CLUSTER>(S, gen)) return give_up();
+        c.phase_c();
+        if (!bar_all<CLUSTER>(S, gen)) return give_up();
+        c.phase_d();
+        if (!bar_all<CLUSTER>(S, gen)) return give_up();
+    }
+    if (sc.ypend && c.warp == C::kYWarp) c.update_yw();
+    __syncthreads();
+    if (c.bid == 0 && c.tid == 0) {
+        sc.ypend = 0;
+        S->sc[0] = sc;
+    }
+}
+
+// The same phases as kernels of their own: the same grid, work split and sums,
+// so the same bits.  Several solves at once (the batched entry point) run these:
+// a persistent kernel holds its stream's hardware queue, and the streams behind
+// it, for the whole iteration.  Also the profiled runs, which time the products.
+// PH 0..2: the start (u; t; v), 3: w and y, 4..7: A..D.
+template <bool MIXED, int NT, int PH>
+__global__ void __launch_bounds__(NT, 1024 / NT) k_lsqr_phase(const PArgs<MIXED> g)
+{
+    pdl_wait();
+    SKL_CTA(MIXED, NT);
+    // slots: A reads 0 and writes 1, B reads 1, C reads 1 and writes 0, D reads 0
+    constexpr int in = (PH == 5 || PH == 6) ? 1 : 0;
+    if (c.tid == 0) sc = g.S->sc[in];
+    __syncthreads();
+    if (PH >= 4 && sc.done) {
+        // A found the end and told slot 1; D and the next A read slot 0
+        if (PH == 6 && c.bid == 0 && c.tid == 0) g.S->sc[0] = sc;
+        return;
+    }
+    if constexpr (PH == 0) c.init_u();
+    if constexpr (PH == 1) {
+        if (c.warp == C::kSWarp) c.init_beta();
+        c.chunks(C::kYWarp);
+        __syncthreads();
+        if (c.bid == 0 && c.tid == 0) g.S->sc[0] = sc;
+    }
+    if constexpr (PH == 2 || PH == 7) c.phase_d();
+    if constexpr (PH == 3) {
+        if (c.warp == C::kYWarp) c.init_alpha();
+        __syncthreads();
+        if (c.warp == C::kYWarp) c.init_yw();
+        if (c.bid == 0 && c.tid == 0) g.S->sc[0] = sc;
+    }
+    if constexpr (PH == 4) {
+        c.phase_a(false);
+        if (sc.done && sc.ypend && c.warp == C::kYWarp) c.update_yw();
+        __syncthreads();
+        if (c.bid == 0 && c.tid == 0) g.S->sc[1] = sc;
+    }
+    if constexpr (PH == 5) c.phase_b();
+    if constexpr (PH == 6) {
+        c.phase_c();
+        __syncthreads();
+        if (c.bid == 0 && c.tid == 0) g.S->sc[0] = sc;
+    }
+}
+
+// ---- column chunks -------------------------------------------------------------
+__global__ void k_chunk_count(const int* __restrict__ cp, const int* __restrict__ cols, int r, int len,
+                              int* __restrict__ cnt)
+{
+    pdl_wait();
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < r; i += gridDim.x * blockDim.x) {
+        const int c = cols[i];
+        cnt[i] = max(1, (cp[c + 1] - cp[c] + len - 1) / len);   // an empty column is a chunk too
+    }
+}
+
+__global__ void k_chunk_fill(const int* __restrict__ cp, const int* __restrict__ cols, int r, int len,
+                             const int* __restrict__ coff, int4* __restrict__ chunks, unsigned* __restrict__ ccnt)
+{
+    pdl_wait();
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < r; i += gridDim.x * blockDim.x) {
+        const int c = cols[i], p1 = cp[c + 1], q0 = coff[i], nq = coff[i + 1] - q0;
+        int p = cp[c];
+        for (int q = 0; q < nq; ++q, p += len) chunks[q0 + q] = make_int4(p, min(p1, p + len), i, nq);
+        ccnt[i] = 0;
+    }
+}
+
+int sm_count_p()
+{
+    static const int v = [] {
+        int dev = 0, s = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&s, cudaDevAttrMultiProcessorCount, dev);
+        return s > 0 ? s : 148;
+    }();
+    return v;
+}
+
+// lanes per row: each lane handles about four nonzeros
+int lanes_row(double avg) { return avg >= 96 ? 32 : avg >= 40 ? 16 : avg >= 16 ? 8 : 4; }
+// lanes per column: about eight per step
+int lanes_col(double avg) { return avg >= 128 ? 32 : avg >= 64 ? 16 : avg >= 24 ? 8 : 4; }
+
+struct PBufs {
+    PState* S;
+    void *us, *vs, *z, *t, *tpart;
+    double *w, *y, *pa, *pb;
+    int4* chunks; int* coff; int* scan; int* cnt; unsigned* ccnt;
+    size_t bytes;
+};
+
+int64_t max_chunks(const LsqrProblem& P, int len) { return P.r + P.nnz / len + 1; }
+
+PBufs pcarve(const LsqrProblem& P, void* work)
+{
+    PBufs B;
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        void* p = (char*)work + off;
+        off += (bytes + 255) & ~(size_t)255;
+        return p;
+    };
+    const size_t vs = P.precision == SKL_PREC_MIXED ? sizeof(float2) : sizeof(double);
+    const int64_t nch = max_chunks(P, 4 * kTU * kChunkSteps);   // the shortest chunks
+    B.S = (PState*)take(sizeof(PState));
+    B.us = take(P.n * vs);
+    B.vs = take(P.r * vs);
+    B.z = take(P.d * vs);
+    B.t = take(P.r * vs);
+    B.tpart = take(nch * vs);
+    B.w = (double*)take(P.r * sizeof(double));
+    B.y = (double*)take(P.r * sizeof(double));
+    B.pa = (double*)take(1024 * sizeof(double));
+    B.pb = (double*)take(1024 * sizeof(double));
+    B.chunks = (int4*)take(nch * sizeof(int4));
+    B.ccnt = (unsigned*)take(P.r * sizeof(unsigned));
+    B.coff = (int*)take((P.r + 1) * sizeof(int));
+    B.cnt = (int*)take(P.r * sizeof(int));
+    B.scan = (int*)take(scan_scratch_ints(P.r) * sizeof(int));
+    B.bytes = off;
+    return B;
+}
+
+// Bytes one iteration reads: both copies of A and both triangles.
+double iter_bytes(const LsqrProblem& P)
+{
+    const double vb = P.precision == SKL_PREC_MIXED ? 4.0 : 8.0;
+    return 24.0 * (double)P.nnz + 16.0 * (double)P.n + vb * (double)P.r * (double)P.r;
+}
+
+size_t vec_smem(const LsqrProblem& P)
+{
+    const size_t vs = P.precision == SKL_PREC_MIXED ? sizeof(float2) : sizeof(double);
+    return (size_t)((std::max(P.r, P.d) + 4) & ~(int64_t)3) * vs;
+}
+
+// CTAs: one per ~100 KB an iteration reads (a barrier costs more with more of
+// them, a CTA streams ~50 KB per us), at least one cluster, at most one per SM;
+// with more than ~400 KB per SM the loads in flight matter and the CTAs get 1,024
+// threads (120,000 x 5,000: 136 -> 107 us per iteration; 31,013 x 1,507, 130 KB
+// per SM: 28 us with 512, 31 with 1,024).
+struct Grid {
+    int ctas, threads;
+};
+Grid grid_of(const LsqrProblem& P)
+{
+    const double bytes = iter_bytes(P);
+    return {(int)std::max<double>(kCluster, std::min<double>(sm_count_p(), std::ceil(bytes / 100e3))),
+            bytes / sm_count_p() > 400e3 ? kBigCta : kSmallCta};
+}
+
+template <bool MIXED, int NT, int PH>
+void launch_phase(const PArgs<MIXED>& g, int G, size_t smem, cudaStream_t st)
+{
+    if (smem > 32 * 1024) allow_max_dynamic_smem((const void*)k_lsqr_phase<MIXED, NT, PH>);
+    launch_k(k_lsqr_phase<MIXED, NT, PH>, (unsigned)G, NT, smem, st, g);
+    SKL_LAUNCHED();
+}
+
+double time_limit_s()
+{
+    static const double v = [] {
+        const char* e = getenv("SKILLS_LSQR_TIMEOUT_S");
+        return e ? atof(e) : 60.0;
+    }();
+    return v;
+}
+
+struct Clock {
+    std::chrono::steady_clock::time_point t0 = std::chrono::steady_clock::now();
+    void check() const
+    {
+        if (std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count() > time_limit_s())
+            fail(SKL_ERR_TIMEOUT, "LSQR exceeded its time limit (SKILLS_LSQR_TIMEOUT_S)");
+    }
+};
+
+// One persistent kernel per kItersPerLaunch iterations.
+template <bool MIXED, int NT>
+const PState* run_persistent(const PArgs<MIXED>& g, int G, size_t smem, void* host_pinned, cudaStream_t st)
+{
+    const bool cluster = G <= kCluster;
+    const void* fn = cluster ? (const void*)k_lsqr_persist<MIXED, NT, true>
+                             : (const void*)k_lsqr_persist<MIXED, NT, false>;
+    allow_max_dynamic_smem(fn);
+    if (cluster) SKL_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)G);
+    cfg.blockDim = dim3(NT);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    if (cluster) {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = kCluster;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    } else {
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    const PState* hs = (const PState*)host_pinned;
+    const Clock clock;
+    for (int start = 1;; start = 0) {
+        int budget = kItersPerLaunch;
+        PArgs<MIXED> a = g;
+        void* args[] = {(void*)&a, (void*)&start, (void*)&budget};
+        SKL_CUDA(cudaLaunchKernelExC(&cfg, fn, args));
+        SKL_LAUNCHED();
+        SKL_CUDA(cudaMemcpyAsync(host_pinned, g.S, sizeof(PState), cudaMemcpyDeviceToHost, st));
+        SKL_CUDA(cudaStreamSynchronize(st));
+        if (hs->timeout) fail(SKL_ERR_TIMEOUT, "a grid barrier's bounded wait gave up (LSQR)");
+        if (hs->sc[0].done) return hs;
+        clock.check();
+        SKL_CUDA(cudaMemsetAsync(&g.S->bar, 0, sizeof(unsigned), st));
+    }
+}
+
+// Phase kernels: a graph of kIterPerGraph iterations, replayed until the state
+// says done; the next replay is queued before the last one's state is read, so
+// the GPU does not wait for the host.  profile: events around the products.
+template <bool MIXED, int NT>
+const PState* run_phases(const PArgs<MIXED>& g, int G, size_t smem, void* host_pinned, cudaStream_t st,
+                         cudaStream_t cap, int profile, LsqrResult& res)
+{
+    launch_phase<MIXED, NT, 0>(g, G, smem, st);
+    launch_phase<MIXED, NT, 1>(g, G, smem, st);
+    launch_phase<MIXED, NT, 2>(g, G, smem, st);
+    launch_phase<MIXED, NT, 3>(g, G, smem, st);
+    struct Owned {
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        cudaEvent_t ev[2] = {nullptr, nullptr};
+        std::vector<cudaEvent_t> pev;
+        ~Owned()
+        {
+            for (cudaEvent_t e : ev)
+                if (e) cudaEventDestroy(e);
+            for (cudaEvent_t e : pev)
+                if (e) cudaEventDestroy(e);
+            if (exec) cudaGraphExecDestroy(exec);
+            if (graph) cudaGraphDestroy(graph);
+        }
+    } o;
+    for (auto& e : o.ev) SKL_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    o.pev.assign(profile ? 8 * kIterPerGraph : 0, nullptr);
+    for (auto& e : o.pev) SKL_CUDA(cudaEventCreate(&e));
+    // capture on the library's stream (the caller's may be the legacy default
+    // stream, which cannot be captured); replay on the caller's
+    SKL_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
+    for (int q = 0; q < kIterPerGraph; ++q) {
+        auto mark = [&](int k) {
+            if (profile) SKL_CUDA(cudaEventRecordWithFlags(o.pev[8 * q + k], cap, cudaEventRecordExternal));
+        };
+        mark(4);
+        launch_phase<MIXED, NT, 4>(g, G, smem, cap);
+        mark(5);
+        mark(0);
+        launch_phase<MIXED, NT, 5>(g, G, smem, cap);
+        mark(1);
+        mark(2);
+        launch_phase<MIXED, NT, 6>(g, G, smem, cap);
+        mark(3);
+        mark(6);
+        launch_phase<MIXED, NT, 7>(g, G, smem, cap);
+        mark(7);
+    }
+    SKL_CUDA(cudaStreamEndCapture(cap, &o.graph));
+    SKL_CUDA(cudaGraphInstantiate(&o.exec, o.graph, 0));
+    const Clock clock;
+    long long it_prev = 0;
+    auto replay = [&](int k) {
+        SKL_CUDA(cudaGraphLaunch(o.exec, st));
+        for (int q = 0; q < 4 * kIterPerGraph; ++q) SKL_LAUNCHED();
+        SKL_CUDA(cudaMemcpyAsync((char*)host_pinned + k * 1024, g.S, sizeof(PState), cudaMemcpyDeviceToHost, st));
+        SKL_CUDA(cudaEventRecord(o.ev[k], st));
+    };
+    static_assert(sizeof(PState) <= 1024, "two states in the pinned scratch");
+    if (!profile) replay(0);
+    for (int k = 0;; k ^= 1) {
+        // a profiled replay is read before the next one overwrites its events
+        replay(profile ? k : k ^ 1);
+        SKL_CUDA(cudaEventSynchronize(o.ev[k]));
+        const PState* hs = (const PState*)((char*)host_pinned + k * 1024);
+        if (profile) {
+            const long long ran = hs->sc[0].it + hs->sc[0].pend - it_prev;
+            it_prev += ran;
+            for (long long q = 0; q < ran && q < kIterPerGraph; ++q)
+                for (int kk = 0; kk < 4; ++kk) {
+                    float ms = 0.f;
+                    SKL_CUDA(cudaEventElapsedTime(&ms, o.pev[8 * q + 2 * kk], o.pev[8 * q + 2 * kk + 1]));
+                    res.prof_ms[kk] += ms;
+                    res.prof_launches[kk] += 1;
+                }
+        }
+        if (hs->sc[0].done) {
+            // the replay still queued returns at once, but it uses the graph
+            if (!profile) SKL_CUDA(cudaEventSynchronize(o.ev[k ^ 1]));
+            return hs;
+        }
+        clock.check();
+    }
+}
+
+template <bool MIXED, int NT>
+LsqrResult persist_impl(const LsqrProblem& P, const double* b, double tol, int64_t max_it, double* y_out, void* work,
+                        void* host_pinned, cudaStream_t st, int profile, cudaStream_t capture_stream)
+{
+    using V = ValT<MIXED>;
+    using MT = MatT<MIXED>;
+    PBufs B = pcarve(P, work);
+    PArgs<MIXED> g{};
+    g.n = (int)P.n;
+    g.r = (int)P.r;
+    g.d = (int)P.d;
+    g.L_n = P.lanes_n ? P.lanes_n : lanes_row(P.n ? (double)P.nnz / P.n : 0.0);
+    g.L_t = P.lanes_t ? P.lanes_t : lanes_col(P.d ? (double)P.nnz / P.d : 0.0);
+    g.rp = P.rp;
+    g.ci = P.ci;
+    g.cv = (const V*)P.cx;
+    g.cp = P.cp;
+    g.ri = P.ri;
+    g.rv = (const V*)P.rx;
+    g.cols = P.cols;
+    g.opscale = P.opscale;
+    g.chunks = B.chunks;
+    g.coff = B.coff;
+    g.ccnt = B.ccnt;
+    g.Mr = (const MT*)P.Mrow;
+    g.Mc = (const MT*)P.M;
+    g.ldm = P.ldm;
+    g.b = b;
+    g.us = (V*)B.us;
+    g.vs = (V*)B.vs;
+    g.z = (V*)B.z;
+    g.t = (V*)B.t;
+    g.tpart = (V*)B.tpart;
+    g.w = B.w;
+    g.y = B.y;
+    g.pa = (V*)B.pa;
+    g.pb = (V*)B.pb;
+    g.S = B.S;
+    const int G = grid_of(P).ctas;
+    // segments per row of the triangle: one round of the 15 (31) warps where the
+    // CTA has fewer rows than that, else about four per warp, which evens out
+    // the rows' lengths
+    const int nloc = (int)((P.r + G - 1) / G), nw = NT / 32 - 1;
+    g.S_seg = std::max(1, std::min(8, nloc <= nw ? nw / nloc : 4 * nw / nloc));
+    // chunks of the columns
+    const int len = g.L_t * kTU * kChunkSteps;
+    const unsigned gr = (unsigned)std::max<int64_t>(1, std::min<int64_t>((P.r + 255) / 256, 152));
+    launch_k(k_chunk_count, gr, 256, 0, st, P.cp, P.cols, (int)P.r, len, B.cnt);
+    SKL_LAUNCHED();
+    scan_exclusive(B.cnt, P.r, B.coff, B.scan, st);
+    launch_k(k_chunk_fill, gr, 256, 0, st, P.cp, P.cols, (int)P.r, len, B.coff, B.chunks, B.ccnt);
+    SKL_LAUNCHED();
+    SKL_CUDA(cudaMemsetAsync(B.z, 0, P.d * sizeof(V), st));
+    PState init{};
+    init.tol = tol;
+    init.max_it = max_it;
+    SKL_CUDA(cudaMemcpyAsync(B.S, &init, sizeof(PState), cudaMemcpyHostToDevice, st));
+    trace_phase(st, "lsqr: init");
+    const size_t smem = vec_smem(P);
+    LsqrResult res;
+    const PState* hs =
+        profile || P.shared_gpu
+            ? run_phases<MIXED, NT>(g, G, smem, host_pinned, st, capture_stream ? capture_stream : st, profile, res)
+            : run_persistent<MIXED, NT>(g, G, smem, host_pinned, st);
+    trace_phase(st, "lsqr: done");
+    res.flag = hs->sc[0].flag;
+    res.it = hs->sc[0].it;
+    SKL_CUDA(cudaMemcpyAsync(y_out, B.y, P.r * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    return res;
+}
+
+}  // namespace
+
+bool lsqr_persist_fits(const LsqrProblem& P)
+{
+    const int G = grid_of(P).ctas;
+    return !P.Ad && P.r > 0 && (P.r + G - 1) / G <= kMaxUnits && vec_smem(P) <= 200 * 1024;
+}
+
+size_t lsqr_persist_workspace_bytes(const LsqrProblem& P) { return pcarve(P, nullptr).bytes; }
+
+LsqrResult lsqr_persist_run(const LsqrProblem& P, const double* b, double tol, int64_t max_it, double* y, void* work,
+                            void* host_pinned, cudaStream_t st, int profile, cudaStream_t capture_stream)
+{
+    const bool big = grid_of(P).threads == kBigCta;
+    auto* fn = P.precision == SKL_PREC_MIXED
+                   ? (big ? persist_impl<true, kBigCta> : persist_impl<true, kSmallCta>)
+                   : (big ? persist_impl<false, kBigCta> : persist_impl<false, kSmallCta>);
+    return fn(P, b, tol, max_it, y, work, host_pinned, st, profile, capture_stream);
+}
+
+}  // namespace skl

@@ -77,6 +77,7 @@ struct Context {
     double* dev_scalars = nullptr;   // small pinned-size scalar area (device)
     void* host_pinned = nullptr;     // pinned host scratch for scalar readback
     size_t host_pinned_bytes = 0;
+    bool batched = false;            // a batched worker's context (slot > 0)
 };
 
 // Device context `slot` of a device (slot 0: single solves; 1..: batched workers).
@@ -269,6 +270,9 @@ struct LsqrProblem {
     const double* opscale = nullptr;
     const void* M = nullptr; const void* Mrow = nullptr; int64_t ldm = 0; int64_t r = 0;
     int precision = SKL_PREC_MIXED;
+    // other solves share the GPU (batched workers): no kernel may hold its
+    // stream's hardware queue for a whole LSQR run
+    bool shared_gpu = false;
     // lanes per CSR row (A z) and per CSC column (A^T u); 0 = by the average
     // row / column length
     int lanes_n = 0, lanes_t = 0;
@@ -286,6 +290,12 @@ size_t lsqr_workspace_bytes(const LsqrProblem& P);
 LsqrResult lsqr_run(const LsqrProblem& P, const double* b, double tol, int64_t max_it, double* y,
                     void* work, unsigned* status, void* host_pinned, cudaStream_t st,
                     int profile = 0, cudaStream_t capture_stream = nullptr);
+// The sparse iteration as one persistent kernel, or as phase kernels with the same
+// bits (k_lsqr_persist.cu), where the problem's vectors fit shared memory.
+bool lsqr_persist_fits(const LsqrProblem& P);
+size_t lsqr_persist_workspace_bytes(const LsqrProblem& P);
+LsqrResult lsqr_persist_run(const LsqrProblem& P, const double* b, double tol, int64_t max_it, double* y, void* work,
+                            void* host_pinned, cudaStream_t st, int profile, cudaStream_t capture_stream);
 // One product in isolation with LSQR's storage and arithmetic: y = A x
 // (trans 'n', CSR kernel) or y = A^T x ('t', CSC kernel, P.cols = 0..d-1,
 // P.r = d).  The stored values are A(:, c) * vscale[c] (vscale nullptr: A's
