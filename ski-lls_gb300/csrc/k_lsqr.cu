@@ -885,6 +885,7 @@ static int64_t spmv_n_blocks(const LsqrProblem& P)
 
 size_t lsqr_workspace_bytes(const LsqrProblem& P)
 {
+    if (P.At) return lsqr_persist_workspace_bytes(P);
     const size_t vs = P.precision == SKL_PREC_MIXED ? sizeof(float2) : sizeof(double);
     size_t b = sizeof(LsqrState) + 256;
     b += 2 * (P.n * sizeof(double) + 256);                   // uh, us

@@ -1,5 +1,4 @@
-// k_lsqr_persist.cu -- the whole LSQR iteration in one persistent kernel
-// (sparse problems).
+// k_lsqr_persist.cu -- the whole LSQR iteration in one persistent kernel.
 //
 // The iteration of k_lsqr.cu (src/IterSolver.cpp:160-284) is five kernels of
 // 5-15 us that each do a few microseconds of work on problems up to a few
@@ -39,6 +38,7 @@
 #include "launch.cuh"
 #include "common.cuh"
 #include "lsqr_types.cuh"
+#include "tc_ptx.cuh"
 
 namespace skl {
 
@@ -176,6 +176,8 @@ SKL_DEV void acc_load(Acc<false>& a, double v) { a.a = v; }
 struct ScaleF {
     ff s, c;
     SKL_DEV ScaleF(double s64, double c64) : s(ff_from_double(s64)), c(ff_from_double(-c64)) {}
+    SKL_DEV explicit ScaleF(float4 v) : s{v.x, v.y}, c{v.z, v.w} {}
+    SKL_DEV float4 pack() const { return make_float4(s.hi, s.lo, c.hi, c.lo); }
     SKL_DEV ff operator()(const Acc<true>& dot, float2 old) const
     {
         ff v{0.f, 0.f};
@@ -585,6 +587,10 @@ struct Cta {
     SKL_DEV void phase_d() const
     {
         for (int i = tid; i < g.r; i += kPT) sv[i] = ld_cg(g.t + i);
+        tri_finish();
+    }
+    SKL_DEV void tri_finish() const
+    {
         __syncthreads();
         tri_units(g.Mc, false, kPW);
         __syncthreads();
@@ -706,6 +712,433 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_lsqr_phase(const PArgs<MIXED>
         __syncthreads();
         if (c.bid == 0 && c.tid == 0) g.S->sc[0] = sc;
     }
+}
+
+// ---- dense problems -------------------------------------------------------------
+// The dense products are bound by A: 1.28 GB at 40,000 x 4,000, read once for A z
+// and again for A^T u.  A row of u needs the whole row's dot first, but only that
+// row: here a CTA holds a few whole rows (a tile) in shared memory, forms their
+// u, and adds u times the tile to its share of A^T u, so that an iteration reads A
+// once (40,000 x 4,000: 463 us per iteration with the two products as kernels of
+// their own at 0.95 of HBM, 340 here, 264 of it the pass; the pass is bound by the
+// float-float arithmetic, ~26 FP32 instructions per entry, and by the sums over
+// the CTA between two of its barriers).  Tried: packed f32x2 arithmetic (487 us: it
+// issues at a quarter of the scalar rate), a tile ring read twice from shared
+// memory with the sums on a warp of their own (440 us), two CTAs of 256 threads per
+// SM (380 us).
+//
+// Storage (k_split_tiles): rows in pairs, columns in K chunks of CW <= 512 (one
+// column per thread); an entry is {hi0, hi1, lo0, lo1} of the pair (one 16-byte
+// read), a chunk is one contiguous bulk copy and a tile RB row pairs.  Threads 0..T-1 keep a ring of chunks in flight
+// (cp.async.bulk, one mbarrier per slot) across tiles, phases and barriers.
+//
+// A tile is in registers before its products start, so its slots are refilled at
+// once and the copies run beside the arithmetic, the barriers and the other
+// phases.  The old u is loaded a tile ahead: it waits ~2 us behind the copies in
+// flight.
+// Phases per iteration: A (M v), BC (the pass over A), R (the CTAs' shares of
+// A^T u added up, in order; beta, y and w beside it), D (M^T t).
+constexpr int kDT = 512;
+constexpr int kDenseMaxD = 8 * kDT;
+
+struct DArgs {
+    const float4* A;          // tiles
+    float2* part;             // [G][K * CW] shares of A^T u
+    float2* tn;               // A^T u, natural column order
+    int CW, ntiles, nslots;
+    int sv_bytes;             // staged-vector bytes before the ring
+    long long* prof;          // 4 summed phase times (ns) of CTA 0, or null
+};
+
+// acc += a x without renormalising acc (the error terms gather in acc.lo, which a
+// few terms leave 2^-22 of acc.hi at most); ff_norm after a handful of terms.
+SKL_DEV void ff_fma_lazy(ff& acc, float ah, float al, ff x)
+{
+    const float p = __fmul_rn(ah, x.hi);
+    const float pe = __fmaf_rn(ah, x.hi, -p);
+    const float pl = __fmaf_rn(ah, x.lo, __fmaf_rn(al, x.hi, pe));
+    float s, e;
+    two_sum(acc.hi, p, s, e);
+    acc.hi = s;
+    acc.lo = __fadd_rn(acc.lo, __fadd_rn(e, pl));
+}
+SKL_DEV void ff_norm(ff& a)
+{
+    const float h = __fadd_rn(a.hi, a.lo);
+    a.lo = __fsub_rn(a.lo, __fsub_rn(h, a.hi));
+    a.hi = h;
+}
+
+SKL_DEV long long now_ns()
+{
+    long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// Sum over the warp of N values per lane (N a power of two): lane l ends with value
+// l / (32 / N).  Halving exchanges, then a plain butterfly: fixed order.
+template <int N>
+SKL_DEV ff warp_sum_n(ff (&v)[N], int lane)
+{
+    int off = 16;
+#pragma unroll
+    for (int n = N; n > 1; n >>= 1, off >>= 1) {
+        const bool up = lane & off;
+#pragma unroll
+        for (int i = 0; i < n / 2; ++i) {
+            const ff send = up ? v[i] : v[i + n / 2];
+            const ff keep = up ? v[i + n / 2] : v[i];
+            v[i] = keep;
+            ff_add(v[i], ff_shfl_xor(send, off));
+        }
+    }
+#pragma unroll
+    for (int o = 32 / N / 2; o > 0; o >>= 1) ff_add(v[0], ff_shfl_xor(v[0], o));
+    return v[0];
+}
+
+template <int K, int RB>
+__global__ void __launch_bounds__(kDT, 1)
+k_lsqr_dense(const PArgs<true> g, const DArgs a, int start, int budget)
+{
+    pdl_wait();
+    SKL_CTA(true, kDT);
+    constexpr int T = K * RB;            // chunks of a tile
+    constexpr int NV = 2 * RB;           // rows of a tile
+    constexpr int kMaxSlots = 64;
+    constexpr int kW = kDT / 32;
+    __shared__ __align__(8) uint64_t bars[kMaxSlots];
+    __shared__ float2 s_part[kW][NV];
+    __shared__ __align__(16) float4 s_u[RB];
+    __shared__ __align__(16) float4 s_scale;
+    __shared__ float2 s_red[C::kYWarp][32];
+    PState* S = g.S;
+    const int tid = c.tid, lane = c.lane, warp = c.warp;
+    const int CW = a.CW, NS = a.nslots;
+    const unsigned chunk_bytes = (unsigned)CW * 16;
+    unsigned char* ring = smem_raw + a.sv_bytes;
+    float2* zs = c.sv;                    // the pass's z, by thread
+    const int mine = (a.ntiles - c.bid + c.G - 1) / c.G;   // this CTA's tiles
+    const bool col_ok = tid < CW;
+    const int col = min(tid, CW - 1);     // a thread past the last column reads it with z = 0
+    unsigned gen = 0;
+    if (tid < NS) tc::mbar_init(smem_u32(bars + tid), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    // Chunk sequence of this CTA: tile by tile, over and over (A does not change
+    // between iterations), round the ring's slots.  All positions advance by
+    // T per tile and wrap by a compare.
+    const int per_pass = mine * T;
+    auto issue = [&](int q, int slot) {
+        const unsigned bar = smem_u32(bars + slot);
+        tc::mbar_expect_tx(bar, chunk_bytes);
+        const float4* src = a.A + ((int64_t)(c.bid + (q / T) * c.G) * T + q % T) * CW;
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         smem_u32(ring) + (unsigned)slot * chunk_bytes),
+                     "l"(src), "r"(chunk_bytes), "r"(bar)
+                     : "memory");
+    };
+    auto arrived = [&](int slot, unsigned parity) {
+        for (unsigned i = 0; i < tc::kWaitLimit; ++i)
+            if (tc::mbar_try(smem_u32(bars + slot), parity)) return true;
+        return false;
+    };
+    int slot0 = 0;                        // slot and parity of the next tile's first chunk
+    unsigned par0 = 0;
+    int next_q = mine > 0 ? (NS + tid) % per_pass : 0;   // thread t < T: its next chunk to ask for
+    if (mine > 0)
+        for (int q = tid; q < NS; q += kDT) issue(q % per_pass, q);
+    auto slot_of = [&](int q, unsigned& parity) {
+        const int sl = slot0 + q;
+        parity = sl >= NS ? par0 ^ 1u : par0;
+        return sl >= NS ? sl - NS : sl;
+    };
+    // the copies in flight land before the CTA exits
+    auto leave = [&] {
+        if (mine > 0 && tid < NS) {
+            unsigned parity;
+            const int sl = slot_of(tid, parity);
+            arrived(sl, parity);
+        }
+        __syncthreads();
+    };
+    auto give_up = [&] {
+        if (tid == 0) S->timeout = 1;
+        leave();
+    };
+    // the pass over A: u = ia A z - coef u, this CTA's share of A^T u; false on a
+    // copy that did not arrive
+    auto pass = [&]() -> bool {
+        // z of the thread's columns: its own shared-memory entries (registers are
+        // short with 64 of them holding the tile)
+        ff t[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int j = k * CW + tid;
+            float2 zz = make_float2(0.f, 0.f);
+            if (col_ok && j < g.d && sc.ia != 0.0) zz = ld_cg(g.z + j);
+            zs[k * kDT + tid] = zz;
+            t[k] = ff{0.f, 0.f};
+        }
+        // the scales as float pairs in shared memory: kept in registers they were
+        // formed again from FP64 in every tile (~2,500 cycles of it between two
+        // barriers)
+        if (tid == 0) s_scale = ScaleF(sc.ia, sc.coef_n).pack();
+        __syncthreads();
+        Sum<true> ss;
+        // finishing threads: value fv, share fw of the warps; fw = 0 writes u
+        const int fv = tid / kW, fw = tid % kW;
+        const bool fin = fv < NV && fw == 0;
+        float2 un = make_float2(0.f, 0.f);   // the next tile's old u
+        if (fin && c.bid * NV + fv < g.n) un = g.us[c.bid * NV + fv];
+        for (int it = 0; it < mine; ++it) {
+            // each warp waits for the tile's chunks with one lane per chunk
+            bool ok = true;
+            if (lane < T) {
+                unsigned parity;
+                const int sl = slot_of(lane, parity);
+                ok = arrived(sl, parity);
+            }
+            __syncwarp();
+            float4 x[T];
+#pragma unroll
+            for (int q = 0; q < T; ++q) {
+                unsigned parity;
+                x[q] = reinterpret_cast<const float4*>(ring + (unsigned)slot_of(q, parity) * chunk_bytes)[col];
+            }
+            if (__syncthreads_or(!ok)) return false;
+            if (tid < T) {
+                unsigned parity;
+                const int sl = slot_of(tid, parity);
+                issue(next_q, sl);
+                next_q += T;
+                if (next_q >= per_pass) next_q -= per_pass;
+            }
+            slot0 += T;
+            if (slot0 >= NS) {
+                slot0 -= NS;
+                par0 ^= 1u;
+            }
+            const int row = (c.bid + it * c.G) * NV + fv;
+            const float2 uo = un;
+            un = make_float2(0.f, 0.f);
+            if (fin && it + 1 < mine && row + c.G * NV < g.n) un = g.us[row + c.G * NV];
+            ff v[NV];
+#pragma unroll
+            for (int q = 0; q < NV; ++q) v[q] = ff{0.f, 0.f};
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const float2 zz = zs[k * kDT + tid];
+                const ff z{zz.x, zz.y};
+#pragma unroll
+                for (int rb = 0; rb < RB; ++rb) {
+                    ff_fma_lazy(v[2 * rb], x[rb * K + k].x, x[rb * K + k].z, z);
+                    ff_fma_lazy(v[2 * rb + 1], x[rb * K + k].y, x[rb * K + k].w, z);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < NV; ++q) ff_norm(v[q]);
+            const ff s = warp_sum_n<NV>(v, lane);
+            if (lane % (32 / NV) == 0) s_part[warp][lane / (32 / NV)] = make_float2(s.hi, s.lo);
+            __syncthreads();
+            if (tid < NV * kW) {
+                const float2 p = s_part[fw][fv];
+                ff r{p.x, p.y};
+#pragma unroll
+                for (int o = kW / 2; o > 0; o >>= 1) ff_add(r, ff_shfl_xor(r, o));
+                if (fin) {
+                    Acc<true> d;
+                    d.a = r;
+                    const volatile float4& vs = s_scale;
+                    const ff nv = ScaleF(make_float4(vs.x, vs.y, vs.z, vs.w))(d, uo);
+                    float* su = reinterpret_cast<float*>(&s_u[fv >> 1]);
+                    su[fv & 1] = nv.hi;
+                    su[2 + (fv & 1)] = nv.lo;
+                    if (row < g.n) {
+                        g.us[row] = to_v(nv);
+                        ss.add_sq(nv);
+                    }
+                }
+            }
+            __syncthreads();
+#pragma unroll
+            for (int rb = 0; rb < RB; ++rb) {
+                const float4 u = s_u[rb];
+#pragma unroll
+                for (int k = 0; k < K; ++k) ff_fma_lazy(t[k], x[rb * K + k].x, x[rb * K + k].z, ff{u.x, u.z});
+#pragma unroll
+                for (int k = 0; k < K; ++k) ff_fma_lazy(t[k], x[rb * K + k].y, x[rb * K + k].w, ff{u.y, u.w});
+            }
+#pragma unroll
+            for (int k = 0; k < K; ++k) ff_norm(t[k]);
+        }
+        if (col_ok)
+#pragma unroll
+            for (int k = 0; k < K; ++k) a.part[(int64_t)c.bid * K * CW + k * CW + tid] = make_float2(t[k].hi, t[k].lo);
+        const float2 tot = ss.block(red);
+        if (tid == 0) g.pb[c.bid] = tot;
+        return true;
+    };
+    // t = the shares' sum: this CTA's columns, by the first kYWarp warps
+    auto reduce = [&] {
+        const int per = (g.d + c.G - 1) / c.G, c0 = c.bid * per, c1 = min(g.d, c0 + per);
+        for (int b0 = c0; b0 < c1; b0 += 32) {
+            const int col = b0 + lane;
+            if (warp < C::kYWarp) {
+                ff r{0.f, 0.f};
+                if (col < c1)
+                    for (int q = warp; q < c.G; q += C::kYWarp) {
+                        const float2 p = ld_cg(a.part + (int64_t)q * K * CW + col);
+                        ff_add(r, p.x, p.y);
+                    }
+                s_red[warp][lane] = make_float2(r.hi, r.lo);
+            }
+            __syncthreads();
+            if (warp == 0 && col < c1) {
+                ff r{0.f, 0.f};
+                for (int w = 0; w < C::kYWarp; ++w) {
+                    const float2 p = s_red[w][lane];
+                    ff_add(r, p.x, p.y);
+                }
+                a.tn[col] = make_float2(r.hi, r.lo);
+            }
+            __syncthreads();
+        }
+    };
+    auto phase_d = [&] {
+        for (int i = tid; i < g.r; i += kDT) c.sv[i] = ld_cg(a.tn + __ldg(g.cols + i));
+        c.tri_finish();
+    };
+    long long tp = 0;
+    auto lap = [&](int k) {
+        if (a.prof && c.bid == 0 && tid == 0) {
+            const long long t = now_ns();
+            if (k >= 0) a.prof[k] += t - tp;
+            tp = t;
+        }
+    };
+    if (start) {
+        // u = b through the pass itself: u = 0 - (-1) u
+        for (int i = c.bid * kDT + tid; i < g.n; i += c.G * kDT) g.us[i] = store_val<true>(g.b[i]);
+        if (tid == 0) {
+            sc.ia = 0.0;
+            sc.coef_n = -1.0;
+        }
+        if (!bar_all<false>(S, gen)) return give_up();
+        if (!pass()) return give_up();
+        if (!bar_all<false>(S, gen)) return give_up();
+        if (warp == C::kSWarp) c.init_beta();
+        reduce();
+        if (!bar_all<false>(S, gen)) return give_up();
+        phase_d();
+        if (!bar_all<false>(S, gen)) return give_up();
+        if (warp == C::kYWarp) c.init_alpha();
+        __syncthreads();
+        if (warp == C::kYWarp) c.init_yw();
+    } else {
+        if (tid == 0) sc = S->sc[0];
+    }
+    __syncthreads();
+    while (!sc.done) {
+        lap(-1);
+        c.phase_a(budget <= 0);
+        if (sc.done || budget <= 0) break;
+        --budget;
+        if (!bar_all<false>(S, gen)) return give_up();
+        lap(0);
+        if (!pass()) return give_up();
+        if (!bar_all<false>(S, gen)) return give_up();
+        lap(1);
+        const int yp = sc.ypend;
+        __syncthreads();   // beta_scalars clears the flag
+        if (warp == C::kSWarp) c.beta_scalars();
+        else if (warp == C::kYWarp && yp) c.update_yw();
+        reduce();
+        if (!bar_all<false>(S, gen)) return give_up();
+        lap(2);
+        phase_d();
+        if (!bar_all<false>(S, gen)) return give_up();
+        lap(3);
+    }
+    if (sc.ypend && warp == C::kYWarp) c.update_yw();
+    __syncthreads();
+    if (c.bid == 0 && tid == 0) {
+        sc.ypend = 0;
+        S->sc[0] = sc;
+    }
+    leave();
+}
+
+// A (FP64, column-major) to the tile storage, with the range check of the mixed
+// path and ||A||_F^2 partials.  FP64 arithmetic on every element would hold the
+// FP64 pipe for ~2 ms at 40,000 x 4,000: hi and lo are cut from the bits.
+constexpr int kSplitRows = 64, kSplitCols = 32;
+
+// hi = x rounded to 24 bits, lo = the rest rounded to 24: as ff_from_double for
+// magnitudes in [2^-100, 2^100] and 0, except that ties round away
+SKL_DEV ff ff_from_bits(double x)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const unsigned hiw = (unsigned)(b >> 32);
+    const int e = (int)((hiw >> 20) & 0x7ff) - 1023;
+    if (e < -101 || e > 100) return ff_from_double(x);
+    const unsigned sign = hiw & 0x80000000u;
+    const unsigned low = (unsigned)b & 0x1fffffffu;                       // the 29 bits below FP32
+    const unsigned top = ((hiw & 0xfffffu) << 3) | ((unsigned)b >> 29);   // 23 bits
+    const unsigned up = low >> 28;
+    const float h = __uint_as_float(sign | (((unsigned)(e + 127) << 23) + top + up));
+    const int rest = (int)low - (int)(up << 29);                          // in units of 2^(e - 52)
+    const float l = (float)rest * __uint_as_float(sign | ((unsigned)(e - 52 + 127 + 30) << 23)) * 0x1p-30f;
+    return ff{h, l};
+}
+
+__global__ void __launch_bounds__(256)
+k_split_tiles(const double* __restrict__ A, int64_t lda, int n, int d, int K, int CW, int64_t blocks,
+              float4* __restrict__ out, float2* __restrict__ fro, unsigned* __restrict__ status)
+{
+    pdl_wait();
+    __shared__ float2 tile[kSplitCols][kSplitRows + 1];
+    __shared__ ff red[8];
+    ff ss{0.f, 0.f};
+    bool bad = false;
+    const int64_t rtiles = (blocks * 2 + kSplitRows - 1) / kSplitRows;
+    const int ctiles = (K * CW + kSplitCols - 1) / kSplitCols;
+    for (int64_t w = blockIdx.x; w < rtiles * ctiles; w += gridDim.x) {
+        const int64_t r0 = (w % rtiles) * kSplitRows;
+        const int c0 = (int)(w / rtiles) * kSplitCols;
+        double x[kSplitRows * kSplitCols / 256];
+#pragma unroll
+        for (int q = 0; q < kSplitRows * kSplitCols / 256; ++q) {
+            const int e = threadIdx.x + q * 256, i = e % kSplitRows, j = e / kSplitRows;
+            x[q] = (r0 + i < n && c0 + j < d) ? A[(r0 + i) + (int64_t)(c0 + j) * lda] : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < kSplitRows * kSplitCols / 256; ++q) {
+            const int e = threadIdx.x + q * 256, i = e % kSplitRows, j = e / kSplitRows;
+            const unsigned long long m = (unsigned long long)__double_as_longlong(x[q]) & 0x7fffffffffffffffull;
+            // |x| > 2^100 or 0 < |x| < 2^-100 (a NaN is neither)
+            bad |= (m > 0x4630000000000000ull && m <= 0x7ff0000000000000ull) || (m != 0 && m < 0x39b0000000000000ull);
+            const ff f = ff_from_bits(x[q]);
+            ff_fma(ss, f, f);
+            tile[j][i] = make_float2(f.hi, f.lo);
+        }
+        __syncthreads();
+        for (int e = threadIdx.x; e < kSplitRows / 2 * kSplitCols; e += 256) {
+            const int j = e % kSplitCols, p = e / kSplitCols;   // row pair p
+            const int col = c0 + j;
+            const int64_t blk = r0 / 2 + p;
+            if (col < K * CW && blk < blocks) {
+                const float2 e = tile[j][2 * p], o = tile[j][2 * p + 1];
+                out[(blk * K + col / CW) * CW + col % CW] = make_float4(e.x, o.x, e.y, o.y);
+            }
+        }
+        __syncthreads();
+    }
+    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(status, kStatusRange);
+    const ff t = block_sum_ff(ss, red);
+    if (threadIdx.x == 0) fro[blockIdx.x] = make_float2(t.hi, t.lo);
 }
 
 // ---- column chunks -------------------------------------------------------------
@@ -841,48 +1274,6 @@ struct Clock {
     }
 };
 
-// One persistent kernel per kItersPerLaunch iterations.
-template <bool MIXED, int NT>
-const PState* run_persistent(const PArgs<MIXED>& g, int G, size_t smem, void* host_pinned, cudaStream_t st)
-{
-    const bool cluster = G <= kCluster;
-    const void* fn = cluster ? (const void*)k_lsqr_persist<MIXED, NT, true>
-                             : (const void*)k_lsqr_persist<MIXED, NT, false>;
-    allow_max_dynamic_smem(fn);
-    if (cluster) SKL_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)G);
-    cfg.blockDim = dim3(NT);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    if (cluster) {
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = kCluster;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    } else {
-        at[0].id = cudaLaunchAttributeCooperative;
-        at[0].val.cooperative = 1;
-    }
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    const PState* hs = (const PState*)host_pinned;
-    const Clock clock;
-    for (int start = 1;; start = 0) {
-        int budget = kItersPerLaunch;
-        PArgs<MIXED> a = g;
-        void* args[] = {(void*)&a, (void*)&start, (void*)&budget};
-        SKL_CUDA(cudaLaunchKernelExC(&cfg, fn, args));
-        SKL_LAUNCHED();
-        SKL_CUDA(cudaMemcpyAsync(host_pinned, g.S, sizeof(PState), cudaMemcpyDeviceToHost, st));
-        SKL_CUDA(cudaStreamSynchronize(st));
-        if (hs->timeout) fail(SKL_ERR_TIMEOUT, "a grid barrier's bounded wait gave up (LSQR)");
-        if (hs->sc[0].done) return hs;
-        clock.check();
-        SKL_CUDA(cudaMemsetAsync(&g.S->bar, 0, sizeof(unsigned), st));
-    }
-}
-
 // Phase kernels: a graph of kIterPerGraph iterations, replayed until the state
 // says done; the next replay is queued before the last one's state is read, so
 // the GPU does not wait for the host.  profile: events around the products.
@@ -969,6 +1360,55 @@ const PState* run_phases(const PArgs<MIXED>& g, int G, size_t smem, void* host_p
     }
 }
 
+// The launches of a persistent kernel fn(args, more, start, budget) until the
+// state says done.
+const PState* run_cooperative(const void* fn, bool cluster, int G, int threads, size_t smem, PState* S, void* host_pinned,
+                              cudaStream_t st, void* arg0, void* arg1)
+{
+    if (cluster) SKL_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)G);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    if (cluster) {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = kCluster;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    } else {
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    const PState* hs = (const PState*)host_pinned;
+    const Clock clock;
+    for (int start = 1;; start = 0) {
+        int budget = kItersPerLaunch;
+        void* with1[] = {arg0, arg1, (void*)&start, (void*)&budget};
+        void* without[] = {arg0, (void*)&start, (void*)&budget};
+        SKL_CUDA(cudaLaunchKernelExC(&cfg, fn, arg1 ? with1 : without));
+        SKL_LAUNCHED();
+        SKL_CUDA(cudaMemcpyAsync(host_pinned, S, sizeof(PState), cudaMemcpyDeviceToHost, st));
+        SKL_CUDA(cudaStreamSynchronize(st));
+        if (hs->timeout) fail(SKL_ERR_TIMEOUT, "a bounded wait gave up (LSQR's grid barrier or its copies)");
+        if (hs->sc[0].done) return hs;
+        clock.check();
+        SKL_CUDA(cudaMemsetAsync(&S->bar, 0, sizeof(unsigned), st));
+    }
+}
+
+template <bool MIXED, int NT>
+const PState* run_persistent(const PArgs<MIXED>& g, int G, size_t smem, void* host_pinned, cudaStream_t st)
+{
+    const void* fn = G <= kCluster ? (const void*)k_lsqr_persist<MIXED, NT, true>
+                                   : (const void*)k_lsqr_persist<MIXED, NT, false>;
+    allow_max_dynamic_smem(fn);
+    PArgs<MIXED> a = g;
+    return run_cooperative(fn, G <= kCluster, G, NT, smem, g.S, host_pinned, st, (void*)&a, nullptr);
+}
+
 template <bool MIXED, int NT>
 LsqrResult persist_impl(const LsqrProblem& P, const double* b, double tol, int64_t max_it, double* y_out, void* work,
                         void* host_pinned, cudaStream_t st, int profile, cudaStream_t capture_stream)
@@ -1040,19 +1480,174 @@ LsqrResult persist_impl(const LsqrProblem& P, const double* b, double tol, int64
     return res;
 }
 
+// ---- dense host side -------------------------------------------------------------
+// Row pairs of a tile: at most 16 entries per thread (64 registers).
+constexpr int tile_rb(int K) { return K == 1 ? 8 : K <= 4 ? 4 : 2; }
+
+struct DenseShape {
+    int K, CW, RB, ntiles;
+    int64_t blocks;
+    size_t bytes() const { return (size_t)blocks * K * CW * 16; }
+};
+DenseShape dense_shape(int64_t n, int64_t d)
+{
+    DenseShape s;
+    s.K = (int)((d + kDT - 1) / kDT);
+    s.CW = (int)((d + s.K - 1) / s.K);
+    s.RB = tile_rb(s.K);
+    s.ntiles = (int)((n + 2 * s.RB - 1) / (2 * s.RB));
+    s.blocks = (int64_t)s.ntiles * s.RB;
+    return s;
+}
+
+// One CTA per ~100 KB, at most one per SM.
+int dense_ctas(const LsqrProblem& P)
+{
+    const double bytes = 8.0 * (double)P.n * (double)P.d + 4.0 * (double)P.r * (double)P.r;
+    return (int)std::max<double>(1, std::min<double>(sm_count_p(), std::ceil(bytes / 100e3)));
+}
+
+struct DBufs {
+    PState* S;
+    float2 *us, *vs, *z, *part, *tn, *pa, *pb;
+    double *w, *y;
+    long long* prof;
+    size_t bytes;
+};
+DBufs dcarve(const LsqrProblem& P, void* work)
+{
+    DBufs B;
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        void* p = (char*)work + off;
+        off += (bytes + 255) & ~(size_t)255;
+        return p;
+    };
+    const DenseShape s = dense_shape(P.n, P.d);
+    B.S = (PState*)take(sizeof(PState));
+    B.us = (float2*)take(P.n * sizeof(float2));
+    B.vs = (float2*)take(P.r * sizeof(float2));
+    B.z = (float2*)take(P.d * sizeof(float2));
+    B.part = (float2*)take((size_t)sm_count_p() * s.K * s.CW * sizeof(float2));
+    B.tn = (float2*)take(P.d * sizeof(float2));
+    B.pa = (float2*)take(1024 * sizeof(float2));
+    B.pb = (float2*)take(1024 * sizeof(float2));
+    B.w = (double*)take(P.r * sizeof(double));
+    B.y = (double*)take(P.r * sizeof(double));
+    B.prof = (long long*)take(4 * sizeof(long long));
+    B.bytes = off;
+    return B;
+}
+
+const void* dense_kernel(int K)
+{
+    static const void* const f[8] = {
+        (const void*)k_lsqr_dense<1, tile_rb(1)>, (const void*)k_lsqr_dense<2, tile_rb(2)>,
+        (const void*)k_lsqr_dense<3, tile_rb(3)>, (const void*)k_lsqr_dense<4, tile_rb(4)>,
+        (const void*)k_lsqr_dense<5, tile_rb(5)>, (const void*)k_lsqr_dense<6, tile_rb(6)>,
+        (const void*)k_lsqr_dense<7, tile_rb(7)>, (const void*)k_lsqr_dense<8, tile_rb(8)>};
+    return f[K - 1];
+}
+
+LsqrResult dense_impl(const LsqrProblem& P, const double* b, double tol, int64_t max_it, double* y_out, void* work,
+                      void* host_pinned, cudaStream_t st, int profile)
+{
+    const DenseShape s = dense_shape(P.n, P.d);
+    DBufs B = dcarve(P, work);
+    PArgs<true> g{};
+    g.n = (int)P.n;
+    g.r = (int)P.r;
+    g.d = (int)P.d;
+    g.cols = P.cols;
+    g.Mr = (const float*)P.Mrow;
+    g.Mc = (const float*)P.M;
+    g.ldm = P.ldm;
+    g.b = b;
+    g.us = B.us;
+    g.vs = B.vs;
+    g.z = B.z;
+    g.w = B.w;
+    g.y = B.y;
+    g.pa = B.pa;
+    g.pb = B.pb;
+    g.S = B.S;
+    const int G = dense_ctas(P);
+    const int nloc = (int)((P.r + G - 1) / G), nw = kDT / 32 - 1;
+    g.S_seg = std::max(1, std::min(8, nloc <= nw ? nw / nloc : 4 * nw / nloc));
+    DArgs a{};
+    a.A = (const float4*)P.At;
+    a.part = B.part;
+    a.tn = B.tn;
+    a.CW = s.CW;
+    a.ntiles = s.ntiles;
+    a.sv_bytes = (int)((std::max(vec_smem(P), (size_t)s.K * kDT * sizeof(float2)) + 127) & ~(size_t)127);
+    const void* fn = dense_kernel(s.K);
+    allow_max_dynamic_smem(fn);
+    cudaFuncAttributes fa;
+    SKL_CUDA(cudaFuncGetAttributes(&fa, fn));
+    const int room = fa.maxDynamicSharedSizeBytes - a.sv_bytes;
+    a.nslots = std::min(64, room / (s.CW * 16));
+    if (a.nslots < s.K * s.RB) fail(SKL_ERR_INVALID, "dense LSQR: the tile ring does not fit");
+    a.prof = profile ? B.prof : nullptr;
+    SKL_CUDA(cudaMemsetAsync(B.z, 0, P.d * sizeof(float2), st));
+    if (profile) SKL_CUDA(cudaMemsetAsync(B.prof, 0, 4 * sizeof(long long), st));
+    PState init{};
+    init.tol = tol;
+    init.max_it = max_it;
+    SKL_CUDA(cudaMemcpyAsync(B.S, &init, sizeof(PState), cudaMemcpyHostToDevice, st));
+    trace_phase(st, "lsqr: init");
+    const PState* hs = run_cooperative(fn, false, G, kDT, (size_t)a.sv_bytes + (size_t)a.nslots * s.CW * 16, B.S, host_pinned,
+                                       st, (void*)&g, (void*)&a);
+    trace_phase(st, "lsqr: done");
+    LsqrResult res;
+    res.flag = hs->sc[0].flag;
+    res.it = hs->sc[0].it;
+    if (profile) {
+        // M v, the pass over A (both products), M^T t with the shares' sum
+        long long ns[4];
+        SKL_CUDA(cudaMemcpyAsync(host_pinned, B.prof, sizeof ns, cudaMemcpyDeviceToHost, st));
+        SKL_CUDA(cudaStreamSynchronize(st));
+        std::memcpy(ns, host_pinned, sizeof ns);
+        const double ms[4] = {ns[1] * 1e-6, 0.0, ns[0] * 1e-6, (ns[2] + ns[3]) * 1e-6};
+        for (int q = 0; q < 4; ++q) {
+            res.prof_ms[q] = ms[q];
+            res.prof_launches[q] = q == 1 ? 0 : res.it;
+        }
+    }
+    SKL_CUDA(cudaMemcpyAsync(y_out, B.y, P.r * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    return res;
+}
+
 }  // namespace
+
+bool lsqr_dense_tiled(int64_t d, int precision) { return precision == SKL_PREC_MIXED && d >= 1 && d <= kDenseMaxD; }
+size_t lsqr_dense_tile_bytes(int64_t n, int64_t d) { return dense_shape(n, d).bytes(); }
+
+void split_dense_tiles(const double* A, int64_t lda, int64_t n, int64_t d, void* out, float2* fro, unsigned* status,
+                       cudaStream_t st)
+{
+    const DenseShape s = dense_shape(n, d);
+    launch_k(k_split_tiles, kFroParts, 256, 0, st, A, lda, (int)n, (int)d, s.K, s.CW, s.blocks, (float4*)out, fro,
+             status);
+    SKL_LAUNCHED();
+}
 
 bool lsqr_persist_fits(const LsqrProblem& P)
 {
+    if (P.At) return true;
     const int G = grid_of(P).ctas;
     return !P.Ad && P.r > 0 && (P.r + G - 1) / G <= kMaxUnits && vec_smem(P) <= 200 * 1024;
 }
 
-size_t lsqr_persist_workspace_bytes(const LsqrProblem& P) { return pcarve(P, nullptr).bytes; }
+size_t lsqr_persist_workspace_bytes(const LsqrProblem& P)
+{
+    return P.At ? dcarve(P, nullptr).bytes : pcarve(P, nullptr).bytes;
+}
 
 LsqrResult lsqr_persist_run(const LsqrProblem& P, const double* b, double tol, int64_t max_it, double* y, void* work,
                             void* host_pinned, cudaStream_t st, int profile, cudaStream_t capture_stream)
 {
+    if (P.At) return dense_impl(P, b, tol, max_it, y, work, host_pinned, st, profile);
     const bool big = grid_of(P).threads == kBigCta;
     auto* fn = P.precision == SKL_PREC_MIXED
                    ? (big ? persist_impl<true, kBigCta> : persist_impl<true, kSmallCta>)

@@ -949,7 +949,10 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
     const size_t qr_ws = cpqr_workspace_bytes<T>(m, d);
     const size_t inv_ws = trinv_workspace_bytes<T>(d);
     LsqrProblem Pq;
-    Pq.n = n; Pq.d = d; Pq.r = d; Pq.precision = o.precision; Pq.Ad = A; Pq.lda = n;
+    const bool tiled = lsqr_dense_tiled(d, o.precision);
+    Pq.n = n; Pq.d = d; Pq.r = d; Pq.precision = o.precision;
+    if (tiled) Pq.At = A;
+    else Pq.Ad = A, Pq.lda = n;
     const size_t lsqr_ws = lsqr_workspace_bytes(Pq);
     const size_t bkt_scr = build_buckets_scratch_ints(m, N * k) * sizeof(int);
     const size_t dht_ws = dht_scratch_bytes(N, o.precision);
@@ -957,7 +960,8 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
     const int64_t ldm_max = round_up(d, 4);
     Sizer S;
     S.add<double>(n); S.add<unsigned>(N * k); S.add<int>(m + 1); S.add<unsigned>(N * k);
-    S.add<char>(mixed ? (int64_t)(n * d * sizeof(float2)) : 0);
+    const int64_t a2_bytes = tiled ? (int64_t)lsqr_dense_tile_bytes(n, d) : mixed ? (int64_t)(n * d * sizeof(float2)) : 0;
+    S.add<char>(a2_bytes);
     S.add<T>(ld * d); S.add<double>(d); S.add<double>(m); S.add<int>(d); S.add<T>(mn); S.add<int>(4);
     S.add<T>(ldm_max * d); S.add<T>(ldm_max * d); S.add<double>(4); S.add<double>(d);
     S.add<double>(n); S.add<double>(d); S.add<double>(1024); S.add<double>(8);
@@ -969,7 +973,7 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
     unsigned* hidx = Ar.alloc<unsigned>(N * k);
     int* bptr = Ar.alloc<int>(m + 1);
     unsigned* bent = Ar.alloc<unsigned>(N * k);
-    float2* A2 = mixed ? (float2*)Ar.take(n * d * sizeof(float2)) : nullptr;
+    float2* A2 = mixed ? (float2*)Ar.take((size_t)a2_bytes) : nullptr;
     T* SA = Ar.alloc<T>(ld * d);
     double* colscale = Ar.alloc<double>(d);
     double* cvec = Ar.alloc<double>(m);
@@ -990,7 +994,8 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
     SKL_CUDA(cudaEventRecord(ev[1], st));
     if (mixed) {
         SKL_CUDA(cudaMemsetAsync(C.dev_status, 0, sizeof(unsigned), st));
-        split_dense(A, lda, n, d, A2, C.dev_status, st);
+        if (tiled) split_dense_tiles(A, lda, n, d, A2, (float2*)part, C.dev_status, st);
+        else split_dense(A, lda, n, d, A2, C.dev_status, st);
     }
     {
         std::vector<double> ones((size_t)d, 1.0);
@@ -998,6 +1003,14 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
         SKL_CUDA(cudaStreamSynchronize(st));
     }
     if (mixed && (read_status(C, st) & kStatusRange)) return false;
+    double fro = 0.0;   // ||A||_F
+    if (tiled) {
+        std::vector<float2> fp((size_t)kFroParts);
+        SKL_CUDA(cudaMemcpyAsync(fp.data(), part, kFroParts * sizeof(float2), cudaMemcpyDeviceToHost, st));
+        SKL_CUDA(cudaStreamSynchronize(st));
+        for (float2 v : fp) fro += (double)v.x + (double)v.y;
+        fro = std::sqrt(fro);
+    }
     if (host_thread->joinable()) host_thread->join();
     SKL_CUDA(cudaMemcpyAsync(Dd, hD->data(), n * sizeof(double), cudaMemcpyHostToDevice, st));
     if (sample_rows) {
@@ -1048,19 +1061,20 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
     }
     LsqrProblem P;
     P.n = n; P.d = d; P.nnz = n * d;
-    P.Ad = mixed ? (const void*)A2 : (const void*)A;
+    if (tiled) P.At = A2;
+    else P.Ad = mixed ? (const void*)A2 : (const void*)A;
     P.lda = mixed ? n : lda;
     P.Ad64 = A; P.lda64 = lda;
     P.cols = jpvt; P.colscale = colscale;
     P.M = Mc; P.Mrow = Mr; P.ldm = ldm; P.r = rank; P.precision = o.precision;
-    // ||A||_F
-    fro_partials(A, lda, n, d, part, st);
-    std::vector<double> fp(512);
-    SKL_CUDA(cudaMemcpyAsync(fp.data(), part, 512 * sizeof(double), cudaMemcpyDeviceToHost, st));
-    SKL_CUDA(cudaStreamSynchronize(st));
-    double fro = 0.0;
-    for (double v : fp) fro += v;
-    fro = std::sqrt(fro);
+    if (!tiled) {
+        fro_partials(A, lda, n, d, part, st);
+        std::vector<double> fp(512);
+        SKL_CUDA(cudaMemcpyAsync(fp.data(), part, 512 * sizeof(double), cudaMemcpyDeviceToHost, st));
+        SKL_CUDA(cudaStreamSynchronize(st));
+        for (double v : fp) fro += v;
+        fro = std::sqrt(fro);
+    }
     double rnorm = 0.0, be = 0.0;
     auto residual = [&]() {
         residual_and_backward(P, x_dev, b, rs, part, scal, st);

@@ -259,6 +259,8 @@ struct LsqrProblem {
     // dense A: storage-type copy (n x d, lda) and the FP64 original (lda64)
     const void* Ad = nullptr; int64_t lda = 0;
     const double* Ad64 = nullptr; int64_t lda64 = 0;
+    // dense A, mixed path, d <= 4,096: the tile storage of the one-pass products
+    const void* At = nullptr;
     // preconditioner: column i of the pivoted set is A(:, cols[i]) scaled by
     // colscale[cols[i]], times M = R11^{-1} (r x r, column-major M and a
     // row-major copy Mrow, both ldm)
@@ -296,6 +298,14 @@ bool lsqr_persist_fits(const LsqrProblem& P);
 size_t lsqr_persist_workspace_bytes(const LsqrProblem& P);
 LsqrResult lsqr_persist_run(const LsqrProblem& P, const double* b, double tol, int64_t max_it, double* y, void* work,
                             void* host_pinned, cudaStream_t st, int profile, cudaStream_t capture_stream);
+// Tile storage of a dense A for the one-pass products: whether the problem takes
+// it, its bytes, and its build from A (FP64, column-major), with the range check
+// (kStatusRange) and kFroParts partial sums of ||A||_F^2.
+constexpr int kFroParts = 152 * 3;
+bool lsqr_dense_tiled(int64_t d, int precision);
+size_t lsqr_dense_tile_bytes(int64_t n, int64_t d);
+void split_dense_tiles(const double* A, int64_t lda, int64_t n, int64_t d, void* out, float2* fro, unsigned* status,
+                       cudaStream_t st);
 // One product in isolation with LSQR's storage and arithmetic: y = A x
 // (trans 'n', CSR kernel) or y = A^T x ('t', CSC kernel, P.cols = 0..d-1,
 // P.r = d).  The stored values are A(:, c) * vscale[c] (vscale nullptr: A's
