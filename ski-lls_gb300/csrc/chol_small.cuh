@@ -79,7 +79,9 @@ template <> SKL_DEV double t_rcp_chain<double>(double x) { return __drcp_rn(x); 
 
 // Step k = 8 kh + kl: kl is a compile-time index (the inner loop is unrolled
 // by 8) so the pivot and the lane's own column k come from fixed registers.
-template <typename T>
+// BOOST: such a pivot is replaced by that bound (by 1 if its mass is not positive,
+// which sets *bad to 2) and the elimination goes on.
+template <typename T, bool BOOST = false>
 SKL_DEV void warp16_chol(T* A, int ld, const T* __restrict__ mass, T eps, int* bad)
 {
     const unsigned full = 0xffffffffu;
@@ -96,7 +98,9 @@ SKL_DEV void warp16_chol(T* A, int ld, const T* __restrict__ mass, T eps, int* b
             const T ms = mass[k];
             const bool ok = d > T(32) * eps * ms && ms > T(0);
             isbad = isbad || !ok;
-            const T inv = ok ? t_rcp_chain(d) : T(0);
+            const T bound = BOOST ? (ms > T(0) ? T(32) * eps * ms : T(1)) : T(0);
+            const T inv = ok ? t_rcp_chain(d) : BOOST ? t_rcp_chain(bound) : T(0);
+            if (BOOST && !(ms > T(0)) && lane == 0) atomicMax(bad, 2);
             T rk[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) rk[e] = __shfl_sync(full, a[e], 2 * k + (lane & 1));
@@ -109,12 +113,18 @@ SKL_DEV void warp16_chol(T* A, int ld, const T* __restrict__ mass, T eps, int* b
             }
         }
     }
-    if (isbad && lane == 0) *bad = 1;
-    // a failed pivot's row is zero, its diagonal entry too
-    const T d = own_col(a, r, lane);
-    const T sc = d > T(32) * eps * mass[r] ? t_rcp(t_sqrt(d)) : T(0);
+    if (isbad && lane == 0) atomicMax(bad, 1);
+    // a failed pivot's row is zero, its diagonal entry too; boosted, the pivot is
+    // the bound
+    T d = own_col(a, r, lane);
+    const bool good = d > T(32) * eps * mass[r] && mass[r] > T(0);
+    if (BOOST && !good) d = mass[r] > T(0) ? T(32) * eps * mass[r] : T(1);
+    const T sc = good || BOOST ? t_rcp(t_sqrt(d)) : T(0);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) A[r * ld + cb + e] = (cb + e >= r) ? a[e] * sc : T(0);
+    for (int e = 0; e < 8; ++e) {
+        const T v = (BOOST && cb + e == r) ? d : a[e];
+        A[r * ld + cb + e] = (cb + e >= r) ? v * sc : T(0);
+    }
     __syncwarp();
 }
 
@@ -573,7 +583,7 @@ SKL_DEV void inv_unit_lower_offdiag(const T* L, int ldl, T* Y, int ldy, int np, 
 // zeros below) over G, X (upper, zeros below) to Xs.  Blocked right-looking:
 // per 16-block, warp 0 factors the diagonal block and inverts it, then
 // R12 = R11^{-T} G12 and G22 -= R12^T R12 as block products.
-template <typename T>
+template <typename T, bool BOOST = false>
 SKL_DEV void chol_inv_small(T* G, int ldx, int np, const T* __restrict__ mass, T eps, T* Xs, T* tmp,
                             int ldt, int* bad)
 {
@@ -583,7 +593,7 @@ SKL_DEV void chol_inv_small(T* G, int ldx, int np, const T* __restrict__ mass, T
         const int rest = np - k0 - kDB;
         T* G11 = G + k0 * ldx + k0;
         if (threadIdx.x < 32) {
-            warp16_chol<T>(G11, ldx, mass + k0, eps, bad);
+            warp16_chol<T, BOOST>(G11, ldx, mass + k0, eps, bad);
             warp16_inv_upper<T>(G11, ldx, Xs + k0 * ldx + k0, ldx, true);
         }
         __syncthreads();

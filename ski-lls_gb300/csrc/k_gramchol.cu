@@ -21,8 +21,14 @@
 // sweep (zero row and column of M) where the caller carries such columns in
 // LSQR's basis (the mixed sparse path); the small singular values they stand
 // for, taken from S A itself, must then lie below a quarter of the rank rule's
-// threshold, as the pivoted factorization's trailing pivots would.  A sketch
-// that fails a test keeps the pivoted factorization: S A is not touched here.
+// threshold, as the pivoted factorization's trailing pivots would.
+// On the dense mixed path a failed pivot is raised to the bound instead and the
+// same is done again on Q = S A M (at most twice): each pass takes the condition
+// number to about the root of what exceeds ~300.  40,000 x 4,000 (S A 6,800 x 4,000):
+// QR and inverse 20.2 + 1.4 ms, one pass 4.4 ms, two (condition number 1e3 to
+// 1e5) 9.9 ms with LSQR's iterations, x and residual unchanged.  From ~1e6 on
+// most attempts end early and the QR comes on top of one pass's time.
+// A sketch that fails a test keeps the QR: S A is not touched here.
 //
 // Sweep (outer blocks of 256 rows, inner blocks of 64): the same row
 // operations that turn G into R turn I into E = R^{-T}, so one trailing update
@@ -87,6 +93,8 @@ struct TnArgs {
     int e_add;              // E part: tiles below this index add to C, others overwrite
     int g_add;              // G part adds to C
     int upper;              // skip G tiles that lie below the diagonal
+    int tri;                // 1: B is upper triangular (K ends at the tile's last column);
+                            // 2: A^T is too (K starts at the tile's first row)
     float alpha;
     float* Cg; int64_t ldg;
     float* Ce; int64_t lde;
@@ -112,7 +120,8 @@ k_tc_tn(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtens
     // bars: full, conv, empty [kNStages each], tfull[2], tempty[2], done; then the TMEM address
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 3 * kNStages + 5);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nkb = t.nkb;
+    const int kb0 = t.tri == 2 ? row0 / kBK : 0;
+    const int nkb = (t.tri ? min(t.nkb, (col0 + kNT) / kBK) : t.nkb) - kb0;
     const int ngroups = (nkb + kNGroup - 1) / kNGroup;
     auto full = [&](int s) { return smem_u32(bars + s); };
     auto conv = [&](int s) { return smem_u32(bars + kNStages + s); };
@@ -157,8 +166,8 @@ k_tc_tn(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtens
                 if (kb >= kNStages) ok = mbar_wait(empty(s), ((kb / kNStages) - 1) & 1, status);
                 if (!ok) break;
                 mbar_expect_tx(full(s), 2 * kNTile);
-                tma_load_2d(smem_u32(hi(s)), &mapA, t.kA + kb * kBK, t.a0 + blockIdx.y * kNT, full(s));
-                tma_load_2d(smem_u32(hi(s)) + kNTile, mapB, t.kB + kb * kBK, col0, full(s));
+                tma_load_2d(smem_u32(hi(s)), &mapA, t.kA + (kb0 + kb) * kBK, t.a0 + blockIdx.y * kNT, full(s));
+                tma_load_2d(smem_u32(hi(s)) + kNTile, mapB, t.kB + (kb0 + kb) * kBK, col0, full(s));
                 ++issued;
             }
             // the copies this CTA issued have landed before it may exit
@@ -306,6 +315,7 @@ struct GcArgs {
     int* bad; int* ndrop; int* drop; int drop_cap;
     int d;
     T pivot;                // pivots at or below pivot * mass fail
+    int boost;              // a failed pivot becomes that bound (counted in ndrop)
 };
 
 constexpr int kSL = kIB + 4;   // row-major 64 x 64 shared-memory blocks
@@ -337,12 +347,20 @@ SKL_DEV void diag_block(const GcArgs<T>& g, int q, int b, int ql, T* S0, T* S1, 
     for (int k = threadIdx.x; k < np; k += kSmallThreads) mass[k] = k < b ? g.mass[q + k] : T(1);
     __syncthreads();
     // chol_inv_small asks for a pivot above 32 x its eps x mass
-    chol_inv_small<T>(S0, kSL, np, mass, g.pivot / T(32), S1, tmp, 36, &s_any);
+    if (g.boost) chol_inv_small<T, true>(S0, kSL, np, mass, g.pivot / T(32), S1, tmp, 36, &s_any);
+    else chol_inv_small<T>(S0, kSL, np, mass, g.pivot / T(32), S1, tmp, 36, &s_any);
     for (int e = threadIdx.x; e < b * b; e += kSmallThreads) {
         const int i = e % b, c = e / b;
         g.R[(q + i) + (int64_t)(q + c) * g.ldg] = S0[i * kSL + c];
         g.mkk[(ql + i) + (ql + c) * kOB] = S1[i * kSL + c];
         g.E[(q + i) + (int64_t)(q + c) * g.lde] = S1[c * kSL + i];
+    }
+    if (g.boost) {
+        if (threadIdx.x == 0 && s_any) {
+            *g.ndrop = 1;
+            if (s_any > 1) *g.bad = 1;   // a zero (or NaN) column
+        }
+        return;
     }
     if (s_any && threadIdx.x < 32) {
         int n = *g.ndrop;
@@ -576,6 +594,30 @@ k_gc_finish(const double* __restrict__ part, int nparts, const T* __restrict__ g
     }
 }
 
+// out(c, r) = X(r, c) for the rows x cols matrix X; upper: entries below X's
+// diagonal count as zero, and become zero in X.
+__global__ void __launch_bounds__(256)
+k_gc_tr(float* __restrict__ X, int64_t ldx, int rows, int cols, int upper, float* __restrict__ out, int64_t ldo)
+{
+    pdl_wait();
+    __shared__ float tile[32][33];
+    const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    for (int q = ty; q < 32; q += 8) {
+        const int r = r0 + tx, c = c0 + q;
+        float v = 0.f;
+        if (r < rows && c < cols) {
+            if (upper && r > c) X[r + (int64_t)c * ldx] = 0.f;
+            else v = X[r + (int64_t)c * ldx];
+        }
+        tile[q][tx] = v;
+    }
+    __syncthreads();
+    for (int q = ty; q < 32; q += 8) {
+        const int c = c0 + tx, r = r0 + q;
+        if (r < rows && c < cols) out[c + (int64_t)r * ldo] = tile[tx][q];
+    }
+}
+
 // ---- c = argmin || S A M c - S b ||: normal equations and refinement -----------
 // Products of FP32 matrices with FP64-class vectors: float-float accumulation
 // (FP64 FMAs would take 5x as long here); vectors as (hi, lo) pairs.
@@ -759,13 +801,14 @@ struct GramBuffers {
     T* G; T* R; T* mkk; T* gdiag; T* mass; T* partial; int64_t partial_cap;
     int* bad; int* ndrop; double* part; double* out;
     T* dw; T* dt; T* dp; T* dn; int64_t ldp;
+    T* Q; T* QT; T* M2c; T* M2r; T* Racc; int64_t ldq;
     typename GV<T>::type* rv; typename GV<T>::type* tv; typename GV<T>::type* cv; typename GV<T>::type* wv;
     double* rows_part; double* c;
     size_t bytes;
 };
 
 template <typename T>
-GramBuffers<T> gram_carve(void* work, int64_t m, int64_t d)
+GramBuffers<T> gram_carve(void* work, int64_t m, int64_t d, bool multi)
 {
     GramBuffers<T> B;
     size_t used = 0;
@@ -790,7 +833,7 @@ GramBuffers<T> gram_carve(void* work, int64_t m, int64_t d)
     B.ndrop = (int*)take(sizeof(int));
     // dropped columns: their coefficients and two rounds' scratch (d x k), their
     // residuals (m x k)
-    const int64_t kd = std::is_same<T, float>::value ? std::min<int64_t>(kGramDropMax, d / 4) : 0;
+    const int64_t kd = std::is_same<T, float>::value && !multi ? std::min<int64_t>(kGramDropMax, d / 4) : 0;
     B.ldp = (m + 31) / 32 * 32;
     B.dw = (T*)take((size_t)B.ldg * kd * sizeof(T));
     B.dt = (T*)take((size_t)B.ldg * kd * sizeof(T));
@@ -804,6 +847,14 @@ GramBuffers<T> gram_carve(void* work, int64_t m, int64_t d)
     B.wv = (V*)take((size_t)d * sizeof(V));
     B.rows_part = (double*)take((size_t)((d + kResCols - 1) / kResCols) * m * sizeof(double));
     B.c = (double*)take((size_t)d * sizeof(double));
+    if (multi) {   // later passes: Q, its transpose, the pass's inverse (both layouts), R so far
+        B.ldq = (m + 31) / 32 * 32;
+        B.Q = (T*)take((size_t)B.ldq * d * sizeof(T));
+        B.QT = (T*)take((size_t)B.ldg * m * sizeof(T));
+        B.M2c = (T*)take((size_t)B.ldg * d * sizeof(T));
+        B.M2r = (T*)take((size_t)B.ldg * d * sizeof(T));
+        B.Racc = (T*)take((size_t)B.ldg * d * sizeof(T));
+    }
     B.bytes = used;
     return B;
 }
@@ -926,9 +977,9 @@ void sweep_update(const Sweep<double>& S, int64_t j0, int64_t j1, int64_t i0, in
                  S.Ew + i0 + j0 * S.lde, S.lde, nullptr, 0, st);
 }
 
-// C (M x N) = A^T B, A K x M, B K x N
+// C (M x N) = A^T B, A K x M, B K x N; tri as in TnArgs (2: C's upper tiles only)
 void tn_product(int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, const float* B, int64_t ldb, float* C,
-                int64_t ldc, unsigned* status, cudaStream_t st)
+                int64_t ldc, unsigned* status, cudaStream_t st, int tri = 0)
 {
     const CUtensorMap ma = map_f32(A, K, M, lda, kNT);
     const CUtensorMap mb = map_f32(B, K, N, ldb, kNT);
@@ -939,6 +990,8 @@ void tn_product(int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, co
     t.alpha = 1.f;
     t.Cg = C;
     t.ldg = ldc;
+    t.tri = tri;
+    t.upper = tri == 2;
     tn_launch(ma, mb, mb, t, tiles(M), tiles(N), nullptr, status, st);
 }
 
@@ -982,6 +1035,55 @@ void drop_check(const Sweep<double>&, const int*, int, cudaStream_t)
     fail(SKL_ERR_INVALID, "dropped columns: FP32 only");
 }
 
+void tr_launch(float* X, int64_t ldx, int64_t rows, int64_t cols, int upper, float* out, int64_t ldo, cudaStream_t st)
+{
+    launch_k(k_gc_tr, dim3((unsigned)((rows + 31) / 32), (unsigned)((cols + 31) / 32)), 256, 0, st, X, ldx, (int)rows,
+             (int)cols, upper, out, ldo);
+    SKL_LAUNCHED();
+}
+
+// After pass 1 (S.SA = S A, its inverse in Mc / Mr): S becomes the sweep of
+// Q = S A M, with the pass's own inverse in M2c / M2r.
+void next_pass(Sweep<float>& S, float* Mc, float* Mr, int64_t ldm, bool first, cudaStream_t st)
+{
+    GramBuffers<float>& B = S.B;
+    // the last pass's inverse, zeros in its other triangles
+    float* Pc = first ? Mc : B.M2c;
+    float* Pr = first ? Mr : B.M2r;
+    const int64_t ldp = first ? ldm : B.ldg;
+    launch_k(k_gc_zero_other, (unsigned)S.d, 256, 0, st, Pc, Pr, ldp, (int)S.d);
+    SKL_LAUNCHED();
+    if (first) SKL_CUDA(cudaMemcpyAsync(B.Racc, B.R, (size_t)B.ldg * S.d * sizeof(float), cudaMemcpyDeviceToDevice, st));
+    // Q = (last Q) P by products with both operands contiguous along K
+    tr_launch(const_cast<float*>(S.SA), S.ld, S.m, S.d, 0, B.QT, B.ldg, st);
+    tn_product(S.m, S.d, S.d, B.QT, B.ldg, Pc, ldp, B.Q, B.ldq, S.status, st, 1);
+    S.SA = B.Q;
+    S.ld = B.ldq;
+    S.Ew = B.M2c;
+    S.E = B.M2r;
+    S.lde = B.ldg;
+}
+void next_pass(Sweep<double>&, double*, double*, int64_t, bool, cudaStream_t)
+{
+    fail(SKL_ERR_INVALID, "Gram passes: FP32 only");
+}
+
+// M = M (pass's inverse), R = (pass's R) R after a sweep of a later pass.
+void join_pass(Sweep<float>& S, float* Mc, float* Mr, int64_t ldm, cudaStream_t st)
+{
+    GramBuffers<float>& B = S.B;
+    const int64_t d = S.d;
+    launch_k(k_gc_zero_other, (unsigned)d, 256, 0, st, B.M2c, B.M2r, B.ldg, (int)d);
+    SKL_LAUNCHED();
+    tn_product(d, d, d, Mr, ldm, B.M2c, B.ldg, Mc, ldm, S.status, st, 2);
+    transpose_upper<float>(Mc, ldm, d, Mr, st);
+    tr_launch(B.R, B.ldg, d, d, 1, B.QT, B.ldg, st);
+    tr_launch(B.Racc, B.ldg, d, d, 1, B.G, B.ldg, st);   // zeros below R's diagonal
+    tn_product(d, d, d, B.QT, B.ldg, B.Racc, B.ldg, B.G, B.ldg, S.status, st, 2);
+    SKL_CUDA(cudaMemcpyAsync(B.Racc, B.G, (size_t)B.ldg * d * sizeof(float), cudaMemcpyDeviceToDevice, st));
+}
+void join_pass(Sweep<double>&, double*, double*, int64_t, cudaStream_t) {}
+
 void drop_exclude(const Sweep<float>& S, double limit, cudaStream_t st)
 {
     launch_k(k_gc_exclude, (unsigned)S.d, 256, 0, st, S.Ew, S.lde, (float)limit, S.B.mass);
@@ -992,9 +1094,9 @@ void drop_exclude(const Sweep<double>&, double, cudaStream_t) {}
 }  // namespace
 
 template <typename T>
-size_t gram_workspace_bytes(int64_t m, int64_t d)
+size_t gram_workspace_bytes(int64_t m, int64_t d, bool multi)
 {
-    return gram_carve<T>(nullptr, m, d).bytes;
+    return gram_carve<T>(nullptr, m, d, multi && std::is_same<T, float>::value).bytes;
 }
 
 bool gram_enabled()
@@ -1008,21 +1110,25 @@ bool gram_enabled()
 
 template <typename T>
 bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int* jpvt, T* Mc, T* Mr, int64_t ldm,
-                  double abs_thresh, double rel_thresh, double rcond_min, GramResult& res, int* drop, void* work,
+                  double abs_thresh, double rel_thresh, double rcond_min, GramResult& res, int* drop, bool multi, void* work,
                   unsigned* status, void* host_pinned, cudaStream_t st)
 {
     // columns the sweep may drop: only where the caller carries them (FP32)
     const int drop_cap = drop ? (int)std::min<int64_t>(kGramDropMax, d / 4) : 0;
     // A dependent column leaves a pivot of up to ~2e-5 of its mass in the FP32
-    // Gram matrix (measured at 120,000 x 5,000); with nothing to drop a failed
-    // pivot only ends the attempt early, which the bound on M D below would do.
+    // Gram matrix (measured at 120,000 x 5,000), and boosted pivots have to stand
+    // clear of the noise around them: with rows of noise / bound ~ 0.1 above them
+    // the inverse grows exponentially (128 eps overflowed at 200 columns).  With
+    // neither, a failed pivot only ends the attempt early, which the bound on M D
+    // below would do.
+    const bool boost = multi && std::is_same<T, float>::value;
     const T eps = std::is_same<T, float>::value ? T(5.9604644775390625e-08) : T(1.1102230246251565e-16);
-    const T pivot = (drop_cap > 0 ? T(2048) : T(128)) * eps;
-    Sweep<T> S{SA, m, d, ld, gram_carve<T>(work, m, d), Mc, Mr, ldm, status};
+    const T pivot = (drop_cap > 0 || boost ? T(2048) : T(128)) * eps;
+    Sweep<T> S{SA, m, d, ld, gram_carve<T>(work, m, d, boost), Mc, Mr, ldm, status};
     GramBuffers<T>& B = S.B;
     const size_t dsm = (2 * (size_t)kIB * kSL + 64 * 36 + kIB) * sizeof(T);
     const size_t ssm = (4 * (size_t)kIB * kSL + 64 * 36 + kIB) * sizeof(T);
-    const GcArgs<T> ga{B.G, B.R, B.ldg, Mc, Mr, ldm, B.mkk, B.mass, B.bad, B.ndrop, drop, drop_cap, (int)d, pivot};
+    GcArgs<T> ga{B.G, B.R, B.ldg, Mc, Mr, ldm, B.mkk, B.mass, B.bad, B.ndrop, drop, drop_cap, (int)d, pivot, boost ? 1 : 0};
     allow_max_dynamic_smem((const void*)k_gc_diag<T>);
     allow_max_dynamic_smem((const void*)k_gc_step<T>);
 
@@ -1086,10 +1192,12 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
             }
         }
         const int nt = (int)((d + kTrTile - 1) / kTrTile);
-        launch_k(k_gc_transpose<T>, dim3(nt, nt), 256, 0, st, S.E, ldm, (int)d, Mc, ldm, B.gdiag, B.part, B.bad);
+        launch_k(k_gc_transpose<T>, dim3(nt, nt), 256, 0, st, S.E, S.lde, (int)d, S.Ew, S.lde, B.gdiag, B.part, B.bad);
         SKL_LAUNCHED();
         launch_k(k_gc_finish<T>, 1, 1024, 0, st, B.part, nt * nt, B.gdiag, (int)d, B.bad, B.ndrop, status, B.out);
         SKL_LAUNCHED();
+    };
+    auto solve_c = [&] {
         if (c) {
             // c = M M^T-normal equations of the sketched problem, then two steps of
             // refinement against its residual: each contracts the error by the
@@ -1128,6 +1236,7 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
     int ndrop = 0;
     for (int attempt = 0;; ++attempt) {
         factor(attempt);
+        solve_c();
         read_out(8);
         mf2 = hp[2];
         mdf2 = hp[3];
@@ -1136,13 +1245,54 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
         if ((unsigned)hp[6] & kStatusTcTimeout)
             fail(SKL_ERR_TIMEOUT, "a tensor-core product's bounded wait gave up");
         if (hp[5] != 0.0 || !std::isfinite(mf2) || !std::isfinite(mdf2) || !(mf2 > 0.0)) return false;
-        if ((double)eps * mdf2 <= 1.0 / 16) break;
+        if ((double)eps * mdf2 <= 1.0 / 16 && !(boost && ndrop > 0)) break;
+        if (boost) break;
         // dependent columns whose pivots passed: again without them
         if (ndrop == 0 || attempt == 2) return false;
         drop_exclude(S, 1.0 / (64.0 * (double)eps), st);
     }
     // the rank rule's threshold, with a factor 2 for M's own error
     const double thresh = std::max(abs_thresh, rel_thresh * std::sqrt(gmax));
+    const T* R = B.R;
+    if (boost && !((double)eps * mdf2 <= 1.0 / 16 && ndrop == 0)) {
+        // Too ill-conditioned for its Gram matrix, or with boosted pivots: the same
+        // on Q = S A M, whose condition number is about the root of the excess, at
+        // most twice; M and R are the passes' products.  Boosted pivots can make a
+        // pass's inverse grow (at 1e5 and beyond, by size), which costs the product
+        // its digits and ends the attempt: eps ||S A|| ||M_1|| ||M_2|| was at most 30
+        // where LSQR took the QR's iterations.
+        const double unit = (double)eps * std::sqrt(gmax);
+        if (unit * std::sqrt(mf2 * (double)d) > 64.0) return false;
+        for (int pass = 2;; ++pass) {
+            const double before = mf2;
+            next_pass(S, Mc, Mr, ldm, pass == 2, st);
+            ga.Ew = S.Ew;
+            ga.E = S.E;
+            ga.lde = S.lde;
+            factor(0);
+            read_out(8);
+            if ((unsigned)hp[6] & kStatusTcTimeout)
+                fail(SKL_ERR_TIMEOUT, "a tensor-core product's bounded wait gave up");
+            if (hp[5] != 0.0 || !std::isfinite(hp[2]) || !std::isfinite(hp[3]) || !(hp[2] > 0.0)) return false;
+            if (unit * std::sqrt(before * hp[2]) > 64.0) return false;
+            const bool last = (double)eps * hp[3] <= 1.0 / 16 && hp[7] == 0.0;
+            join_pass(S, Mc, Mr, ldm, st);
+            // ||M||_F of the product (the masses stay the pass's: only out[2] counts)
+            const int nt = (int)((d + kTrTile - 1) / kTrTile);
+            launch_k(k_gc_transpose<T>, dim3(nt, nt), 256, 0, st, Mr, ldm, (int)d, Mc, ldm, B.gdiag, B.part, B.bad);
+            launch_k(k_gc_finish<T>, 1, 1024, 0, st, B.part, nt * nt, B.gdiag, (int)d, B.bad, B.ndrop, status, B.out);
+            SKL_LAUNCHED();
+            SKL_LAUNCHED();
+            if (last) solve_c();
+            read_out(8);
+            mf2 = hp[2];
+            if (!std::isfinite(mf2) || !(1.0 / std::sqrt(mf2) > 2.0 * thresh)) return false;
+            if (last) break;
+            if (pass == 3) return false;
+        }
+        R = B.Racc;
+        ndrop = 0;
+    }
     if (!(1.0 / std::sqrt(mf2) > 2.0 * thresh)) return false;
     if (ndrop > 0) {
         drop_check(S, drop, ndrop, st);
@@ -1150,7 +1300,7 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
         if (!(std::sqrt(hp[0]) <= 0.25 * thresh)) return false;
     }
     SKL_CUDA(cudaMemsetAsync(B.out, 0, 2 * sizeof(double), st));
-    inf_norm_upper<T>(B.R, B.ldg, d, B.rows_part, B.out, st);
+    inf_norm_upper<T>(R, B.ldg, d, B.rows_part, B.out, st);
     inf_norm_upper<T>(Mc, ldm, d, B.rows_part, B.out + 1, st);
     read_out(2);
     const double nr = hp[0], nm = hp[1];
@@ -1170,11 +1320,11 @@ void gram_unit_dropped(const int* drop, int64_t k, float* Mc, float* Mr, int64_t
 }
 void gram_unit_dropped(const int*, int64_t, double*, double*, int64_t, cudaStream_t) {}
 
-template size_t gram_workspace_bytes<float>(int64_t, int64_t);
-template size_t gram_workspace_bytes<double>(int64_t, int64_t);
+template size_t gram_workspace_bytes<float>(int64_t, int64_t, bool);
+template size_t gram_workspace_bytes<double>(int64_t, int64_t, bool);
 template bool gram_precond<float>(const float*, int64_t, int64_t, int64_t, double*, int*, float*, float*, int64_t, double,
-                                  double, double, GramResult&, int*, void*, unsigned*, void*, cudaStream_t);
+                                  double, double, GramResult&, int*, bool, void*, unsigned*, void*, cudaStream_t);
 template bool gram_precond<double>(const double*, int64_t, int64_t, int64_t, double*, int*, double*, double*, int64_t,
-                                   double, double, double, GramResult&, int*, void*, unsigned*, void*, cudaStream_t);
+                                   double, double, double, GramResult&, int*, bool, void*, unsigned*, void*, cudaStream_t);
 
 }  // namespace skl

@@ -314,7 +314,7 @@ static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, do
     // ---- workspace layout (sized once, then carved) ----
     const size_t qr_ws = cpqr_workspace_bytes<T>(m, d);
     const size_t inv_ws = std::max(trinv_workspace_bytes<T>(d) + (size_t)d * d * sizeof(T),
-                                   gram_enabled() && m >= d ? gram_workspace_bytes<T>(m, d) : 0);
+                                   gram_enabled() && m >= d ? gram_workspace_bytes<T>(m, d, false) : 0);
     LsqrProblem Pq;
     Pq.n = n; Pq.d = d; Pq.nnz = nnz; Pq.r = d; Pq.precision = o.precision;
     const size_t lsqr_ws = lsqr_workspace_bytes(Pq);
@@ -474,7 +474,7 @@ static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, do
     // randomized CPQR, rank by its diagonal
     const bool gram = gram_enabled() && m >= d &&
                       gram_precond<T>(SA, m, d, ld, cvec, jpvt, Mc, Mr, ldm, 0.0, rel, o.rcond_threshold, gres,
-                                      carry_unresolved ? drop : nullptr, work, C.dev_status, C.host_pinned, st);
+                                      carry_unresolved ? drop : nullptr, false, work, C.dev_status, C.host_pinned, st);
     if (gram) {
         info.rank = d - gres.dropped;
         info.unresolved_cols = gres.dropped;
@@ -947,7 +947,8 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
     const int64_t mn = std::min(m, d);
     info.sketch_rows = m;
     const size_t qr_ws = cpqr_workspace_bytes<T>(m, d);
-    const size_t inv_ws = trinv_workspace_bytes<T>(d);
+    const size_t inv_ws = std::max(trinv_workspace_bytes<T>(d),
+                                   gram_enabled() ? gram_workspace_bytes<T>(m, d, true) : 0);
     LsqrProblem Pq;
     const bool tiled = lsqr_dense_tiled(d, o.precision);
     Pq.n = n; Pq.d = d; Pq.r = d; Pq.precision = o.precision;
@@ -1028,37 +1029,47 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
     if (cpqr_on) dht_hash_rhs(b, n, Dd, N, bptr, bent, (int)k, m, cvec, work, work_bytes, st);
     trace_phase(st, "dense sketch");
     SKL_CUDA(cudaEventRecord(ev[3], st));
-    // ---- QR (pivoted for the CPQR path) ----
+    // ---- factorization: Cholesky of a well-conditioned sketch's Gram matrix,
+    // else QR (pivoted for the CPQR path) ----
     SKL_CUDA(cudaMemsetAsync(C.dev_status, 0, sizeof(unsigned), st));
-    cpqr<T>(SA, m, d, ld, jpvt, tau, work, C.dev_status, st, cpqr_on ? cvec : nullptr,
-            cpqr_on ? 1 : 0, o.profile ? info.qr_prof_ms : nullptr);
-    {
-        const unsigned qs = read_status(C, st);
-        if (qs & kStatusTcTimeout) fail(SKL_ERR_TIMEOUT, "a kernel's bounded wait gave up (tensor-core product or sample QRP exchange)");
-        if (qs & kQrSelectBit) fail(SKL_ERR_NONFINITE, "non-finite values in the sketch factorization");
-    }
-    trace_phase(st, "dense qr");
-    SKL_CUDA(cudaEventRecord(ev[4], st));
-    // ---- rank: leading |R_ii| > rcond (absolute, :79-89); noCPQR keeps all ----
+    // the reference's absolute rank rule (:79-89), floored at the working precision's
+    // resolution of the sketch (FP32 cannot resolve |R_ii| below eps*|R_00|);
+    // noCPQR keeps all columns, by the QR where that resolution is reached
+    const double floor_rel = mixed ? 5.960464477539063e-08 : 0.0;
     int64_t rank = d;
-    if (cpqr_on) {
-        // the reference's absolute rule, floored at the working precision's
-        // resolution of the sketch (FP32 cannot resolve |R_ii| below eps*|R_00|)
-        const double floor_rel = mixed ? 5.960464477539063e-08 : 0.0;
-        rank = count_rank<T>(SA, ld, mn, o.rcond, floor_rel, dint, (int*)C.host_pinned, st);
-        if (rank == 0) fail(SKL_ERR_RANK_ZERO, "sketch has no diagonal entry above rcond");
+    int64_t ldm = round_up(d, 4);
+    GramResult gres;
+    const bool gram = gram_enabled() &&
+                      gram_precond<T>(SA, m, d, ld, cpqr_on ? cvec : nullptr, jpvt, Mc, Mr, ldm,
+                                      cpqr_on ? o.rcond : 0.0, floor_rel, 0.0, gres, nullptr, true, work,
+                                      C.dev_status, C.host_pinned, st);
+    if (gram) {
+        SKL_CUDA(cudaEventRecord(ev[4], st));
+    } else {
+        cpqr<T>(SA, m, d, ld, jpvt, tau, work, C.dev_status, st, cpqr_on ? cvec : nullptr,
+                cpqr_on ? 1 : 0, o.profile ? info.qr_prof_ms : nullptr);
+        {
+            const unsigned qs = read_status(C, st);
+            if (qs & kStatusTcTimeout) fail(SKL_ERR_TIMEOUT, "a kernel's bounded wait gave up (tensor-core product or sample QRP exchange)");
+            if (qs & kQrSelectBit) fail(SKL_ERR_NONFINITE, "non-finite values in the sketch factorization");
+        }
+        trace_phase(st, "dense qr");
+        SKL_CUDA(cudaEventRecord(ev[4], st));
+        if (cpqr_on) {
+            rank = count_rank<T>(SA, ld, mn, o.rcond, floor_rel, dint, (int*)C.host_pinned, st);
+            if (rank == 0) fail(SKL_ERR_RANK_ZERO, "sketch has no diagonal entry above rcond");
+        }
+        ldm = round_up(rank, 4);
+        trinv_upper<T>(SA, ld, rank, 0.0, Mc, ldm, norms, work, st);
+        transpose_upper<T>(Mc, ldm, rank, Mr, st);
+        SKL_CUDA(cudaMemcpyAsync(C.host_pinned, norms, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
+        SKL_CUDA(cudaStreamSynchronize(st));
+        gres.norm_r = ((double*)C.host_pinned)[0];
+        gres.norm_m = ((double*)C.host_pinned)[1];
     }
     info.rank = rank;
     info.success = 1;
-    const int64_t ldm = round_up(rank, 4);
-    trinv_upper<T>(SA, ld, rank, 0.0, Mc, ldm, norms, work, st);
-    transpose_upper<T>(Mc, ldm, rank, Mr, st);
-    SKL_CUDA(cudaMemcpyAsync(C.host_pinned, norms, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
-    SKL_CUDA(cudaStreamSynchronize(st));
-    {
-        double nr = ((double*)C.host_pinned)[0], nm = ((double*)C.host_pinned)[1];
-        info.rcond_r11 = (nr > 0 && nm > 0) ? 1.0 / (nr * nm) : 0.0;
-    }
+    info.rcond_r11 = (gres.norm_r > 0 && gres.norm_m > 0) ? 1.0 / (gres.norm_r * gres.norm_m) : 0.0;
     LsqrProblem P;
     P.n = n; P.d = d; P.nnz = n * d;
     if (tiled) P.At = A2;

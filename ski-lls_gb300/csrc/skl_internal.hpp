@@ -230,6 +230,7 @@ void inf_norm_upper(const T* X, int64_t ld, int64_t r, double* part, double* out
 // depend on the others at FP32 resolution (distance at most a quarter of the
 // rule's threshold): res.dropped of them are listed, their rows and columns of
 // M and entries of c are zero.
+// multi (FP32): up to two more passes on SA M for ill-conditioned sketches.
 // Otherwise false: SA and c are untouched, Mc and Mr undefined.
 constexpr int kGramDropMax = 512;
 struct GramResult {
@@ -237,10 +238,10 @@ struct GramResult {
     int64_t dropped = 0;
 };
 template <typename T>
-size_t gram_workspace_bytes(int64_t m, int64_t d);
+size_t gram_workspace_bytes(int64_t m, int64_t d, bool multi);
 template <typename T>
 bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int* jpvt, T* Mc, T* Mr, int64_t ldm,
-                  double abs_thresh, double rel_thresh, double rcond_min, GramResult& res, int* drop, void* work,
+                  double abs_thresh, double rel_thresh, double rcond_min, GramResult& res, int* drop, bool multi, void* work,
                   unsigned* status, void* host_pinned, cudaStream_t st);
 // M(j, j) = 1 for the k dropped columns (LSQR carries them unpreconditioned).
 void gram_unit_dropped(const int* drop, int64_t k, float* Mc, float* Mr, int64_t ldm, cudaStream_t st);
