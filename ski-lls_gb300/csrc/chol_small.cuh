@@ -14,12 +14,9 @@ namespace skl {
 constexpr int kSmallThreads = 1024;
 
 // ---- small dense algebra on b x b (b <= 64) row-major shared-memory blocks --
-// The factorizations are blocked by 16: the 16 x 16 diagonal blocks are
-// factored and inverted by one warp (a step is a __syncwarp, not a block
-// barrier), and everything else is a block product over the whole CTA
-// (blk_mul).  A 64 x 64 Cholesky plus inverse is then 4 warp factorizations
-// and ~14 block barriers instead of 128 one-barrier elimination steps, each of
-// which had to wait for all 32 warps of the CTA.  Matrices are padded to
+// The modified LU is blocked by 16: the 16 x 16 diagonal blocks are factored and
+// inverted by one warp (a step is a __syncwarp, not a block barrier), and
+// everything else is a block product over the whole CTA (blk_mul).  Matrices are padded to
 // np = round_up(b, 16) rows/columns (identity for the Cholesky, zeros for the
 // LU input, which the modified LU turns into identity factors).
 constexpr int kDB = 16;   // diagonal block
@@ -30,24 +27,6 @@ constexpr int kDB = 16;   // diagonal block
 // loops stay rolled (register elements picked by selects): a one-warp
 // straight-line version would wait on instruction fetch.
 template <typename T>
-SKL_DEV T sel8(const T (&a)[8], int i)
-{
-    T v = a[0];
-#pragma unroll
-    for (int e = 1; e < 8; ++e) v = (i == e) ? a[e] : v;
-    return v;
-}
-
-// Element k of the lane's own row (k in either half of the row).
-template <typename T>
-SKL_DEV T own_col(const T (&a)[8], int k, int lane)
-{
-    const T mine = sel8(a, k & 7);
-    const T other = __shfl_xor_sync(0xffffffffu, mine, 1);
-    return ((k >> 3) == (lane & 1)) ? mine : other;
-}
-
-template <typename T>
 SKL_DEV void row_load(const T* A, int ld, T (&a)[8])
 {
     const int lane = threadIdx.x & 31, r = lane >> 1, cb = (lane & 1) * 8;
@@ -55,10 +34,6 @@ SKL_DEV void row_load(const T* A, int ld, T (&a)[8])
     for (int e = 0; e < 8; ++e) a[e] = A[r * ld + cb + e];
 }
 
-// In-place Cholesky of the symmetric 16 x 16 block A (both triangles hold the
-// current values): R (upper, normalised, zeros below) over A.  Rows stay
-// unnormalised during the elimination and are scaled by 1/sqrt(d) at the end.
-// Sets *bad when a pivot is not above 32 eps times its mass.
 template <typename T>
 SKL_DEV T t_rcp(T x);
 template <> SKL_DEV float t_rcp<float>(float x) { return __frcp_rn(x); }
@@ -76,57 +51,6 @@ template <> SKL_DEV float t_rcp_chain<float>(float x)
     return y;
 }
 template <> SKL_DEV double t_rcp_chain<double>(double x) { return __drcp_rn(x); }
-
-// Step k = 8 kh + kl: kl is a compile-time index (the inner loop is unrolled
-// by 8) so the pivot and the lane's own column k come from fixed registers.
-// BOOST: such a pivot is replaced by that bound (by 1 if its mass is not positive,
-// which sets *bad to 2) and the elimination goes on.
-template <typename T, bool BOOST = false>
-SKL_DEV void warp16_chol(T* A, int ld, const T* __restrict__ mass, T eps, int* bad)
-{
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31, r = lane >> 1, cb = (lane & 1) * 8;
-    T a[8];
-    row_load(A, ld, a);
-    bool isbad = false;
-#pragma unroll 1
-    for (int kh = 0; kh < 2; ++kh) {
-#pragma unroll
-        for (int kl = 0; kl < 8; ++kl) {
-            const int k = kh * 8 + kl;
-            const T d = __shfl_sync(full, a[kl], 2 * k + kh);
-            const T ms = mass[k];
-            const bool ok = d > T(32) * eps * ms && ms > T(0);
-            isbad = isbad || !ok;
-            const T bound = BOOST ? (ms > T(0) ? T(32) * eps * ms : T(1)) : T(0);
-            const T inv = ok ? t_rcp_chain(d) : BOOST ? t_rcp_chain(bound) : T(0);
-            if (BOOST && !(ms > T(0)) && lane == 0) atomicMax(bad, 2);
-            T rk[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) rk[e] = __shfl_sync(full, a[e], 2 * k + (lane & 1));
-            const T other = __shfl_xor_sync(full, a[kl], 1);
-            const T g = (kh == (lane & 1) ? a[kl] : other) * inv;   // A[r][k] = A[k][r]
-            if (r > k) {
-#pragma unroll
-                for (int e = 0; e < 8; ++e)
-                    if (cb + e > k) a[e] -= g * rk[e];
-            }
-        }
-    }
-    if (isbad && lane == 0) atomicMax(bad, 1);
-    // a failed pivot's row is zero, its diagonal entry too; boosted, the pivot is
-    // the bound
-    T d = own_col(a, r, lane);
-    const bool good = d > T(32) * eps * mass[r] && mass[r] > T(0);
-    if (BOOST && !good) d = mass[r] > T(0) ? T(32) * eps * mass[r] : T(1);
-    const T sc = good || BOOST ? t_rcp(t_sqrt(d)) : T(0);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        const T v = (BOOST && cb + e == r) ? d : a[e];
-        A[r * ld + cb + e] = (cb + e >= r) ? v * sc : T(0);
-    }
-    __syncwarp();
-}
 
 // X = U^{-1} for the upper 16 x 16 block U (entries below its diagonal never
 // read): X's upper triangle, and zeros below it when zero_lower.  A zero
@@ -241,7 +165,8 @@ SKL_DEV void warp16_mlu(T* A, int ld, T* sg)
 }
 
 // Operand views for blk_mul, in the coordinates (r, s) of op(X):
-enum : int { kMFull = 0, kMUpper = 1, kMUpperUnit = 2, kMLowerUnit = 3 };
+// kMLower: zeros are stored above the diagonal.
+enum : int { kMFull = 0, kMUpper = 1, kMUpperUnit = 2, kMLowerUnit = 3, kMLower = 4 };
 
 template <typename T, bool TR, int MASK>
 SKL_DEV T op_at(const T* X, int ld, int r, int s)
@@ -260,7 +185,7 @@ SKL_DEV void k_range(int i0, int c0, int tr, int tc, int kk, int& klo, int& khi)
     klo = 0;
     khi = kk;
     if (MA == kMUpper) klo = i0;
-    if (MA == kMLowerUnit) khi = min(khi, i0 + tr);
+    if (MA == kMLowerUnit || MA == kMLower) khi = min(khi, i0 + tr);
     if (MB == kMUpper || MB == kMUpperUnit) khi = min(khi, c0 + tc);
     if (MB == kMLowerUnit) klo = max(klo, c0);
 }
@@ -579,42 +504,130 @@ SKL_DEV void inv_unit_lower_offdiag(const T* L, int ldl, T* Y, int ldy, int np, 
     }
 }
 
-// Cholesky G = R^T R (np x np, np a multiple of 16) with X = R^{-1}: R (upper,
-// zeros below) over G, X (upper, zeros below) to Xs.  Blocked right-looking:
-// per 16-block, warp 0 factors the diagonal block and inverts it, then
-// R12 = R11^{-T} G12 and G22 -= R12^T R12 as block products.
+// Cholesky G = R^T R (np x np, np a multiple of 16, both triangles given) with
+// X = R^{-1}: R (upper, zeros below) over G, X (upper, zeros below) to Xs.
+// Gaussian elimination of [G | I] on 16 warps, in place: row i of the work
+// matrix holds G's Schur complement at the columns not yet eliminated and row i
+// of R^{-T} at the others (unnormalised until the end).  Warp w keeps rows 4 w ..
+// 4 w + 3 in registers, two columns per lane.  In round r warp r eliminates its
+// four rows among themselves with shuffles and publishes them with their
+// multiples by the pivots' reciprocals; one barrier later the warps below
+// subtract the four products, whose row factors are the same published rows (the
+// complement is symmetric).  Bound by the chain through warp r in FP32, by the
+// FP64 pipe and that chain in FP64.  64 x 64: 20,600 cycles (FP64 157,000); with
+// blocks of 16 factored and inverted by one warp and block products over 32
+// warps between them ~37,000 (260,000); with a rolled loop of one pivot per
+// barrier 31,000 (144,000).
+// A pivot that is not above 32 eps times its mass sets *bad to 1 and leaves zeros
+// in its row of R and its row and column of X.  BOOST: it is replaced by that
+// bound (by 1 if the mass is not positive, which sets *bad to 2).
 template <typename T, bool BOOST = false>
-SKL_DEV void chol_inv_small(T* G, int ldx, int np, const T* __restrict__ mass, T eps, T* Xs, T* tmp,
-                            int ldt, int* bad)
+SKL_DEV void chol_inv_small(T* G, int ldx, int np, const T* __restrict__ mass, T eps, T* Xs, int* bad)
 {
-    for (int e = threadIdx.x; e < np * np; e += kSmallThreads) Xs[(e / np) * ldx + e % np] = T(0);
+    constexpr int kRows = 4, kWarps = 64 / kRows;
+    struct alignas(16) Quad { T v[kRows]; };
+    // by column: the four rows of a round, and those times their pivots' reciprocals
+    __shared__ Quad s_row[2][64], s_mul[2][64];
+    const unsigned full = 0xffffffffu;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i0 = kRows * warp;
     __syncthreads();
-    for (int k0 = 0; k0 < np; k0 += kDB) {
-        const int rest = np - k0 - kDB;
-        T* G11 = G + k0 * ldx + k0;
-        if (threadIdx.x < 32) {
-            warp16_chol<T, BOOST>(G11, ldx, mass + k0, eps, bad);
-            warp16_inv_upper<T>(G11, ldx, Xs + k0 * ldx + k0, ldx, true);
-        }
-        __syncthreads();
-        if (rest > 0) {
-            T* G12 = G11 + kDB;
-            blk_mul<T, true, kMFull, false, kMFull>(kDB, rest, kDB, Xs + k0 * ldx + k0, ldx, G12, ldx,
-                                                    nullptr, T(1), G12, ldx);
-            blk_mul<T, true, kMFull, false, kMFull, true>(rest, rest, kDB, G12, ldx, G12, ldx, nullptr,
-                                                          T(-1), G11 + kDB * ldx + kDB, ldx);
+    if (warp < kWarps) {
+        T a[kRows][2];
+#pragma unroll
+        for (int j = 0; j < kRows; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int c = lane + 32 * h;
+                a[j][h] = i0 < np && c < np ? G[(i0 + j) * ldx + c] : T(0);
+            }
+#pragma unroll 1
+        for (int r = 0; kRows * r < np; ++r) {
+            const int k0 = kRows * r;
+            const bool up = k0 >= 32;             // the half that holds the round's columns
+            const int rl = lane - (k0 & 31);      // 0..3: the lane's column of that half is k0 + rl
+            T dd[kRows];
+            int flag = 0;
+            if (warp == r) {
+                T l[kRows][2];
+#pragma unroll
+                for (int j = 0; j < kRows; ++j) {
+                    const int src = (k0 & 31) + j;
+                    const T cur = up ? a[j][1] : a[j][0];
+                    const T d = __shfl_sync(full, cur, src);
+                    const T ms = mass[k0 + j], bound = T(32) * eps * ms;
+                    const bool pos = ms > T(0), ok = pos && d > bound;
+                    dd[j] = ok ? d : BOOST ? (pos ? bound : T(1)) : T(0);
+                    const T inv = ok || BOOST ? t_rcp_chain(dd[j]) : T(0);
+                    flag = max(flag, ok ? 0 : BOOST && !pos ? 2 : 1);
+                    // from here on the pivot's column belongs to R^{-T}: 1 in its row
+                    if (rl == j) {
+#pragma unroll
+                        for (int q = j; q < kRows; ++q) {
+                            const T v = q == j ? T(1) : T(0);
+                            if (up) a[q][1] = v;
+                            else a[q][0] = v;
+                        }
+                    }
+                    l[j][0] = a[j][0] * inv;
+                    l[j][1] = a[j][1] * inv;
+#pragma unroll
+                    for (int q = j + 1; q < kRows; ++q) {
+                        const T f = __shfl_sync(full, cur, src + q - j);
+                        a[q][0] -= f * l[j][0];
+                        a[q][1] -= f * l[j][1];
+                    }
+                }
+                // the round's columns right of a pivot: eliminated in the rows below
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    Quad vr, vl;
+#pragma unroll
+                    for (int j = 0; j < kRows; ++j) {
+                        vr.v[j] = a[j][h];
+                        vl.v[j] = (h == 1) == up && rl > j && rl < kRows ? T(0) : l[j][h];
+                    }
+                    s_row[r & 1][lane + 32 * h] = vr;
+                    s_mul[r & 1][lane + 32 * h] = vl;
+                }
+            }
+            asm volatile("bar.sync 1, 512;" ::: "memory");
+            if (warp == r) {
+                if (flag && lane == 0) atomicMax(bad, flag);
+                T sc[kRows];
+#pragma unroll
+                for (int j = 0; j < kRows; ++j) sc[j] = dd[j] > T(0) ? t_rcp(t_sqrt(dd[j])) : T(0);
+#pragma unroll
+                for (int j = 0; j < kRows; ++j)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int k = k0 + j, c = lane + 32 * h;
+                        if (c >= np) continue;
+                        const T v = a[j][h] * sc[j];
+                        G[k * ldx + c] = c < k ? T(0) : c == k ? dd[j] * sc[j] : v;
+                        Xs[c * ldx + k] = c > k ? T(0) : v;
+                    }
+            } else if (warp > r && i0 < np) {
+                if (rl >= 0 && rl < kRows) {
+#pragma unroll
+                    for (int q = 0; q < kRows; ++q) {
+                        if (up) a[q][1] = T(0);
+                        else a[q][0] = T(0);
+                    }
+                }
+                const Quad m0 = s_mul[r & 1][lane], m1 = s_mul[r & 1][lane + 32];
+#pragma unroll
+                for (int q = 0; q < kRows; ++q) {
+                    const Quad f = s_row[r & 1][i0 + q];
+#pragma unroll
+                    for (int j = 0; j < kRows; ++j) {
+                        a[q][0] -= f.v[j] * m0.v[j];
+                        a[q][1] -= f.v[j] * m1.v[j];
+                    }
+                }
+            }
         }
     }
-    // R's strict lower part (the off-diagonal blocks kept G's values)
-    for (int e = threadIdx.x; e < np * np; e += kSmallThreads) {
-        const int i = e / np, c = e % np;
-        if (c < i) G[i * ldx + c] = T(0);
-    }
     __syncthreads();
-    if constexpr (std::is_same<T, float>::value)
-        inv_offdiag_tc(G, ldx, Xs, ldx, nullptr, 0, nullptr, 0, np, tmp, ldt);
-    else
-        inv_upper_offdiag<T>(G, ldx, Xs, ldx, np, tmp, ldt);
 }
 
 // Modified LU of A (np x np) in place (L strict lower, U upper), signs to

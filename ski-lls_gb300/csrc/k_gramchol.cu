@@ -25,7 +25,7 @@
 // On the dense mixed path a failed pivot is raised to the bound instead and the
 // same is done again on Q = S A M (at most twice): each pass takes the condition
 // number to about the root of what exceeds ~300.  40,000 x 4,000 (S A 6,800 x 4,000):
-// QR and inverse 20.2 + 1.4 ms, one pass 4.4 ms, two (condition number 1e3 to
+// QR and inverse 20.2 + 1.4 ms, one pass 4.1 ms, two (condition number 1e3 to
 // 1e5) 9.9 ms with LSQR's iterations, x and residual unchanged.  From ~1e6 on
 // most attempts end early and the QR comes on top of one pass's time.
 // A sketch that fails a test keeps the QR: S A is not touched here.
@@ -332,6 +332,43 @@ SKL_DEV void tile_load(const T* __restrict__ X, int64_t ld, int r0, int c0, int 
     }
 }
 
+// V -= U^T U (64 x 64).  FP64: 2 x 2 tiles of the upper triangle on 17 full warps,
+// mirrored: the FP64 pipe bounds it (134,000 cycles with all tiles).
+template <typename T>
+SKL_DEV void sub_gram(const T* U, T* V)
+{
+    if constexpr (std::is_same<T, float>::value) {
+        blk_mul<T, true, kMFull, false, kMFull, true>(kIB, kIB, kIB, U, kSL, U, kSL, nullptr, T(-1), V, kSL);
+    } else {
+        // tile t of the triangle: row i of tiles holds columns i .. 31
+        int t = threadIdx.x, i = 0;
+        if (t < 32 * 33 / 2) {
+            while (t >= 32 - i) t -= 32 - i++;
+            const int r0 = 2 * i, c0 = 2 * (i + t);
+            T a00 = 0, a01 = 0, a10 = 0, a11 = 0;
+#pragma unroll 4
+            for (int k = 0; k < kIB; ++k) {
+                const T x0 = U[k * kSL + r0], x1 = U[k * kSL + r0 + 1];
+                const T y0 = U[k * kSL + c0], y1 = U[k * kSL + c0 + 1];
+                a00 += x0 * y0;
+                a01 += x0 * y1;
+                a10 += x1 * y0;
+                a11 += x1 * y1;
+            }
+            auto sub = [&](int r, int c, T v) {
+                const T w = V[r * kSL + c] - v;
+                V[r * kSL + c] = w;
+                V[c * kSL + r] = w;
+            };
+            sub(r0, c0, a00);
+            sub(r0, c0 + 1, a01);
+            if (c0 > r0) sub(r0 + 1, c0, a10);
+            sub(r0 + 1, c0 + 1, a11);
+        }
+        __syncthreads();
+    }
+}
+
 // R_ss and X = R_ss^{-1} of the b x b (b <= 64) diagonal block S0 (symmetric,
 // identity beyond b) at row q: R to R, X^T to E, X to mkk at offset ql.  A
 // failed pivot drops the column: its row of
@@ -339,7 +376,7 @@ SKL_DEV void tile_load(const T* __restrict__ X, int64_t ld, int r0, int c0, int 
 // column were not there, and its index joins the list; more than drop_cap of
 // them set *bad.
 template <typename T>
-SKL_DEV void diag_block(const GcArgs<T>& g, int q, int b, int ql, T* S0, T* S1, T* tmp, T* mass)
+SKL_DEV void diag_block(const GcArgs<T>& g, int q, int b, int ql, T* S0, T* S1, T* mass)
 {
     __shared__ int s_any;
     const int np = small_np(b);
@@ -347,8 +384,8 @@ SKL_DEV void diag_block(const GcArgs<T>& g, int q, int b, int ql, T* S0, T* S1, 
     for (int k = threadIdx.x; k < np; k += kSmallThreads) mass[k] = k < b ? g.mass[q + k] : T(1);
     __syncthreads();
     // chol_inv_small asks for a pivot above 32 x its eps x mass
-    if (g.boost) chol_inv_small<T, true>(S0, kSL, np, mass, g.pivot / T(32), S1, tmp, 36, &s_any);
-    else chol_inv_small<T>(S0, kSL, np, mass, g.pivot / T(32), S1, tmp, 36, &s_any);
+    if (g.boost) chol_inv_small<T, true>(S0, kSL, np, mass, g.pivot / T(32), S1, &s_any);
+    else chol_inv_small<T>(S0, kSL, np, mass, g.pivot / T(32), S1, &s_any);
     for (int e = threadIdx.x; e < b * b; e += kSmallThreads) {
         const int i = e % b, c = e / b;
         g.R[(q + i) + (int64_t)(q + c) * g.ldg] = S0[i * kSL + c];
@@ -392,7 +429,6 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_gc_diag(const GcArgs<T> g,
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* S0 = (T*)smem_raw;
     T* S1 = S0 + kIB * kSL;
-    T* tmp = S1 + kIB * kSL;
     // both triangles from G's upper one, identity beyond b
     for (int e = threadIdx.x; e < kIB * kIB; e += kSmallThreads) {
         const int i = e % kIB, c = e / kIB;
@@ -401,7 +437,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_gc_diag(const GcArgs<T> g,
         S0[i * kSL + c] = v;
         S0[c * kSL + i] = v;
     }
-    diag_block<T>(g, q, b, 0, S0, S1, tmp, tmp + 64 * 36);
+    diag_block<T>(g, q, b, 0, S0, S1, S1 + kIB * kSL);
 }
 
 // ---- one inner step of a 256-block ---------------------------------------------
@@ -452,7 +488,6 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_gc_step(const GcArgs<T> g,
     T* P = X + kIB * kSL;
     T* U = P + kIB * kSL;
     T* V = U + kIB * kSL;
-    T* tmp = V + kIB * kSL;
     const int q = j0 + s * kIB;
     auto width = [&](int blk) { return min(kIB, g.d - (j0 + blk * kIB)); };
     const int bs = width(s), bI = width(I), bJ = width(J);
@@ -469,9 +504,9 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_gc_step(const GcArgs<T> g,
             V[c * kSL + i] = v;
         }
         __syncthreads();
-        blk_mul<T, true, kMFull, false, kMFull>(kIB, kIB, kIB, X, kSL, P, kSL, nullptr, T(1), U, kSL);
-        blk_mul<T, true, kMFull, false, kMFull, true>(kIB, kIB, kIB, U, kSL, U, kSL, nullptr, T(-1), V, kSL);
-        diag_block<T>(g, cI, bI, I * kIB, V, P, tmp, tmp + 64 * 36);
+        blk_mul<T, true, kMLower, false, kMFull>(kIB, kIB, kIB, X, kSL, P, kSL, nullptr, T(1), U, kSL);
+        sub_gram<T>(U, V);
+        diag_block<T>(g, cI, bI, I * kIB, V, P, V + kIB * kSL);
         return;
     }
     // V = row s of the target's columns
@@ -482,7 +517,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_gc_step(const GcArgs<T> g,
     } else {
         tile_load<T>(is_e ? g.Ew : g.G, is_e ? g.lde : g.ldg, q, cJ, bs, bJ, P);
         __syncthreads();
-        blk_mul<T, true, kMFull, false, kMFull>(kIB, kIB, kIB, X, kSL, P, kSL, nullptr, T(1), V, kSL);
+        blk_mul<T, true, kMLower, false, kMFull>(kIB, kIB, kIB, X, kSL, P, kSL, nullptr, T(1), V, kSL);
     }
     if (I == s) {
         for (int e = threadIdx.x; e < kIB * kIB; e += kSmallThreads) {
@@ -505,7 +540,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_gc_step(const GcArgs<T> g,
         __syncthreads();
         tile_load<T>(g.G, g.ldg, q, cI, bs, bI, P);
         __syncthreads();
-        blk_mul<T, true, kMFull, false, kMFull>(kIB, kIB, kIB, X, kSL, P, kSL, nullptr, T(1), U, kSL);
+        blk_mul<T, true, kMLower, false, kMFull>(kIB, kIB, kIB, X, kSL, P, kSL, nullptr, T(1), U, kSL);
         u = U;
     }
     blk_mul<T, true, kMFull, false, kMFull>(kIB, kIB, kIB, u, kSL, V, kSL, nullptr, T(1), P, kSL);
@@ -1126,8 +1161,8 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
     const T pivot = (drop_cap > 0 || boost ? T(2048) : T(128)) * eps;
     Sweep<T> S{SA, m, d, ld, gram_carve<T>(work, m, d, boost), Mc, Mr, ldm, status};
     GramBuffers<T>& B = S.B;
-    const size_t dsm = (2 * (size_t)kIB * kSL + 64 * 36 + kIB) * sizeof(T);
-    const size_t ssm = (4 * (size_t)kIB * kSL + 64 * 36 + kIB) * sizeof(T);
+    const size_t dsm = (2 * (size_t)kIB * kSL + kIB) * sizeof(T);
+    const size_t ssm = (4 * (size_t)kIB * kSL + kIB) * sizeof(T);
     GcArgs<T> ga{B.G, B.R, B.ldg, Mc, Mr, ldm, B.mkk, B.mass, B.bad, B.ndrop, drop, drop_cap, (int)d, pivot, boost ? 1 : 0};
     allow_max_dynamic_smem((const void*)k_gc_diag<T>);
     allow_max_dynamic_smem((const void*)k_gc_step<T>);

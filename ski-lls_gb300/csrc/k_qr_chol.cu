@@ -28,8 +28,7 @@ k_chol_small1(const T* __restrict__ G, int b, T* __restrict__ R1, T* __restrict_
     const int LDX = np + 4;
     T* S0 = (T*)smem_raw;
     T* S1 = S0 + (size_t)np * LDX;
-    T* tmp = S1 + (size_t)np * LDX;
-    T* mass = tmp + 64 * 36;
+    T* mass = S1 + (size_t)np * LDX;
     __shared__ int s_bad;
     const T eps = std::is_same<T, float>::value ? T(5.9604645e-08) : T(1.1102230246251565e-16);
     if (threadIdx.x == 0) s_bad = 0;
@@ -40,7 +39,7 @@ k_chol_small1(const T* __restrict__ G, int b, T* __restrict__ R1, T* __restrict_
     }
     for (int k = threadIdx.x; k < np; k += kSmallThreads) mass[k] = k < b ? G[k * b + k] : T(1);
     __syncthreads();
-    chol_inv_small<T>(S0, LDX, np, mass, eps, S1, tmp, 36, &s_bad);
+    chol_inv_small<T>(S0, LDX, np, mass, eps, S1, &s_bad);
     for (int e = threadIdx.x; e < b * b; e += kSmallThreads) {
         const int i = e / b, c = e % b;
         R1[e] = S0[i * LDX + c];     // row-major b x b
@@ -99,7 +98,7 @@ k_chol_small2(const T* __restrict__ G, int b, const T* __restrict__ R1g, const T
         if (threadIdx.x == 0) *fail = 1;
         return;
     }
-    chol_inv_small<T>(S1, LDX, np, mass, eps, S2, tmp, 36, &s_bad);  // R2 over S1, X2 -> S2
+    chol_inv_small<T>(S1, LDX, np, mass, eps, S2, &s_bad);  // R2 over S1, X2 -> S2
     if (s_bad) {
         if (threadIdx.x == 0) *fail = 1;
         return;
