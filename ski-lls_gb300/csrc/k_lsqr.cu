@@ -1405,10 +1405,10 @@ __global__ void k_axpy_sign(int n, double sgn, const double* __restrict__ dc, do
         c[i] = fma(sgn, dc[i], c[i]);
 }
 
-__global__ void __launch_bounds__(kLThreads)
-k_residual_csr(const int* __restrict__ rp, const int* __restrict__ ci, const double* __restrict__ cx,
-               int n, const double* __restrict__ x, const double* __restrict__ b,
-               double* __restrict__ r, double* __restrict__ part);
+// r = b - A x over the CSR rows, kResGrid partial sums of r^2
+constexpr int kResGrid = 912;
+static void residual_csr(const LsqrProblem& P, const double* x, const double* b, double* r, double* part,
+                         cudaStream_t st);
 __global__ void k_sum_parts(const double* __restrict__ part, int np, double* __restrict__ out);
 
 static void vec_norm(const double* x, int64_t n, double* part, double* out, cudaStream_t st)
@@ -1449,92 +1449,181 @@ void sketch_refine_apply(const LsqrProblem& P, double sgn, const double* dc, dou
     SKL_LAUNCHED();
     SKL_CUDA(cudaMemsetAsync(x, 0, P.d * sizeof(double), st));
     precond_apply(P, c, x, nullptr, st);
-    const int np = 512;
-    launch_k(k_residual_csr, np, kLThreads, 0, st, P.rp, P.ci, P.cx64, (int)P.n, x, b, rs, part);
-    launch_k(k_sum_parts, 1, kLThreads, 0, st, part, np, rnorm);
+    residual_csr(P, x, b, rs, part, st);
+    launch_k(k_sum_parts, 1, kLThreads, 0, st, part, kResGrid, rnorm);
     SKL_LAUNCHED();
     SKL_LAUNCHED();
 }
 
 // ------------------------------------------------- FP64 residual checks --
 // r = b - A x with plain FP64 (CSR rows or dense columns); partial ||r||^2.
+// Grids of 152 x 6 CTAs of 256 threads, partial sums by CTA.
+constexpr int kResWarps = kLThreads / 32;
+
+// L (4..32) lanes per row, of the order of the mean row length: short rows are
+// bound by the chain row pointer, index, x, so they need rows in flight rather
+// than lanes (1,000,000 rows of 10: 121 us; 589 with a warp per row).  A row
+// beyond 32 L entries is left to its whole warp.
 __global__ void __launch_bounds__(kLThreads)
 k_residual_csr(const int* __restrict__ rp, const int* __restrict__ ci, const double* __restrict__ cx,
-               int n, const double* __restrict__ x, const double* __restrict__ b,
+               int n, int L, const double* __restrict__ x, const double* __restrict__ b,
                double* __restrict__ r, double* __restrict__ part)
 {
     pdl_wait();
-    __shared__ double red[kLThreads / 32];
-    const int lane = threadIdx.x & 31;
+    __shared__ double red[kResWarps];
+    const int lane = threadIdx.x & 31, gl = lane & (L - 1);
+    const int per_warp = 32 / L;
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
     double ss = 0.0;
-    for (int i = gw; i < n; i += nw) {
+    auto finish = [&](int i, double acc) {
+        const double v = b[i] - acc;
+        r[i] = v;
+        ss += v * v;
+    };
+    for (int base = gw * per_warp; base < n; base += nw * per_warp) {
+        const int i = base + lane / L;
+        const int p0 = i < n ? rp[i] : 0, p1 = i < n ? rp[i + 1] : 0;
+        const bool by_warp = p1 - p0 > 32 * L;
         double acc = 0.0;
-        for (int p = rp[i] + lane; p < rp[i + 1]; p += 32) acc = fma(cx[p], x[ci[p]], acc);
-        acc = warp_sum(acc);
-        if (lane == 0) {
-            double v = b[i] - acc;
-            r[i] = v;
-            ss += v * v;
+        if (!by_warp)
+            for (int p = p0 + gl; p < p1; p += L) acc = fma(cx[p], x[ci[p]], acc);
+        for (int o = L / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (i < n && !by_warp && gl == 0) finish(i, acc);
+        unsigned todo = __ballot_sync(0xffffffffu, by_warp && gl == 0);
+        while (todo) {
+            const int src = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const int q0 = __shfl_sync(0xffffffffu, p0, src), q1 = __shfl_sync(0xffffffffu, p1, src);
+            acc = 0.0;
+            for (int p = q0 + lane; p < q1; p += 32) acc = fma(cx[p], x[ci[p]], acc);
+            acc = warp_sum(acc);
+            if (lane == src) finish(i, acc);
         }
     }
     ss = block_sum(ss, red);
     if (threadIdx.x == 0) part[blockIdx.x] = ss;
 }
 
+// 32 rows per CTA, its warps sharing the columns: bound by the FP64 pipe and HBM
+// together (40,000 x 4,000: 324 us; 1,789 with a thread per row, which had 40,000
+// threads with one or two loads each in flight).
 __global__ void __launch_bounds__(kLThreads)
 k_residual_dense(const double* __restrict__ A, int64_t lda, int n, int d,
                  const double* __restrict__ x, const double* __restrict__ b,
                  double* __restrict__ r, double* __restrict__ part)
 {
     pdl_wait();
-    __shared__ double red[kLThreads / 32];
+    __shared__ double s_acc[kResWarps][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double ss = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        double acc = 0.0;
-        for (int j = 0; j < d; ++j) acc = fma(A[i + (int64_t)j * lda], x[j], acc);
-        double v = b[i] - acc;
-        r[i] = v;
-        ss += v * v;
+    for (int i0 = blockIdx.x * 32; i0 < n; i0 += gridDim.x * 32) {
+        const int i = i0 + lane;
+        const double* col = A + min(i, n - 1);
+        double acc[2] = {0.0, 0.0};
+        int j = warp;
+        for (; j + 7 * kResWarps < d; j += 8 * kResWarps) {
+            double v[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q] = col[(int64_t)(j + q * kResWarps) * lda];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) acc[q & 1] = fma(v[q], x[j + q * kResWarps], acc[q & 1]);
+        }
+        for (; j < d; j += kResWarps) acc[0] = fma(col[(int64_t)j * lda], x[j], acc[0]);
+        s_acc[warp][lane] = acc[0] + acc[1];
+        __syncthreads();
+        if (warp == 0 && i < n) {
+            double s = s_acc[0][lane];
+#pragma unroll
+            for (int w = 1; w < kResWarps; ++w) s += s_acc[w][lane];
+            const double v = b[i] - s;
+            r[i] = v;
+            ss += v * v;
+        }
+        __syncthreads();
     }
-    ss = block_sum(ss, red);
-    if (threadIdx.x == 0) part[blockIdx.x] = ss;
+    if (warp == 0) {
+        ss = warp_sum(ss);
+        if (lane == 0) part[blockIdx.x] = ss;
+    }
 }
 
-// g = A^T r over all d columns, partial ||g||^2
+// g = A^T r over all d columns, partial ||g||^2.  A warp per column, columns beyond
+// 1,024 entries by the CTA: with one warp the longest decides (power-law columns up
+// to 20,000 entries: 110 us; 404 before).
 __global__ void __launch_bounds__(kLThreads)
 k_atr_csc(const int* __restrict__ cp, const int* __restrict__ ri, const double* __restrict__ rx,
           int d, const double* __restrict__ r, double* __restrict__ part)
 {
     pdl_wait();
-    __shared__ double red[kLThreads / 32];
-    const int lane = threadIdx.x & 31;
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
+    constexpr int kLong = 1024;
+    __shared__ double red[kResWarps];
+    __shared__ int s_len[kResWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double ss = 0.0;
-    for (int j = gw; j < d; j += nw) {
-        double acc = 0.0;
-        for (int p = cp[j] + lane; p < cp[j + 1]; p += 32) acc = fma(rx[p], r[ri[p]], acc);
-        acc = warp_sum(acc);
-        if (lane == 0) ss += acc * acc;
+    for (int j0 = blockIdx.x * kResWarps; j0 < d; j0 += gridDim.x * kResWarps) {
+        const int j = j0 + warp;
+        const int p0 = j < d ? cp[j] : 0, p1 = j < d ? cp[j + 1] : 0;
+        if (lane == 0) s_len[warp] = p1 - p0;
+        if (p1 - p0 <= kLong) {
+            double acc = 0.0;
+#pragma unroll 4
+            for (int p = p0 + lane; p < p1; p += 32) acc = fma(rx[p], r[ri[p]], acc);
+            acc = warp_sum(acc);
+            if (lane == 0) ss += acc * acc;
+        }
+        __syncthreads();
+        for (int w = 0; w < kResWarps; ++w) {
+            if (s_len[w] <= kLong) continue;   // uniform in the CTA
+            const int q0 = cp[j0 + w], q1 = q0 + s_len[w];
+            double acc = 0.0;
+#pragma unroll 4
+            for (int p = q0 + threadIdx.x; p < q1; p += kLThreads) acc = fma(rx[p], r[ri[p]], acc);
+            acc = block_sum(acc, red);
+            if (threadIdx.x == 0) ss += acc * acc;
+        }
+        __syncthreads();
     }
     ss = block_sum(ss, red);
     if (threadIdx.x == 0) part[blockIdx.x] = ss;
 }
 
+// Two columns per CTA at a time, which share the loads of r (40,000 x 4,000: 310 us,
+// 634 with one column and 512 CTAs).
 __global__ void __launch_bounds__(kLThreads)
 k_atr_dense(const double* __restrict__ A, int64_t lda, int n, int d, const double* __restrict__ r,
             double* __restrict__ part)
 {
     pdl_wait();
-    __shared__ double red[kLThreads / 32];
+    __shared__ double red[kResWarps];
     double ss = 0.0;
-    for (int j = blockIdx.x; j < d; j += gridDim.x) {
-        double acc = 0.0;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) acc = fma(A[i + (int64_t)j * lda], r[i], acc);
-        acc = block_sum(acc, red);
-        ss += acc * acc;
+    for (int j = 2 * blockIdx.x; j < d; j += 2 * gridDim.x) {
+        const double* a0 = A + (int64_t)j * lda;
+        const double* a1 = j + 1 < d ? a0 + lda : a0;
+        double s0 = 0.0, s1 = 0.0;
+        int i = threadIdx.x;
+        for (; i + 3 * kLThreads < n; i += 4 * kLThreads) {
+            double u[4], v0[4], v1[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                u[q] = r[i + q * kLThreads];
+                v0[q] = a0[i + q * kLThreads];
+                v1[q] = a1[i + q * kLThreads];
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                s0 = fma(v0[q], u[q], s0);
+                s1 = fma(v1[q], u[q], s1);
+            }
+        }
+        for (; i < n; i += kLThreads) {
+            const double u = r[i];
+            s0 = fma(a0[i], u, s0);
+            s1 = fma(a1[i], u, s1);
+        }
+        s0 = block_sum(s0, red);
+        s1 = block_sum(s1, red);
+        ss += s0 * s0 + (j + 1 < d ? s1 * s1 : 0.0);
     }
     if (threadIdx.x == 0) part[blockIdx.x] = ss;
 }
@@ -1549,22 +1638,30 @@ __global__ void k_sum_parts(const double* __restrict__ part, int np, double* __r
     if (threadIdx.x == 0) *out = sqrt(s);
 }
 
+static void residual_csr(const LsqrProblem& P, const double* x, const double* b, double* r, double* part,
+                         cudaStream_t st)
+{
+    // lanes per row: the power of two at or above half the mean row length, 4 to 32
+    const int64_t mean = P.n > 0 ? P.nnz / P.n : 0;
+    int L = 4;
+    while (L < 32 && 2 * L < mean) L *= 2;
+    launch_k(k_residual_csr, kResGrid, kLThreads, 0, st, P.rp, P.ci, P.cx64, (int)P.n, L, x, b, r, part);
+}
+
 // out[0] = ||b - A x||, out[1] = ||A^T (b - A x)||; FP64 throughout.
 void residual_and_backward(const LsqrProblem& P, const double* x, const double* b, double* r,
                            double* part, double* out, cudaStream_t st)
 {
-    const int np = 512;
     if (P.Ad64) {
-        launch_k(k_residual_dense, np, kLThreads, 0, st, P.Ad64, P.lda64, (int)P.n, (int)P.d, x, b, r, part);
-        launch_k(k_sum_parts, 1, kLThreads, 0, st, part, np, out);
-        launch_k(k_atr_dense, np, kLThreads, 0, st, P.Ad64, P.lda64, (int)P.n, (int)P.d, r, part);
-        launch_k(k_sum_parts, 1, kLThreads, 0, st, part, np, out + 1);
+        launch_k(k_residual_dense, kResGrid, kLThreads, 0, st, P.Ad64, P.lda64, (int)P.n, (int)P.d, x, b, r, part);
+        launch_k(k_sum_parts, 1, kLThreads, 0, st, part, kResGrid, out);
+        launch_k(k_atr_dense, kResGrid, kLThreads, 0, st, P.Ad64, P.lda64, (int)P.n, (int)P.d, r, part);
     } else {
-        launch_k(k_residual_csr, np, kLThreads, 0, st, P.rp, P.ci, P.cx64, (int)P.n, x, b, r, part);
-        launch_k(k_sum_parts, 1, kLThreads, 0, st, part, np, out);
-        launch_k(k_atr_csc, np, kLThreads, 0, st, P.cp, P.ri, P.rx64, (int)P.d, r, part);
-        launch_k(k_sum_parts, 1, kLThreads, 0, st, part, np, out + 1);
+        residual_csr(P, x, b, r, part, st);
+        launch_k(k_sum_parts, 1, kLThreads, 0, st, part, kResGrid, out);
+        launch_k(k_atr_csc, kResGrid, kLThreads, 0, st, P.cp, P.ri, P.rx64, (int)P.d, r, part);
     }
+    launch_k(k_sum_parts, 1, kLThreads, 0, st, part, kResGrid, out + 1);
     for (int q = 0; q < 4; ++q) SKL_LAUNCHED();
 }
 
