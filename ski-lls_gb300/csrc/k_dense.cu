@@ -12,10 +12,10 @@
 // into its m sketch rows by a fixed-order gather over S's bucket lists, so
 // HDA never exists in HBM.  The DHT of a real length-N vector is computed from
 // a complex FFT of half length L = N/2 (even/odd packing) and H = Re F - Im F.
-// The FFT is a Stockham autosort pass sequence with radices 7, 5, 4, 3, 2:
-// FP32 columns stay in shared memory (each pass reads its butterflies into
-// registers, synchronises, writes back in place); FP64 columns, or lengths
-// beyond shared memory, ping-pong through a global scratch slab per CTA.
+// FP32 columns run a decimation-in-frequency FFT in place in shared memory; FP64
+// columns, or lengths beyond shared memory, Stockham passes with radices 7, 5, 4,
+// 3, 2 through a global scratch slab per CTA; the right-hand side (one FP64
+// column) the same passes over the whole GPU.
 #include <cmath>
 
 #include "skl_internal.hpp"
@@ -25,9 +25,7 @@
 namespace skl {
 
 constexpr int kFftThreads = 1024;
-constexpr int kFftMaxPerThread = 32;            // complex values per thread (registers)
 constexpr int kFftMaxRadices = 32;
-constexpr int kFftDhtStage = 26;               // unpack values per thread (L <= 26 * 1024)
 constexpr int kFftSmemMaxL = 25 * 1024;        // shared-memory path limit
 
 template <typename T> struct Cplx;
@@ -180,27 +178,6 @@ SKL_DEV void butterfly_store(typename Cplx<T>::type* y, int p, int i, const type
     for (int q = 0; q < R; ++q) y[j + q * p] = v[q];
 }
 
-// One pass in place on `buf` (all threads load, sync, store).
-template <typename T, int R>
-SKL_DEV void pass_inplace(typename Cplx<T>::type* buf, int L, int p)
-{
-    using C = typename Cplx<T>::type;
-    const int nb = L / R;
-    C v[kFftMaxPerThread];
-    int cnt = 0;
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-        butterfly_load<T, R>(buf, L, p, i, v + cnt * R);
-        ++cnt;
-    }
-    __syncthreads();
-    cnt = 0;
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-        butterfly_store<T, R>(buf, p, i, v + cnt * R);
-        ++cnt;
-    }
-    __syncthreads();
-}
-
 template <typename T, int R>
 SKL_DEV void pass_pingpong(const typename Cplx<T>::type* x, typename Cplx<T>::type* y, int L, int p)
 {
@@ -220,8 +197,7 @@ struct FftPlan {
     int radix[kFftMaxRadices];
 };
 
-// Complex forward FFT of length L on buf (in place for shared memory; with a
-// second buffer `alt` the passes ping-pong and the result ends in *res).
+// Complex forward FFT of length L, ping-pong between buf and alt; the result's buffer.
 template <typename T>
 SKL_DEV typename Cplx<T>::type* fft_run(const FftPlan& P, typename Cplx<T>::type* buf,
                                         typename Cplx<T>::type* alt)
@@ -232,108 +208,66 @@ SKL_DEV typename Cplx<T>::type* fft_run(const FftPlan& P, typename Cplx<T>::type
     C* y = alt;
     for (int s = 0; s < P.nr; ++s) {
         const int R = P.radix[s];
-        if (!alt) {
-            switch (R) {
-            case 2: pass_inplace<T, 2>(x, P.L, p); break;
-            case 3: pass_inplace<T, 3>(x, P.L, p); break;
-            case 4: pass_inplace<T, 4>(x, P.L, p); break;
-            case 5: pass_inplace<T, 5>(x, P.L, p); break;
-            default: pass_inplace<T, 7>(x, P.L, p); break;
-            }
-        } else {
-            switch (R) {
-            case 2: pass_pingpong<T, 2>(x, y, P.L, p); break;
-            case 3: pass_pingpong<T, 3>(x, y, P.L, p); break;
-            case 4: pass_pingpong<T, 4>(x, y, P.L, p); break;
-            case 5: pass_pingpong<T, 5>(x, y, P.L, p); break;
-            default: pass_pingpong<T, 7>(x, y, P.L, p); break;
-            }
-            C* t = x;
-            x = y;
-            y = t;
+        switch (R) {
+        case 2: pass_pingpong<T, 2>(x, y, P.L, p); break;
+        case 3: pass_pingpong<T, 3>(x, y, P.L, p); break;
+        case 4: pass_pingpong<T, 4>(x, y, P.L, p); break;
+        case 5: pass_pingpong<T, 5>(x, y, P.L, p); break;
+        default: pass_pingpong<T, 7>(x, y, P.L, p); break;
         }
+        C* t = x;
+        x = y;
+        y = t;
         p *= R;
     }
     return x;
 }
 
-// Column transform.  Input column a (n entries, FP64) times D/sqrt(N), zero
-// padded to N = 2L; output H (N reals) written over the complex buffer as
-// reals (H[k] at ((T*)buf)[k]) -- the caller provides the buffers.
+// z[t] = x[2t] + i x[2t+1] of the column a (n entries, zeros beyond) times D scale.
 template <typename T>
-SKL_DEV typename Cplx<T>::type* dht_column(const FftPlan& P, const double* __restrict__ a, int n,
-                                           const double* __restrict__ D, double scale,
-                                           typename Cplx<T>::type* buf,
-                                           typename Cplx<T>::type* alt)
+SKL_DEV typename Cplx<T>::type dht_packed(const double* __restrict__ a, int n, const double* __restrict__ D, T sc,
+                                          int t)
 {
-    using C = typename Cplx<T>::type;
-    const int L = P.L;
-    // pack z[t] = x[2t] + i x[2t+1]
-    const T sc = (T)scale;
-    for (int t = threadIdx.x; t < L; t += blockDim.x) {
-        const int i0 = 2 * t, i1 = 2 * t + 1;
-        T x0 = i0 < n ? (T)a[i0] : T(0);
-        T x1 = i1 < n ? (T)a[i1] : T(0);
-        if (i0 < n && D[i0] < 0) x0 = -x0;
-        if (i1 < n && D[i1] < 0) x1 = -x1;
-        C z;
-        z.x = x0 * sc;
-        z.y = x1 * sc;
-        buf[t] = z;
-    }
-    __syncthreads();
-    C* Z = fft_run<T>(P, buf, alt);
-    // unpack: X[k] = (Z[k] + conj(Z[L-k]))/2 - i/2 e^{-2 pi i k/N} (Z[k] - conj(Z[L-k]))
-    // H[k] = Re X[k] - Im X[k] (k < L), H[N-k] = Re X[k] + Im X[k] (0 < k < L),
-    // H[L] = Re Z[0] - Im Z[0].
-    const int N = 2 * L;
-    auto hvals = [&](int kk, T& hk, T& hnk) {
-        const C zk = Z[kk % L];
-        const C zc = Z[(L - kk) % L];
-        const T er = (zk.x + zc.x) * T(0.5), ei = (zk.y - zc.y) * T(0.5);   // even part
-        const T or_ = (zk.y + zc.y) * T(0.5), oi = -(zk.x - zc.x) * T(0.5); // odd part
-        const C w = twiddle<T>(kk, 2 * L);
-        const T xr = er + (w.x * or_ - w.y * oi);
-        const T xi = ei + (w.x * oi + w.y * or_);
-        hk = xr - xi;
-        hnk = xr + xi;
-    };
-    if (alt) {
-        // ping-pong path: write the reals into the other buffer
-        C* other = (Z == buf) ? alt : buf;
-        T* H = reinterpret_cast<T*>(other);
-        for (int kk = threadIdx.x; kk < L; kk += blockDim.x) {
-            T hk, hnk;
-            hvals(kk, hk, hnk);
-            H[kk] = hk;
-            if (kk != 0) H[N - kk] = hnk;
-        }
-        if (threadIdx.x == 0) H[L] = Z[0].x - Z[0].y;
-        __syncthreads();
-        return other;
-    }
-    // in place (shared memory): stage in registers, synchronise, write
-    T hv[2 * kFftDhtStage];
-    int cnt = 0;
-    for (int kk = threadIdx.x; kk < L; kk += blockDim.x) {
-        hvals(kk, hv[cnt], hv[cnt + 1]);
-        cnt += 2;
-    }
-    T hL = T(0);
-    if (threadIdx.x == 0) hL = Z[0].x - Z[0].y;
-    __syncthreads();
-    T* H = reinterpret_cast<T*>(Z);
-    cnt = 0;
-    for (int kk = threadIdx.x; kk < L; kk += blockDim.x) {
-        H[kk] = hv[cnt];
-        if (kk != 0) H[N - kk] = hv[cnt + 1];
-        cnt += 2;
-    }
-    if (threadIdx.x == 0) H[L] = hL;
-    __syncthreads();
-    return Z;
+    const int i0 = 2 * t, i1 = 2 * t + 1;
+    T x0 = i0 < n ? (T)a[i0] : T(0);
+    T x1 = i1 < n ? (T)a[i1] : T(0);
+    if (i0 < n && D[i0] < 0) x0 = -x0;
+    if (i1 < n && D[i1] < 0) x1 = -x1;
+    typename Cplx<T>::type z;
+    z.x = x0 * sc;
+    z.y = x1 * sc;
+    return z;
 }
 
+// H[k] and H[N-k] from Z[k] = zk, Z[L-k] = zc and w = exp(-2 pi i k / N):
+// X[k] = (Z[k] + conj(Z[L-k]))/2 - i/2 w (Z[k] - conj(Z[L-k])),
+// H[k] = Re X[k] - Im X[k], H[N-k] = Re X[k] + Im X[k]; also H[0], H[L] for k = 0.
+template <typename T>
+SKL_DEV void dht_pair(typename Cplx<T>::type zk, typename Cplx<T>::type zc, typename Cplx<T>::type w, T& hk, T& hnk)
+{
+    const T er = (zk.x + zc.x) * T(0.5), ei = (zk.y - zc.y) * T(0.5);   // even part
+    const T or_ = (zk.y + zc.y) * T(0.5), oi = -(zk.x - zc.x) * T(0.5); // odd part
+    const T xr = er + (w.x * or_ - w.y * oi);
+    const T xi = ei + (w.x * oi + w.y * or_);
+    hk = xr - xi;
+    hnk = xr + xi;
+}
+
+// Bucket sums of one transformed column: SA[h] = sum over the bucket of h
+// (increasing source row) of alpha * (+-1/sqrt(k)) * H[i], the order of csc_mv 'n'.
+template <typename T>
+SKL_DEV T bucket_sum(const T* H, const int* __restrict__ bptr, const unsigned* __restrict__ bent, int h, T av)
+{
+    T acc = T(0);
+    for (int q = bptr[h]; q < bptr[h + 1]; ++q) {
+        const unsigned e = bent[q];
+        const T hv = H[e & 0x7fffffffu];
+        acc += (e & 0x80000000u) ? -av * hv : av * hv;
+    }
+    return acc;
+}
+
+// FP64 columns, or lengths beyond shared memory: a CTA per column, ping-pong in gscratch.
 template <typename T>
 __global__ void __launch_bounds__(kFftThreads)
 k_dht_hash(const double* __restrict__ A, int64_t lda, int n, int d, const double* __restrict__ D,
@@ -343,32 +277,341 @@ k_dht_hash(const double* __restrict__ A, int64_t lda, int n, int d, const double
 {
     pdl_wait();
     using C = typename Cplx<T>::type;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    C* buf;
-    C* alt = nullptr;
-    if (gscratch) {
-        buf = gscratch + (size_t)blockIdx.x * 2 * P.L;
-        alt = buf + P.L;
-    } else {
-        buf = reinterpret_cast<C*>(smem_raw);
-    }
-    const int N = 2 * P.L;
+    C* buf = gscratch + (size_t)blockIdx.x * 2 * P.L;
+    C* alt = buf + P.L;
+    const int L = P.L, N = 2 * L;
     for (int j = blockIdx.x; j < d; j += gridDim.x) {
-        C* Z = dht_column<T>(P, A + (int64_t)j * lda, n, D, scale, buf, alt);
-        const T* H = reinterpret_cast<const T*>(Z);
+        for (int t = threadIdx.x; t < L; t += blockDim.x)
+            buf[t] = dht_packed<T>(A + (int64_t)j * lda, n, D, (T)scale, t);
+        __syncthreads();
+        const C* Z = fft_run<T>(P, buf, alt);
+        T* H = reinterpret_cast<T*>(Z == buf ? alt : buf);
+        for (int kk = threadIdx.x; kk < L; kk += blockDim.x) {
+            T hk, hnk;
+            dht_pair<T>(Z[kk], Z[(L - kk) % L], twiddle<T>(kk, N), hk, hnk);
+            H[kk] = hk;
+            if (kk != 0) H[N - kk] = hnk;
+        }
+        if (threadIdx.x == 0) H[L] = Z[0].x - Z[0].y;
+        __syncthreads();
         if (Yout) {
             for (int k = threadIdx.x; k < N; k += blockDim.x) Yout[k + (int64_t)j * ldy] = (double)H[k];
         }
         if (SA) {
-            // SA[h, j] = sum over the bucket of h (increasing source row) of
-            // alpha * (+-1/sqrt(k)) * H[i]  -- the order of csc_mv 'n'
-            const T av = (T)alpha_v;
-            for (int h = threadIdx.x; h < m; h += blockDim.x) {
-                T acc = T(0);
-                for (int q = bptr[h]; q < bptr[h + 1]; ++q) {
-                    const unsigned e = bent[q];
-                    const T hv = H[e & 0x7fffffffu];
-                    acc += (e & 0x80000000u) ? -av * hv : av * hv;
+            for (int h = threadIdx.x; h < m; h += blockDim.x)
+                SA[h + (int64_t)j * ld] = bucket_sum<T>(H, bptr, bent, h, (T)alpha_v);
+        }
+        __syncthreads();
+    }
+}
+
+// One column over the whole GPU (the right-hand side, FP64): a launch per pass.
+// A single CTA takes 1,380 us for 40,000 rows, these ~10 launches 58 us.
+__global__ void k_dht_load(const double* __restrict__ a, int n, const double* __restrict__ D, double scale, int L,
+                           double2* __restrict__ z)
+{
+    pdl_wait();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < L) z[t] = dht_packed<double>(a, n, D, scale, t);
+}
+template <int R>
+__global__ void k_dht_pass(const double2* __restrict__ x, double2* __restrict__ y, int L, int p)
+{
+    pdl_wait();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= L / R) return;
+    double2 v[R];
+    butterfly_load<double, R>(x, L, p, i, v);
+    butterfly_store<double, R>(y, p, i, v);
+}
+__global__ void k_dht_unpack(const double2* __restrict__ Z, int L, double* __restrict__ H)
+{
+    pdl_wait();
+    const int kk = blockIdx.x * blockDim.x + threadIdx.x;
+    if (kk >= L) return;
+    double hk, hnk;
+    dht_pair<double>(Z[kk], Z[(L - kk) % L], twiddle<double>(kk, 2 * L), hk, hnk);
+    H[kk] = hk;
+    if (kk != 0) H[2 * L - kk] = hnk;
+    else H[L] = Z[0].x - Z[0].y;
+}
+__global__ void k_dht_gather(const double* __restrict__ H, const int* __restrict__ bptr,
+                             const unsigned* __restrict__ bent, int m, double alpha_v, double* __restrict__ Sb)
+{
+    pdl_wait();
+    const int h = blockIdx.x * blockDim.x + threadIdx.x;
+    if (h < m) Sb[h] = bucket_sum<double>(H, bptr, bent, h, alpha_v);
+}
+
+// ---- FP32 columns in shared memory ----------------------------------------------
+// A CTA per column at a time.  The FFT is decimation in frequency in place: a pass
+// of radix R = R1 R2 (two radices in registers between one load and one store of
+// shared memory) reads and writes the same places, so no thread holds more than
+// R values and no second buffer is needed; the results end in digit-reversed
+// order, which the last two steps undo through tables made once per call:
+// part[p] (the partner's place and the frequency at p) for the unpacking, done in
+// place pair by pair, and the bucket entries with source rows replaced by places.
+// The column is read once, with the next column's lines on their way to L2; the
+// signs are bits in shared memory, and the FP64 values are rounded to FP32 on
+// their bits (a warp's FP64 conversion holds the pipe for 16 cycles: 10 us of a
+// column of 40,000).  Passes with odd R come last: their short strides then meet
+// each bank once.  40,000 x 4,000: 1,516 us, 2,690 with one radix per pass,
+// autosorted through local memory (floor: 188 us for the read).
+constexpr int kDifThreads = 512;
+constexpr int kDifMaxPasses = 16;
+struct DifPlan {
+    int L, np;
+    int r1[kDifMaxPasses], r2[kDifMaxPasses];
+};
+
+// Forward DFT of the R values v[off + q step].
+template <int R, int NV>
+SKL_DEV void dft_at(float2 (&v)[NV], int off, int step)
+{
+    if constexpr (R == 2 || R == 4) {
+        float2 w[R];
+#pragma unroll
+        for (int q = 0; q < R; ++q) w[q] = v[off + q * step];
+        dft_small<float, R>(w);
+#pragma unroll
+        for (int q = 0; q < R; ++q) v[off + q * step] = w[q];
+    } else if constexpr (R > 1) {
+        // symmetric halves: X_q, X_{R-q} = x0 + sum cos a_h -+ i sum sin b_h
+        constexpr int H = (R - 1) / 2;
+        constexpr Roots<R> w{};
+        const float2 x0 = v[off];
+        float2 a[H], b[H];
+        float2 s = x0;
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+            const float2 u = v[off + (h + 1) * step], t = v[off + (R - 1 - h) * step];
+            a[h] = cadd(u, t);
+            b[h] = csub(u, t);
+            s = cadd(s, a[h]);
+        }
+        v[off] = s;
+#pragma unroll
+        for (int q = 1; q <= H; ++q) {
+            float2 m = x0, y = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int h = 0; h < H; ++h) {
+                const float c = (float)w.re[q * (h + 1) % R], sn = -(float)w.im[q * (h + 1) % R];
+                m.x = fmaf(c, a[h].x, m.x);
+                m.y = fmaf(c, a[h].y, m.y);
+                y.x = fmaf(sn, b[h].x, y.x);
+                y.y = fmaf(sn, b[h].y, y.y);
+            }
+            v[off + q * step] = make_float2(m.x + y.y, m.y - y.x);
+            v[off + (R - q) * step] = make_float2(m.x - y.y, m.y + y.x);
+        }
+    }
+}
+
+// One pass over blocks of B values: butterfly j < S = B / (R1 R2) of a block.
+template <int R1, int R2>
+SKL_DEV void dif_pass(float2* z, int L, int B)
+{
+    constexpr int R = R1 * R2;
+    const int S = B / R, nb = L / R;
+    const unsigned magic = S > 1 ? (unsigned)(((1ull << 32) + S - 1) / S) : 0u;   // i / S, exact for i < 2^16
+    for (int i = threadIdx.x; i < nb; i += kDifThreads) {
+        const int blk = S > 1 ? (int)__umulhi((unsigned)i, magic) : i;
+        const int j = i - blk * S;
+        float2* x = z + blk * B + j;
+        float2 v[R];
+#pragma unroll
+        for (int q = 0; q < R; ++q) v[q] = x[q * S];
+#pragma unroll
+        for (int q2 = 0; q2 < R2; ++q2) dft_at<R1, R>(v, q2, R2);   // v[t1 R2 + q2]
+        if constexpr (R2 > 1) {
+#pragma unroll
+            for (int t1 = 1; t1 < R1; ++t1)
+#pragma unroll
+                for (int q2 = 1; q2 < R2; ++q2) v[t1 * R2 + q2] = cmul(v[t1 * R2 + q2], small_root<float, R>(t1 * q2));
+#pragma unroll
+            for (int t1 = 0; t1 < R1; ++t1) dft_at<R2, R>(v, t1 * R2, 1);
+        }
+        if (S > 1) {
+            // times exp(-2 pi i j t / B), t = t1 + R1 t2: powers of two values of their own
+            const float2 w1 = twiddle<float>(j, B);
+            const float2 w2 = R2 > 1 ? twiddle<float>(R1 * j, B) : w1;
+            float2 u2 = make_float2(1.f, 0.f);
+#pragma unroll
+            for (int t2 = 0; t2 < R2; ++t2) {
+                float2 u = u2;
+#pragma unroll
+                for (int t1 = 0; t1 < R1; ++t1) {
+                    if (t1 > 0) u = t2 == 0 && t1 == 1 ? w1 : cmul(u, w1);
+                    if (t1 > 0 || t2 > 0) v[t1 * R2 + t2] = cmul(v[t1 * R2 + t2], u);
+                }
+                if (t2 + 1 < R2) u2 = t2 == 0 ? w2 : cmul(u2, w2);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < R; ++q) x[q * S] = v[q];
+    }
+    __syncthreads();
+}
+
+SKL_DEV void dif_run(const DifPlan& P, float2* z)
+{
+    int B = P.L;
+    for (int s = 0; s < P.np; ++s) {
+        const int r1 = P.r1[s], r2 = P.r2[s];
+        switch (8 * r1 + r2) {
+        case 8 * 7 + 3: dif_pass<7, 3>(z, P.L, B); break;
+        case 8 * 7 + 2: dif_pass<7, 2>(z, P.L, B); break;
+        case 8 * 5 + 5: dif_pass<5, 5>(z, P.L, B); break;
+        case 8 * 5 + 4: dif_pass<5, 4>(z, P.L, B); break;
+        case 8 * 5 + 3: dif_pass<5, 3>(z, P.L, B); break;
+        case 8 * 5 + 2: dif_pass<5, 2>(z, P.L, B); break;
+        case 8 * 4 + 4: dif_pass<4, 4>(z, P.L, B); break;
+        case 8 * 4 + 3: dif_pass<4, 3>(z, P.L, B); break;
+        case 8 * 4 + 2: dif_pass<4, 2>(z, P.L, B); break;
+        case 8 * 3 + 3: dif_pass<3, 3>(z, P.L, B); break;
+        case 8 * 3 + 2: dif_pass<3, 2>(z, P.L, B); break;
+        case 8 * 7 + 1: dif_pass<7, 1>(z, P.L, B); break;
+        case 8 * 5 + 1: dif_pass<5, 1>(z, P.L, B); break;
+        case 8 * 4 + 1: dif_pass<4, 1>(z, P.L, B); break;
+        case 8 * 3 + 1: dif_pass<3, 1>(z, P.L, B); break;
+        default: dif_pass<2, 1>(z, P.L, B); break;
+        }
+        B /= r1 * r2;
+    }
+}
+
+// Place of frequency k: its digits, first pass's first.
+SKL_DEV int dif_place(const DifPlan& P, int k)
+{
+    int S = P.L, pos = 0;
+    for (int s = 0; s < P.np; ++s)
+        for (int h = 0; h < 2; ++h) {
+            const int r = h ? P.r2[s] : P.r1[s];
+            S /= r;
+            pos += (k % r) * S;
+            k /= r;
+        }
+    return pos;
+}
+
+// part[p] = partner's place | frequency << 16 at the place p of frequency k;
+// place[i], i < N: where H[i] ends, as an index of floats.
+__global__ void k_dif_tables(DifPlan P, unsigned* __restrict__ part, unsigned* __restrict__ place)
+{
+    pdl_wait();
+    const int k = blockIdx.x * blockDim.x + threadIdx.x, L = P.L;
+    if (k >= L) return;
+    const int p = dif_place(P, k);
+    part[p] = (unsigned)dif_place(P, k ? L - k : 0) | ((unsigned)k << 16);
+    place[k] = 2 * p;
+    place[k ? 2 * L - k : L] = 2 * p + 1;
+}
+__global__ void k_dif_entries(const int* __restrict__ bptr, const unsigned* __restrict__ bent, int m,
+                              const unsigned* __restrict__ place, unsigned* __restrict__ out)
+{
+    pdl_wait();
+    const int total = bptr[m];
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < total; q += gridDim.x * blockDim.x) {
+        const unsigned e = bent[q];
+        out[q] = place[e & 0x7fffffffu] | (e & 0x80000000u);
+    }
+}
+
+// (float)a by its bits (round to nearest even); zeros, infinities, NaN and what
+// is not normal in FP32 by the conversion.
+SKL_DEV float round_f32(double a)
+{
+    const unsigned hi = (unsigned)__double2hiint(a), lo = (unsigned)__double2loint(a);
+    const unsigned ex = (hi >> 20) & 0x7ffu;
+    if (ex - 897u >= 253u) return (float)a;
+    unsigned f = ((ex - 896u) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
+    f += ((lo & 0x1fffffffu) + (f & 1u)) > 0x10000000u ? 1u : 0u;
+    return __uint_as_float(f | (hi & 0x80000000u));
+}
+
+__global__ void __launch_bounds__(kDifThreads, 1)
+k_dht_hash_smem(const double* __restrict__ A, int64_t lda, int n, int d, const double* __restrict__ D, DifPlan P,
+                double scale, const int* __restrict__ bptr, const unsigned* __restrict__ ent, int m, double alpha_v,
+                float* __restrict__ SA, int64_t ld, double* __restrict__ Yout, int64_t ldy,
+                const unsigned* __restrict__ part, const unsigned* __restrict__ place)
+{
+    pdl_wait();
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float2* z = reinterpret_cast<float2*>(smem_raw);
+    const float* H = reinterpret_cast<const float*>(z);
+    const int L = P.L, N = 2 * L;
+    unsigned* sgn = reinterpret_cast<unsigned*>(z + L);   // bit i: D[i] < 0
+    for (int w = threadIdx.x; w < (N + 31) / 32 * 32; w += kDifThreads) {
+        const unsigned bits = __ballot_sync(0xffffffffu, w < n && D[w] < 0);
+        if ((threadIdx.x & 31) == 0) sgn[w / 32] = bits;
+    }
+    __syncthreads();
+    const float sc = (float)scale, av = (float)alpha_v;
+    for (int j = blockIdx.x; j < d; j += gridDim.x) {
+        const double* a = A + (int64_t)j * lda;
+        if (j + (int)gridDim.x < d) {
+            const char* nx = reinterpret_cast<const char*>(a + (int64_t)gridDim.x * lda);
+            for (int64_t o = (int64_t)threadIdx.x * 128; o < (int64_t)n * 8; o += kDifThreads * 128)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + o));
+        }
+        // x[2t] + i x[2t+1] with D's signs, scaled; pairs of loads where they align
+        const bool vec = ((reinterpret_cast<uintptr_t>(a) & 15) == 0);
+        auto put = [&](int t, double x0, double x1) {
+            const unsigned w = sgn[t >> 4] >> (2 * (t & 15));
+            z[t] = make_float2(__uint_as_float(__float_as_uint(round_f32(x0)) ^ (w << 31)) * sc,
+                               __uint_as_float(__float_as_uint(round_f32(x1)) ^ ((w >> 1) << 31)) * sc);
+        };
+        const int full = vec ? n / 2 : 0;
+        constexpr int U = 8;
+        int t = threadIdx.x;
+        for (; t + (U - 1) * kDifThreads < full; t += U * kDifThreads) {
+            double2 v[U];
+#pragma unroll
+            for (int q = 0; q < U; ++q) v[q] = reinterpret_cast<const double2*>(a)[t + q * kDifThreads];
+#pragma unroll
+            for (int q = 0; q < U; ++q) put(t + q * kDifThreads, v[q].x, v[q].y);
+        }
+#pragma unroll 4
+        for (; t < L; t += kDifThreads)
+            put(t, 2 * t < n ? a[2 * t] : 0.0, 2 * t + 1 < n ? a[2 * t + 1] : 0.0);
+        __syncthreads();
+        dif_run(P, z);
+        // the pair of places (p, p2) holds Z[k], Z[L-k]: H[k], H[N-k] to p, H[L-k],
+        // H[L+k] to p2 (exp(-2 pi i (L-k) / N) = -conj of k's)
+#pragma unroll 4
+        for (int p = threadIdx.x; p < L; p += kDifThreads) {
+            const unsigned e = part[p];
+            const int p2 = e & 0xffffu, k = e >> 16;
+            if (p2 < p) continue;
+            const float2 zk = z[p], zc = z[p2];
+            const float2 w = twiddle<float>(k, N);
+            float2 h, g;
+            dht_pair<float>(zk, zc, w, h.x, h.y);
+            if (k == 0) h.y = zk.x - zk.y;
+            if (p2 != p) {
+                dht_pair<float>(zc, zk, make_float2(-w.x, w.y), g.x, g.y);
+                z[p2] = g;
+            }
+            z[p] = h;
+        }
+        __syncthreads();
+        if (Yout) {
+            for (int k = threadIdx.x; k < N; k += kDifThreads) Yout[k + (int64_t)j * ldy] = (double)H[place[k]];
+        }
+        if (SA) {
+            for (int h = threadIdx.x; h < m; h += kDifThreads) {
+                // the bucket's sum in its order, four entries' loads at a time
+                float acc = 0.f;
+                const int q1 = bptr[h + 1];
+                for (int q = bptr[h]; q < q1; q += 4) {
+                    unsigned e[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) e[c] = q + c < q1 ? ent[q + c] : 0u;
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const float hv = H[e[c] & 0x7fffffffu];
+                        if (q + c < q1) acc += (e[c] & 0x80000000u) ? -av * hv : av * hv;
+                    }
                 }
                 SA[h + (int64_t)j * ld] = acc;
             }
@@ -437,6 +680,43 @@ static size_t smem_optin_bytes()
     return v;
 }
 
+// Passes of one or two radices, R1 R2 <= 25: the largest left with the largest that
+// fits; multiples of 4 first, odd ones (and a lone 2) last.
+static DifPlan dif_plan(const FftPlan& P)
+{
+    int cnt[8] = {};
+    for (int s = 0; s < P.nr; ++s) ++cnt[P.radix[s]];
+    cnt[4] += cnt[2] / 2;
+    cnt[2] %= 2;
+    DifPlan Q{};
+    Q.L = P.L;
+    auto push = [&](int a, int b) {
+        Q.r1[Q.np] = a;
+        Q.r2[Q.np++] = b;
+    };
+    for (int f : {7, 5, 4, 3, 2})
+        while (cnt[f] > 0) {
+            --cnt[f];
+            int g = 1;
+            for (int c : {5, 4, 3, 2})
+                if (c <= f && cnt[c] > 0 && f * c <= 25) {
+                    g = c;
+                    --cnt[c];
+                    break;
+                }
+            push(f, g);
+        }
+    // stable: multiples of 4, then the others, each by falling size
+    for (int i = 1; i < Q.np; ++i)
+        for (int j = i; j > 0; --j) {
+            auto key = [&](int q) { const int R = Q.r1[q] * Q.r2[q]; return (R % 4 == 0 ? 1000 : 0) + R; };
+            if (key(j - 1) >= key(j)) break;
+            std::swap(Q.r1[j - 1], Q.r1[j]);
+            std::swap(Q.r2[j - 1], Q.r2[j]);
+        }
+    return Q;
+}
+
 template <typename T>
 static void launch_dht(const double* A, int64_t lda, int64_t n, int64_t d, const double* D,
                        int64_t N, const int* bptr, const unsigned* bent, int k, int64_t m, T* SA,
@@ -447,31 +727,45 @@ static void launch_dht(const double* A, int64_t lda, int64_t n, int64_t d, const
     FftPlan P;
     if (N & 1) fail(SKL_ERR_INVALID, "DHT length must be even");
     if (!factor_plan(N / 2, P)) fail(SKL_ERR_INVALID, "DHT length must factor into 2,3,5,7");
-    const size_t need = (size_t)P.L * sizeof(C);
-    const bool in_smem = std::is_same<T, float>::value && need + 1024 <= smem_optin_bytes() &&
-                         P.L <= kFftSmemMaxL;
     const double scale = 1.0 / std::sqrt((double)N);
     const double alpha_v = (1.0 / std::sqrt((double)k)) * (1.0 / std::sqrt((double)k));
     unsigned grid = (unsigned)std::min<int64_t>(d, 152);
-    if (in_smem) {
-        allow_max_dynamic_smem((const void*)k_dht_hash<T>);
-        launch_k(k_dht_hash<T>, grid, kFftThreads, need, st, A, lda, (int)n, (int)d, D, P, scale, bptr,
-                                                        bent, (int)m, alpha_v, SA, ld, Yout, ldy,
-                                                        nullptr);
-    } else {
-        const size_t per = 2 * (size_t)P.L * sizeof(C);
-        grid = (unsigned)std::min<int64_t>(grid, (int64_t)(gscratch_bytes / per));
-        if (grid == 0) fail(SKL_ERR_ALLOC, "DHT scratch too small");
-        launch_k(k_dht_hash<T>, grid, kFftThreads, 0, st, A, lda, (int)n, (int)d, D, P, scale, bptr, bent,
-                                                     (int)m, alpha_v, SA, ld, Yout, ldy,
-                                                     (C*)gscratch_buf);
+    if constexpr (std::is_same<T, float>::value) {
+        // in shared memory where the column, the signs and (in the scratch) the tables fit
+        const size_t need = (size_t)P.L * sizeof(C) + (size_t)((N + 31) / 32) * 4;
+        const size_t tables = ((size_t)P.L + N + (SA ? (size_t)N * k : 0)) * 4;
+        const DifPlan Q = dif_plan(P);
+        if (P.L <= kFftSmemMaxL && need + 1024 <= smem_optin_bytes() && tables <= gscratch_bytes) {
+            unsigned* part = (unsigned*)gscratch_buf;
+            unsigned* place = part + P.L;
+            unsigned* ent = place + N;
+            launch_k(k_dif_tables, (unsigned)((P.L + 255) / 256), 256, 0, st, Q, part, place);
+            SKL_LAUNCHED();
+            if (SA) {
+                launch_k(k_dif_entries, (unsigned)std::min<int64_t>((N * k + 255) / 256, 1216), 256, 0, st, bptr, bent,
+                         (int)m, (const unsigned*)place, ent);
+                SKL_LAUNCHED();
+            }
+            allow_max_dynamic_smem((const void*)k_dht_hash_smem);
+            launch_k(k_dht_hash_smem, grid, kDifThreads, need, st, A, lda, (int)n, (int)d, D, Q, scale, bptr,
+                     (const unsigned*)ent, (int)m, alpha_v, SA, ld, Yout, ldy, (const unsigned*)part,
+                     (const unsigned*)place);
+            SKL_LAUNCHED();
+            return;
+        }
     }
+    const size_t per = 2 * (size_t)P.L * sizeof(C);
+    grid = (unsigned)std::min<int64_t>(grid, (int64_t)(gscratch_bytes / per));
+    if (grid == 0) fail(SKL_ERR_ALLOC, "DHT scratch too small");
+    launch_k(k_dht_hash<T>, grid, kFftThreads, 0, st, A, lda, (int)n, (int)d, D, P, scale, bptr, bent,
+             (int)m, alpha_v, SA, ld, Yout, ldy, (C*)gscratch_buf);
     SKL_LAUNCHED();
 }
 
 void dht_load_kernels()
 {
     cudaFuncAttributes fa;
+    SKL_CUDA(cudaFuncGetAttributes(&fa, k_dht_hash_smem));
     SKL_CUDA(cudaFuncGetAttributes(&fa, k_dht_hash<float>));
     SKL_CUDA(cudaFuncGetAttributes(&fa, k_dht_hash<double>));
 }
@@ -502,8 +796,32 @@ void dht_hash_rhs(const double* b, int64_t n, const double* D, int64_t N, const 
                   const unsigned* bent, int k, int64_t m, double* Sb, void* scratch,
                   size_t scratch_bytes, cudaStream_t st)
 {
-    launch_dht<double>(b, n, n, 1, D, N, bptr, bent, k, m, Sb, m, nullptr, 0, scratch,
-                       scratch_bytes, st);
+    FftPlan P;
+    if (N & 1) fail(SKL_ERR_INVALID, "DHT length must be even");
+    if (!factor_plan(N / 2, P)) fail(SKL_ERR_INVALID, "DHT length must factor into 2,3,5,7");
+    if (scratch_bytes < 2 * (size_t)P.L * sizeof(double2)) fail(SKL_ERR_ALLOC, "DHT scratch too small");
+    const double scale = 1.0 / std::sqrt((double)N);
+    const double alpha_v = (1.0 / std::sqrt((double)k)) * (1.0 / std::sqrt((double)k));
+    double2* x = (double2*)scratch;
+    double2* y = x + P.L;
+    constexpr int kT = 64;   // small blocks: a pass has a few thousand butterflies
+    auto blocks = [](int64_t c) { return (unsigned)((c + kT - 1) / kT); };
+    launch_k(k_dht_load, blocks(P.L), kT, 0, st, b, (int)n, D, scale, P.L, x);
+    SKL_LAUNCHED();
+    int p = 1;
+    for (int s = 0; s < P.nr; ++s) {
+        const int R = P.radix[s];
+        auto* f = R == 2 ? k_dht_pass<2> : R == 3 ? k_dht_pass<3> : R == 4 ? k_dht_pass<4> : R == 5 ? k_dht_pass<5>
+                                                                                                  : k_dht_pass<7>;
+        launch_k(f, blocks(P.L / R), kT, 0, st, (const double2*)x, y, P.L, p);
+        SKL_LAUNCHED();
+        std::swap(x, y);
+        p *= R;
+    }
+    launch_k(k_dht_unpack, blocks(P.L), kT, 0, st, (const double2*)x, P.L, (double*)y);
+    launch_k(k_dht_gather, blocks(m), kT, 0, st, (const double*)y, bptr, bent, (int)m, alpha_v, Sb);
+    SKL_LAUNCHED();
+    SKL_LAUNCHED();
 }
 
 // Per-block partial sums of squares of a dense column-major matrix (512
