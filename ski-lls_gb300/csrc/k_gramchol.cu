@@ -66,21 +66,24 @@ constexpr int kIB = 64;    // inner block
 // ---- C = alpha A^T B + beta C on the tensor cores (FP32, 3xTF32) -------------
 // 128 x 128 tiles of C, one per CTA; K in stages of 32 rows.  Both operands
 // are column-major with K contiguous, loaded by TMA with the 128-byte swizzle
-// and split in shared memory into hi and lo TF32 parts (hi in place), as in
-// k_tc.cu; the accumulator lives in tensor memory for 64 rows of K and is then
-// added into registers, because the tensor core's own FP32 accumulation over
-// thousands of rows is several times less accurate than FP32 adds.  A stage is
-// 12 MMAs of 128 x 128 x 8 (~768 cycles) against ~1,750 cycles of shared-memory
-// traffic (TMA write, split, MMA reads): the split bounds it.
+// and split into hi and lo TF32 parts: A's go to tensor memory, from where the
+// MMAs take them, B's stay in shared memory (hi in place).  The accumulator lives
+// in tensor memory for 64 rows of K and is then added into registers, because the
+// tensor core's own FP32 accumulation over thousands of rows is several times
+// less accurate than FP32 adds.  A stage is 12 MMAs of 128 x 128 x 8 (~768
+// cycles) against ~1,125 cycles of shared-memory traffic (TMA write, split, MMA
+// reads of B); with A's parts in shared memory too that was ~1,750.  The Gram
+// matrix of 15,000 x 10,000: 7.5 ms, 1,500 cycles a stage; 1,990 with A in shared
+// memory, 1,650 with conversions instead of integer rounding for the hi parts.
 constexpr int kNT = 128;
-constexpr int kNStages = 3;
+constexpr int kNStages = 4;
 constexpr int kNTile = kNT * kBK * 4;               // 16 KB
-constexpr int kNStage = 4 * kNTile;                 // A hi, B hi, A lo, B lo
+constexpr int kNStage = 3 * kNTile;                 // A, B (then its hi), B lo
 constexpr int kNThreads = 512;                      // producer, MMA, 6 splitter, 8 drainer warps
 constexpr int kNSplit = 192;                        // splitter threads (16 warps in all: 128 registers each)
 constexpr int kNGroup = 2;                          // stages per accumulation
 constexpr int kNSmem = kNStages * kNStage + 1024 + 1024;
-constexpr unsigned kNTmemCols = 2 * kNT;
+constexpr unsigned kNTmemCols = 2 * kNT + kNStages * 2 * kBK;   // accumulators; A hi and lo by stage
 
 // Output tiles: blockIdx.y = row tile, blockIdx.x = column tile, first nE tiles
 // of the E part (columns from 0), then the G part (columns from g0).  A row
@@ -129,8 +132,10 @@ k_tc_tn(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtens
     auto tfull = [&](int q) { return smem_u32(bars + 3 * kNStages + q); };
     auto tempty = [&](int q) { return smem_u32(bars + 3 * kNStages + 2 + q); };
     const unsigned done = smem_u32(bars + 3 * kNStages + 4);
-    auto hi = [&](int s) { return smem + s * kNStage; };                 // A then B
-    auto lo = [&](int s) { return smem + s * kNStage + 2 * kNTile; };
+    auto raw_a = [&](int s) { return smem + s * kNStage; };
+    auto hi_b = [&](int s) { return smem + s * kNStage + kNTile; };
+    auto lo_b = [&](int s) { return smem + s * kNStage + 2 * kNTile; };
+    auto tmem_a = [&](unsigned base, int s) { return base + 2 * kNT + (unsigned)(s * 2 * kBK); };   // hi, then lo
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kNStages; ++s) {
@@ -166,8 +171,8 @@ k_tc_tn(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtens
                 if (kb >= kNStages) ok = mbar_wait(empty(s), ((kb / kNStages) - 1) & 1, status);
                 if (!ok) break;
                 mbar_expect_tx(full(s), 2 * kNTile);
-                tma_load_2d(smem_u32(hi(s)), &mapA, t.kA + (kb0 + kb) * kBK, t.a0 + blockIdx.y * kNT, full(s));
-                tma_load_2d(smem_u32(hi(s)) + kNTile, mapB, t.kB + (kb0 + kb) * kBK, col0, full(s));
+                tma_load_2d(smem_u32(raw_a(s)), &mapA, t.kA + (kb0 + kb) * kBK, t.a0 + blockIdx.y * kNT, full(s));
+                tma_load_2d(smem_u32(hi_b(s)), mapB, t.kB + (kb0 + kb) * kBK, col0, full(s));
                 ++issued;
             }
             // the copies this CTA issued have landed before it may exit
@@ -187,15 +192,14 @@ k_tc_tn(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtens
                 if (!ok) break;
                 tc_fence_after();
                 const unsigned d = tmem + (unsigned)(buf * kNT);
-                const unsigned ah = smem_u32(hi(s)), bh = ah + kNTile;
-                const unsigned al = smem_u32(lo(s)), bl = al + kNTile;
+                const unsigned ah = tmem_a(tmem, s), al = ah + kBK;
+                const unsigned bh = smem_u32(hi_b(s)), bl = smem_u32(lo_b(s));
 #pragma unroll
                 for (int k8 = 0; k8 < kBK / 8; ++k8) {
                     const unsigned off = k8 * 32;   // 8 TF32 values along K
-                    mma_tf32(d, sw128_desc(al + off), sw128_desc(bh + off), idesc,
-                             (first && k8 == 0) ? 0u : 1u);
-                    mma_tf32(d, sw128_desc(ah + off), sw128_desc(bl + off), idesc, 1u);
-                    mma_tf32(d, sw128_desc(ah + off), sw128_desc(bh + off), idesc, 1u);
+                    mma_tf32_ta(d, al + k8 * 8, sw128_desc(bh + off), idesc, (first && k8 == 0) ? 0u : 1u);
+                    mma_tf32_ta(d, ah + k8 * 8, sw128_desc(bl + off), idesc, 1u);
+                    mma_tf32_ta(d, ah + k8 * 8, sw128_desc(bh + off), idesc, 1u);
                 }
                 mma_commit(empty(s));
                 if ((kb % kNGroup) == kNGroup - 1 || kb == nkb - 1) mma_commit(tfull(buf));
@@ -205,25 +209,51 @@ k_tc_tn(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtens
             mbar_wait(done, 0, status);
         }
     } else if (warp < 8) {
-        // warps 2..7: split both tiles into hi / lo
-        const int e0 = threadIdx.x - 64;
+        // warps 2..7 split into hi / lo.  Warps 4..7: their quadrant's 32 rows of A
+        // to tensor memory; warps 2 to 5 share B's 32 groups of 32 float4.
+        constexpr int kShare = 6;   // of warps 4, 5, whose schedulers have no other splitter
+        const int quad = warp & 3;
+        const int g0 = warp < 4 ? 2 * kShare + (warp - 2) * (16 - kShare) : warp < 6 ? (warp - 4) * kShare : 0;
+        const int ng = warp < 4 ? 16 - kShare : warp < 6 ? kShare : 0;
         for (int kb = 0; kb < nkb; ++kb) {
             const int s = kb % kNStages;
-            if (!mbar_wait(full(s), (kb / kNStages) & 1, status)) break;
-            float4* h = reinterpret_cast<float4*>(hi(s));
-            float4* l = reinterpret_cast<float4*>(lo(s));
+            if (!__all_sync(0xffffffffu, mbar_wait(full(s), (kb / kNStages) & 1, status))) break;
+            if (warp >= 4) {
+                tc_fence_after();
+                const unsigned char* rowp = raw_a(s) + (quad * 32 + lane) * 128;
+                float h[kBK], l[kBK];
+#pragma unroll
+                for (int c = 0; c < kBK / 4; ++c) {
+                    const float4 v = *reinterpret_cast<const float4*>(rowp + ((c ^ (lane & 7)) << 4));
+                    const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        h[4 * c + q] = tf32_hi_int(x[q]);
+                        l[4 * c + q] = tf32_hi(x[q] - h[4 * c + q]);
+                    }
+                }
+                const unsigned ta = tmem_a(tmem, s) + ((unsigned)(quad * 32) << 16);
+                tmem_st32(ta, h);
+                tmem_st32(ta + kBK, l);
+            }
+            float4* h = reinterpret_cast<float4*>(hi_b(s)) + g0 * 32 + lane;
+            float4* l = reinterpret_cast<float4*>(lo_b(s)) + g0 * 32 + lane;
 #pragma unroll 4
-            for (int e = e0; e < 2 * kNTile / 16; e += kNSplit) {
-                const float4 v = h[e];
+            for (int e = 0; e < ng; ++e) {
+                const float4 v = h[e * 32];
                 float4 a, b;
-                a.x = tf32_hi(v.x); b.x = tf32_hi(v.x - a.x);
-                a.y = tf32_hi(v.y); b.y = tf32_hi(v.y - a.y);
-                a.z = tf32_hi(v.z); b.z = tf32_hi(v.z - a.z);
-                a.w = tf32_hi(v.w); b.w = tf32_hi(v.w - a.w);
-                h[e] = a;
-                l[e] = b;
+                a.x = tf32_hi_int(v.x); b.x = tf32_hi(v.x - a.x);
+                a.y = tf32_hi_int(v.y); b.y = tf32_hi(v.y - a.y);
+                a.z = tf32_hi_int(v.z); b.z = tf32_hi(v.z - a.z);
+                a.w = tf32_hi_int(v.w); b.w = tf32_hi(v.w - a.w);
+                h[e * 32] = a;
+                l[e * 32] = b;
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            if (warp >= 4) {
+                tmem_st_wait();
+                tc_fence_before();
+            }
             mbar_arrive(conv(s));
         }
     } else {

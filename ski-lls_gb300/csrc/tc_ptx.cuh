@@ -97,6 +97,17 @@ __device__ __forceinline__ void mma_tf32(unsigned d_tmem, uint64_t a, uint64_t b
         : "memory");
 }
 
+// The same with A (K columns of 32 bits, a row per lane) in tensor memory.
+__device__ __forceinline__ void mma_tf32_ta(unsigned d_tmem, unsigned a_tmem, uint64_t b, uint32_t idesc,
+                                            unsigned accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
 __device__ __forceinline__ void mma_commit(unsigned bar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
@@ -124,6 +135,24 @@ __device__ __forceinline__ void tmem_ld32(unsigned taddr, float (&v)[32])
     for (int q = 0; q < 32; ++q) v[q] = __uint_as_float(r[q]);
 }
 
+// 32 consecutive TMEM columns of this warp's lane quadrant; tmem_st_wait before
+// they are used.
+__device__ __forceinline__ void tmem_st32(unsigned taddr, const float (&v)[32])
+{
+    unsigned r[32];
+#pragma unroll
+    for (int q = 0; q < 32; ++q) r[q] = __float_as_uint(v[q]);
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
+        "%13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31};" ::"r"(r[0]),
+        "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
+        "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
+        "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]), "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
 // a rounded to the nearest TF32 value (low 13 significand bits zero).  The
 // splits are hi = rna(a) and lo = rna(a - hi): both exact TF32 operands, with
 // |a - hi - lo| <= 2^-24 |a|, so the three products carry ~2^-24 per term.
@@ -132,6 +161,14 @@ __device__ __forceinline__ float tf32_hi(float a)
     unsigned r;
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(a));
     return __uint_as_float(r);
+}
+
+// The same on the integer pipe (a conversion holds its pipe for 8 cycles a warp),
+// but for NaN, which it may turn into -0: for the hi part only, whose lo part
+// a - hi stays NaN through tf32_hi.
+__device__ __forceinline__ float tf32_hi_int(float a)
+{
+    return __uint_as_float((__float_as_uint(a) + 0x1000u) & 0xffffe000u);
 }
 
 // ---- host side ---------------------------------------------------------------
