@@ -1,8 +1,12 @@
 // k_gemm.cuh -- tiled CUDA-core GEMM for the QR / inverse building blocks.
 //
 // C = alpha * op(A) * op(B) + beta * C, column-major, op(X) = X or X^T.
-// 64x64 output tile per CTA, 256 threads with a 4x4 micro-tile each, K in
-// steps of 16 through shared memory.  Split-K writes per-split partials that
+// 64x64 output tile per CTA (FP64: 32x32), 256 threads with a 4x4 (2x2)
+// micro-tile each, K in steps of 16 through shared memory.  FP64 is bound by its
+// pipe (2 FMAs per cycle and SM), not by loads, so small tiles, which spread over
+// the SMs evenly, are the better ones at every size: the products with K = 256
+// of a 1,000 x 1,000 factorization took 282 us each with 64x64 tiles (16 to 144
+// of them), 77 to 134 with 32x32; the Gram matrix of 1,700 x 1,000 2,602 -> 1,513 us.  Split-K writes per-split partials that
 // a fixed-order reduction combines (bitwise reproducible).
 #pragma once
 #include <cstdint>
@@ -13,7 +17,9 @@
 
 namespace skl {
 
-constexpr int kGBM = 64, kGBN = 64, kGBK = 16;
+constexpr int kGBK = 16;
+template <typename T>
+constexpr int kGTile = sizeof(T) == 8 ? 32 : 64;
 
 // TRI = 0: general.  TRI = 1: op(A) is upper triangular (terms with k < row
 // vanish).  TRI = 2: op(B) is upper triangular (terms with k > col vanish).
@@ -28,12 +34,13 @@ k_gemm(int M, int N, int K, T alpha, const T* __restrict__ A, int64_t lda,
        T* __restrict__ partial, int64_t bsa = 0, int64_t bsb = 0, int64_t bsc = 0)
 {
     pdl_wait();
-    __shared__ T As[kGBK][kGBM + 1];
-    __shared__ T Bs[kGBK][kGBN + 1];
+    constexpr int BT = kGTile<T>, MI = BT / 16;
+    __shared__ T As[kGBK][BT + 1];
+    __shared__ T Bs[kGBK][BT + 1];
     const int tid = threadIdx.x;
     const int tx = tid & 15, ty = tid >> 4;     // 16 x 16 threads
-    const int m0 = blockIdx.x * kGBM, n0 = blockIdx.y * kGBN;
-    if (TRI == 3 && n0 + kGBN <= m0) return;
+    const int m0 = blockIdx.x * BT, n0 = blockIdx.y * BT;
+    if (TRI == 3 && n0 + BT <= m0) return;
     if (BAT) {
         A += blockIdx.z * bsa;
         B += blockIdx.z * bsb;
@@ -43,19 +50,19 @@ k_gemm(int M, int N, int K, T alpha, const T* __restrict__ A, int64_t lda,
     int k_begin = BAT ? 0 : blockIdx.z * kchunk;
     int k_end = BAT ? K : min(K, k_begin + kchunk);
     if (TRI == 1) k_begin = max(k_begin, m0 / kGBK * kGBK);
-    if (TRI == 2) k_end = min(k_end, n0 + kGBN);
-    T acc[4][4];
+    if (TRI == 2) k_end = min(k_end, n0 + BT);
+    T acc[MI][MI];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < MI; ++i)
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj) acc[i][jj] = T(0);
+        for (int jj = 0; jj < MI; ++jj) acc[i][jj] = T(0);
 
     for (int k0 = k_begin; k0 < k_end; k0 += kGBK) {
-        // load op(A)[m0:m0+64, k0:k0+16] -> As[k][m]
+        // load op(A)[m0:m0+BT, k0:k0+16] -> As[k][m]
 #pragma unroll
-        for (int e = tid; e < kGBM * kGBK; e += 256) {
+        for (int e = tid; e < BT * kGBK; e += 256) {
             int mm, kk;
-            if (!TA) { mm = e % kGBM; kk = e / kGBM; }
+            if (!TA) { mm = e % BT; kk = e / BT; }
             else { kk = e % kGBK; mm = e / kGBK; }
             int gm = m0 + mm, gk = k0 + kk;
             T v = T(0);
@@ -63,12 +70,12 @@ k_gemm(int M, int N, int K, T alpha, const T* __restrict__ A, int64_t lda,
                 v = TA ? A[gk + (int64_t)gm * lda] : A[gm + (int64_t)gk * lda];
             As[kk][mm] = v;
         }
-        // load op(B)[k0:k0+16, n0:n0+64] -> Bs[k][n]
+        // load op(B)[k0:k0+16, n0:n0+BT] -> Bs[k][n]
 #pragma unroll
-        for (int e = tid; e < kGBN * kGBK; e += 256) {
+        for (int e = tid; e < BT * kGBK; e += 256) {
             int nn, kk;
             if (!TB) { kk = e % kGBK; nn = e / kGBK; }
-            else { nn = e % kGBN; kk = e / kGBN; }
+            else { nn = e % BT; kk = e / BT; }
             int gn = n0 + nn, gk = k0 + kk;
             T v = T(0);
             if (gn < N && gk < k_end && (TRI != 2 || gk <= gn))
@@ -78,24 +85,24 @@ k_gemm(int M, int N, int K, T alpha, const T* __restrict__ A, int64_t lda,
         __syncthreads();
 #pragma unroll
         for (int kk = 0; kk < kGBK; ++kk) {
-            T a[4], b[4];
+            T a[MI], b[MI];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[kk][tx + 16 * i];
+            for (int i = 0; i < MI; ++i) a[i] = As[kk][tx + 16 * i];
 #pragma unroll
-            for (int jj = 0; jj < 4; ++jj) b[jj] = Bs[kk][ty + 16 * jj];
+            for (int jj = 0; jj < MI; ++jj) b[jj] = Bs[kk][ty + 16 * jj];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < MI; ++i)
 #pragma unroll
-                for (int jj = 0; jj < 4; ++jj) acc[i][jj] = fma(a[i], b[jj], acc[i][jj]);
+                for (int jj = 0; jj < MI; ++jj) acc[i][jj] = fma(a[i], b[jj], acc[i][jj]);
         }
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < MI; ++i) {
         int gm = m0 + tx + 16 * i;
         if (gm >= M) continue;
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
+        for (int jj = 0; jj < MI; ++jj) {
             int gn = n0 + ty + 16 * jj;
             if (gn >= N) continue;
             if (partial) {
@@ -417,11 +424,15 @@ inline void splitk_reduce_launch(int M, int N, int splits, T alpha, const T* par
 // must hold splits*M*N entries when splits > 1.
 constexpr int kSplitMinK = 64;
 constexpr int kSplitMax = 128;
-inline int gemm_splits(int M, int N, int K)
+// FP64: six tiles per SM, so that a last one weighs little.
+template <typename T>
+inline int gemm_splits(int M, int N, int K, int tri)
 {
-    int tiles = ((M + kGBM - 1) / kGBM) * ((N + kGBN - 1) / kGBN);
+    constexpr int BT = kGTile<T>, kWant = (sizeof(T) == 8 ? 6 : 2) * 152;
+    int64_t tiles = (int64_t)((M + BT - 1) / BT) * ((N + BT - 1) / BT);
+    if (tri == 3 && sizeof(T) == 8) tiles = (tiles + 1) / 2;
     int s = 1;
-    while (tiles * s < 2 * 152 && K / (s * 2) >= kSplitMinK && s < kSplitMax) s *= 2;
+    while (tiles * s < kWant && K / (s * 2) >= kSplitMinK && s < kSplitMax) s *= 2;
     return s;
 }
 
@@ -453,7 +464,7 @@ inline void gemm_launch_generic(bool ta, bool tb, int M, int N, int K, T alpha, 
                                 T* partial, int64_t partial_cap, int tri, cudaStream_t st)
 {
     if (M <= 0 || N <= 0) return;
-    int splits = (K > 0 && partial && (tri == 0 || tri == 3)) ? gemm_splits(M, N, K) : 1;
+    int splits = (K > 0 && partial && (tri == 0 || tri == 3)) ? gemm_splits<T>(M, N, K, tri) : 1;
     while (splits > 1 && (int64_t)splits * M * N > partial_cap) splits >>= 1;
     int kchunk = K;
     if (splits > 1) {
@@ -462,7 +473,7 @@ inline void gemm_launch_generic(bool ta, bool tb, int M, int N, int K, T alpha, 
         splits = (K + kchunk - 1) / kchunk;
     }
     if (K <= 0) { kchunk = 0; splits = 1; }
-    dim3 grid((M + kGBM - 1) / kGBM, (N + kGBN - 1) / kGBN, splits);
+    dim3 grid((M + kGTile<T> - 1) / kGTile<T>, (N + kGTile<T> - 1) / kGTile<T>, splits);
     T* part = splits > 1 ? partial : nullptr;
     if (tri == 1) launch_k(k_gemm<T, false, false, 1>, grid, 256, 0, st, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, kchunk, part,
                                   (int64_t)0, (int64_t)0, (int64_t)0);
@@ -559,7 +570,7 @@ void trmm(int tri, int M, int N, int K, T alpha, const T* A, int64_t lda, const 
                    st);
 }
 
-// C = alpha * A^T * B + beta * C on the 64 x 64 tiles on and above the diagonal
+// C = alpha * A^T * B + beta * C on the tiles on and above the diagonal
 // of C (the other tiles are not written, or hold nothing of use).
 template <typename T>
 void gemm_upper(int M, int N, int K, T alpha, const T* A, int64_t lda, const T* B, int64_t ldb, T beta,
@@ -577,7 +588,7 @@ void trmm_batched(int tri, int M, int N, int K, T alpha, const T* A, int64_t lda
                   int batch, cudaStream_t st)
 {
     if (M <= 0 || N <= 0 || batch <= 0) return;
-    dim3 grid((M + kGBM - 1) / kGBM, (N + kGBN - 1) / kGBN, batch);
+    dim3 grid((M + kGTile<T> - 1) / kGTile<T>, (N + kGTile<T> - 1) / kGTile<T>, batch);
     if (tri == 1)
         launch_k(k_gemm<T, false, false, 1, true>, grid, 256, 0, st, M, N, K, alpha, A, lda, B, ldb, beta, C,
                                                                 ldc, K, nullptr, bsa, bsb, bsc);
