@@ -4,8 +4,9 @@
 // 5-15 us that each do a few microseconds of work on problems up to a few
 // thousand columns: 30-40 us per iteration went into ramp-up, tails, the
 // launches between them and a host round trip per four iterations (20,000 x
-// 1,000: 36 us per iteration, here 22; 31,013 x 1,507: 40 -> 24; 2,000 x 60: 30 ->
-// 14; 1e6 x 1e4, which streams 0.6 GB: 288 -> 205).  Here the CTAs stay resident and the phases are separated by grid barriers:
+// 1,000: 36 us per iteration, here 19; 31,013 x 1,507: 40 -> 21; 2,000 x 60: 30 ->
+// 13; 1e6 x 1e4, which streams 0.6 GB: 288 -> 196).  Here the CTAs stay resident and
+// the phases are separated by grid barriers:
 //   A  z = M v        rows of the triangle, v in shared memory
 //   B  u = A z - (alpha / beta) u,  partial ||u||^2      z in shared memory
 //   C  t = A^T u      column chunks
@@ -27,6 +28,11 @@
 // FP64 is slow enough (see Sum) that the scalar recurrences of one lane take 2-5
 // us: a warp of their own runs them beside phases A (alpha) and C (beta), and
 // another one updates y and w of the previous iteration beside phase C.
+// On small problems an iteration is latency, ~1.5 us per barrier (a release add and
+// an acquire poll by one thread; fences of its own around them cost 0.3 us more)
+// and ~2.5 to 4 us per phase.  What a phase reads that the previous one does not
+// write (first row and chunk, old u and v, column numbers) is on its way before
+// the staged vector arrives: 21.4 -> 19.1 us per iteration at 20,000 x 1,000.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -112,14 +118,12 @@ SKL_DEV bool bar_all(PState* S, unsigned& gen)
         __syncthreads();
         if (threadIdx.x == 0) {
             gen += gridDim.x;
-            __threadfence();
-            atomicAdd(&S->bar, 1u);
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&S->bar) : "memory");
             unsigned v = 0, k = 0;
             do {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&S->bar) : "memory");
             } while (v < gen && ++k < kBarLimit);
             s_ok = v >= gen;
-            __threadfence();
         }
         __syncthreads();
         return s_ok != 0;
@@ -135,9 +139,15 @@ template <bool MIXED>
 struct Sum {
     ff a{0.f, 0.f};
     SKL_DEV void add_sq(ff x) { ff_fma(a, x, x); }
+    // the CTA's sum, in thread 0; red is free again after the next barrier
     SKL_DEV float2 block(ff* red) const
     {
-        const ff t = block_sum_ff(a, red);
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const ff w = warp_sum_ff(a);
+        if (lane == 0) red[warp] = w;
+        __syncthreads();
+        ff t{0.f, 0.f};
+        if (warp == 0) t = warp_sum_ff(lane < (int)(blockDim.x >> 5) ? red[lane] : t);
         return make_float2(t.hi, t.lo);
     }
 };
@@ -172,12 +182,30 @@ SKL_DEV double val64(double v) { return v; }
 SKL_DEV void acc_load(Acc<true>& a, float2 v) { a.a = ff{v.x, v.y}; }
 SKL_DEV void acc_load(Acc<false>& a, double v) { a.a = v; }
 
-// s * dot - c * old, with s and c as the caller split them once
+// s = sqrt(x), r = 1 / s (0 for x = 0), each to about an ulp: the reciprocal root
+// first, the root from it with one Newton correction.  Shorter than sqrt and a
+// division after it, and several of them can overlap (an FP64 instruction's
+// latency is what one lane waits for).
+SKL_DEV void sqrt_rcp(double x, double& s, double& r)
+{
+    if (x > 1e-280 && x < 1e280) {
+        r = rsqrt(x);
+        s = x * r;
+        s = fma(fma(-s, s, x), 0.5 * r, s);
+    } else {
+        s = sqrt(x);
+        r = s > 0.0 ? 1.0 / s : 0.0;
+    }
+}
+
+// s * dot - c * old, with s and c split once per phase by one thread: the FP64
+// conversions of a whole CTA's warps took ~1,500 to 3,000 cycles of phases B and D
 struct ScaleF {
     ff s, c;
     SKL_DEV ScaleF(double s64, double c64) : s(ff_from_double(s64)), c(ff_from_double(-c64)) {}
     SKL_DEV explicit ScaleF(float4 v) : s{v.x, v.y}, c{v.z, v.w} {}
     SKL_DEV float4 pack() const { return make_float4(s.hi, s.lo, c.hi, c.lo); }
+    SKL_DEV bool pos() const { return s.hi > 0.f; }
     SKL_DEV ff operator()(const Acc<true>& dot, float2 old) const
     {
         ff v{0.f, 0.f};
@@ -189,6 +217,7 @@ struct ScaleF {
 struct ScaleD {
     double s, c;
     SKL_DEV ScaleD(double s64, double c64) : s(s64), c(c64) {}
+    SKL_DEV bool pos() const { return s > 0.0; }
     SKL_DEV double operator()(const Acc<false>& dot, double old) const { return dot.a * s - c * old; }
 };
 template <bool MIXED> using Scale = typename std::conditional<MIXED, ScaleF, ScaleD>::type;
@@ -274,7 +303,19 @@ struct Cta {
     V* sv;                  // staged vector, max(r, d) entries
     V* s_unit;              // kMaxUnits segment sums
     RedT<MIXED>* red;
+    float4* scale;          // the phase's scales
     int tid, lane, warp, G, bid, nloc;
+
+    // set by one thread beside the staging of the phase's vector, read after its barrier
+    SKL_DEV void put_scale(double s, double c) const
+    {
+        if constexpr (MIXED) *scale = ScaleF(s, c).pack();
+    }
+    SKL_DEV Scale<MIXED> get_scale(double s, double c) const
+    {
+        if constexpr (MIXED) return ScaleF(*scale);
+        else return ScaleD(s, c);
+    }
 
     // Rows of the triangle this CTA owns, longest first: local row k is the q-th
     // longest, q = k G + bid (k even) or (k + 1) G - 1 - bid (k odd).
@@ -377,17 +418,21 @@ struct Cta {
     // sc.done decided; z is written unless it is set or `last`.
     SKL_DEV void phase_a(bool last) const
     {
+        const int i0 = tid < nloc ? tri_row(tid, true) : -1;
+        const int c0 = i0 >= 0 ? __ldg(g.cols + i0) : 0;
         for (int i = tid; i < g.r; i += kPT) sv[i] = ld_cg(g.vs + i);
         __syncthreads();
         if (warp < kSWarp) {
             tri_units(g.Mr, true, kSWarp);
         } else if (sc.pend) {
-            const double a = sqrt(sum_partials(g.pa, G));
+            const double a2 = sum_partials(g.pa, G);
             if (lane == 0) {
                 // the reference skips the A^T u step when beta == 0 (IterSolver.cpp:242)
-                const double alpha = sc.beta > 0.0 ? a : sc.alpha;
-                sc.alpha = alpha;
-                sc.ia = alpha > 0.0 ? 1.0 / alpha : 0.0;
+                double alpha = sc.alpha;
+                if (sc.beta > 0.0) {
+                    sqrt_rcp(a2, alpha, sc.ia);
+                    sc.alpha = alpha;
+                }
                 sc.coef_n = alpha * sc.ib;
                 sc.t2 = -sc.sn * alpha * sc.irho;
                 sc.rhobar = -sc.cs * alpha;
@@ -413,29 +458,28 @@ struct Cta {
             const int i = tri_row(k, true);
             if (i < 0) continue;
             const Acc<MIXED> a = tri_sum(k);
-            const int c = __ldg(g.cols + i);
+            const int c = k == tid ? c0 : __ldg(g.cols + i);
             g.z[c] = g.opscale ? store_val<MIXED>(a.value() * g.opscale[c]) : acc_store(a);
         }
     }
 
     // ---- B: u = A z / alpha - (alpha / beta) u; partial ||u||^2
-    SKL_DEV void phase_b() const
+    // row pointers of this lane's first row: the same in every iteration
+    SKL_DEV int2 first_row() const
+    {
+        const int per = 32 / g.L_n, i = (bid * kPW + warp) * per + lane / g.L_n;
+        return i < g.n ? make_int2(__ldg(g.rp + i), __ldg(g.rp + i + 1)) : make_int2(0, 0);
+    }
+    SKL_DEV void phase_b(int2 row0) const
     {
         const int L = g.L_n, l = lane & (L - 1), per = 32 / L, rstep = G * kPW * per;
-        for (int j = tid; j < g.d; j += kPT) sv[j] = ld_cg(g.z + j);
-        __syncthreads();
-        const Scale<MIXED> sc2(sc.ia, sc.coef_n);
+        if (tid == kPT - 1) put_scale(sc.ia, sc.coef_n);
         Sum<MIXED> ss;
         // the next row's entries and old u are loaded before this row's products
         int cc[4], nc[4];
         V aa[4], na[4], uo{}, nuo{};
-        auto load_row = [&](int i, int& p0, int& p1, int (&c)[4], V (&a)[4], V& u) {
-            p0 = p1 = 0;
-            if (i < g.n) {
-                p0 = __ldg(g.rp + i) + l;
-                p1 = __ldg(g.rp + i + 1);
-                if (l == 0) u = ld_cg(g.us + i);
-            }
+        auto load_entries = [&](int i, int p0, int p1, int (&c)[4], V (&a)[4], V& u) {
+            if (i < g.n && l == 0) u = ld_cg(g.us + i);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const bool ok = p0 + k * L < p1;
@@ -445,8 +489,19 @@ struct Cta {
             }
         };
         int base = (bid * kPW + warp) * per;
-        int i = base + lane / L, p0, p1, np0, np1;
-        load_row(i, p0, p1, cc, aa, uo);
+        auto load_row = [&](int i, int& p0, int& p1, int (&c)[4], V (&a)[4], V& u) {
+            p0 = p1 = 0;
+            if (i < g.n) {
+                p0 = __ldg(g.rp + i) + l;
+                p1 = __ldg(g.rp + i + 1);
+            }
+            load_entries(i, p0, p1, c, a, u);
+        };
+        int i = base + lane / L, p0 = row0.x + l, p1 = row0.y, np0, np1;
+        load_entries(i, p0, p1, cc, aa, uo);
+        for (int j = tid; j < g.d; j += kPT) sv[j] = ld_cg(g.z + j);
+        __syncthreads();
+        const Scale<MIXED> sc2 = get_scale(sc.ia, sc.coef_n);
         for (; base < g.n; base += rstep) {
             load_row(i + rstep, np0, np1, nc, na, nuo);
             Acc<MIXED> acc, acc2;
@@ -487,17 +542,19 @@ struct Cta {
     // beta and the Givens rotation (one warp, beside the chunks of phase C)
     SKL_DEV void beta_scalars() const
     {
-        const double beta = sqrt(sum_partials(g.pb, G));
+        const double b2 = sum_partials(g.pb, G);
         if (lane == 0) {
+            double beta, ib, rho, irho;
+            sqrt_rcp(b2, beta, ib);
+            sqrt_rcp(fma(sc.rhobar, sc.rhobar, b2), rho, irho);
             sc.beta = beta;
-            sc.ib = beta > 0.0 ? 1.0 / beta : 0.0;
+            sc.ib = ib;
             sc.coef_t = beta * sc.ia;
-            const double rho = sqrt(sc.rhobar * sc.rhobar + beta * beta);
-            sc.irho = 1.0 / rho;
-            sc.cs = sc.rhobar * sc.irho;
-            sc.sn = beta * sc.irho;
-            sc.t1 = sc.cs * sc.phibar * sc.irho;
-            if (beta > 0.0) sc.nrm_a = sqrt(sc.nrm_a * sc.nrm_a + sc.alpha * sc.alpha + beta * beta);
+            sc.irho = irho;
+            sc.cs = sc.rhobar * irho;
+            sc.sn = beta * irho;
+            sc.t1 = sc.cs * sc.phibar * irho;
+            if (beta > 0.0) sc.nrm_a = sqrt(sc.nrm_a * sc.nrm_a + sc.alpha * sc.alpha + b2);
             sc.phibar = sc.sn * sc.phibar;
             sc.pend = 1;
             sc.ypend = 0;
@@ -505,17 +562,23 @@ struct Cta {
     }
 
     // ---- C: t(i) = A(:, c)^T u by chunks, on the first nw warps of each CTA
-    SKL_DEV void chunks(int nw) const
+    // (ch0: this lane's first chunk, the same in every iteration)
+    SKL_DEV int4 first_chunk(int nw) const
+    {
+        const int q = (bid * nw + warp) * (32 / g.L_t) + lane / g.L_t;
+        return warp < nw && q < __ldg(g.coff + g.r) ? __ldg(g.chunks + q) : make_int4(0, 0, 0, 0);
+    }
+    SKL_DEV void chunks(int nw, const int4 ch0) const
     {
         if (warp >= nw) return;
         const int Lt = g.L_t, lt = lane & (Lt - 1), pert = 32 / Lt;
-        const int total = __ldg(g.coff + g.r);
-        for (int q0 = (bid * nw + warp) * pert; q0 < total; q0 += G * nw * pert) {
+        const int total = __ldg(g.coff + g.r), first = (bid * nw + warp) * pert;
+        for (int q0 = first; q0 < total; q0 += G * nw * pert) {
             const int q = q0 + lane / Lt;
             Acc<MIXED> acc, acc2;
-            int4 ch = make_int4(0, 0, 0, 0);
+            int4 ch = ch0;
             if (q < total) {
-                ch = __ldg(g.chunks + q);
+                if (q0 != first) ch = __ldg(g.chunks + q);
                 for (int p = ch.x + lt; p < ch.y; p += kTU * Lt) {
                     int rr[kTU];
                     V aa[kTU], uu[kTU];
@@ -574,35 +637,41 @@ struct Cta {
             }
         }
     }
-    SKL_DEV void phase_c() const
+    SKL_DEV void phase_c(const int4 ch0) const
     {
         const int yp = sc.ypend;
         __syncthreads();   // beta_scalars clears the flag
         if (warp == kSWarp) beta_scalars();
         else if (warp == kYWarp && yp) update_yw();
-        chunks(kYWarp);
+        chunks(kYWarp, ch0);
     }
 
     // ---- D: v = M^T t / beta - (beta / alpha) v; partial ||v||^2
     SKL_DEV void phase_d() const
     {
+        if (tid == kPT - 1) put_scale(sc.ib, sc.coef_t);
         for (int i = tid; i < g.r; i += kPT) sv[i] = ld_cg(g.t + i);
         tri_finish();
     }
     SKL_DEV void tri_finish() const
     {
+        const bool has_old = (__double_as_longlong(sc.coef_t) << 1) != 0;   // coef_t != 0
+        // this thread's first entry of v, on its way beside the products
+        const int j0 = tid < nloc ? tri_row(tid, false) : -1;
+        V old0{};
+        if (j0 >= 0 && has_old) old0 = g.vs[j0];
         __syncthreads();
         tri_units(g.Mc, false, kPW);
         __syncthreads();
         Sum<MIXED> ss;
-        const double ib = sc.ib, coef_t = sc.coef_t;
-        const Scale<MIXED> sc2(ib, coef_t);
+        const Scale<MIXED> sc2 = get_scale(sc.ib, sc.coef_t);
         for (int k = tid; k < nloc; k += kPT) {
             const int j = tri_row(k, false);
             if (j < 0) continue;
-            const V old = coef_t != 0.0 ? g.vs[j] : V{};
+            V old = old0;
+            if (k != tid) old = has_old ? g.vs[j] : V{};
             const auto nv = sc2(tri_sum(k), old);
-            if (ib > 0.0) g.vs[j] = to_v(nv);   // v stays when beta = 0 (IterSolver.cpp:242)
+            if (sc2.pos()) g.vs[j] = to_v(nv);   // v stays when beta = 0 (IterSolver.cpp:242)
             ss.add_sq(nv);
         }
         const V tot = ss.block(red);
@@ -615,8 +684,9 @@ struct Cta {
     __shared__ PScal sc;                                                                                 \
     __shared__ ValT<MIXED> s_unit[kMaxUnits];                                                            \
     __shared__ RedT<MIXED> red[NT / 32];                                                                 \
+    __shared__ __align__(16) float4 s_phase_scale;                                                       \
     using C = Cta<MIXED, NT>;                                                                            \
-    const C c{g, sc, reinterpret_cast<ValT<MIXED>*>(smem_raw), s_unit, red, (int)threadIdx.x,   \
+    const C c{g, sc, reinterpret_cast<ValT<MIXED>*>(smem_raw), s_unit, red, &s_phase_scale, (int)threadIdx.x,   \
                        (int)threadIdx.x & 31, (int)threadIdx.x >> 5, (int)gridDim.x, (int)blockIdx.x,    \
                        (g.r + (int)gridDim.x - 1) / (int)gridDim.x}
 
@@ -632,11 +702,13 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_lsqr_persist(const PArgs<MIXE
     auto give_up = [&] {
         if (c.tid == 0) S->timeout = 1;
     };
+    const int4 ch0 = c.first_chunk(C::kYWarp);
+    const int2 row0 = c.first_row();
     if (start) {
         c.init_u();
         if (!bar_all<CLUSTER>(S, gen)) return give_up();
         if (c.warp == C::kSWarp) c.init_beta();
-        c.chunks(C::kYWarp);
+        c.chunks(C::kYWarp, ch0);
         if (!bar_all<CLUSTER>(S, gen)) return give_up();
         c.phase_d();
         if (!bar_all<CLUSTER>(S, gen)) return give_up();
@@ -652,9 +724,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_lsqr_persist(const PArgs<MIXE
         if (sc.done || budget <= 0) break;
         --budget;
         if (!bar_all<CLUSTER>(S, gen)) return give_up();
-        c.phase_b();
+        c.phase_b(row0);
         if (!bar_all<CLUSTER>(S, gen)) return give_up();
-        c.phase_c();
+        c.phase_c(ch0);
         if (!bar_all<CLUSTER>(S, gen)) return give_up();
         c.phase_d();
         if (!bar_all<CLUSTER>(S, gen)) return give_up();
@@ -689,7 +761,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_lsqr_phase(const PArgs<MIXED>
     if constexpr (PH == 0) c.init_u();
     if constexpr (PH == 1) {
         if (c.warp == C::kSWarp) c.init_beta();
-        c.chunks(C::kYWarp);
+        c.chunks(C::kYWarp, c.first_chunk(C::kYWarp));
         __syncthreads();
         if (c.bid == 0 && c.tid == 0) g.S->sc[0] = sc;
     }
@@ -706,9 +778,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_lsqr_phase(const PArgs<MIXED>
         __syncthreads();
         if (c.bid == 0 && c.tid == 0) g.S->sc[1] = sc;
     }
-    if constexpr (PH == 5) c.phase_b();
+    if constexpr (PH == 5) c.phase_b(c.first_row());
     if constexpr (PH == 6) {
-        c.phase_c();
+        c.phase_c(c.first_chunk(C::kYWarp));
         __syncthreads();
         if (c.bid == 0 && c.tid == 0) g.S->sc[0] = sc;
     }
@@ -874,11 +946,12 @@ k_lsqr_dense(const PArgs<true> g, const DArgs a, int start, int budget)
         // z of the thread's columns: its own shared-memory entries (registers are
         // short with 64 of them holding the tile)
         ff t[K];
+        const bool use_z = (__double_as_longlong(sc.ia) << 1) != 0;   // sc.ia != 0
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             const int j = k * CW + tid;
             float2 zz = make_float2(0.f, 0.f);
-            if (col_ok && j < g.d && sc.ia != 0.0) zz = ld_cg(g.z + j);
+            if (col_ok && j < g.d && use_z) zz = ld_cg(g.z + j);
             zs[k * kDT + tid] = zz;
             t[k] = ff{0.f, 0.f};
         }
@@ -1008,6 +1081,7 @@ k_lsqr_dense(const PArgs<true> g, const DArgs a, int start, int budget)
         }
     };
     auto phase_d = [&] {
+        if (tid == kDT - 1) c.put_scale(sc.ib, sc.coef_t);
         for (int i = tid; i < g.r; i += kDT) c.sv[i] = ld_cg(a.tn + __ldg(g.cols + i));
         c.tri_finish();
     };
