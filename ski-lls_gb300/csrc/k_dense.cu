@@ -351,6 +351,8 @@ __global__ void k_dht_gather(const double* __restrict__ H, const int* __restrict
 // order, which the last two steps undo through tables made once per call:
 // part[p] (the partner's place and the frequency at p) for the unpacking, done in
 // place pair by pair, and the bucket entries with source rows replaced by places.
+// The transform without a sketch computes both where it needs them: it uses no
+// scratch, so that calls which share one may overlap.
 // The column is read once, with the next column's lines on their way to L2; the
 // signs are bits in shared memory, and the FP64 values are rounded to FP32 on
 // their bits (a warp's FP64 conversion holds the pipe for 16 cycles: 10 us of a
@@ -494,6 +496,26 @@ SKL_DEV int dif_place(const DifPlan& P, int k)
     return pos;
 }
 
+SKL_DEV int dif_frequency(const DifPlan& P, int p)
+{
+    int S = P.L, k = 0, mul = 1;
+    for (int s = 0; s < P.np; ++s)
+        for (int h = 0; h < 2; ++h) {
+            const int r = h ? P.r2[s] : P.r1[s];
+            S /= r;
+            const int t = p / S;
+            p -= t * S;
+            k += t * mul;
+            mul *= r;
+        }
+    return k;
+}
+// Where H[i] ends, as an index of floats.
+SKL_DEV int dif_output(const DifPlan& P, int i)
+{
+    return i < P.L ? 2 * dif_place(P, i) : 2 * dif_place(P, i == P.L ? 0 : 2 * P.L - i) + 1;
+}
+
 // part[p] = partner's place | frequency << 16 at the place p of frequency k;
 // place[i], i < N: where H[i] ends, as an index of floats.
 __global__ void k_dif_tables(DifPlan P, unsigned* __restrict__ part, unsigned* __restrict__ place)
@@ -533,7 +555,7 @@ __global__ void __launch_bounds__(kDifThreads, 1)
 k_dht_hash_smem(const double* __restrict__ A, int64_t lda, int n, int d, const double* __restrict__ D, DifPlan P,
                 double scale, const int* __restrict__ bptr, const unsigned* __restrict__ ent, int m, double alpha_v,
                 float* __restrict__ SA, int64_t ld, double* __restrict__ Yout, int64_t ldy,
-                const unsigned* __restrict__ part, const unsigned* __restrict__ place)
+                const unsigned* __restrict__ part)
 {
     pdl_wait();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -580,8 +602,15 @@ k_dht_hash_smem(const double* __restrict__ A, int64_t lda, int n, int d, const d
         // H[L+k] to p2 (exp(-2 pi i (L-k) / N) = -conj of k's)
 #pragma unroll 4
         for (int p = threadIdx.x; p < L; p += kDifThreads) {
-            const unsigned e = part[p];
-            const int p2 = e & 0xffffu, k = e >> 16;
+            int p2, k;
+            if (SA) {
+                const unsigned e = part[p];
+                p2 = e & 0xffffu;
+                k = e >> 16;
+            } else {
+                k = dif_frequency(P, p);
+                p2 = dif_place(P, k ? L - k : 0);
+            }
             if (p2 < p) continue;
             const float2 zk = z[p], zc = z[p2];
             const float2 w = twiddle<float>(k, N);
@@ -596,7 +625,7 @@ k_dht_hash_smem(const double* __restrict__ A, int64_t lda, int n, int d, const d
         }
         __syncthreads();
         if (Yout) {
-            for (int k = threadIdx.x; k < N; k += kDifThreads) Yout[k + (int64_t)j * ldy] = (double)H[place[k]];
+            for (int k = threadIdx.x; k < N; k += kDifThreads) Yout[k + (int64_t)j * ldy] = (double)H[dif_output(P, k)];
         }
         if (SA) {
             for (int h = threadIdx.x; h < m; h += kDifThreads) {
@@ -731,25 +760,25 @@ static void launch_dht(const double* A, int64_t lda, int64_t n, int64_t d, const
     const double alpha_v = (1.0 / std::sqrt((double)k)) * (1.0 / std::sqrt((double)k));
     unsigned grid = (unsigned)std::min<int64_t>(d, 152);
     if constexpr (std::is_same<T, float>::value) {
-        // in shared memory where the column, the signs and (in the scratch) the tables fit
+        // in shared memory where the column, the signs and (in the scratch) a sketch's
+        // tables fit
         const size_t need = (size_t)P.L * sizeof(C) + (size_t)((N + 31) / 32) * 4;
-        const size_t tables = ((size_t)P.L + N + (SA ? (size_t)N * k : 0)) * 4;
+        const size_t tables = SA ? ((size_t)P.L + N + (size_t)N * k) * 4 : 0;
         const DifPlan Q = dif_plan(P);
         if (P.L <= kFftSmemMaxL && need + 1024 <= smem_optin_bytes() && tables <= gscratch_bytes) {
             unsigned* part = (unsigned*)gscratch_buf;
             unsigned* place = part + P.L;
             unsigned* ent = place + N;
-            launch_k(k_dif_tables, (unsigned)((P.L + 255) / 256), 256, 0, st, Q, part, place);
-            SKL_LAUNCHED();
             if (SA) {
+                launch_k(k_dif_tables, (unsigned)((P.L + 255) / 256), 256, 0, st, Q, part, place);
                 launch_k(k_dif_entries, (unsigned)std::min<int64_t>((N * k + 255) / 256, 1216), 256, 0, st, bptr, bent,
                          (int)m, (const unsigned*)place, ent);
+                SKL_LAUNCHED();
                 SKL_LAUNCHED();
             }
             allow_max_dynamic_smem((const void*)k_dht_hash_smem);
             launch_k(k_dht_hash_smem, grid, kDifThreads, need, st, A, lda, (int)n, (int)d, D, Q, scale, bptr,
-                     (const unsigned*)ent, (int)m, alpha_v, SA, ld, Yout, ldy, (const unsigned*)part,
-                     (const unsigned*)place);
+                     (const unsigned*)ent, (int)m, alpha_v, SA, ld, Yout, ldy, (const unsigned*)part);
             SKL_LAUNCHED();
             return;
         }

@@ -45,3 +45,28 @@ def test_sketch_and_right_hand_side(n, d, m, k):
     SA, Sb = skl.sketch_dense(A, b, D, N, m, k, rows, vals, precision="mixed")
     assert np.linalg.norm(SA - SA_ref) <= 2e-6 * np.linalg.norm(SA_ref)
     assert np.linalg.norm(Sb - Sb_ref) <= 1e-12 * np.linalg.norm(Sb_ref)
+
+
+def test_transforms_without_scratch_may_overlap():
+    """FP32 transforms in shared memory of two lengths, on two streams at once through the
+    entry point whose calls share one scratch: the results of the calls alone, bit for bit."""
+    import torch
+    rng = np.random.default_rng(3)
+    jobs = []
+    for N, d in ((40000, 304), (30000, 456)):
+        A = torch.from_numpy(rng.standard_normal((d, N))).cuda()
+        D = torch.from_numpy(np.where(rng.random(N) < 0.5, -1.0, 1.0)).cuda()
+        Y = torch.zeros((d, N), dtype=torch.float64, device="cuda")
+        skl.dht_device_noalloc(A.data_ptr(), N, N, d, D.data_ptr(), N, Y.data_ptr(), N)
+        torch.cuda.synchronize()
+        jobs.append((A, D, N, d, Y.clone(), Y, torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    for _ in range(5):
+        for A, D, N, d, _, Y, st in jobs:
+            Y.zero_()
+        torch.cuda.synchronize()
+        for A, D, N, d, _, Y, st in jobs:
+            skl.dht_device_noalloc(A.data_ptr(), N, N, d, D.data_ptr(), N, Y.data_ptr(), N, stream=st.cuda_stream)
+        torch.cuda.synchronize()
+        for A, D, N, d, ref, Y, st in jobs:
+            assert torch.equal(ref, Y)
