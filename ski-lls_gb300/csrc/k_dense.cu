@@ -348,16 +348,17 @@ __global__ void k_dht_gather(const double* __restrict__ H, const int* __restrict
 // of radix R = R1 R2 (two radices in registers between one load and one store of
 // shared memory) reads and writes the same places, so no thread holds more than
 // R values and no second buffer is needed; the results end in digit-reversed
-// order, which the last two steps undo through tables made once per call:
-// part[p] (the partner's place and the frequency at p) for the unpacking, done in
-// place pair by pair, and the bucket entries with source rows replaced by places.
+// order, which the last two steps undo through tables made once per call: the
+// places of each pair of frequencies for the unpacking, done in place, and the
+// bucket entries with source rows replaced by places.
 // The transform without a sketch computes both where it needs them: it uses no
 // scratch, so that calls which share one may overlap.
 // The column is read once, with the next column's lines on their way to L2; the
 // signs are bits in shared memory, and the FP64 values are rounded to FP32 on
 // their bits (a warp's FP64 conversion holds the pipe for 16 cycles: 10 us of a
 // column of 40,000).  Passes with odd R come last: their short strides then meet
-// each bank once.  40,000 x 4,000: 1,516 us, 2,690 with one radix per pass,
+// each bank once.  40,000 x 4,000: 1,350 us (cycles of a column: load 14,000, FFT
+// 20,000, the rest unpacking and buckets), 2,690 with one radix per pass,
 // autosorted through local memory (floor: 188 us for the read).
 constexpr int kDifThreads = 512;
 constexpr int kDifMaxPasses = 16;
@@ -496,35 +497,21 @@ SKL_DEV int dif_place(const DifPlan& P, int k)
     return pos;
 }
 
-SKL_DEV int dif_frequency(const DifPlan& P, int p)
-{
-    int S = P.L, k = 0, mul = 1;
-    for (int s = 0; s < P.np; ++s)
-        for (int h = 0; h < 2; ++h) {
-            const int r = h ? P.r2[s] : P.r1[s];
-            S /= r;
-            const int t = p / S;
-            p -= t * S;
-            k += t * mul;
-            mul *= r;
-        }
-    return k;
-}
 // Where H[i] ends, as an index of floats.
 SKL_DEV int dif_output(const DifPlan& P, int i)
 {
     return i < P.L ? 2 * dif_place(P, i) : 2 * dif_place(P, i == P.L ? 0 : 2 * P.L - i) + 1;
 }
 
-// part[p] = partner's place | frequency << 16 at the place p of frequency k;
-// place[i], i < N: where H[i] ends, as an index of floats.
+// part[k], k <= L / 2: the places of frequencies k and L - k (upper half);
+// place[i], i < N: dif_output.
 __global__ void k_dif_tables(DifPlan P, unsigned* __restrict__ part, unsigned* __restrict__ place)
 {
     pdl_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x, L = P.L;
     if (k >= L) return;
     const int p = dif_place(P, k);
-    part[p] = (unsigned)dif_place(P, k ? L - k : 0) | ((unsigned)k << 16);
+    if (k <= L / 2) part[k] = (unsigned)p | ((unsigned)dif_place(P, k ? L - k : 0) << 16);
     place[k] = 2 * p;
     place[k ? 2 * L - k : L] = 2 * p + 1;
 }
@@ -601,26 +588,23 @@ k_dht_hash_smem(const double* __restrict__ A, int64_t lda, int n, int d, const d
         // the pair of places (p, p2) holds Z[k], Z[L-k]: H[k], H[N-k] to p, H[L-k],
         // H[L+k] to p2 (exp(-2 pi i (L-k) / N) = -conj of k's)
 #pragma unroll 4
-        for (int p = threadIdx.x; p < L; p += kDifThreads) {
-            int p2, k;
+        for (int k = threadIdx.x; k <= L / 2; k += kDifThreads) {
+            int p, p2;
             if (SA) {
-                const unsigned e = part[p];
-                p2 = e & 0xffffu;
-                k = e >> 16;
+                const unsigned e = part[k];
+                p = e & 0xffffu;
+                p2 = e >> 16;
             } else {
-                k = dif_frequency(P, p);
+                p = dif_place(P, k);
                 p2 = dif_place(P, k ? L - k : 0);
             }
-            if (p2 < p) continue;
             const float2 zk = z[p], zc = z[p2];
             const float2 w = twiddle<float>(k, N);
             float2 h, g;
             dht_pair<float>(zk, zc, w, h.x, h.y);
             if (k == 0) h.y = zk.x - zk.y;
-            if (p2 != p) {
-                dht_pair<float>(zc, zk, make_float2(-w.x, w.y), g.x, g.y);
-                z[p2] = g;
-            }
+            dht_pair<float>(zc, zk, make_float2(-w.x, w.y), g.x, g.y);
+            if (p2 != p) z[p2] = g;
             z[p] = h;
         }
         __syncthreads();
@@ -628,21 +612,34 @@ k_dht_hash_smem(const double* __restrict__ A, int64_t lda, int n, int d, const d
             for (int k = threadIdx.x; k < N; k += kDifThreads) Yout[k + (int64_t)j * ldy] = (double)H[dif_output(P, k)];
         }
         if (SA) {
-            for (int h = threadIdx.x; h < m; h += kDifThreads) {
-                // the bucket's sum in its order, four entries' loads at a time
-                float acc = 0.f;
-                const int q1 = bptr[h + 1];
-                for (int q = bptr[h]; q < q1; q += 4) {
-                    unsigned e[4];
+            // buckets h and h + 512: each sum in its order, eight entries' loads at a time
+            auto step = [&](int q, int q1, const unsigned (&e)[4], float& acc) {
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) e[c] = q + c < q1 ? ent[q + c] : 0u;
+                for (int c = 0; c < 4; ++c) {
+                    const float hv = H[e[c] & 0x7fffffffu];
+                    if (q + c < q1) acc += (e[c] & 0x80000000u) ? -av * hv : av * hv;
+                }
+            };
+            for (int h = threadIdx.x; h < m; h += 2 * kDifThreads) {
+                const int h2 = h + kDifThreads;
+                const bool two = h2 < m;
+                int q = bptr[h], r = two ? bptr[h2] : 0;
+                const int q1 = bptr[h + 1], r1 = two ? bptr[h2 + 1] : 0;
+                float a0 = 0.f, a1 = 0.f;
+                while (q < q1 || r < r1) {
+                    unsigned e[4], f[4];
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
-                        const float hv = H[e[c] & 0x7fffffffu];
-                        if (q + c < q1) acc += (e[c] & 0x80000000u) ? -av * hv : av * hv;
+                        e[c] = q + c < q1 ? ent[q + c] : 0u;
+                        f[c] = r + c < r1 ? ent[r + c] : 0u;
                     }
+                    step(q, q1, e, a0);
+                    step(r, r1, f, a1);
+                    q += 4;
+                    r += 4;
                 }
-                SA[h + (int64_t)j * ld] = acc;
+                SA[h + (int64_t)j * ld] = a0;
+                if (two) SA[h2 + (int64_t)j * ld] = a1;
             }
         }
         __syncthreads();
