@@ -749,8 +749,10 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_lsqr_phase(const PArgs<MIXED>
 {
     pdl_wait();
     SKL_CTA(MIXED, NT);
-    // slots: A reads 0 and writes 1, B reads 1, C reads 1 and writes 0, D reads 0
-    constexpr int in = (PH == 5 || PH == 6) ? 1 : 0;
+    // slots: no phase writes the one that its own CTAs read.  1 reads 0 and writes 1,
+    // 2 reads 1, 3 reads 1 and writes 0; A reads 0 and writes 1, B reads 1, C reads 1
+    // and writes 0, D reads 0
+    constexpr int in = (PH == 2 || PH == 3 || PH == 5 || PH == 6) ? 1 : 0;
     if (c.tid == 0) sc = g.S->sc[in];
     __syncthreads();
     if (PH >= 4 && sc.done) {
@@ -763,7 +765,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_lsqr_phase(const PArgs<MIXED>
         if (c.warp == C::kSWarp) c.init_beta();
         c.chunks(C::kYWarp, c.first_chunk(C::kYWarp));
         __syncthreads();
-        if (c.bid == 0 && c.tid == 0) g.S->sc[0] = sc;
+        if (c.bid == 0 && c.tid == 0) g.S->sc[1] = sc;
     }
     if constexpr (PH == 2 || PH == 7) c.phase_d();
     if constexpr (PH == 3) {
