@@ -756,8 +756,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_lsqr_phase(const PArgs<MIXED>
     if (c.tid == 0) sc = g.S->sc[in];
     __syncthreads();
     if (PH >= 4 && sc.done) {
-        // A found the end and told slot 1; D and the next A read slot 0
-        if (PH == 6 && c.bid == 0 && c.tid == 0) g.S->sc[0] = sc;
+        // A found the end and told slot 1, D and the next A read slot 0; where the
+        // start found it (alpha beta = 0), slot 0 knows and B and C read slot 1
+        if ((PH == 4 || PH == 6) && c.bid == 0 && c.tid == 0) g.S->sc[PH == 4 ? 1 : 0] = sc;
         return;
     }
     if constexpr (PH == 0) c.init_u();
