@@ -61,6 +61,7 @@ constexpr int kTU = 8;                    // entries per lane per step (columns)
 constexpr int kChunkSteps = 2;
 constexpr unsigned kBarLimit = 1u << 23;  // polls before a grid barrier gives up
 constexpr int kItersPerLaunch = 256;
+constexpr int kNormParts = 152;
 
 // Scalars of the iteration: one copy per CTA in the persistent kernel, two
 // slots in memory otherwise (a phase kernel reads one and writes the other).
@@ -69,6 +70,7 @@ struct PScal {
     double ia, ib, coef_n, coef_t;         // 1/alpha, 1/beta, alpha/beta, beta/alpha
     double cs, sn, irho, t1, t2;
     double y_t1, y_t2, y_ia;               // the outstanding update of y and w
+    double bs;                             // the right-hand side's scale, a power of two
     long long it;
     int done, flag;
     int pend;              // a finished iteration's alpha scalars are outstanding
@@ -96,6 +98,7 @@ struct PArgs {
     unsigned* ccnt;           // finished chunks of a column with several
     const MT* Mr; const MT* Mc; int64_t ldm;
     const double* b;
+    const double* bpart;      // kNormParts partial sums of ||b||^2
     V* us; V* vs; V* z; V* t; V* tpart;
     double* w; double* y;
     V* pa; V* pb;
@@ -354,28 +357,24 @@ struct Cta {
         return a;
     }
 
-    // u = b, partial ||b||^2
-    SKL_DEV void init_u() const
-    {
-        Sum<MIXED> ss;
-        for (int i = bid * kPT + tid; i < g.n; i += G * kPT) {
-            const V x = store_val<MIXED>(g.b[i]);
-            g.us[i] = x;
-            if constexpr (MIXED) ss.add_sq(ff{x.x, x.y});
-            else ss.add_sq(x);
-        }
-        const V tot = ss.block(red);
-        if (tid == 0) g.pb[bid] = tot;
-    }
-    // beta_1 (one warp)
+    // beta_1 (one warp).  Mixed: the pairs hold b times a power of two that brings
+    // ||b|| to [1, 2), so that neither they nor A^T b leave the float range; y is
+    // scaled back at the end (k_lsqr_y).
     SKL_DEV void init_beta() const
     {
-        const double beta = sqrt(sum_partials(g.pb, G));
+        const double beta = sqrt(sum_partials(g.bpart, kNormParts));
         if (lane == 0) {
-            sc.beta = beta;
-            sc.ib = beta > 0.0 ? 1.0 / beta : 0.0;
+            const long long e = (__double_as_longlong(beta) >> 52) & 0x7ff;   // 1 .. 1534 for a sum that is finite
+            sc.bs = MIXED && beta > 0.0 && e < 0x7ff ? __longlong_as_double((2046 - e) << 52) : 1.0;
+            sc.beta = beta * sc.bs;
+            sc.ib = beta > 0.0 ? 1.0 / sc.beta : 0.0;
             sc.coef_t = 0.0;
         }
+    }
+    // u = b, once sc.bs is known to the CTA
+    SKL_DEV void init_u() const
+    {
+        for (int i = bid * kPT + tid; i < g.n; i += G * kPT) g.us[i] = store_val<MIXED>(g.b[i] * sc.bs);
     }
     // alpha_1 (one warp); w = v, y = 0 by the warp that updates them later
     SKL_DEV void init_alpha() const
@@ -705,9 +704,10 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_lsqr_persist(const PArgs<MIXE
     const int4 ch0 = c.first_chunk(C::kYWarp);
     const int2 row0 = c.first_row();
     if (start) {
+        if (c.warp == C::kSWarp) c.init_beta();
+        __syncthreads();
         c.init_u();
         if (!bar_all<CLUSTER>(S, gen)) return give_up();
-        if (c.warp == C::kSWarp) c.init_beta();
         c.chunks(C::kYWarp, ch0);
         if (!bar_all<CLUSTER>(S, gen)) return give_up();
         c.phase_d();
@@ -749,10 +749,10 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_lsqr_phase(const PArgs<MIXED>
 {
     pdl_wait();
     SKL_CTA(MIXED, NT);
-    // slots: no phase writes the one that its own CTAs read.  1 reads 0 and writes 1,
-    // 2 reads 1, 3 reads 1 and writes 0; A reads 0 and writes 1, B reads 1, C reads 1
-    // and writes 0, D reads 0
-    constexpr int in = (PH == 2 || PH == 3 || PH == 5 || PH == 6) ? 1 : 0;
+    // slots: no phase writes the one that its own CTAs read.  0 reads 0 and writes 1,
+    // 1 and 2 read 1, 3 reads 1 and writes 0; A reads 0 and writes 1, B reads 1, C
+    // reads 1 and writes 0, D reads 0
+    constexpr int in = (PH == 0 || PH == 4 || PH == 7) ? 0 : 1;
     if (c.tid == 0) sc = g.S->sc[in];
     __syncthreads();
     if (PH >= 4 && sc.done) {
@@ -761,13 +761,13 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_lsqr_phase(const PArgs<MIXED>
         if ((PH == 4 || PH == 6) && c.bid == 0 && c.tid == 0) g.S->sc[PH == 4 ? 1 : 0] = sc;
         return;
     }
-    if constexpr (PH == 0) c.init_u();
-    if constexpr (PH == 1) {
+    if constexpr (PH == 0) {
         if (c.warp == C::kSWarp) c.init_beta();
-        c.chunks(C::kYWarp, c.first_chunk(C::kYWarp));
         __syncthreads();
         if (c.bid == 0 && c.tid == 0) g.S->sc[1] = sc;
+        c.init_u();
     }
+    if constexpr (PH == 1) c.chunks(C::kYWarp, c.first_chunk(C::kYWarp));
     if constexpr (PH == 2 || PH == 7) c.phase_d();
     if constexpr (PH == 3) {
         if (c.warp == C::kYWarp) c.init_alpha();
@@ -1098,7 +1098,9 @@ k_lsqr_dense(const PArgs<true> g, const DArgs a, int start, int budget)
     };
     if (start) {
         // u = b through the pass itself: u = 0 - (-1) u
-        for (int i = c.bid * kDT + tid; i < g.n; i += c.G * kDT) g.us[i] = store_val<true>(g.b[i]);
+        if (warp == C::kSWarp) c.init_beta();
+        __syncthreads();
+        c.init_u();
         if (tid == 0) {
             sc.ia = 0.0;
             sc.coef_n = -1.0;
@@ -1106,7 +1108,6 @@ k_lsqr_dense(const PArgs<true> g, const DArgs a, int start, int budget)
         if (!bar_all<false>(S, gen)) return give_up();
         if (!pass()) return give_up();
         if (!bar_all<false>(S, gen)) return give_up();
-        if (warp == C::kSWarp) c.init_beta();
         reduce();
         if (!bar_all<false>(S, gen)) return give_up();
         phase_d();
@@ -1218,6 +1219,38 @@ k_split_tiles(const double* __restrict__ A, int64_t lda, int n, int d, int K, in
     if (threadIdx.x == 0) fro[blockIdx.x] = make_float2(t.hi, t.lo);
 }
 
+// ---- start and end -------------------------------------------------------------
+// kNormParts partial sums of ||b||^2, FP64 as b is: squares of pairs leave the
+// float range where ||b|| is below 1e-19 or above 1e19.  3 us of a solve.
+__global__ void __launch_bounds__(256) k_lsqr_norm(const double* __restrict__ b, int64_t n, double* __restrict__ part)
+{
+    pdl_wait();
+    __shared__ double red[8];
+    double s = 0.0;
+    for (int64_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += kNormParts * 256) s = fma(b[i], b[i], s);
+    s = block_sum(s, red);
+    if (threadIdx.x == 0) part[blockIdx.x] = s;
+}
+
+// y for the caller: the scale of b taken out
+__global__ void k_lsqr_y(const double* __restrict__ y, int r, const PState* __restrict__ S, double* __restrict__ out)
+{
+    pdl_wait();
+    const double inv = 1.0 / S->sc[0].bs;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < r; i += gridDim.x * blockDim.x) out[i] = y[i] * inv;
+}
+
+void norm_launch(const double* b, int64_t n, double* part, cudaStream_t st)
+{
+    launch_k(k_lsqr_norm, kNormParts, 256, 0, st, b, n, part);
+    SKL_LAUNCHED();
+}
+void y_launch(const double* y, int64_t r, const PState* S, double* out, cudaStream_t st)
+{
+    launch_k(k_lsqr_y, (unsigned)std::min<int64_t>((r + 255) / 256, 152), 256, 0, st, y, (int)r, S, out);
+    SKL_LAUNCHED();
+}
+
 // ---- column chunks -------------------------------------------------------------
 __global__ void k_chunk_count(const int* __restrict__ cp, const int* __restrict__ cols, int r, int len,
                               int* __restrict__ cnt)
@@ -1260,7 +1293,7 @@ int lanes_col(double avg) { return avg >= 128 ? 32 : avg >= 64 ? 16 : avg >= 24 
 struct PBufs {
     PState* S;
     void *us, *vs, *z, *t, *tpart;
-    double *w, *y, *pa, *pb;
+    double *w, *y, *pa, *pb, *bpart;
     int4* chunks; int* coff; int* scan; int* cnt; unsigned* ccnt;
     size_t bytes;
 };
@@ -1288,6 +1321,7 @@ PBufs pcarve(const LsqrProblem& P, void* work)
     B.y = (double*)take(P.r * sizeof(double));
     B.pa = (double*)take(1024 * sizeof(double));
     B.pb = (double*)take(1024 * sizeof(double));
+    B.bpart = (double*)take(kNormParts * sizeof(double));
     B.chunks = (int4*)take(nch * sizeof(int4));
     B.ccnt = (unsigned*)take(P.r * sizeof(unsigned));
     B.coff = (int*)take((P.r + 1) * sizeof(int));
@@ -1523,6 +1557,7 @@ LsqrResult persist_impl(const LsqrProblem& P, const double* b, double tol, int64
     g.y = B.y;
     g.pa = (V*)B.pa;
     g.pb = (V*)B.pb;
+    g.bpart = B.bpart;
     g.S = B.S;
     const int G = grid_of(P).ctas;
     // segments per row of the triangle: one round of the 15 (31) warps where the
@@ -1543,6 +1578,7 @@ LsqrResult persist_impl(const LsqrProblem& P, const double* b, double tol, int64
     init.tol = tol;
     init.max_it = max_it;
     SKL_CUDA(cudaMemcpyAsync(B.S, &init, sizeof(PState), cudaMemcpyHostToDevice, st));
+    norm_launch(b, P.n, B.bpart, st);
     trace_phase(st, "lsqr: init");
     const size_t smem = vec_smem(P);
     LsqrResult res;
@@ -1553,7 +1589,7 @@ LsqrResult persist_impl(const LsqrProblem& P, const double* b, double tol, int64
     trace_phase(st, "lsqr: done");
     res.flag = hs->sc[0].flag;
     res.it = hs->sc[0].it;
-    SKL_CUDA(cudaMemcpyAsync(y_out, B.y, P.r * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    y_launch(B.y, P.r, B.S, y_out, st);
     return res;
 }
 
@@ -1588,7 +1624,7 @@ int dense_ctas(const LsqrProblem& P)
 struct DBufs {
     PState* S;
     float2 *us, *vs, *z, *part, *tn, *pa, *pb;
-    double *w, *y;
+    double *w, *y, *bpart;
     long long* prof;
     size_t bytes;
 };
@@ -1612,6 +1648,7 @@ DBufs dcarve(const LsqrProblem& P, void* work)
     B.pb = (float2*)take(1024 * sizeof(float2));
     B.w = (double*)take(P.r * sizeof(double));
     B.y = (double*)take(P.r * sizeof(double));
+    B.bpart = (double*)take(kNormParts * sizeof(double));
     B.prof = (long long*)take(4 * sizeof(long long));
     B.bytes = off;
     return B;
@@ -1648,6 +1685,7 @@ LsqrResult dense_impl(const LsqrProblem& P, const double* b, double tol, int64_t
     g.y = B.y;
     g.pa = B.pa;
     g.pb = B.pb;
+    g.bpart = B.bpart;
     g.S = B.S;
     const int G = dense_ctas(P);
     const int nloc = (int)((P.r + G - 1) / G), nw = kDT / 32 - 1;
@@ -1673,6 +1711,7 @@ LsqrResult dense_impl(const LsqrProblem& P, const double* b, double tol, int64_t
     init.tol = tol;
     init.max_it = max_it;
     SKL_CUDA(cudaMemcpyAsync(B.S, &init, sizeof(PState), cudaMemcpyHostToDevice, st));
+    norm_launch(b, P.n, B.bpart, st);
     trace_phase(st, "lsqr: init");
     const PState* hs = run_cooperative(fn, false, G, kDT, (size_t)a.sv_bytes + (size_t)a.nslots * s.CW * 16, B.S, host_pinned,
                                        st, (void*)&g, (void*)&a);
@@ -1692,7 +1731,7 @@ LsqrResult dense_impl(const LsqrProblem& P, const double* b, double tol, int64_t
             res.prof_launches[q] = q == 1 ? 0 : res.it;
         }
     }
-    SKL_CUDA(cudaMemcpyAsync(y_out, B.y, P.r * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    y_launch(B.y, P.r, B.S, y_out, st);
     return res;
 }
 
