@@ -850,32 +850,52 @@ void dht_hash_rhs(const double* b, int64_t n, const double* D, int64_t N, const 
     SKL_LAUNCHED();
 }
 
-// Per-block partial sums of squares of a dense column-major matrix (512
-// blocks): FP32 sums per thread, FP64 per block -- ||A||_F only normalises the
-// reported backward error.
-__global__ void k_fro_partial(const double* __restrict__ A, int64_t lda, int64_t n, int64_t d,
-                              double* __restrict__ out)
+// kFroParts partial sums of squares of a dense column-major matrix, in FP64: its
+// entries may be as small or large as FP64 holds squares of.
+__global__ void __launch_bounds__(256)
+k_fro_partial(const double* __restrict__ A, int64_t lda, int64_t n, int64_t d, double* __restrict__ out)
 {
     pdl_wait();
-    __shared__ double red[32];
+    __shared__ double red[8];
     double acc = 0.0;
-    for (int64_t j = blockIdx.x; j < d; j += gridDim.x) {
-        float s = 0.f;
-        for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-            float v = (float)A[i + j * lda];
-            s = fmaf(v, v, s);
+    for (int64_t j = blockIdx.x; j < d; j += gridDim.x)
+#pragma unroll 4
+        for (int64_t i = threadIdx.x; i < n; i += 256) {
+            const double v = A[i + j * lda];
+            acc = fma(v, v, acc);
         }
-        acc += (double)s;
-    }
     acc = block_sum(acc, red);
     if (threadIdx.x == 0) out[blockIdx.x] = acc;
 }
 
-void fro_partials(const double* A, int64_t lda, int64_t n, int64_t d, double* out512,
-                  cudaStream_t st)
+void fro_partials(const double* A, int64_t lda, int64_t n, int64_t d, double* out, cudaStream_t st)
 {
-    SKL_CUDA(cudaMemsetAsync(out512, 0, 512 * sizeof(double), st));
-    launch_k(k_fro_partial, 512, 256, 0, st, A, lda, n, d, out512);
+    launch_k(k_fro_partial, kFroParts, 256, 0, st, A, lda, n, d, out);
+    SKL_LAUNCHED();
+}
+
+// kStatusRange where a column that is not zero has a sum of squares outside
+// [2^-120, 2^126].
+__global__ void __launch_bounds__(256)
+k_column_range(const float* __restrict__ X, int64_t ld, int m, unsigned* __restrict__ status)
+{
+    pdl_wait();
+    __shared__ float red[8];
+    const float* x = X + blockIdx.x * ld;
+    float s = 0.f;
+    bool any = false;
+    for (int i = threadIdx.x; i < m; i += 256) {
+        s = fmaf(x[i], x[i], s);
+        any |= x[i] != 0.f;
+    }
+    s = block_sum(s, red);
+    any = __syncthreads_or(any);
+    if (threadIdx.x == 0 && any && !(s >= 0x1p-120f && s <= 0x1p126f)) atomicOr(status, kStatusRange);
+}
+
+void check_column_range(const float* X, int64_t ld, int64_t m, int64_t d, unsigned* status, cudaStream_t st)
+{
+    launch_k(k_column_range, (unsigned)d, 256, 0, st, X, ld, (int)m, status);
     SKL_LAUNCHED();
 }
 

@@ -1151,7 +1151,9 @@ k_lsqr_dense(const PArgs<true> g, const DArgs a, int start, int budget)
 
 // A (FP64, column-major) to the tile storage, with the range check of the mixed
 // path and ||A||_F^2 partials.  FP64 arithmetic on every element would hold the
-// FP64 pipe for ~2 ms at 40,000 x 4,000: hi and lo are cut from the bits.
+// FP64 pipe for ~2 ms at 40,000 x 4,000: hi and lo are cut from the bits, and the
+// squares are summed in float pairs, in three sums, so that none of the admitted
+// values' squares leaves the float range.
 constexpr int kSplitRows = 64, kSplitCols = 32;
 
 // hi = x rounded to 24 bits, lo = the rest rounded to 24: as ff_from_double for
@@ -1174,12 +1176,12 @@ SKL_DEV ff ff_from_bits(double x)
 
 __global__ void __launch_bounds__(256)
 k_split_tiles(const double* __restrict__ A, int64_t lda, int n, int d, int K, int CW, int64_t blocks,
-              float4* __restrict__ out, float2* __restrict__ fro, unsigned* __restrict__ status)
+              float4* __restrict__ out, double* __restrict__ fro, unsigned* __restrict__ status)
 {
     pdl_wait();
     __shared__ float2 tile[kSplitCols][kSplitRows + 1];
     __shared__ ff red[8];
-    ff ss{0.f, 0.f};
+    ff ss{0.f, 0.f}, big{0.f, 0.f}, small{0.f, 0.f};   // of x, of x 2^-60, of x 2^60
     bool bad = false;
     const int64_t rtiles = (blocks * 2 + kSplitRows - 1) / kSplitRows;
     const int ctiles = (K * CW + kSplitCols - 1) / kSplitCols;
@@ -1199,7 +1201,16 @@ k_split_tiles(const double* __restrict__ A, int64_t lda, int n, int d, int K, in
             // |x| > 2^100 or 0 < |x| < 2^-100 (a NaN is neither)
             bad |= (m > 0x4630000000000000ull && m <= 0x7ff0000000000000ull) || (m != 0 && m < 0x39b0000000000000ull);
             const ff f = ff_from_bits(x[q]);
-            ff_fma(ss, f, f);
+            const float mag = fabsf(f.hi);
+            if (mag <= 0x1p40f && mag >= 0x1p-40f) {
+                ff_fma(ss, f, f);
+            } else if (mag > 1.f) {
+                const ff g{f.hi * 0x1p-60f, f.lo * 0x1p-60f};
+                ff_fma(big, g, g);
+            } else if (mag > 0.f) {
+                const ff g{f.hi * 0x1p60f, f.lo * 0x1p60f};
+                ff_fma(small, g, g);
+            }
             tile[j][i] = make_float2(f.hi, f.lo);
         }
         __syncthreads();
@@ -1215,8 +1226,9 @@ k_split_tiles(const double* __restrict__ A, int64_t lda, int n, int d, int K, in
         __syncthreads();
     }
     if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(status, kStatusRange);
-    const ff t = block_sum_ff(ss, red);
-    if (threadIdx.x == 0) fro[blockIdx.x] = make_float2(t.hi, t.lo);
+    const double t = ff_to_double(block_sum_ff(ss, red)) + ff_to_double(block_sum_ff(big, red)) * 0x1p120 +
+                     ff_to_double(block_sum_ff(small, red)) * 0x1p-120;
+    if (threadIdx.x == 0) fro[blockIdx.x] = t;
 }
 
 // ---- start and end -------------------------------------------------------------
@@ -1740,7 +1752,7 @@ LsqrResult dense_impl(const LsqrProblem& P, const double* b, double tol, int64_t
 bool lsqr_dense_tiled(int64_t d, int precision) { return precision == SKL_PREC_MIXED && d >= 1 && d <= kDenseMaxD; }
 size_t lsqr_dense_tile_bytes(int64_t n, int64_t d) { return dense_shape(n, d).bytes(); }
 
-void split_dense_tiles(const double* A, int64_t lda, int64_t n, int64_t d, void* out, float2* fro, unsigned* status,
+void split_dense_tiles(const double* A, int64_t lda, int64_t n, int64_t d, void* out, double* fro, unsigned* status,
                        cudaStream_t st)
 {
     const DenseShape s = dense_shape(n, d);

@@ -995,7 +995,7 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
     SKL_CUDA(cudaEventRecord(ev[1], st));
     if (mixed) {
         SKL_CUDA(cudaMemsetAsync(C.dev_status, 0, sizeof(unsigned), st));
-        if (tiled) split_dense_tiles(A, lda, n, d, A2, (float2*)part, C.dev_status, st);
+        if (tiled) split_dense_tiles(A, lda, n, d, A2, part, C.dev_status, st);
         else split_dense(A, lda, n, d, A2, C.dev_status, st);
     }
     {
@@ -1005,11 +1005,12 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
     }
     if (mixed && (read_status(C, st) & kStatusRange)) return false;
     double fro = 0.0;   // ||A||_F
-    if (tiled) {
-        std::vector<float2> fp((size_t)kFroParts);
-        SKL_CUDA(cudaMemcpyAsync(fp.data(), part, kFroParts * sizeof(float2), cudaMemcpyDeviceToHost, st));
+    {
+        if (!tiled) fro_partials(A, lda, n, d, part, st);
+        std::vector<double> fp((size_t)kFroParts);
+        SKL_CUDA(cudaMemcpyAsync(fp.data(), part, kFroParts * sizeof(double), cudaMemcpyDeviceToHost, st));
         SKL_CUDA(cudaStreamSynchronize(st));
-        for (float2 v : fp) fro += (double)v.x + (double)v.y;
+        for (double v : fp) fro += v;
         fro = std::sqrt(fro);
     }
     if (host_thread->joinable()) host_thread->join();
@@ -1029,9 +1030,15 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
     if (cpqr_on) dht_hash_rhs(b, n, Dd, N, bptr, bent, (int)k, m, cvec, work, work_bytes, st);
     trace_phase(st, "dense sketch");
     SKL_CUDA(cudaEventRecord(ev[3], st));
+    SKL_CUDA(cudaMemsetAsync(C.dev_status, 0, sizeof(unsigned), st));
+    // A as a whole so large or small that squares of the sketch leave the float range:
+    // FP64 (a small column of an ordinary A stays, as the rank rule's business)
+    if (mixed && (fro >= 0x1p60 || (fro > 0.0 && fro < 0x1p-50))) {
+        check_column_range((const float*)SA, ld, m, d, C.dev_status, st);
+        if (read_status(C, st) & kStatusRange) return false;
+    }
     // ---- factorization: Cholesky of a well-conditioned sketch's Gram matrix,
     // else QR (pivoted for the CPQR path) ----
-    SKL_CUDA(cudaMemsetAsync(C.dev_status, 0, sizeof(unsigned), st));
     // the reference's absolute rank rule (:79-89), floored at the working precision's
     // resolution of the sketch (FP32 cannot resolve |R_ii| below eps*|R_00|);
     // noCPQR keeps all columns, by the QR where that resolution is reached
@@ -1078,14 +1085,6 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
     P.Ad64 = A; P.lda64 = lda;
     P.cols = jpvt; P.colscale = colscale;
     P.M = Mc; P.Mrow = Mr; P.ldm = ldm; P.r = rank; P.precision = o.precision;
-    if (!tiled) {
-        fro_partials(A, lda, n, d, part, st);
-        std::vector<double> fp(512);
-        SKL_CUDA(cudaMemcpyAsync(fp.data(), part, 512 * sizeof(double), cudaMemcpyDeviceToHost, st));
-        SKL_CUDA(cudaStreamSynchronize(st));
-        for (double v : fp) fro += v;
-        fro = std::sqrt(fro);
-    }
     double rnorm = 0.0, be = 0.0;
     auto residual = [&]() {
         residual_and_backward(P, x_dev, b, rs, part, scal, st);

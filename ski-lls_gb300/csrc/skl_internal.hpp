@@ -146,8 +146,12 @@ void dht_hash(const double* A, int64_t lda, int64_t n, int64_t d, const double* 
 void dht_hash_rhs(const double* b, int64_t n, const double* D, int64_t N, const int* bptr,
                   const unsigned* bent, int k, int64_t m, double* Sb, void* scratch,
                   size_t scratch_bytes, cudaStream_t st);
-void fro_partials(const double* A, int64_t lda, int64_t n, int64_t d, double* out512,
-                  cudaStream_t st);
+// kFroParts partial sums of ||A||_F^2
+constexpr int kFroParts = 152 * 3;
+void fro_partials(const double* A, int64_t lda, int64_t n, int64_t d, double* out, cudaStream_t st);
+// kStatusRange in *status where a nonzero column of the FP32 sketch has a sum of
+// squares outside [2^-120, 2^126]
+void check_column_range(const float* X, int64_t ld, int64_t m, int64_t d, unsigned* status, cudaStream_t st);
 
 // -------------------------------------------------------------- k_qr.cu --
 template <typename T>
@@ -302,10 +306,9 @@ LsqrResult lsqr_persist_run(const LsqrProblem& P, const double* b, double tol, i
 // Tile storage of a dense A for the one-pass products: whether the problem takes
 // it, its bytes, and its build from A (FP64, column-major), with the range check
 // (kStatusRange) and kFroParts partial sums of ||A||_F^2.
-constexpr int kFroParts = 152 * 3;
 bool lsqr_dense_tiled(int64_t d, int precision);
 size_t lsqr_dense_tile_bytes(int64_t n, int64_t d);
-void split_dense_tiles(const double* A, int64_t lda, int64_t n, int64_t d, void* out, float2* fro, unsigned* status,
+void split_dense_tiles(const double* A, int64_t lda, int64_t n, int64_t d, void* out, double* fro, unsigned* status,
                        cudaStream_t st);
 // One product in isolation with LSQR's storage and arithmetic: y = A x
 // (trans 'n', CSR kernel) or y = A^T x ('t', CSC kernel, P.cols = 0..d-1,
