@@ -100,8 +100,9 @@ struct PArgs {
     const double* b;
     const double* bpart;      // kNormParts partial sums of ||b||^2
     V* us; V* vs; V* z; V* t; V* tpart;
+    double* vh;               // v in FP64; vs holds its pairs (FP64 path: vh itself)
     double* w; double* y;
-    V* pa; V* pb;
+    double* pa; double* pb;   // partials of ||v||^2, ||u||^2
     PState* S;
 };
 
@@ -133,44 +134,39 @@ SKL_DEV bool bar_all(PState* S, unsigned& gen)
     }
 }
 
-// Sums of squares: float-float on the mixed path.  GB300 issues two FP64 FMAs
-// per SM and cycle, so one FP64 instruction of a warp holds the pipe for 16
-// cycles whatever its active lanes: an epilogue of ten of them in each of 32
-// warps is 2.7 us, and the mixed path's vector updates and norms therefore run
-// in float-float too; FP64 is left to the scalars of one lane and to y and w.
+// Sum of ||u||^2.  GB300 issues two FP64 FMAs per SM and cycle, so one FP64
+// instruction of a warp holds the pipe for 16 cycles whatever its active lanes: an
+// epilogue of ten of them in each of 32 warps is 2.7 us.  The mixed path's u of a
+// sparse problem is a float pair, and its squares are summed in pairs up to the warp,
+// FP64 from there (the warps' 2^-48 average out over a few thousand of them).  What
+// has one value per row of the triangle or of a tile (v, the dense u and their
+// norms, y, w) is FP64 altogether: one or two warps of a CTA hold it.
 template <bool MIXED>
 struct Sum {
     ff a{0.f, 0.f};
     SKL_DEV void add_sq(ff x) { ff_fma(a, x, x); }
-    // the CTA's sum, in thread 0; red is free again after the next barrier
-    SKL_DEV float2 block(ff* red) const
-    {
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        const ff w = warp_sum_ff(a);
-        if (lane == 0) red[warp] = w;
-        __syncthreads();
-        ff t{0.f, 0.f};
-        if (warp == 0) t = warp_sum_ff(lane < (int)(blockDim.x >> 5) ? red[lane] : t);
-        return make_float2(t.hi, t.lo);
-    }
+    SKL_DEV double warp() const { return ff_to_double(warp_sum_ff(a)); }
 };
 template <>
 struct Sum<false> {
     double a = 0.0;
     SKL_DEV void add_sq(double x) { a = fma(x, x, a); }
-    SKL_DEV double block(double* red) const { return block_sum(a, red); }
+    SKL_DEV double warp() const { return warp_sum(a); }
 };
 
-// Fixed-order sum of the CTAs' partials (one warp; every lane gets it).
-SKL_DEV double sum_partials(const float2* p, int np)
+// The first nw warps' sums added up in thread 0; red is free again after the next
+// barrier
+SKL_DEV double sum_warps(double w, int nw, double* red)
 {
-    ff s{0.f, 0.f};
-    for (int i = threadIdx.x & 31; i < np; i += 32) {
-        const float2 v = __ldcg(p + i);
-        ff_add(s, v.x, v.y);
-    }
-    return ff_to_double(warp_sum_ff(s));
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0 && warp < nw) red[warp] = w;
+    __syncthreads();
+    double t = 0.0;
+    if (warp == 0) t = warp_sum(lane < nw ? red[lane] : 0.0);
+    return t;
 }
+
+// Fixed-order sum of the CTAs' partials (one warp; every lane gets it).
 SKL_DEV double sum_partials(const double* p, int np)
 {
     double s = 0.0;
@@ -180,8 +176,6 @@ SKL_DEV double sum_partials(const double* p, int np)
 
 SKL_DEV float2 acc_store(const Acc<true>& a) { return make_float2(a.a.hi, a.a.lo); }
 SKL_DEV double acc_store(const Acc<false>& a) { return a.a; }
-SKL_DEV double val64(float2 v) { return (double)v.x + (double)v.y; }
-SKL_DEV double val64(double v) { return v; }
 SKL_DEV void acc_load(Acc<true>& a, float2 v) { a.a = ff{v.x, v.y}; }
 SKL_DEV void acc_load(Acc<false>& a, double v) { a.a = v; }
 
@@ -202,13 +196,12 @@ SKL_DEV void sqrt_rcp(double x, double& s, double& r)
 }
 
 // s * dot - c * old, with s and c split once per phase by one thread: the FP64
-// conversions of a whole CTA's warps took ~1,500 to 3,000 cycles of phases B and D
+// conversions of a whole CTA's warps took ~3,000 cycles of phase B
 struct ScaleF {
     ff s, c;
     SKL_DEV ScaleF(double s64, double c64) : s(ff_from_double(s64)), c(ff_from_double(-c64)) {}
     SKL_DEV explicit ScaleF(float4 v) : s{v.x, v.y}, c{v.z, v.w} {}
     SKL_DEV float4 pack() const { return make_float4(s.hi, s.lo, c.hi, c.lo); }
-    SKL_DEV bool pos() const { return s.hi > 0.f; }
     SKL_DEV ff operator()(const Acc<true>& dot, float2 old) const
     {
         ff v{0.f, 0.f};
@@ -220,11 +213,9 @@ struct ScaleF {
 struct ScaleD {
     double s, c;
     SKL_DEV ScaleD(double s64, double c64) : s(s64), c(c64) {}
-    SKL_DEV bool pos() const { return s > 0.0; }
     SKL_DEV double operator()(const Acc<false>& dot, double old) const { return dot.a * s - c * old; }
 };
 template <bool MIXED> using Scale = typename std::conditional<MIXED, ScaleF, ScaleD>::type;
-template <bool MIXED> using RedT = typename std::conditional<MIXED, ff, double>::type;
 SKL_DEV float2 to_v(ff x) { return make_float2(x.hi, x.lo); }
 SKL_DEV double to_v(double x) { return x; }
 
@@ -305,7 +296,7 @@ struct Cta {
     PScal& sc;              // shared memory
     V* sv;                  // staged vector, max(r, d) entries
     V* s_unit;              // kMaxUnits segment sums
-    RedT<MIXED>* red;
+    double* red;
     float4* scale;          // the phase's scales
     int tid, lane, warp, G, bid, nloc;
 
@@ -397,7 +388,7 @@ struct Cta {
     SKL_DEV void init_yw() const
     {
         for (int i = bid * 32 + lane; i < g.r; i += G * 32) {
-            g.w[i] = val64(ld_cg(g.vs + i)) * sc.ia;
+            g.w[i] = __ldcg(g.vh + i) * sc.ia;
             g.y[i] = 0.0;
         }
     }
@@ -406,7 +397,7 @@ struct Cta {
     {
         const double t1 = sc.y_t1, t2 = sc.y_t2, ia = sc.y_ia;
         for (int i = bid * 32 + lane; i < g.r; i += G * 32) {
-            const double v = ia != 0.0 ? val64(ld_cg(g.vs + i)) * ia : 0.0;
+            const double v = ia != 0.0 ? __ldcg(g.vh + i) * ia : 0.0;
             const double wi = g.w[i];
             g.y[i] += t1 * wi;
             g.w[i] = t2 * wi + v;
@@ -534,7 +525,7 @@ struct Cta {
                 aa[k] = na[k];
             }
         }
-        const V tot = ss.block(red);
+        const double tot = sum_warps(ss.warp(), kPW, red);
         if (tid == 0) g.pb[bid] = tot;
     }
 
@@ -648,7 +639,6 @@ struct Cta {
     // ---- D: v = M^T t / beta - (beta / alpha) v; partial ||v||^2
     SKL_DEV void phase_d() const
     {
-        if (tid == kPT - 1) put_scale(sc.ib, sc.coef_t);
         for (int i = tid; i < g.r; i += kPT) sv[i] = ld_cg(g.t + i);
         tri_finish();
     }
@@ -657,23 +647,29 @@ struct Cta {
         const bool has_old = (__double_as_longlong(sc.coef_t) << 1) != 0;   // coef_t != 0
         // this thread's first entry of v, on its way beside the products
         const int j0 = tid < nloc ? tri_row(tid, false) : -1;
-        V old0{};
-        if (j0 >= 0 && has_old) old0 = g.vs[j0];
+        double old0 = 0.0;
+        if (j0 >= 0 && has_old) old0 = g.vh[j0];
         __syncthreads();
         tri_units(g.Mc, false, kPW);
         __syncthreads();
-        Sum<MIXED> ss;
-        const Scale<MIXED> sc2 = get_scale(sc.ib, sc.coef_t);
+        const double ib = sc.ib, coef = sc.coef_t;
+        double ss = 0.0;
         for (int k = tid; k < nloc; k += kPT) {
             const int j = tri_row(k, false);
             if (j < 0) continue;
-            V old = old0;
-            if (k != tid) old = has_old ? g.vs[j] : V{};
-            const auto nv = sc2(tri_sum(k), old);
-            if (sc2.pos()) g.vs[j] = to_v(nv);   // v stays when beta = 0 (IterSolver.cpp:242)
-            ss.add_sq(nv);
+            double old = old0;
+            if (k != tid) old = has_old ? g.vh[j] : 0.0;
+            const double nv = fma(-coef, old, tri_sum(k).value() * ib);
+            if (ib > 0.0) {   // v stays when beta = 0 (IterSolver.cpp:242)
+                g.vh[j] = nv;
+                if constexpr (MIXED) g.vs[j] = store_val<true>(nv);
+            }
+            ss = fma(nv, nv, ss);
         }
-        const V tot = ss.block(red);
+        // only the warps that own rows hold a sum
+        const int nw = min(kPW, (nloc + 31) / 32);
+        if (warp < nw) ss = warp_sum(ss);
+        const double tot = sum_warps(ss, nw, red);
         if (tid == 0) g.pa[bid] = tot;
     }
 };
@@ -682,7 +678,7 @@ struct Cta {
     extern __shared__ __align__(16) unsigned char smem_raw[];                                            \
     __shared__ PScal sc;                                                                                 \
     __shared__ ValT<MIXED> s_unit[kMaxUnits];                                                            \
-    __shared__ RedT<MIXED> red[NT / 32];                                                                 \
+    __shared__ double red[NT / 32];                                                                      \
     __shared__ __align__(16) float4 s_phase_scale;                                                       \
     using C = Cta<MIXED, NT>;                                                                            \
     const C c{g, sc, reinterpret_cast<ValT<MIXED>*>(smem_raw), s_unit, red, &s_phase_scale, (int)threadIdx.x,   \
@@ -795,9 +791,11 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_lsqr_phase(const PArgs<MIXED>
 // row: here a CTA holds a few whole rows (a tile) in shared memory, forms their
 // u, and adds u times the tile to its share of A^T u, so that an iteration reads A
 // once (40,000 x 4,000: 463 us per iteration with the two products as kernels of
-// their own at 0.95 of HBM, 340 here, 264 of it the pass; the pass is bound by the
-// float-float arithmetic, ~26 FP32 instructions per entry, and by the sums over
-// the CTA between two of its barriers).  Tried: packed f32x2 arithmetic (487 us: it
+// their own at 0.95 of HBM, 360 here; the pass is bound by the float-float
+// arithmetic, ~26 FP32 instructions per entry, and by the sums over the CTA between
+// two of its barriers).  u and its norm are FP64, formed by one warp between the
+// barriers, and A^T u is summed four rows at a time: 340 us with pairs and one chain,
+// which left x 25 % further off.  Tried: packed f32x2 arithmetic (487 us: it
 // issues at a quarter of the scalar rate), a tile ring read twice from shared
 // memory with the sums on a warp of their own (440 us), two CTAs of 256 threads per
 // SM (380 us).
@@ -818,6 +816,7 @@ constexpr int kDenseMaxD = 8 * kDT;
 
 struct DArgs {
     const float4* A;          // tiles
+    double* uh;               // u
     float2* part;             // [G][K * CW] shares of A^T u
     float2* tn;               // A^T u, natural column order
     int CW, ntiles, nslots;
@@ -836,6 +835,12 @@ SKL_DEV void ff_fma_lazy(ff& acc, float ah, float al, ff x)
     two_sum(acc.hi, p, s, e);
     acc.hi = s;
     acc.lo = __fadd_rn(acc.lo, __fadd_rn(e, pl));
+}
+// a x, unnormalised
+SKL_DEV ff ff_mul_lazy(float ah, float al, ff x)
+{
+    const float p = __fmul_rn(ah, x.hi);
+    return {p, __fmaf_rn(ah, x.lo, __fmaf_rn(al, x.hi, __fmaf_rn(ah, x.hi, -p)))};
 }
 SKL_DEV void ff_norm(ff& a)
 {
@@ -886,7 +891,6 @@ k_lsqr_dense(const PArgs<true> g, const DArgs a, int start, int budget)
     __shared__ __align__(8) uint64_t bars[kMaxSlots];
     __shared__ float2 s_part[kW][NV];
     __shared__ __align__(16) float4 s_u[RB];
-    __shared__ __align__(16) float4 s_scale;
     __shared__ float2 s_red[C::kYWarp][32];
     PState* S = g.S;
     const int tid = c.tid, lane = c.lane, warp = c.warp;
@@ -958,17 +962,11 @@ k_lsqr_dense(const PArgs<true> g, const DArgs a, int start, int budget)
             zs[k * kDT + tid] = zz;
             t[k] = ff{0.f, 0.f};
         }
-        // the scales as float pairs in shared memory: kept in registers they were
-        // formed again from FP64 in every tile (~2,500 cycles of it between two
-        // barriers)
-        if (tid == 0) s_scale = ScaleF(sc.ia, sc.coef_n).pack();
-        __syncthreads();
-        Sum<true> ss;
-        // finishing threads: value fv, share fw of the warps; fw = 0 writes u
-        const int fv = tid / kW, fw = tid % kW;
-        const bool fin = fv < NV && fw == 0;
-        float2 un = make_float2(0.f, 0.f);   // the next tile's old u
-        if (fin && c.bid * NV + fv < g.n) un = g.us[c.bid * NV + fv];
+        double ss = 0.0;
+        // warp 0 finishes the tile's rows: lane l row l % NV, and lanes below NV write u
+        const bool fin = tid < NV;
+        double un = 0.0;                     // the next tile's old u
+        if (fin && c.bid * NV + tid < g.n) un = a.uh[c.bid * NV + tid];
         for (int it = 0; it < mine; ++it) {
             // each warp waits for the tile's chunks with one lane per chunk
             bool ok = true;
@@ -997,10 +995,10 @@ k_lsqr_dense(const PArgs<true> g, const DArgs a, int start, int budget)
                 slot0 -= NS;
                 par0 ^= 1u;
             }
-            const int row = (c.bid + it * c.G) * NV + fv;
-            const float2 uo = un;
-            un = make_float2(0.f, 0.f);
-            if (fin && it + 1 < mine && row + c.G * NV < g.n) un = g.us[row + c.G * NV];
+            const int row = (c.bid + it * c.G) * NV + tid;
+            const double uc = -sc.coef_n * un;   // off the chain below
+            un = 0.0;
+            if (fin && it + 1 < mine && row + c.G * NV < g.n) un = a.uh[row + c.G * NV];
             ff v[NV];
 #pragma unroll
             for (int q = 0; q < NV; ++q) v[q] = ff{0.f, 0.f};
@@ -1019,42 +1017,63 @@ k_lsqr_dense(const PArgs<true> g, const DArgs a, int start, int budget)
             const ff s = warp_sum_n<NV>(v, lane);
             if (lane % (32 / NV) == 0) s_part[warp][lane / (32 / NV)] = make_float2(s.hi, s.lo);
             __syncthreads();
-            if (tid < NV * kW) {
-                const float2 p = s_part[fw][fv];
-                ff r{p.x, p.y};
+            if (warp == 0) {
+                // 32 / NV lanes share a row's warps
+                constexpr int kPer = kW * NV / 32;
+                ff r[kPer];
 #pragma unroll
-                for (int o = kW / 2; o > 0; o >>= 1) ff_add(r, ff_shfl_xor(r, o));
+                for (int w = 0; w < kPer; ++w) {
+                    const float2 p = s_part[(lane / NV) * kPer + w][lane % NV];
+                    r[w] = ff{p.x, p.y};
+                }
+#pragma unroll
+                for (int h = kPer / 2; h > 0; h >>= 1)
+#pragma unroll
+                    for (int w = 0; w < h; ++w) ff_add(r[w], r[w + h]);
+#pragma unroll
+                for (int o = 16; o >= NV; o >>= 1) ff_add(r[0], ff_shfl_xor(r[0], o));
                 if (fin) {
-                    Acc<true> d;
-                    d.a = r;
-                    const volatile float4& vs = s_scale;
-                    const ff nv = ScaleF(make_float4(vs.x, vs.y, vs.z, vs.w))(d, uo);
-                    float* su = reinterpret_cast<float*>(&s_u[fv >> 1]);
-                    su[fv & 1] = nv.hi;
-                    su[2 + (fv & 1)] = nv.lo;
+                    const double nv = fma((double)r[0].lo, sc.ia, fma((double)r[0].hi, sc.ia, uc));
+                    const float2 nf = store_val<true>(nv);
+                    float* su = reinterpret_cast<float*>(&s_u[lane >> 1]);
+                    su[lane & 1] = nf.x;
+                    su[2 + (lane & 1)] = nf.y;
                     if (row < g.n) {
-                        g.us[row] = to_v(nv);
-                        ss.add_sq(nv);
+                        a.uh[row] = nv;
+                        ss = fma(nv, nv, ss);
                     }
                 }
             }
             __syncthreads();
+            // A^T u: up to four rows' products first, then one normalised addition to the
+            // running sum, whose rounding errors the long chain would gather
+            constexpr int GR = RB == 8 ? 1 : 2;
 #pragma unroll
-            for (int rb = 0; rb < RB; ++rb) {
-                const float4 u = s_u[rb];
+            for (int r0 = 0; r0 < RB; r0 += GR) {
+                float4 u[GR];
 #pragma unroll
-                for (int k = 0; k < K; ++k) ff_fma_lazy(t[k], x[rb * K + k].x, x[rb * K + k].z, ff{u.x, u.z});
+                for (int q = 0; q < GR; ++q) u[q] = s_u[r0 + q];
 #pragma unroll
-                for (int k = 0; k < K; ++k) ff_fma_lazy(t[k], x[rb * K + k].y, x[rb * K + k].w, ff{u.y, u.w});
+                for (int k = 0; k < K; ++k) {
+                    ff w;
+#pragma unroll
+                    for (int q = 0; q < GR; ++q) {
+                        const float4 xx = x[(r0 + q) * K + k];
+                        if (q == 0) w = ff_mul_lazy(xx.x, xx.z, ff{u[q].x, u[q].z});
+                        else ff_fma_lazy(w, xx.x, xx.z, ff{u[q].x, u[q].z});
+                        ff_fma_lazy(w, xx.y, xx.w, ff{u[q].y, u[q].w});
+                    }
+                    ff_add(t[k], w);
+                }
             }
-#pragma unroll
-            for (int k = 0; k < K; ++k) ff_norm(t[k]);
         }
         if (col_ok)
 #pragma unroll
             for (int k = 0; k < K; ++k) a.part[(int64_t)c.bid * K * CW + k * CW + tid] = make_float2(t[k].hi, t[k].lo);
-        const float2 tot = ss.block(red);
-        if (tid == 0) g.pb[c.bid] = tot;
+        if (warp == 0) {
+            ss = warp_sum(ss);
+            if (lane == 0) g.pb[c.bid] = ss;
+        }
         return true;
     };
     // t = the shares' sum: this CTA's columns, by the first kYWarp warps
@@ -1063,28 +1082,41 @@ k_lsqr_dense(const PArgs<true> g, const DArgs a, int start, int budget)
         for (int b0 = c0; b0 < c1; b0 += 32) {
             const int col = b0 + lane;
             if (warp < C::kYWarp) {
+                // four shares at a time, in pairs: short chains round less
                 ff r{0.f, 0.f};
                 if (col < c1)
-                    for (int q = warp; q < c.G; q += C::kYWarp) {
-                        const float2 p = ld_cg(a.part + (int64_t)q * K * CW + col);
-                        ff_add(r, p.x, p.y);
+                    for (int q = warp; q < c.G; q += 4 * C::kYWarp) {
+                        ff p[4];
+#pragma unroll
+                        for (int h = 0; h < 4; ++h) {
+                            const int qq = q + h * C::kYWarp;
+                            const float2 v = qq < c.G ? ld_cg(a.part + (int64_t)qq * K * CW + col) : make_float2(0.f, 0.f);
+                            p[h] = ff{v.x, v.y};
+                        }
+                        ff_add(p[0], p[1]);
+                        ff_add(p[2], p[3]);
+                        ff_add(p[0], p[2]);
+                        ff_add(r, p[0]);
                     }
                 s_red[warp][lane] = make_float2(r.hi, r.lo);
             }
             __syncthreads();
             if (warp == 0 && col < c1) {
-                ff r{0.f, 0.f};
-                for (int w = 0; w < C::kYWarp; ++w) {
-                    const float2 p = s_red[w][lane];
-                    ff_add(r, p.x, p.y);
+                static_assert(C::kYWarp % 2 == 0, "sums in pairs");
+                double s = 0.0;
+#pragma unroll
+                for (int w = 0; w < C::kYWarp; w += 2) {
+                    const float2 p = s_red[w][lane], q = s_red[w + 1][lane];
+                    ff r{p.x, p.y};
+                    ff_add(r, q.x, q.y);
+                    s += ff_to_double(r);
                 }
-                a.tn[col] = make_float2(r.hi, r.lo);
+                a.tn[col] = store_val<true>(s);
             }
             __syncthreads();
         }
     };
     auto phase_d = [&] {
-        if (tid == kDT - 1) c.put_scale(sc.ib, sc.coef_t);
         for (int i = tid; i < g.r; i += kDT) c.sv[i] = ld_cg(a.tn + __ldg(g.cols + i));
         c.tri_finish();
     };
@@ -1100,7 +1132,7 @@ k_lsqr_dense(const PArgs<true> g, const DArgs a, int start, int budget)
         // u = b through the pass itself: u = 0 - (-1) u
         if (warp == C::kSWarp) c.init_beta();
         __syncthreads();
-        c.init_u();
+        for (int i = c.bid * kDT + tid; i < g.n; i += c.G * kDT) a.uh[i] = g.b[i] * sc.bs;
         if (tid == 0) {
             sc.ia = 0.0;
             sc.coef_n = -1.0;
@@ -1305,7 +1337,7 @@ int lanes_col(double avg) { return avg >= 128 ? 32 : avg >= 64 ? 16 : avg >= 24 
 struct PBufs {
     PState* S;
     void *us, *vs, *z, *t, *tpart;
-    double *w, *y, *pa, *pb, *bpart;
+    double *vh, *w, *y, *pa, *pb, *bpart;
     int4* chunks; int* coff; int* scan; int* cnt; unsigned* ccnt;
     size_t bytes;
 };
@@ -1329,6 +1361,7 @@ PBufs pcarve(const LsqrProblem& P, void* work)
     B.z = take(P.d * vs);
     B.t = take(P.r * vs);
     B.tpart = take(nch * vs);
+    B.vh = P.precision == SKL_PREC_MIXED ? (double*)take(P.r * sizeof(double)) : (double*)B.vs;
     B.w = (double*)take(P.r * sizeof(double));
     B.y = (double*)take(P.r * sizeof(double));
     B.pa = (double*)take(1024 * sizeof(double));
@@ -1565,10 +1598,11 @@ LsqrResult persist_impl(const LsqrProblem& P, const double* b, double tol, int64
     g.z = (V*)B.z;
     g.t = (V*)B.t;
     g.tpart = (V*)B.tpart;
+    g.vh = B.vh;
     g.w = B.w;
     g.y = B.y;
-    g.pa = (V*)B.pa;
-    g.pb = (V*)B.pb;
+    g.pa = B.pa;
+    g.pb = B.pb;
     g.bpart = B.bpart;
     g.S = B.S;
     const int G = grid_of(P).ctas;
@@ -1635,8 +1669,8 @@ int dense_ctas(const LsqrProblem& P)
 
 struct DBufs {
     PState* S;
-    float2 *us, *vs, *z, *part, *tn, *pa, *pb;
-    double *w, *y, *bpart;
+    float2 *vs, *z, *part, *tn;
+    double *uh, *vh, *w, *y, *pa, *pb, *bpart;
     long long* prof;
     size_t bytes;
 };
@@ -1651,13 +1685,14 @@ DBufs dcarve(const LsqrProblem& P, void* work)
     };
     const DenseShape s = dense_shape(P.n, P.d);
     B.S = (PState*)take(sizeof(PState));
-    B.us = (float2*)take(P.n * sizeof(float2));
+    B.uh = (double*)take(P.n * sizeof(double));
+    B.vh = (double*)take(P.r * sizeof(double));
     B.vs = (float2*)take(P.r * sizeof(float2));
     B.z = (float2*)take(P.d * sizeof(float2));
     B.part = (float2*)take((size_t)sm_count_p() * s.K * s.CW * sizeof(float2));
     B.tn = (float2*)take(P.d * sizeof(float2));
-    B.pa = (float2*)take(1024 * sizeof(float2));
-    B.pb = (float2*)take(1024 * sizeof(float2));
+    B.pa = (double*)take(1024 * sizeof(double));
+    B.pb = (double*)take(1024 * sizeof(double));
     B.w = (double*)take(P.r * sizeof(double));
     B.y = (double*)take(P.r * sizeof(double));
     B.bpart = (double*)take(kNormParts * sizeof(double));
@@ -1690,8 +1725,8 @@ LsqrResult dense_impl(const LsqrProblem& P, const double* b, double tol, int64_t
     g.Mc = (const float*)P.M;
     g.ldm = P.ldm;
     g.b = b;
-    g.us = B.us;
     g.vs = B.vs;
+    g.vh = B.vh;
     g.z = B.z;
     g.w = B.w;
     g.y = B.y;
@@ -1704,6 +1739,7 @@ LsqrResult dense_impl(const LsqrProblem& P, const double* b, double tol, int64_t
     g.S_seg = std::max(1, std::min(8, nloc <= nw ? nw / nloc : 4 * nw / nloc));
     DArgs a{};
     a.A = (const float4*)P.At;
+    a.uh = B.uh;
     a.part = B.part;
     a.tn = B.tn;
     a.CW = s.CW;
