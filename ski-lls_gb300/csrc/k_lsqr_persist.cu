@@ -1785,7 +1785,21 @@ LsqrResult dense_impl(const LsqrProblem& P, const double* b, double tol, int64_t
 
 }  // namespace
 
-bool lsqr_dense_tiled(int64_t d, int precision) { return precision == SKL_PREC_MIXED && d >= 1 && d <= kDenseMaxD; }
+// SKILLS_LSQR_PERSIST=0: the kernels of k_lsqr.cu for every problem, none of which
+// waits for the whole GPU.
+static bool persist_enabled()
+{
+    static const bool v = [] {
+        const char* e = getenv("SKILLS_LSQR_PERSIST");
+        return !(e && e[0] == '0');
+    }();
+    return v;
+}
+
+bool lsqr_dense_tiled(int64_t d, int precision)
+{
+    return persist_enabled() && precision == SKL_PREC_MIXED && d >= 1 && d <= kDenseMaxD;
+}
 size_t lsqr_dense_tile_bytes(int64_t n, int64_t d) { return dense_shape(n, d).bytes(); }
 
 void split_dense_tiles(const double* A, int64_t lda, int64_t n, int64_t d, void* out, double* fro, unsigned* status,
@@ -1800,6 +1814,7 @@ void split_dense_tiles(const double* A, int64_t lda, int64_t n, int64_t d, void*
 bool lsqr_persist_fits(const LsqrProblem& P)
 {
     if (P.At) return true;
+    if (!persist_enabled()) return false;
     const int G = grid_of(P).ctas;
     return !P.Ad && P.r > 0 && (P.r + G - 1) / G <= kMaxUnits && vec_smem(P) <= 200 * 1024;
 }
