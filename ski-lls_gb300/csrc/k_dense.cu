@@ -351,8 +351,10 @@ __global__ void k_dht_gather(const double* __restrict__ H, const int* __restrict
 // order, which the last two steps undo through tables made once per call: the
 // places of each pair of frequencies for the unpacking, done in place, and the
 // bucket entries with source rows replaced by places.
-// The transform without a sketch computes both where it needs them: it uses no
-// scratch, so that calls which share one may overlap.
+// The transform without a sketch computes places where it needs them (two per
+// frequency and column): it uses no scratch, so that calls which share one may
+// overlap.  40,000 x 1,000: 489 us; 1,342 with a division per digit, 711 for the
+// autosorted passes before this kernel.
 // The column is read once, with the next column's lines on their way to L2; the
 // signs are bits in shared memory, and the FP64 values are rounded to FP32 on
 // their bits (a warp's FP64 conversion holds the pipe for 16 cycles: 10 us of a
@@ -365,6 +367,11 @@ constexpr int kDifMaxPasses = 16;
 struct DifPlan {
     int L, np;
     int r1[kDifMaxPasses], r2[kDifMaxPasses];
+    // the digits of a frequency, first pass's first: radix, stride of its place, and
+    // ceil(2^32 / radix) (quotients exact below 2^16)
+    int nd;
+    int dr[kFftMaxRadices], ds[kFftMaxRadices];
+    unsigned dm[kFftMaxRadices];
 };
 
 // Forward DFT of the R values v[off + q step].
@@ -483,28 +490,20 @@ SKL_DEV void dif_run(const DifPlan& P, float2* z)
     }
 }
 
-// Place of frequency k: its digits, first pass's first.
+// Place of frequency k.
 SKL_DEV int dif_place(const DifPlan& P, int k)
 {
-    int S = P.L, pos = 0;
-    for (int s = 0; s < P.np; ++s)
-        for (int h = 0; h < 2; ++h) {
-            const int r = h ? P.r2[s] : P.r1[s];
-            S /= r;
-            pos += (k % r) * S;
-            k /= r;
-        }
+    int pos = 0;
+    for (int h = 0; h < P.nd; ++h) {
+        const int q = (int)__umulhi((unsigned)k, P.dm[h]);
+        pos += (k - q * P.dr[h]) * P.ds[h];
+        k = q;
+    }
     return pos;
 }
 
-// Where H[i] ends, as an index of floats.
-SKL_DEV int dif_output(const DifPlan& P, int i)
-{
-    return i < P.L ? 2 * dif_place(P, i) : 2 * dif_place(P, i == P.L ? 0 : 2 * P.L - i) + 1;
-}
-
 // part[k], k <= L / 2: the places of frequencies k and L - k (upper half);
-// place[i], i < N: dif_output.
+// place[i], i < N: where H[i] ends, as an index of floats.
 __global__ void k_dif_tables(DifPlan P, unsigned* __restrict__ part, unsigned* __restrict__ place)
 {
     pdl_wait();
@@ -609,7 +608,12 @@ k_dht_hash_smem(const double* __restrict__ A, int64_t lda, int n, int d, const d
         }
         __syncthreads();
         if (Yout) {
-            for (int k = threadIdx.x; k < N; k += kDifThreads) Yout[k + (int64_t)j * ldy] = (double)H[dif_output(P, k)];
+            double* y = Yout + (int64_t)j * ldy;
+            for (int k = threadIdx.x; k < L; k += kDifThreads) {
+                const float2 h = z[dif_place(P, k)];   // H[k], H[N-k] (H[L] for k = 0)
+                y[k] = (double)h.x;
+                y[k ? N - k : L] = (double)h.y;
+            }
         }
         if (SA) {
             // buckets h and h + 512: each sum in its order, eight entries' loads at a time
@@ -739,6 +743,15 @@ static DifPlan dif_plan(const FftPlan& P)
             if (key(j - 1) >= key(j)) break;
             std::swap(Q.r1[j - 1], Q.r1[j]);
             std::swap(Q.r2[j - 1], Q.r2[j]);
+        }
+    int S = Q.L;
+    for (int s = 0; s < Q.np; ++s)
+        for (int r : {Q.r1[s], Q.r2[s]}) {
+            if (r == 1) continue;
+            S /= r;
+            Q.dr[Q.nd] = r;
+            Q.ds[Q.nd] = S;
+            Q.dm[Q.nd++] = (unsigned)(((1ull << 32) + r - 1) / r);
         }
     return Q;
 }
