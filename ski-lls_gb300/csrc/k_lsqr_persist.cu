@@ -468,6 +468,8 @@ struct Cta {
         // the next row's entries and old u are loaded before this row's products
         int cc[4], nc[4];
         V aa[4], na[4], uo{}, nuo{};
+        const int n_long = 4 * L + min(8 * L, 64);
+        bool any_long = false;
         auto load_entries = [&](int i, int p0, int p1, int (&c)[4], V (&a)[4], V& u) {
             if (i < g.n && l == 0) u = ld_cg(g.us + i);
 #pragma unroll
@@ -500,17 +502,20 @@ struct Cta {
                 acc.fma_mv(aa[k], sv[cc[k]]);
                 acc2.fma_mv(aa[k + 1], sv[cc[k + 1]]);
             }
-            for (int p = p0 + 4 * L; p < p1; p += 2 * L) {   // rows longer than 4 L
-                const int c0 = __ldg(g.ci + p);
-                acc.fma_mv(__ldg(g.cv + p), sv[c0]);
-                if (p + L < p1) {
-                    const int c1 = __ldg(g.ci + p + L);
-                    acc2.fma_mv(__ldg(g.cv + p + L), sv[c1]);
+            const bool lng = p1 - (p0 - l) > n_long;
+            any_long |= lng;
+            if (!lng)
+                for (int p = p0 + 4 * L; p < p1; p += 2 * L) {   // rows longer than 4 L
+                    const int c0 = __ldg(g.ci + p);
+                    acc.fma_mv(__ldg(g.cv + p), sv[c0]);
+                    if (p + L < p1) {
+                        const int c1 = __ldg(g.ci + p + L);
+                        acc2.fma_mv(__ldg(g.cv + p + L), sv[c1]);
+                    }
                 }
-            }
             acc.add(acc2);
             for (int o = L / 2; o > 0; o >>= 1) acc.add(acc.shfl_xor(o));
-            if (i < g.n && l == 0) {
+            if (i < g.n && l == 0 && !lng) {
                 const auto nv = sc2(acc, uo);
                 g.us[i] = to_v(nv);
                 ss.add_sq(nv);
@@ -525,6 +530,44 @@ struct Cta {
                 aa[k] = na[k];
             }
         }
+        // the long rows that this warp passed over, a row at a time: as two entries a
+        // lane and step above, their steps wait for one another (20,000 x 1,000 with
+        // 100 full rows: 115 us per iteration, 26 so); a loop of its own, since inside
+        // the other one its registers would spill
+        if (__any_sync(0xffffffffu, any_long))
+            for (base = (bid * kPW + warp) * per; base < g.n; base += rstep) {
+                i = base + lane / L;
+                p0 = i < g.n ? __ldg(g.rp + i) : 0;
+                p1 = i < g.n ? __ldg(g.rp + i + 1) : 0;
+                unsigned todo = __ballot_sync(0xffffffffu, p1 - p0 > n_long && l == 0);
+                while (todo) {
+                    const int src = __ffs(todo) - 1, row = base + src / L;
+                    todo &= todo - 1;
+                    const int q1 = __shfl_sync(0xffffffffu, p1, src);
+                    Acc<MIXED> acc, acc2;
+                    for (int p = __shfl_sync(0xffffffffu, p0, src) + lane; p < q1; p += 128) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const bool ok = p + 32 * k < q1;
+                            cc[k] = ok ? __ldg(g.ci + p + 32 * k) : 0;
+                            if (ok) aa[k] = __ldg(g.cv + p + 32 * k);
+                            else aa[k] = V{};
+                        }
+#pragma unroll
+                        for (int k = 0; k < 4; k += 2) {
+                            acc.fma_mv(aa[k], sv[cc[k]]);
+                            acc2.fma_mv(aa[k + 1], sv[cc[k + 1]]);
+                        }
+                    }
+                    acc.add(acc2);
+                    acc = warp_reduce<MIXED>(acc);
+                    if (lane == 0) {
+                        const auto nv = sc2(acc, ld_cg(g.us + row));
+                        g.us[row] = to_v(nv);
+                        ss.add_sq(nv);
+                    }
+                }
+            }
         const double tot = sum_warps(ss.warp(), kPW, red);
         if (tid == 0) g.pb[bid] = tot;
     }
@@ -669,8 +712,8 @@ struct Cta {
         // only the warps that own rows hold a sum
         const int nw = min(kPW, (nloc + 31) / 32);
         if (warp < nw) ss = warp_sum(ss);
-        const double tot = sum_warps(ss, nw, red);
-        if (tid == 0) g.pa[bid] = tot;
+        if (nw > 1) ss = sum_warps(ss, nw, red);
+        if (tid == 0) g.pa[bid] = ss;
     }
 };
 
