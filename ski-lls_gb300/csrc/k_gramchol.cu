@@ -1301,7 +1301,6 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
     int ndrop = 0;
     for (int attempt = 0;; ++attempt) {
         factor(attempt);
-        solve_c();
         read_out(8);
         mf2 = hp[2];
         mdf2 = hp[3];
@@ -1348,7 +1347,6 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
             launch_k(k_gc_finish<T>, 1, 1024, 0, st, B.part, nt * nt, B.gdiag, (int)d, B.bad, B.ndrop, status, B.out);
             SKL_LAUNCHED();
             SKL_LAUNCHED();
-            if (last) solve_c();
             read_out(8);
             mf2 = hp[2];
             if (!std::isfinite(mf2) || !(1.0 / std::sqrt(mf2) > 2.0 * thresh)) return false;
@@ -1373,6 +1371,7 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
     res.norm_r = nr;
     res.norm_m = nm;
     res.dropped = ndrop;
+    solve_c();
     if (c) SKL_CUDA(cudaMemcpyAsync(c, B.c, d * sizeof(double), cudaMemcpyDeviceToDevice, st));
     return true;
 }
