@@ -43,6 +43,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <cstring>
 #include <limits>
 #include <mutex>
 #include <type_traits>
@@ -829,23 +830,87 @@ k_gc_ratio_max(const float* __restrict__ p, const float* __restrict__ w, int k, 
     if (threadIdx.x == 0) *out = mx;
 }
 
-// Excludes (infinite mass) the columns with ||M e_j||^2 >= limit from the next
+// The block's largest |x_i| of n entries and its smallest index (n if all are zero or
+// not numbers), in thread 0.
+SKL_DEV void block_argmax(const float* __restrict__ x, int n, float& w, int& at)
+{
+    __shared__ float s_w[8];
+    __shared__ int s_i[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    w = 0.f;
+    at = n;
+    auto take = [&](float v, int i) {
+        if (v > w || (v == w && i < at)) {
+            w = v;
+            at = i;
+        }
+    };
+    for (int i = threadIdx.x; i < n; i += 256) take(fabsf(x[i]), i);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float v = __shfl_xor_sync(0xffffffffu, w, o);
+        const int i = __shfl_xor_sync(0xffffffffu, at, o);
+        take(v, i);
+    }
+    if (lane == 0) {
+        s_w[warp] = w;
+        s_i[warp] = at;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int q = 1; q < 8; ++q) take(s_w[q], s_i[q]);
+    __syncthreads();
+}
+
+// The sweep drops the last of a set of dependent columns, whose coefficients w on the
+// others (a column of W per dropped one) may be large: those that stay are then
+// nearly dependent themselves.  In another attempt the column with the largest |w_i|
+// goes instead if that exceeds 1, and j stays, which multiplies the volume of those
+// that stay by |w_i|; a pivoted QR chooses so.  LSQR, which carries the dropped
+// columns, pays for the difference where they are not exactly dependent, which FP32
+// cannot tell below ~3e-7 (120,000 x 5,000, 50 columns at a distance of 1e-6: 2,650
+// iterations, 1,026 with the exchange, 1,028 with the QR).
+// want[t] = the column to leave out, *big = max |w_i| (bits of a float >= 0).
+__global__ void __launch_bounds__(256)
+k_gc_exchange(const int* __restrict__ drop, const float* __restrict__ W, int64_t ldw, int d, int* __restrict__ want,
+              int* __restrict__ big)
+{
+    pdl_wait();
+    const int t = blockIdx.x;
+    float w;
+    int at;
+    block_argmax(W + t * ldw, d, w, at);
+    if (threadIdx.x != 0) return;
+    want[t] = w > 1.02f && at < d ? at : drop[t];   // 2 % above 1: equal ones stay
+    atomicMax(big, __float_as_int(w));
+}
+__global__ void k_gc_leave_out(const int* __restrict__ want, int k, float* __restrict__ mass)
+{
+    pdl_wait();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < k) mass[want[t]] = std::numeric_limits<float>::infinity();
+}
+
+// Excludes (infinite mass) a column for each with ||M e_j||^2 >= limit from the next
 // attempt: a dependent column that follows two nearly parallel ones has the
 // Gram matrix's noise amplified in its pivot, which then passes, but its column
-// of M is as large as the noise is small.
+// of M, (-w, 1) / R_jj, is as large as the noise is small.  The largest entry's column
+// goes, by 2 % as above.
 __global__ void __launch_bounds__(256)
 k_gc_exclude(const float* __restrict__ Mc, int64_t ldm, float limit, float* __restrict__ mass)
 {
     pdl_wait();
     __shared__ float red[8];
     const int j = blockIdx.x;
+    const float* m = Mc + (int64_t)j * ldm;
     float s = 0.f;
-    for (int i = threadIdx.x; i <= j; i += 256) {
-        const float v = Mc[i + (int64_t)j * ldm];
-        s = fmaf(v, v, s);
-    }
+    for (int i = threadIdx.x; i <= j; i += 256) s = fmaf(m[i], m[i], s);
     s = block_sum(s, red);
-    if (threadIdx.x == 0 && !(s < limit)) mass[j] = std::numeric_limits<float>::infinity();
+    if (s < limit) return;   // the same in every thread
+    float w;
+    int at;
+    block_argmax(m, j, w, at);
+    if (threadIdx.x == 0) mass[w > 1.02f * fabsf(m[j]) && at < j ? at : j] = std::numeric_limits<float>::infinity();
 }
 
 // M's diagonal entries of the dropped columns
@@ -865,7 +930,7 @@ struct GramBuffers {
     int64_t ldg;
     T* G; T* R; T* mkk; T* gdiag; T* mass; T* partial; int64_t partial_cap;
     int* bad; int* ndrop; double* part; double* out;
-    T* dw; T* dt; T* dp; T* dn; int64_t ldp;
+    T* dw; T* dt; T* dp; T* dn; int* want; int64_t ldp;
     T* Q; T* QT; T* M2c; T* M2r; T* Racc; int64_t ldq;
     typename GV<T>::type* rv; typename GV<T>::type* tv; typename GV<T>::type* cv; typename GV<T>::type* wv;
     double* rows_part; double* c;
@@ -904,6 +969,7 @@ GramBuffers<T> gram_carve(void* work, int64_t m, int64_t d, bool multi)
     B.dt = (T*)take((size_t)B.ldg * kd * sizeof(T));
     B.dp = (T*)take((size_t)B.ldp * kd * sizeof(T));
     B.dn = (T*)take((size_t)2 * kd * sizeof(T));
+    B.want = (int*)take((size_t)kd * sizeof(int));
     B.part = (double*)take((size_t)2 * nt * nt * sizeof(double));
     B.out = (double*)take(8 * sizeof(double));
     B.rv = (V*)take((size_t)m * sizeof(V));
@@ -1060,45 +1126,80 @@ void tn_product(int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, co
     tn_launch(ma, mb, mb, t, tiles(M), tiles(N), nullptr, status, st);
 }
 
-// Whether the k dropped columns of S A depend on the others at FP32 resolution.
-// From S A itself (the Gram matrix cannot tell 1e-4 from 0): p = the residual of
-// column j against the kept columns with coefficients w (the normal equations',
-// refined once).  (w, -1) is then a vector that S A maps to p, so the dropped
-// columns' singular values are about ||p|| / (1 + ||w||^2)^(1/2), which is what the
-// trailing pivots of a pivoted QR show; out[0] = the largest such ratio squared.
-void drop_check(const Sweep<float>& S, const int* drop, int k, cudaStream_t st)
+// W (dt, zeros at the dropped columns) = the dropped columns' coefficients on the
+// columns before them that stay; P (dp) = the dropped columns of S A.
+void drop_coefs(const Sweep<float>& S, const int* drop, int k, cudaStream_t st)
+{
+    const GramBuffers<float>& B = S.B;
+    const int m = (int)S.m, d = (int)S.d;
+    launch_k(k_gc_drop_gather, dim3(16, (unsigned)k), 256, 0, st, drop, B.R, B.ldg, d, S.SA, S.ld, m, B.dw, B.ldg,
+             B.dp, B.ldp);
+    launch_k(k_gc_zero_other, (unsigned)d, 256, 0, st, S.Ew, S.E, S.lde, d);
+    SKL_LAUNCHED();
+    SKL_LAUNCHED();
+    tn_product(d, k, d, S.E, S.lde, B.dw, B.ldg, B.dt, B.ldg, S.status, st);
+}
+void drop_coefs(const Sweep<double>&, const int*, int, cudaStream_t)
+{
+    fail(SKL_ERR_INVALID, "dropped columns: FP32 only");
+}
+
+// Whether the k dropped columns of S A depend on the others at FP32 resolution
+// (after drop_coefs).  From S A itself (the Gram matrix cannot tell 1e-4 from 0):
+// p = the residual of column j against the columns that stay, with coefficients w
+// from the normal equations.  (w, -1) is then a vector that S A maps to p, so the
+// dropped columns' singular values are about ||p|| / (1 + ||w||^2)^(1/2), which is
+// what the trailing pivots of a pivoted QR show; out[0] = the largest such ratio
+// squared.  W is a good start where only columns before j matter; a column that an
+// exchange left out depends on later ones too, and takes two steps from zero.
+void drop_check(const Sweep<float>& S, int k, bool from_w, cudaStream_t st)
 {
     const GramBuffers<float>& B = S.B;
     const int m = (int)S.m, d = (int)S.d;
     float* Mc = S.Ew;
     float* Mr = S.E;
-    launch_k(k_gc_drop_gather, dim3(16, (unsigned)k), 256, 0, st, drop, B.R, B.ldg, d, S.SA, S.ld, m, B.dw, B.ldg,
-             B.dp, B.ldp);
-    launch_k(k_gc_zero_other, (unsigned)d, 256, 0, st, Mc, Mr, S.lde, d);
-    SKL_LAUNCHED();
-    SKL_LAUNCHED();
     float* part = (float*)B.rows_part;
     const int64_t cap = (int64_t)((d + kResCols - 1) / kResCols) * m * 2;
+    auto norms = [&](const float* X, int64_t ld, int rows, float* out) {
+        launch_k(k_gc_colnorm, (unsigned)k, 256, 0, st, X, ld, rows, out);
+        SKL_LAUNCHED();
+    };
     auto residual = [&](const float* W) {
         gemm<float>(false, false, m, k, d, -1.f, S.SA, S.ld, W, B.ldg, 1.f, B.dp, B.ldp, part, cap, st);
     };
-    tn_product(d, k, d, Mr, S.lde, B.dw, B.ldg, B.dt, B.ldg, S.status, st);
-    launch_k(k_gc_colnorm, (unsigned)k, 256, 0, st, B.dt, B.ldg, d, B.dn);
-    SKL_LAUNCHED();
-    residual(B.dt);
-    tn_product(d, k, m, S.SA, S.ld, B.dp, B.ldp, B.dw, B.ldg, S.status, st);
-    tn_product(d, k, d, Mc, S.lde, B.dw, B.ldg, B.dt, B.ldg, S.status, st);
-    tn_product(d, k, d, Mr, S.lde, B.dt, B.ldg, B.dw, B.ldg, S.status, st);
-    residual(B.dw);
-    launch_k(k_gc_colnorm, (unsigned)k, 256, 0, st, B.dp, B.ldp, m, B.dn + k);
+    if (from_w) {
+        norms(B.dt, B.ldg, d, B.dn);
+        residual(B.dt);
+    }
+    for (int s = from_w ? 1 : 0; s < 2; ++s) {
+        tn_product(d, k, m, S.SA, S.ld, B.dp, B.ldp, B.dw, B.ldg, S.status, st);
+        tn_product(d, k, d, Mc, S.lde, B.dw, B.ldg, B.dt, B.ldg, S.status, st);
+        tn_product(d, k, d, Mr, S.lde, B.dt, B.ldg, B.dw, B.ldg, S.status, st);
+        residual(B.dw);
+        if (s == 0) norms(B.dw, B.ldg, d, B.dn);
+    }
+    norms(B.dp, B.ldp, m, B.dn + k);
     launch_k(k_gc_ratio_max, 1, 256, 0, st, B.dn + k, B.dn, k, B.out);
     SKL_LAUNCHED();
+}
+void drop_check(const Sweep<double>&, int, bool, cudaStream_t) {}
+
+// After drop_coefs: the columns that another attempt would leave out, to B.want, and
+// the largest |w| of a dropped column (its bits to the low half of out[0]).
+void drop_exchange(const Sweep<float>& S, const int* drop, int k, cudaStream_t st)
+{
+    const GramBuffers<float>& B = S.B;
+    SKL_CUDA(cudaMemsetAsync(B.out, 0, sizeof(double), st));
+    launch_k(k_gc_exchange, (unsigned)k, 256, 0, st, drop, (const float*)B.dt, B.ldg, (int)S.d, B.want, (int*)B.out);
     SKL_LAUNCHED();
 }
-void drop_check(const Sweep<double>&, const int*, int, cudaStream_t)
+void drop_exchange(const Sweep<double>&, const int*, int, cudaStream_t) {}
+void leave_out(const Sweep<float>& S, int k, cudaStream_t st)
 {
-    fail(SKL_ERR_INVALID, "dropped columns: FP32 only");
+    launch_k(k_gc_leave_out, (unsigned)((k + 127) / 128), 128, 0, st, (const int*)S.B.want, k, S.B.mass);
+    SKL_LAUNCHED();
 }
+void leave_out(const Sweep<double>&, int, cudaStream_t) {}
 
 void tr_launch(float* X, int64_t ldx, int64_t rows, int64_t cols, int upper, float* out, int64_t ldo, cudaStream_t st)
 {
@@ -1297,7 +1398,7 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
         SKL_CUDA(cudaMemcpyAsync(hp, B.out, count * sizeof(double), cudaMemcpyDeviceToHost, st));
         SKL_CUDA(cudaStreamSynchronize(st));
     };
-    double mf2 = 0.0, mdf2 = 0.0, gmax = 0.0;
+    double mf2 = 0.0, mdf2 = 0.0, gmax = 0.0, thresh = 0.0;
     int ndrop = 0;
     for (int attempt = 0;; ++attempt) {
         factor(attempt);
@@ -1309,14 +1410,36 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
         if ((unsigned)hp[6] & kStatusTcTimeout)
             fail(SKL_ERR_TIMEOUT, "a tensor-core product's bounded wait gave up");
         if (hp[5] != 0.0 || !std::isfinite(mf2) || !std::isfinite(mdf2) || !(mf2 > 0.0)) return false;
-        if ((double)eps * mdf2 <= 1.0 / 16 && !(boost && ndrop > 0)) break;
+        // the rank rule's threshold (below: with a factor 2 for M's own error)
+        thresh = std::max(abs_thresh, rel_thresh * std::sqrt(gmax));
         if (boost) break;
-        // dependent columns whose pivots passed: again without them
-        if (ndrop == 0 || attempt == 2) return false;
-        drop_exclude(S, 1.0 / (64.0 * (double)eps), st);
+        const bool well = (double)eps * mdf2 <= 1.0 / 16;
+        if (ndrop == 0) {
+            if (well) break;
+            return false;
+        }
+        drop_coefs(S, drop, ndrop, st);
+        bool again = !well;
+        if (attempt == 0) {
+            // a sweep more (a fifth of a rank-deficient solve) where a choice is worse
+            // than the best by more than 2
+            drop_exchange(S, drop, ndrop, st);
+            read_out(1);
+            float w;
+            std::memcpy(&w, hp, sizeof w);
+            again = again || w > 2.f;
+            if (again) leave_out(S, ndrop, st);
+        }
+        if (!again) {
+            drop_check(S, ndrop, attempt == 0, st);
+            read_out(1);
+            if (std::sqrt(hp[0]) <= 0.25 * thresh) break;
+            return false;
+        }
+        if (attempt == 2) return false;
+        // and without dependent columns whose pivots passed
+        if (!well) drop_exclude(S, 1.0 / (64.0 * (double)eps), st);
     }
-    // the rank rule's threshold, with a factor 2 for M's own error
-    const double thresh = std::max(abs_thresh, rel_thresh * std::sqrt(gmax));
     const T* R = B.R;
     if (boost && !((double)eps * mdf2 <= 1.0 / 16 && ndrop == 0)) {
         // Too ill-conditioned for its Gram matrix, or with boosted pivots: the same
@@ -1357,11 +1480,6 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
         ndrop = 0;
     }
     if (!(1.0 / std::sqrt(mf2) > 2.0 * thresh)) return false;
-    if (ndrop > 0) {
-        drop_check(S, drop, ndrop, st);
-        read_out(1);
-        if (!(std::sqrt(hp[0]) <= 0.25 * thresh)) return false;
-    }
     SKL_CUDA(cudaMemsetAsync(B.out, 0, 2 * sizeof(double), st));
     inf_norm_upper<T>(R, B.ldg, d, B.rows_part, B.out, st);
     inf_norm_upper<T>(Mc, ldm, d, B.rows_part, B.out + 1, st);
