@@ -930,7 +930,7 @@ struct GramBuffers {
     int64_t ldg;
     T* G; T* R; T* mkk; T* gdiag; T* mass; T* partial; int64_t partial_cap;
     int* bad; int* ndrop; double* part; double* out;
-    T* dw; T* dt; T* dp; T* dn; int* want; int64_t ldp;
+    T* Gkeep; T* dw; T* dt; T* dp; T* dn; int* want; int64_t ldp;
     T* Q; T* QT; T* M2c; T* M2r; T* Racc; int64_t ldq;
     typename GV<T>::type* rv; typename GV<T>::type* tv; typename GV<T>::type* cv; typename GV<T>::type* wv;
     double* rows_part; double* c;
@@ -965,6 +965,7 @@ GramBuffers<T> gram_carve(void* work, int64_t m, int64_t d, bool multi)
     // residuals (m x k)
     const int64_t kd = std::is_same<T, float>::value && !multi ? std::min<int64_t>(kGramDropMax, d / 4) : 0;
     B.ldp = (m + 31) / 32 * 32;
+    B.Gkeep = (T*)take(kd > 0 ? (size_t)B.ldg * d * sizeof(T) : 0);
     B.dw = (T*)take((size_t)B.ldg * kd * sizeof(T));
     B.dt = (T*)take((size_t)B.ldg * kd * sizeof(T));
     B.dp = (T*)take((size_t)B.ldp * kd * sizeof(T));
@@ -1323,7 +1324,13 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
     }
 
     auto factor = [&](int attempt) {
-        sweep_gram(S, st);
+        // the sweep works in place; a copy of the Gram matrix (30 us at 5,000 columns, the
+        // product 1.5 ms) is there for attempts without some of the columns
+        const size_t gbytes = (size_t)B.ldg * d * sizeof(T);
+        if (attempt == 0) sweep_gram(S, st);
+        if (drop_cap > 0 && !ga.boost)
+            SKL_CUDA(cudaMemcpyAsync(attempt == 0 ? B.Gkeep : B.G, attempt == 0 ? B.G : B.Gkeep, gbytes,
+                                     cudaMemcpyDeviceToDevice, st));
         launch_k(k_gc_init<T>, 64, 256, 0, st, B.G, B.ldg, (int)d, B.gdiag, B.mass, attempt == 0, B.mkk, jpvt, B.bad, B.ndrop);
         SKL_LAUNCHED();
         bool bulk_pending = false;
