@@ -26,8 +26,15 @@
 // same is done again on Q = S A M (at most twice): each pass takes the condition
 // number to about the root of what exceeds ~300.  40,000 x 4,000 (S A 6,800 x 4,000):
 // QR and inverse 20.2 + 1.4 ms, one pass ~3.3 ms, two (condition number 1e3 to
-// 1e5) 7.5 ms with LSQR's iterations, x and residual unchanged.  From ~1e6 on
-// most attempts end early and the QR comes on top of one pass's time.
+// 1e5) 7.5 ms with LSQR's iterations, x and residual unchanged.  Beyond, by size
+// (12,007 x 1,201: from 1e7 on), attempts end early and the QR comes on top of a
+// pass's time.
+// The sparse path takes the later passes where no pivot failed but the bound on M D
+// does, or where the dropped columns are all at least four thresholds away from
+// dependence (120,000 x 5,000, S A 8,500 x 5,000: 11.2 and 16 to 19 ms; the QR and
+// inverse 26.9 + 2 ms).  Columns between a quarter of the threshold and four of
+// them, and more than 512 failed pivots, end in the QR after an attempt of 0.2 to
+// 7.5 ms.
 // A sketch that fails a test keeps the QR: S A is not touched here.
 //
 // Sweep (outer blocks of 256 rows, inner blocks of 64): the same row
@@ -815,19 +822,40 @@ k_gc_colnorm(const float* __restrict__ X, int64_t ld, int m, float* __restrict__
     if (threadIdx.x == 0) out[blockIdx.x] = s;
 }
 
-// out[0] = max_t p[t] / (1 + w[t]) (a NaN counts as infinity); one block
+// *out = max(*out, ||upper triangle of X||_1); one block per column
+template <typename T>
+__global__ void __launch_bounds__(256)
+k_gc_one_norm(const T* __restrict__ X, int64_t ld, double* __restrict__ out)
+{
+    pdl_wait();
+    __shared__ double red[8];
+    const T* x = X + (int64_t)blockIdx.x * ld;
+    double s = 0.0;
+    for (int i = threadIdx.x; i <= (int)blockIdx.x; i += 256) s += fabs((double)x[i]);
+    s = block_sum(s, red);
+    // sums >= 0 compare like their bits
+    if (threadIdx.x == 0) atomicMax((unsigned long long*)out, (unsigned long long)__double_as_longlong(s));
+}
+
+// out[0] = max_t p[t] / (1 + w[t]) (a NaN counts as infinity), out[1] = the smallest
+// (as 0); one block
 __global__ void __launch_bounds__(256)
 k_gc_ratio_max(const float* __restrict__ p, const float* __restrict__ w, int k, double* __restrict__ out)
 {
     pdl_wait();
     __shared__ double red[8];
-    double mx = 0.0;
+    double mx = 0.0, mi = 0.0;   // of r and 1 / r
     for (int t = threadIdx.x; t < k; t += 256) {
         const float r = p[t] / (1.f + w[t]);
         mx = fmax(mx, r >= 0.f ? (double)r : HUGE_VAL);
+        mi = fmax(mi, r > 0.f ? 1.0 / (double)r : HUGE_VAL);
     }
     mx = block_max(mx, red);
-    if (threadIdx.x == 0) *out = mx;
+    mi = block_max(mi, red);
+    if (threadIdx.x == 0) {
+        out[0] = mx;
+        out[1] = 1.0 / mi;
+    }
 }
 
 // The block's largest |x_i| of n entries and its smallest index (n if all are zero or
@@ -938,7 +966,7 @@ struct GramBuffers {
 };
 
 template <typename T>
-GramBuffers<T> gram_carve(void* work, int64_t m, int64_t d, bool multi)
+GramBuffers<T> gram_carve(void* work, int64_t m, int64_t d, bool multi, bool drops)
 {
     GramBuffers<T> B;
     size_t used = 0;
@@ -963,7 +991,7 @@ GramBuffers<T> gram_carve(void* work, int64_t m, int64_t d, bool multi)
     B.ndrop = (int*)take(sizeof(int));
     // dropped columns: their coefficients and two rounds' scratch (d x k), their
     // residuals (m x k)
-    const int64_t kd = std::is_same<T, float>::value && !multi ? std::min<int64_t>(kGramDropMax, d / 4) : 0;
+    const int64_t kd = std::is_same<T, float>::value && drops ? std::min<int64_t>(kGramDropMax, d / 4) : 0;
     B.ldp = (m + 31) / 32 * 32;
     B.Gkeep = (T*)take(kd > 0 ? (size_t)B.ldg * d * sizeof(T) : 0);
     B.dw = (T*)take((size_t)B.ldg * kd * sizeof(T));
@@ -1261,9 +1289,9 @@ void drop_exclude(const Sweep<double>&, double, cudaStream_t) {}
 }  // namespace
 
 template <typename T>
-size_t gram_workspace_bytes(int64_t m, int64_t d, bool multi)
+size_t gram_workspace_bytes(int64_t m, int64_t d, bool multi, bool drops)
 {
-    return gram_carve<T>(nullptr, m, d, multi && std::is_same<T, float>::value).bytes;
+    return gram_carve<T>(nullptr, m, d, multi && std::is_same<T, float>::value, drops).bytes;
 }
 
 bool gram_enabled()
@@ -1288,10 +1316,13 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
     // the inverse grows exponentially (128 eps overflowed at 200 columns).  With
     // neither, a failed pivot only ends the attempt early, which the bound on M D
     // below would do.
-    const bool boost = multi && std::is_same<T, float>::value;
+    // Where columns may be dropped, pivots are only raised for sketches that turn out
+    // to need later passes.
+    const bool passes = multi && std::is_same<T, float>::value;
+    bool boost = passes && !drop;
     const T eps = std::is_same<T, float>::value ? T(5.9604644775390625e-08) : T(1.1102230246251565e-16);
-    const T pivot = (drop_cap > 0 || boost ? T(2048) : T(128)) * eps;
-    Sweep<T> S{SA, m, d, ld, gram_carve<T>(work, m, d, boost), Mc, Mr, ldm, status};
+    const T pivot = (drop || passes ? T(2048) : T(128)) * eps;
+    Sweep<T> S{SA, m, d, ld, gram_carve<T>(work, m, d, passes, drop != nullptr), Mc, Mr, ldm, status};
     GramBuffers<T>& B = S.B;
     const size_t dsm = (2 * (size_t)kIB * kSL + kIB) * sizeof(T);
     const size_t ssm = (4 * (size_t)kIB * kSL + kIB) * sizeof(T);
@@ -1323,15 +1354,15 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
         SKL_CUDA(cudaEventCreateWithFlags(&evB, cudaEventDisableTiming));
     }
 
-    auto factor = [&](int attempt) {
+    // again: on the first sweep's Gram matrix
+    auto factor = [&](bool again, bool all_columns) {
         // the sweep works in place; a copy of the Gram matrix (30 us at 5,000 columns, the
         // product 1.5 ms) is there for attempts without some of the columns
         const size_t gbytes = (size_t)B.ldg * d * sizeof(T);
-        if (attempt == 0) sweep_gram(S, st);
-        if (drop_cap > 0 && !ga.boost)
-            SKL_CUDA(cudaMemcpyAsync(attempt == 0 ? B.Gkeep : B.G, attempt == 0 ? B.G : B.Gkeep, gbytes,
-                                     cudaMemcpyDeviceToDevice, st));
-        launch_k(k_gc_init<T>, 64, 256, 0, st, B.G, B.ldg, (int)d, B.gdiag, B.mass, attempt == 0, B.mkk, jpvt, B.bad, B.ndrop);
+        if (!again) sweep_gram(S, st);
+        if (drop_cap > 0 && (again || !ga.boost))
+            SKL_CUDA(cudaMemcpyAsync(again ? B.G : B.Gkeep, again ? B.Gkeep : B.G, gbytes, cudaMemcpyDeviceToDevice, st));
+        launch_k(k_gc_init<T>, 64, 256, 0, st, B.G, B.ldg, (int)d, B.gdiag, B.mass, all_columns, B.mkk, jpvt, B.bad, B.ndrop);
         SKL_LAUNCHED();
         bool bulk_pending = false;
         for (int64_t j0 = 0; j0 < d; j0 += kOB) {
@@ -1407,8 +1438,7 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
     };
     double mf2 = 0.0, mdf2 = 0.0, gmax = 0.0, thresh = 0.0;
     int ndrop = 0;
-    for (int attempt = 0;; ++attempt) {
-        factor(attempt);
+    auto read_sweep = [&] {
         read_out(8);
         mf2 = hp[2];
         mdf2 = hp[3];
@@ -1416,19 +1446,38 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
         ndrop = (int)hp[7];
         if ((unsigned)hp[6] & kStatusTcTimeout)
             fail(SKL_ERR_TIMEOUT, "a tensor-core product's bounded wait gave up");
-        if (hp[5] != 0.0 || !std::isfinite(mf2) || !std::isfinite(mdf2) || !(mf2 > 0.0)) return false;
         // the rank rule's threshold (below: with a factor 2 for M's own error)
         thresh = std::max(abs_thresh, rel_thresh * std::sqrt(gmax));
+        return hp[5] == 0.0 && std::isfinite(mf2) && std::isfinite(mdf2) && mf2 > 0.0;
+    };
+    // sigma_min > 2 thresh: from ||M||_F, or where many small singular values make that
+    // too large, from ||M||_2^2 <= ||M||_1 ||M||_inf
+    auto resolves = [&] {
+        if (1.0 / std::sqrt(mf2) > 2.0 * thresh) return true;
+        if (!drop || !std::isfinite(mf2)) return false;
+        SKL_CUDA(cudaMemsetAsync(B.out, 0, 2 * sizeof(double), st));
+        inf_norm_upper<T>(Mc, ldm, d, B.rows_part, B.out, st);
+        launch_k(k_gc_one_norm<T>, (unsigned)d, 256, 0, st, (const T*)Mc, ldm, B.out + 1);
+        SKL_LAUNCHED();
+        read_out(2);
+        return 1.0 / std::sqrt(hp[0] * hp[1]) > 2.0 * thresh;
+    };
+    for (int attempt = 0;; ++attempt) {
+        factor(attempt > 0, attempt == 0);
+        if (!read_sweep()) return false;
         if (boost) break;
         const bool well = (double)eps * mdf2 <= 1.0 / 16;
         if (ndrop == 0) {
             if (well) break;
-            return false;
+            // condition number beyond ~1e3: later passes, as on the dense path
+            if (!passes || !resolves()) return false;
+            ga.boost = boost = true;
+            break;
         }
         drop_coefs(S, drop, ndrop, st);
         bool again = !well;
         if (attempt == 0) {
-            // a sweep more (a fifth of a rank-deficient solve) where a choice is worse
+            // a sweep more (a tenth of a rank-deficient solve) where a choice is worse
             // than the best by more than 2
             drop_exchange(S, drop, ndrop, st);
             read_out(1);
@@ -1439,9 +1488,15 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
         }
         if (!again) {
             drop_check(S, ndrop, attempt == 0, st);
-            read_out(1);
+            read_out(2);
             if (std::sqrt(hp[0]) <= 0.25 * thresh) break;
-            return false;
+            // none of them dependent, nor close to what the rule decides on: later
+            // passes with all columns resolve them
+            if (!passes || !(std::sqrt(hp[1]) >= 4.0 * thresh)) return false;
+            ga.boost = boost = true;
+            factor(true, true);
+            if (!read_sweep()) return false;
+            break;
         }
         if (attempt == 2) return false;
         // and without dependent columns whose pivots passed
@@ -1463,7 +1518,7 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
             ga.Ew = S.Ew;
             ga.E = S.E;
             ga.lde = S.lde;
-            factor(0);
+            factor(false, true);
             read_out(8);
             if ((unsigned)hp[6] & kStatusTcTimeout)
                 fail(SKL_ERR_TIMEOUT, "a tensor-core product's bounded wait gave up");
@@ -1479,14 +1534,14 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
             SKL_LAUNCHED();
             read_out(8);
             mf2 = hp[2];
-            if (!std::isfinite(mf2) || !(1.0 / std::sqrt(mf2) > 2.0 * thresh)) return false;
+            if (!std::isfinite(mf2) || !resolves()) return false;
             if (last) break;
             if (pass == 3) return false;
         }
         R = B.Racc;
         ndrop = 0;
     }
-    if (!(1.0 / std::sqrt(mf2) > 2.0 * thresh)) return false;
+    if (!resolves()) return false;
     SKL_CUDA(cudaMemsetAsync(B.out, 0, 2 * sizeof(double), st));
     inf_norm_upper<T>(R, B.ldg, d, B.rows_part, B.out, st);
     inf_norm_upper<T>(Mc, ldm, d, B.rows_part, B.out + 1, st);
@@ -1509,8 +1564,8 @@ void gram_unit_dropped(const int* drop, int64_t k, float* Mc, float* Mr, int64_t
 }
 void gram_unit_dropped(const int*, int64_t, double*, double*, int64_t, cudaStream_t) {}
 
-template size_t gram_workspace_bytes<float>(int64_t, int64_t, bool);
-template size_t gram_workspace_bytes<double>(int64_t, int64_t, bool);
+template size_t gram_workspace_bytes<float>(int64_t, int64_t, bool, bool);
+template size_t gram_workspace_bytes<double>(int64_t, int64_t, bool, bool);
 template bool gram_precond<float>(const float*, int64_t, int64_t, int64_t, double*, int*, float*, float*, int64_t, double,
                                   double, double, GramResult&, int*, bool, void*, unsigned*, void*, cudaStream_t);
 template bool gram_precond<double>(const double*, int64_t, int64_t, int64_t, double*, int*, double*, double*, int64_t,

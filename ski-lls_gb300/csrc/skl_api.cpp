@@ -314,7 +314,7 @@ static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, do
     // ---- workspace layout (sized once, then carved) ----
     const size_t qr_ws = cpqr_workspace_bytes<T>(m, d);
     const size_t inv_ws = std::max(trinv_workspace_bytes<T>(d) + (size_t)d * d * sizeof(T),
-                                   gram_enabled() && m >= d ? gram_workspace_bytes<T>(m, d, false) : 0);
+                                   gram_enabled() && m >= d ? gram_workspace_bytes<T>(m, d, mixed, mixed) : 0);
     LsqrProblem Pq;
     Pq.n = n; Pq.d = d; Pq.nnz = nnz; Pq.r = d; Pq.precision = o.precision;
     const size_t lsqr_ws = lsqr_workspace_bytes(Pq);
@@ -474,7 +474,7 @@ static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, do
     // randomized CPQR, rank by its diagonal
     const bool gram = gram_enabled() && m >= d &&
                       gram_precond<T>(SA, m, d, ld, cvec, jpvt, Mc, Mr, ldm, 0.0, rel, o.rcond_threshold, gres,
-                                      carry_unresolved ? drop : nullptr, false, work, C.dev_status, C.host_pinned, st);
+                                      carry_unresolved ? drop : nullptr, carry_unresolved, work, C.dev_status, C.host_pinned, st);
     if (gram) {
         info.rank = d - gres.dropped;
         info.unresolved_cols = gres.dropped;
@@ -948,7 +948,7 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
     info.sketch_rows = m;
     const size_t qr_ws = cpqr_workspace_bytes<T>(m, d);
     const size_t inv_ws = std::max(trinv_workspace_bytes<T>(d),
-                                   gram_enabled() ? gram_workspace_bytes<T>(m, d, true) : 0);
+                                   gram_enabled() ? gram_workspace_bytes<T>(m, d, true, false) : 0);
     LsqrProblem Pq;
     const bool tiled = lsqr_dense_tiled(d, o.precision);
     Pq.n = n; Pq.d = d; Pq.r = d; Pq.precision = o.precision;

@@ -242,7 +242,7 @@ struct GramResult {
     int64_t dropped = 0;
 };
 template <typename T>
-size_t gram_workspace_bytes(int64_t m, int64_t d, bool multi);
+size_t gram_workspace_bytes(int64_t m, int64_t d, bool multi, bool drops);
 template <typename T>
 bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int* jpvt, T* Mc, T* Mr, int64_t ldm,
                   double abs_thresh, double rel_thresh, double rcond_min, GramResult& res, int* drop, bool multi, void* work,
