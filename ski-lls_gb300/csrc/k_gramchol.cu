@@ -941,6 +941,14 @@ k_gc_exclude(const float* __restrict__ Mc, int64_t ldm, float limit, float* __re
     if (threadIdx.x == 0) mass[w > 1.02f * fabsf(m[j]) && at < j ? at : j] = std::numeric_limits<float>::infinity();
 }
 
+__global__ void __launch_bounds__(256)
+k_gc_narrow(const double* __restrict__ X, int64_t ld, int rows, float* __restrict__ out)
+{
+    pdl_wait();
+    const int64_t o = blockIdx.y * ld;
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < rows; i += gridDim.x * 256) out[o + i] = (float)X[o + i];
+}
+
 // M's diagonal entries of the dropped columns
 __global__ void k_gc_drop_unit(const int* __restrict__ drop, int k, float* __restrict__ Mc,
                                float* __restrict__ Mr, int64_t ldm)
@@ -1554,6 +1562,31 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
     solve_c();
     if (c) SKL_CUDA(cudaMemcpyAsync(c, B.c, d * sizeof(double), cudaMemcpyDeviceToDevice, st));
     return true;
+}
+
+static size_t up256(size_t b) { return (b + 255) & ~(size_t)255; }
+
+size_t gram_probe_bytes(int64_t m, int64_t d, int64_t ld)
+{
+    if (d < kGramProbeCols) return 0;
+    return up256((size_t)ld * d * sizeof(float)) + up256(kGramDropMax * sizeof(int)) +
+           gram_workspace_bytes<float>(m, d, false, true);
+}
+
+bool gram_probe(const double* SA, int64_t m, int64_t d, int64_t ld, int* jpvt, double* Mc, double* Mr, void* work,
+                unsigned* status, void* host_pinned, cudaStream_t st)
+{
+    if (d < kGramProbeCols) return true;
+    float* SAf = (float*)work;
+    int* drop = (int*)((char*)work + up256((size_t)ld * d * sizeof(float)));
+    void* rest = (char*)drop + up256(kGramDropMax * sizeof(int));
+    launch_k(k_gc_narrow, dim3((unsigned)((m + 1023) / 1024), (unsigned)d), 256, 0, st, SA, ld, (int)m, SAf);
+    SKL_LAUNCHED();
+    const double rel = 2.0 * std::sqrt((double)m) * 5.960464477539063e-08;
+    GramResult res;
+    const bool found = gram_precond<float>(SAf, m, d, ld, nullptr, jpvt, (float*)Mc, (float*)Mr, (d + 3) / 4 * 4, 0.0,
+                                           rel, 0.0, res, drop, false, rest, status, host_pinned, st);
+    return !(found && res.dropped > 0);
 }
 
 void gram_unit_dropped(const int* drop, int64_t k, float* Mc, float* Mr, int64_t ldm, cudaStream_t st)

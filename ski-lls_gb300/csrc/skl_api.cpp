@@ -294,6 +294,14 @@ struct SparseDev {
     const int64_t* Ap; const int64_t* Ai; const double* Ax; const double* b;
 };
 
+// Workspace of the Gram route, the FP64 path's probe included.
+template <typename T>
+static size_t gram_bytes(int64_t m, int64_t d, int64_t ld, bool multi, bool drops)
+{
+    const size_t probe = std::is_same<T, double>::value ? gram_probe_bytes(m, d, ld) : 0;
+    return std::max(gram_workspace_bytes<T>(m, d, multi, drops), probe);
+}
+
 // ------------------------------------------------------- sparse solve ---
 template <typename T>
 static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, double* x_dev,
@@ -314,7 +322,7 @@ static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, do
     // ---- workspace layout (sized once, then carved) ----
     const size_t qr_ws = cpqr_workspace_bytes<T>(m, d);
     const size_t inv_ws = std::max(trinv_workspace_bytes<T>(d) + (size_t)d * d * sizeof(T),
-                                   gram_enabled() && m >= d ? gram_workspace_bytes<T>(m, d, mixed, mixed) : 0);
+                                   gram_enabled() && m >= d ? gram_bytes<T>(m, d, ld, mixed, mixed) : 0);
     LsqrProblem Pq;
     Pq.n = n; Pq.d = d; Pq.nnz = nnz; Pq.r = d; Pq.precision = o.precision;
     const size_t lsqr_ws = lsqr_workspace_bytes(Pq);
@@ -473,6 +481,7 @@ static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, do
     // Cholesky of its Gram matrix, the rank proven from M; any other one:
     // randomized CPQR, rank by its diagonal
     const bool gram = gram_enabled() && m >= d &&
+                      gram_probe(SA, m, d, ld, jpvt, Mc, Mr, work, C.dev_status, C.host_pinned, st) &&
                       gram_precond<T>(SA, m, d, ld, cvec, jpvt, Mc, Mr, ldm, 0.0, rel, o.rcond_threshold, gres,
                                       carry_unresolved ? drop : nullptr, carry_unresolved, work, C.dev_status, C.host_pinned, st);
     if (gram) {
@@ -948,7 +957,7 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
     info.sketch_rows = m;
     const size_t qr_ws = cpqr_workspace_bytes<T>(m, d);
     const size_t inv_ws = std::max(trinv_workspace_bytes<T>(d),
-                                   gram_enabled() ? gram_workspace_bytes<T>(m, d, true, false) : 0);
+                                   gram_enabled() ? gram_bytes<T>(m, d, ld, true, false) : 0);
     LsqrProblem Pq;
     const bool tiled = lsqr_dense_tiled(d, o.precision);
     Pq.n = n; Pq.d = d; Pq.r = d; Pq.precision = o.precision;
@@ -1047,6 +1056,7 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
     int64_t ldm = round_up(d, 4);
     GramResult gres;
     const bool gram = gram_enabled() &&
+                      gram_probe(SA, m, d, ld, jpvt, Mc, Mr, work, C.dev_status, C.host_pinned, st) &&
                       gram_precond<T>(SA, m, d, ld, cpqr_on ? cvec : nullptr, jpvt, Mc, Mr, ldm,
                                       cpqr_on ? o.rcond : 0.0, floor_rel, 0.0, gres, nullptr, true, work,
                                       C.dev_status, C.host_pinned, st);
