@@ -1145,10 +1145,12 @@ LsqrResult lsqr_run(const LsqrProblem& P, const double* b, double tol, int64_t m
 // ------------------------------------------------------------- tuning --
 // Times the CSR product A z and the CSC product A^T u of this problem's matrix
 // for each lanes-per-row (column) choice, median of three launches after one
-// warm-up, and keeps the fastest in P.lanes_n / P.lanes_t.
+// warm-up, and keeps the fastest in P.lanes_n / P.lanes_t: the kernels, or the
+// persistent kernel's phases, that the solve will run.
 void tune_lsqr_products(LsqrProblem& P, void* work, cudaStream_t st)
 {
     if (P.Ad || P.n <= 0 || P.r <= 0) return;
+    if (lsqr_persist_fits(P)) return lsqr_persist_tune(P, work, st);
     LsqrBufs B = carve(P, work);
     LsqrState init{};
     init.ib = 1.0;

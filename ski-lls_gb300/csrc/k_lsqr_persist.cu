@@ -1608,13 +1608,12 @@ const PState* run_persistent(const PArgs<MIXED>& g, int G, size_t smem, void* ho
     return run_cooperative(fn, G <= kCluster, G, NT, smem, g.S, host_pinned, st, (void*)&a, nullptr);
 }
 
+// The kernels' arguments, and the column chunks that they name.
 template <bool MIXED, int NT>
-LsqrResult persist_impl(const LsqrProblem& P, const double* b, double tol, int64_t max_it, double* y_out, void* work,
-                        void* host_pinned, cudaStream_t st, int profile, cudaStream_t capture_stream)
+PArgs<MIXED> persist_args(const LsqrProblem& P, const PBufs& B, const double* b, cudaStream_t st)
 {
     using V = ValT<MIXED>;
     using MT = MatT<MIXED>;
-    PBufs B = pcarve(P, work);
     PArgs<MIXED> g{};
     g.n = (int)P.n;
     g.r = (int)P.r;
@@ -1663,6 +1662,16 @@ LsqrResult persist_impl(const LsqrProblem& P, const double* b, double tol, int64
     launch_k(k_chunk_fill, gr, 256, 0, st, P.cp, P.cols, (int)P.r, len, B.coff, B.chunks, B.ccnt);
     SKL_LAUNCHED();
     SKL_CUDA(cudaMemsetAsync(B.z, 0, P.d * sizeof(V), st));
+    return g;
+}
+
+template <bool MIXED, int NT>
+LsqrResult persist_impl(const LsqrProblem& P, const double* b, double tol, int64_t max_it, double* y_out, void* work,
+                        void* host_pinned, cudaStream_t st, int profile, cudaStream_t capture_stream)
+{
+    PBufs B = pcarve(P, work);
+    const PArgs<MIXED> g = persist_args<MIXED, NT>(P, B, b, st);
+    const int G = grid_of(P).ctas;
     PState init{};
     init.tol = tol;
     init.max_it = max_it;
@@ -1680,6 +1689,54 @@ LsqrResult persist_impl(const LsqrProblem& P, const double* b, double tol, int64
     res.it = hs->sc[0].it;
     y_launch(B.y, P.r, B.S, y_out, st);
     return res;
+}
+
+// Lanes per row and column by time: phases B and C at each choice, median of three
+// after a warm-up.  The persistent kernel runs the same phases on the same grid.
+template <bool MIXED, int NT>
+void persist_tune(LsqrProblem& P, void* work, cudaStream_t st)
+{
+    const PBufs B = pcarve(P, work);
+    struct Events {
+        cudaEvent_t e[2] = {nullptr, nullptr};
+        ~Events()
+        {
+            for (cudaEvent_t v : e)
+                if (v) cudaEventDestroy(v);
+        }
+    } ev;
+    for (auto& e : ev.e) SKL_CUDA(cudaEventCreate(&e));
+    PState init{};
+    for (PScal& sc : init.sc) sc.alpha = sc.beta = sc.rhobar = sc.phibar = sc.ia = sc.ib = sc.bs = 1.0;
+    SKL_CUDA(cudaMemcpyAsync(B.S, &init, sizeof(PState), cudaMemcpyHostToDevice, st));
+    SKL_CUDA(cudaMemsetAsync(B.us, 0, P.n * sizeof(ValT<MIXED>), st));
+    const int G = grid_of(P).ctas;
+    const size_t smem = vec_smem(P);
+    auto time_of = [&](auto&& launch) {
+        launch();
+        float t[3];
+        for (float& v : t) {
+            SKL_CUDA(cudaEventRecord(ev.e[0], st));
+            launch();
+            SKL_CUDA(cudaEventRecord(ev.e[1], st));
+            SKL_CUDA(cudaEventSynchronize(ev.e[1]));
+            SKL_CUDA(cudaEventElapsedTime(&v, ev.e[0], ev.e[1]));
+        }
+        std::sort(t, t + 3);
+        return t[1];
+    };
+    float best_n = 1e30f, best_t = 1e30f;
+    int ln = 0, lt = 0;
+    for (int L : {4, 8, 16, 32}) {
+        P.lanes_n = P.lanes_t = L;
+        const PArgs<MIXED> g = persist_args<MIXED, NT>(P, B, nullptr, st);
+        const float tn = time_of([&] { launch_phase<MIXED, NT, 5>(g, G, smem, st); });
+        if (tn < best_n) best_n = tn, ln = L;
+        const float tt = time_of([&] { launch_phase<MIXED, NT, 6>(g, G, smem, st); });
+        if (tt < best_t) best_t = tt, lt = L;
+    }
+    P.lanes_n = ln;
+    P.lanes_t = lt;
 }
 
 // ---- dense host side -------------------------------------------------------------
@@ -1876,6 +1933,14 @@ LsqrResult lsqr_persist_run(const LsqrProblem& P, const double* b, double tol, i
                    ? (big ? persist_impl<true, kBigCta> : persist_impl<true, kSmallCta>)
                    : (big ? persist_impl<false, kBigCta> : persist_impl<false, kSmallCta>);
     return fn(P, b, tol, max_it, y, work, host_pinned, st, profile, capture_stream);
+}
+
+void lsqr_persist_tune(LsqrProblem& P, void* work, cudaStream_t st)
+{
+    const bool big = grid_of(P).threads == kBigCta;
+    auto* fn = P.precision == SKL_PREC_MIXED ? (big ? persist_tune<true, kBigCta> : persist_tune<true, kSmallCta>)
+                                             : (big ? persist_tune<false, kBigCta> : persist_tune<false, kSmallCta>);
+    fn(P, work, st);
 }
 
 }  // namespace skl

@@ -229,10 +229,11 @@ static void check_opts(const skl_opts& o)
 // ------------------------------------------------------------ autotuning --
 // opts.autotune = 1: the first solve of a shape class times the candidates of
 // each tunable launch shape on its own data -- the sketch's block size, the
-// CPQR's panel width (whole factorizations of a copy of the sketch), the lanes
-// per row / column of LSQR's two sparse products -- and caches the fastest
-// for the process (skl_finalize clears the cache).  Shape class: precision
-// and half-octave buckets of n, d, nnz per row and m.
+// CPQR's panel width (whole factorizations of a copy of the sketch, the first time
+// that a solve of the class takes the CPQR), the lanes per row / column of LSQR's
+// two sparse products -- and caches the fastest for the process (skl_finalize
+// clears the cache).  Shape class: precision and half-octave buckets of n, d, nnz per
+// row and m.
 struct Tuned {
     int sketch_threads = 0, nb = 0, lanes_n = 0, lanes_t = 0;
 };
@@ -433,32 +434,6 @@ static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, do
     trace_phase(st, "sketch");
     SKL_CUDA(cudaEventRecord(ev[3], st));
     // ---- factorization of the sketch, c = coefficients of S b ----
-    if (tuning && mixed) {
-        // whole factorizations of a copy of the sketch at each panel width
-        T* SAc = nullptr;
-        double* cc = nullptr;
-        SKL_CUDA(cudaMallocAsync((void**)&SAc, (size_t)ld * d * sizeof(T), st));
-        SKL_CUDA(cudaMallocAsync((void**)&cc, (size_t)m * sizeof(double), st));
-        float best = 1e30f;
-        int last_nb = 0;
-        for (int cap : {64, 48, 32}) {
-            const int nbw = cpqr_panel_width(m, d, cap);
-            if (nbw == last_nb) continue;
-            last_nb = nbw;
-            const float t = time_median3(st, [&] {
-                SKL_CUDA(cudaMemcpyAsync(SAc, SA, (size_t)ld * d * sizeof(T), cudaMemcpyDeviceToDevice, st));
-                SKL_CUDA(cudaMemcpyAsync(cc, cvec, (size_t)m * sizeof(double), cudaMemcpyDeviceToDevice, st));
-                cpqr<T>(SAc, m, d, ld, jpvt, tau, work, C.dev_status, st, cc, 1, nullptr, nbw);
-            });
-            if (t < best) {
-                best = t;
-                tuned.nb = nbw;
-            }
-        }
-        SKL_CUDA(cudaFreeAsync(SAc, st));
-        SKL_CUDA(cudaFreeAsync(cc, st));
-        SKL_CUDA(cudaMemsetAsync(C.dev_status, 0, sizeof(unsigned), st));
-    }
     // ---- the rank rule ----
     // FP64: SPQR's default tolerance 20 (m + d) eps relative to the largest
     // (equilibrated) column.  FP32: an exactly dependent column leaves |R_ii|
@@ -491,6 +466,36 @@ static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, do
         info.success = 1;
         SKL_CUDA(cudaEventRecord(ev[4], st));
     } else {
+        if (o.autotune && mixed && tuned.nb == 0) {
+            // whole factorizations of a copy of the sketch at each panel width
+            T* SAc = nullptr;
+            double* cc = nullptr;
+            SKL_CUDA(cudaMallocAsync((void**)&SAc, (size_t)ld * d * sizeof(T), st));
+            SKL_CUDA(cudaMallocAsync((void**)&cc, (size_t)m * sizeof(double), st));
+            float best = 1e30f;
+            int last_nb = 0;
+            for (int cap : {64, 48, 32}) {
+                const int nbw = cpqr_panel_width(m, d, cap);
+                if (nbw == last_nb) continue;
+                last_nb = nbw;
+                const float t = time_median3(st, [&] {
+                    SKL_CUDA(cudaMemcpyAsync(SAc, SA, (size_t)ld * d * sizeof(T), cudaMemcpyDeviceToDevice, st));
+                    SKL_CUDA(cudaMemcpyAsync(cc, cvec, (size_t)m * sizeof(double), cudaMemcpyDeviceToDevice, st));
+                    cpqr<T>(SAc, m, d, ld, jpvt, tau, work, C.dev_status, st, cc, 1, nullptr, nbw);
+                });
+                if (t < best) {
+                    best = t;
+                    tuned.nb = nbw;
+                }
+            }
+            SKL_CUDA(cudaFreeAsync(SAc, st));
+            SKL_CUDA(cudaFreeAsync(cc, st));
+            SKL_CUDA(cudaMemsetAsync(C.dev_status, 0, sizeof(unsigned), st));
+            if (have_tuned) {
+                std::lock_guard<std::mutex> lk(g_tune_mu);
+                g_tune[tkey].nb = tuned.nb;
+            }
+        }
         cpqr<T>(SA, m, d, ld, jpvt, tau, work, C.dev_status, st, cvec, 1,
                 o.profile ? info.qr_prof_ms : nullptr, tuned.nb);
         {

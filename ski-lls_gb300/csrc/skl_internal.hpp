@@ -318,6 +318,8 @@ bool lsqr_persist_fits(const LsqrProblem& P);
 size_t lsqr_persist_workspace_bytes(const LsqrProblem& P);
 LsqrResult lsqr_persist_run(const LsqrProblem& P, const double* b, double tol, int64_t max_it, double* y, void* work,
                             void* host_pinned, cudaStream_t st, int profile, cudaStream_t capture_stream);
+// tune_lsqr_products on those phases
+void lsqr_persist_tune(LsqrProblem& P, void* work, cudaStream_t st);
 // Tile storage of a dense A for the one-pass products: whether the problem takes
 // it, its bytes, and its build from A (FP64, column-major), with the range check
 // (kStatusRange) and kFroParts partial sums of ||A||_F^2.
