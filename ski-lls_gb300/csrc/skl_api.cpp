@@ -121,19 +121,34 @@ skl_status run_guarded(void (*fn)(void*), void* arg)
 }
 
 // -------------------------------------------------------------- arena ----
-void Arena::reserve(size_t bytes)
+// SKILLS_WORKSPACE_MB=<n>: no arena beyond n MiB (a solve that needs more fails with
+// SKL_ERR_ALLOC, as where the device has no more).
+static size_t arena_limit()
 {
-    if (bytes <= cap_) return;
+    const char* e = std::getenv("SKILLS_WORKSPACE_MB");
+    return e ? (size_t)std::max(0ll, std::atoll(e)) << 20 : ~(size_t)0;
+}
+
+bool Arena::try_reserve(size_t bytes)
+{
+    if (bytes <= cap_) return true;
     release();
     bytes = (bytes + ((size_t)1 << 20) - 1) & ~(((size_t)1 << 20) - 1);
-    cudaError_t e = cudaMalloc((void**)&base_, bytes);
-    if (e != cudaSuccess) {
+    if (bytes > arena_limit()) return false;
+    if (cudaMalloc((void**)&base_, bytes) != cudaSuccess) {
         cudaGetLastError();
         base_ = nullptr;
-        fail(SKL_ERR_ALLOC, "device allocation of " + std::to_string(bytes >> 20) + " MiB failed");
+        return false;
     }
     cap_ = bytes;
     used_ = 0;
+    return true;
+}
+
+void Arena::reserve(size_t bytes)
+{
+    if (!try_reserve(bytes))
+        fail(SKL_ERR_ALLOC, "device allocation of " + std::to_string((bytes + ((size_t)1 << 20) - 1) >> 20) + " MiB failed");
 }
 
 void* Arena::take(size_t bytes)
@@ -321,9 +336,12 @@ static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, do
     info.sketch_rows = m;
 
     // ---- workspace layout (sized once, then carved) ----
+    // the Gram route where it applies and its workspace can be had, which is larger
+    // than the QR's
+    bool use_gram = gram_enabled() && m >= d;
     const size_t qr_ws = cpqr_workspace_bytes<T>(m, d);
-    const size_t inv_ws = std::max(trinv_workspace_bytes<T>(d) + (size_t)d * d * sizeof(T),
-                                   gram_enabled() && m >= d ? gram_bytes<T>(m, d, ld, mixed, mixed) : 0);
+    const size_t inv_ws = trinv_workspace_bytes<T>(d) + (size_t)d * d * sizeof(T);
+    const size_t gram_ws = use_gram ? gram_bytes<T>(m, d, ld, mixed, mixed) : 0;
     LsqrProblem Pq;
     Pq.n = n; Pq.d = d; Pq.nnz = nnz; Pq.r = d; Pq.precision = o.precision;
     const size_t lsqr_ws = lsqr_workspace_bytes(Pq);
@@ -337,11 +355,13 @@ static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, do
     S.add<int>(d); S.add<T>(mn); S.add<int>(4);
     S.add<T>(round_up(d, 4) * d); S.add<T>(round_up(d, 4) * d); S.add<double>(4);
     S.add<double>(d); S.add<double>(n); S.add<double>(d); S.add<double>(1024); S.add<double>(8);
-    S.add<char>((int64_t)std::max({qr_ws, inv_ws, lsqr_ws, csr_scr, bkt_scr}));
     S.add<float2>(d);
     S.add<double>(m);
     S.add<int>(kGramDropMax);
-    C.arena.reserve(S.bytes());
+    size_t work_bytes = std::max({qr_ws, inv_ws, lsqr_ws, csr_scr, bkt_scr});
+    use_gram = use_gram && C.arena.try_reserve(S.bytes() + std::max(work_bytes, gram_ws));
+    if (use_gram) work_bytes = std::max(work_bytes, gram_ws);
+    else C.arena.reserve(S.bytes() + work_bytes);
     C.arena.reset();
     Arena& Ar = C.arena;
     int* cp = Ar.alloc<int>(d + 1);
@@ -369,7 +389,7 @@ static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, do
     double* xacc = Ar.alloc<double>(d);
     double* part = Ar.alloc<double>(1024);
     double* scal = Ar.alloc<double>(8);
-    void* work = Ar.take(std::max({qr_ws, inv_ws, lsqr_ws, csr_scr, bkt_scr}));
+    void* work = Ar.take(work_bytes);
     float2* ysplit = Ar.alloc<float2>(d);
     int* drop = Ar.alloc<int>(kGramDropMax);
     double* gm = Ar.alloc<double>(m);   // S r_s during the sketch-solution refinement
@@ -455,7 +475,7 @@ static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, do
     // a well-conditioned sketch (but for exactly dependent columns, carried below):
     // Cholesky of its Gram matrix, the rank proven from M; any other one:
     // randomized CPQR, rank by its diagonal
-    const bool gram = gram_enabled() && m >= d &&
+    const bool gram = use_gram &&
                       gram_probe(SA, m, d, ld, jpvt, Mc, Mr, work, C.dev_status, C.host_pinned, st) &&
                       gram_precond<T>(SA, m, d, ld, cvec, jpvt, Mc, Mr, ldm, 0.0, rel, o.rcond_threshold, gres,
                                       carry_unresolved ? drop : nullptr, carry_unresolved, work, C.dev_status, C.host_pinned, st);
@@ -961,8 +981,10 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
     const int64_t mn = std::min(m, d);
     info.sketch_rows = m;
     const size_t qr_ws = cpqr_workspace_bytes<T>(m, d);
-    const size_t inv_ws = std::max(trinv_workspace_bytes<T>(d),
-                                   gram_enabled() ? gram_bytes<T>(m, d, ld, true, false) : 0);
+    const size_t inv_ws = trinv_workspace_bytes<T>(d);
+    // as on the sparse path: the Gram route where its workspace can be had
+    bool use_gram = gram_enabled();
+    const size_t gram_ws = use_gram ? gram_bytes<T>(m, d, ld, true, false) : 0;
     LsqrProblem Pq;
     const bool tiled = lsqr_dense_tiled(d, o.precision);
     Pq.n = n; Pq.d = d; Pq.r = d; Pq.precision = o.precision;
@@ -971,7 +993,7 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
     const size_t lsqr_ws = lsqr_workspace_bytes(Pq);
     const size_t bkt_scr = build_buckets_scratch_ints(m, N * k) * sizeof(int);
     const size_t dht_ws = dht_scratch_bytes(N, o.precision);
-    const size_t work_bytes = std::max({qr_ws, inv_ws, lsqr_ws, bkt_scr, dht_ws});
+    size_t work_bytes = std::max({qr_ws, inv_ws, lsqr_ws, bkt_scr, dht_ws});
     const int64_t ldm_max = round_up(d, 4);
     Sizer S;
     S.add<double>(n); S.add<unsigned>(N * k); S.add<int>(m + 1); S.add<unsigned>(N * k);
@@ -980,8 +1002,10 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
     S.add<T>(ld * d); S.add<double>(d); S.add<double>(m); S.add<int>(d); S.add<T>(mn); S.add<int>(4);
     S.add<T>(ldm_max * d); S.add<T>(ldm_max * d); S.add<double>(4); S.add<double>(d);
     S.add<double>(n); S.add<double>(d); S.add<double>(1024); S.add<double>(8);
-    S.add<char>((int64_t)work_bytes); S.add<float2>(d);
-    C.arena.reserve(S.bytes());
+    S.add<float2>(d);
+    use_gram = use_gram && C.arena.try_reserve(S.bytes() + std::max(work_bytes, gram_ws));
+    if (use_gram) work_bytes = std::max(work_bytes, gram_ws);
+    else C.arena.reserve(S.bytes() + work_bytes);
     C.arena.reset();
     Arena& Ar = C.arena;
     double* Dd = Ar.alloc<double>(n);
@@ -1060,7 +1084,7 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
     int64_t rank = d;
     int64_t ldm = round_up(d, 4);
     GramResult gres;
-    const bool gram = gram_enabled() &&
+    const bool gram = use_gram &&
                       gram_probe(SA, m, d, ld, jpvt, Mc, Mr, work, C.dev_status, C.host_pinned, st) &&
                       gram_precond<T>(SA, m, d, ld, cpqr_on ? cvec : nullptr, jpvt, Mc, Mr, ldm,
                                       cpqr_on ? o.rcond : 0.0, floor_rel, 0.0, gres, nullptr, true, work,

@@ -41,7 +41,8 @@ void reset_launch_count();
 // Grow-only device arena; one per device context, bump-allocated per solve.
 class Arena {
 public:
-    void reserve(size_t bytes);
+    void reserve(size_t bytes);        // or SKL_ERR_ALLOC
+    bool try_reserve(size_t bytes);    // false: nothing is reserved
     void reset() { used_ = 0; }
     void* take(size_t bytes);
     template <typename T>
