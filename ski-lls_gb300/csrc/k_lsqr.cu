@@ -1142,6 +1142,23 @@ LsqrResult lsqr_run(const LsqrProblem& P, const double* b, double tol, int64_t m
     return run_impl<false>(P, b, tol, max_it, y, work, host_pinned, st, profile, capture_stream);
 }
 
+void split_dense_load();
+
+// The dense mixed kernels, loaded (CUDA does so at their first use).
+void lsqr_load_dense_kernels()
+{
+    cudaFuncAttributes fa;
+    SKL_CUDA(cudaFuncGetAttributes(&fa, k_spmv_n_dense<true>));
+    SKL_CUDA(cudaFuncGetAttributes(&fa, k_spmv_n_dense_reduce<true>));
+    SKL_CUDA(cudaFuncGetAttributes(&fa, k_spmv_t_dense<true>));
+    SKL_CUDA(cudaFuncGetAttributes(&fa, k_tri_n<true>));
+    SKL_CUDA(cudaFuncGetAttributes(&fa, k_tri_t<true>));
+    SKL_CUDA(cudaFuncGetAttributes(&fa, k_lsqr_init_u<true>));
+    SKL_CUDA(cudaFuncGetAttributes(&fa, k_lsqr_init_v<true>));
+    SKL_CUDA(cudaFuncGetAttributes(&fa, k_lsqr_update<true>));
+    split_dense_load();
+}
+
 // ------------------------------------------------------------- tuning --
 // Times the CSR product A z and the CSC product A^T u of this problem's matrix
 // for each lanes-per-row (column) choice, median of three launches after one
@@ -1738,6 +1755,12 @@ __global__ void k_split_dense(const double* __restrict__ A, int64_t lda, int64_t
         out[e] = make_float2(f.hi, f.lo);
     }
     if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(status, kStatusRange);
+}
+
+void split_dense_load()
+{
+    cudaFuncAttributes fa;
+    SKL_CUDA(cudaFuncGetAttributes(&fa, k_split_dense));
 }
 
 void split_dense(const double* A, int64_t lda, int64_t n, int64_t d, float2* out,

@@ -16,7 +16,8 @@
 // has four barriers; each CTA reduces the norms' partials itself, in the same
 // order, and runs the scalar recurrences redundantly.  Small problems run as
 // one 16-CTA cluster (hardware barrier, no co-residency to ask for, so several
-// of them share the GPU), larger ones as a cooperative grid of one CTA per SM.
+// of them share the GPU), larger ones as a grid of one CTA per SM, whose CTAs first
+// make sure that all of them run (meet_all).
 //
 // Work split: phases A and D deal the triangle's rows (columns) to the CTAs in
 // snake order, so that every CTA has long and short ones, and cut each into S
@@ -36,8 +37,11 @@
 #include <algorithm>
 #include <chrono>
 #include <cmath>
+#include <cstddef>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
+#include <utility>
 #include <vector>
 
 #include "skl_internal.hpp"
@@ -82,8 +86,11 @@ struct PState {
     double tol;
     long long max_it;
     unsigned bar;          // grid barrier arrivals of this launch
+    unsigned meet;         // its CTAs that have started; kMeetOff: called off
     int timeout;
 };
+constexpr unsigned kMeetOff = 1u << 31;
+constexpr long long kMeetNs = 20000000;   // a launch waits this long for its CTAs
 
 template <bool MIXED>
 struct PArgs {
@@ -132,6 +139,40 @@ SKL_DEV bool bar_all(PState* S, unsigned& gen)
         __syncthreads();
         return s_ok != 0;
     }
+}
+
+SKL_DEV long long now_ns()
+{
+    long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// Whether all CTAs of the grid run at once, the same answer in each.  With one that
+// does not start within kMeetNs (another stream's kernel holds an SM) the launch is
+// called off and the CTAs leave, the late ones too, so that the solve can go on in
+// kernels that share the GPU.  A cooperative launch would wait for that kernel's
+// end, which may itself wait for what the caller does after the solve.
+SKL_DEV bool meet_all(PState* S)
+{
+    __shared__ int s_all;
+    if (threadIdx.x == 0) {
+        const unsigned G = gridDim.x;
+        const long long t0 = now_ns();
+        unsigned v = atomicAdd(&S->meet, 1u) + 1;
+        for (unsigned k = 0; !(v & kMeetOff) && v < G; ++k) {
+            if (now_ns() - t0 > kMeetNs || k >= kBarLimit) {
+                // called off unless the last one has arrived meanwhile
+                const unsigned was = atomicCAS(&S->meet, v, v | kMeetOff);
+                v = was == v ? v | kMeetOff : was;
+            } else {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&S->meet) : "memory");
+            }
+        }
+        s_all = !(v & kMeetOff);
+    }
+    __syncthreads();
+    return s_all != 0;
 }
 
 // Sum of ||u||^2.  GB300 issues two FP64 FMAs per SM and cycle, so one FP64
@@ -736,6 +777,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_lsqr_persist(const PArgs<MIXE
     pdl_wait();
     SKL_CTA(MIXED, NT);
     PState* S = g.S;
+    if constexpr (!CLUSTER)
+        if (!meet_all(S)) return;
     unsigned gen = 0;
     auto give_up = [&] {
         if (c.tid == 0) S->timeout = 1;
@@ -892,13 +935,6 @@ SKL_DEV void ff_norm(ff& a)
     a.hi = h;
 }
 
-SKL_DEV long long now_ns()
-{
-    long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
 // Sum over the warp of N values per lane (N a power of two): lane l ends with value
 // l / (32 / N).  Halving exchanges, then a plain butterfly: fixed order.
 template <int N>
@@ -936,6 +972,7 @@ k_lsqr_dense(const PArgs<true> g, const DArgs a, int start, int budget)
     __shared__ __align__(16) float4 s_u[RB];
     __shared__ float2 s_red[C::kYWarp][32];
     PState* S = g.S;
+    if (!meet_all(S)) return;
     const int tid = c.tid, lane = c.lane, warp = c.warp;
     const int CW = a.CW, NS = a.nslots;
     const unsigned chunk_bytes = (unsigned)CW * 16;
@@ -1475,15 +1512,18 @@ struct Clock {
 
 // Phase kernels: a graph of kIterPerGraph iterations, replayed until the state
 // says done; the next replay is queued before the last one's state is read, so
-// the GPU does not wait for the host.  profile: events around the products.
+// the GPU does not wait for the host.  start: from b, else from slot 0's state.
+// profile: events around the products.
 template <bool MIXED, int NT>
 const PState* run_phases(const PArgs<MIXED>& g, int G, size_t smem, void* host_pinned, cudaStream_t st,
-                         cudaStream_t cap, int profile, LsqrResult& res)
+                         cudaStream_t cap, bool start, int profile, LsqrResult& res)
 {
-    launch_phase<MIXED, NT, 0>(g, G, smem, st);
-    launch_phase<MIXED, NT, 1>(g, G, smem, st);
-    launch_phase<MIXED, NT, 2>(g, G, smem, st);
-    launch_phase<MIXED, NT, 3>(g, G, smem, st);
+    if (start) {
+        launch_phase<MIXED, NT, 0>(g, G, smem, st);
+        launch_phase<MIXED, NT, 1>(g, G, smem, st);
+        launch_phase<MIXED, NT, 2>(g, G, smem, st);
+        launch_phase<MIXED, NT, 3>(g, G, smem, st);
+    }
     struct Owned {
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
@@ -1560,9 +1600,10 @@ const PState* run_phases(const PArgs<MIXED>& g, int G, size_t smem, void* host_p
 }
 
 // The launches of a persistent kernel fn(args, more, start, budget) until the
-// state says done.
-const PState* run_cooperative(const void* fn, bool cluster, int G, int threads, size_t smem, PState* S, void* host_pinned,
-                              cudaStream_t st, void* arg0, void* arg1)
+// state says done, or one is called off (meet_all): false, with the state of the
+// launches before it.
+bool run_resident(const void* fn, bool cluster, int G, int threads, size_t smem, PState* S, void* host_pinned,
+                  cudaStream_t st, void* arg0, void* arg1)
 {
     if (cluster) SKL_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
@@ -1575,12 +1616,9 @@ const PState* run_cooperative(const void* fn, bool cluster, int G, int threads, 
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = kCluster;
         at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    } else {
-        at[0].id = cudaLaunchAttributeCooperative;
-        at[0].val.cooperative = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
     }
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
     const PState* hs = (const PState*)host_pinned;
     const Clock clock;
     for (int start = 1;; start = 0) {
@@ -1592,20 +1630,35 @@ const PState* run_cooperative(const void* fn, bool cluster, int G, int threads, 
         SKL_CUDA(cudaMemcpyAsync(host_pinned, S, sizeof(PState), cudaMemcpyDeviceToHost, st));
         SKL_CUDA(cudaStreamSynchronize(st));
         if (hs->timeout) fail(SKL_ERR_TIMEOUT, "a bounded wait gave up (LSQR's grid barrier or its copies)");
-        if (hs->sc[0].done) return hs;
+        if (hs->meet & kMeetOff) return false;
+        if (hs->sc[0].done) return true;
         clock.check();
-        SKL_CUDA(cudaMemsetAsync(&S->bar, 0, sizeof(unsigned), st));
+        static_assert(offsetof(PState, meet) == offsetof(PState, bar) + sizeof(unsigned), "reset together");
+        SKL_CUDA(cudaMemsetAsync(&S->bar, 0, 2 * sizeof(unsigned), st));
     }
 }
 
+// The phase kernels loaded before a persistent launch can be called off: loading one
+// (CUDA does so at its first use) may itself wait for the kernel that holds the SM.
+template <bool MIXED, int NT, int... PH>
+void load_phases(std::integer_sequence<int, PH...>)
+{
+    cudaFuncAttributes fa;
+    (SKL_CUDA(cudaFuncGetAttributes(&fa, k_lsqr_phase<MIXED, NT, PH>)), ...);
+}
+
 template <bool MIXED, int NT>
-const PState* run_persistent(const PArgs<MIXED>& g, int G, size_t smem, void* host_pinned, cudaStream_t st)
+bool run_persistent(const PArgs<MIXED>& g, int G, size_t smem, void* host_pinned, cudaStream_t st)
 {
     const void* fn = G <= kCluster ? (const void*)k_lsqr_persist<MIXED, NT, true>
                                    : (const void*)k_lsqr_persist<MIXED, NT, false>;
     allow_max_dynamic_smem(fn);
+    if (G > kCluster) {
+        static std::once_flag once;
+        std::call_once(once, [] { load_phases<MIXED, NT>(std::make_integer_sequence<int, 8>{}); });
+    }
     PArgs<MIXED> a = g;
-    return run_cooperative(fn, G <= kCluster, G, NT, smem, g.S, host_pinned, st, (void*)&a, nullptr);
+    return run_resident(fn, G <= kCluster, G, NT, smem, g.S, host_pinned, st, (void*)&a, nullptr);
 }
 
 // The kernels' arguments, and the column chunks that they name.
@@ -1680,10 +1733,13 @@ LsqrResult persist_impl(const LsqrProblem& P, const double* b, double tol, int64
     trace_phase(st, "lsqr: init");
     const size_t smem = vec_smem(P);
     LsqrResult res;
-    const PState* hs =
-        profile || P.shared_gpu
-            ? run_phases<MIXED, NT>(g, G, smem, host_pinned, st, capture_stream ? capture_stream : st, profile, res)
-            : run_persistent<MIXED, NT>(g, G, smem, host_pinned, st);
+    const PState* hs = (const PState*)host_pinned;
+    const bool phases = profile || P.shared_gpu;
+    if (phases || !run_persistent<MIXED, NT>(g, G, smem, host_pinned, st)) {
+        // the state is the start's unless a launch before the one called off ended
+        const bool start = phases || hs->sc[0].it == 0;
+        hs = run_phases<MIXED, NT>(g, G, smem, host_pinned, st, capture_stream ? capture_stream : st, start, profile, res);
+    }
     trace_phase(st, "lsqr: done");
     res.flag = hs->sc[0].flag;
     res.it = hs->sc[0].it;
@@ -1846,6 +1902,8 @@ LsqrResult dense_impl(const LsqrProblem& P, const double* b, double tol, int64_t
     a.ntiles = s.ntiles;
     a.sv_bytes = (int)((std::max(vec_smem(P), (size_t)s.K * kDT * sizeof(float2)) + 127) & ~(size_t)127);
     const void* fn = dense_kernel(s.K);
+    static std::once_flag once;
+    std::call_once(once, [] { lsqr_load_dense_kernels(); });   // as load_phases
     allow_max_dynamic_smem(fn);
     cudaFuncAttributes fa;
     SKL_CUDA(cudaFuncGetAttributes(&fa, fn));
@@ -1861,10 +1919,14 @@ LsqrResult dense_impl(const LsqrProblem& P, const double* b, double tol, int64_t
     SKL_CUDA(cudaMemcpyAsync(B.S, &init, sizeof(PState), cudaMemcpyHostToDevice, st));
     norm_launch(b, P.n, B.bpart, st);
     trace_phase(st, "lsqr: init");
-    const PState* hs = run_cooperative(fn, false, G, kDT, (size_t)a.sv_bytes + (size_t)a.nslots * s.CW * 16, B.S, host_pinned,
-                                       st, (void*)&g, (void*)&a);
-    trace_phase(st, "lsqr: done");
     LsqrResult res;
+    if (!run_resident(fn, false, G, kDT, (size_t)a.sv_bytes + (size_t)a.nslots * s.CW * 16, B.S, host_pinned, st,
+                      (void*)&g, (void*)&a)) {
+        res.called_off = true;
+        return res;
+    }
+    const PState* hs = (const PState*)host_pinned;
+    trace_phase(st, "lsqr: done");
     res.flag = hs->sc[0].flag;
     res.it = hs->sc[0].it;
     if (profile) {

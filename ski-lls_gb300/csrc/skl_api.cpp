@@ -988,9 +988,12 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
     LsqrProblem Pq;
     const bool tiled = lsqr_dense_tiled(d, o.precision);
     Pq.n = n; Pq.d = d; Pq.r = d; Pq.precision = o.precision;
-    if (tiled) Pq.At = A;
-    else Pq.Ad = A, Pq.lda = n;
-    const size_t lsqr_ws = lsqr_workspace_bytes(Pq);
+    Pq.Ad = A, Pq.lda = n;
+    size_t lsqr_ws = lsqr_workspace_bytes(Pq);
+    if (tiled) {
+        Pq.At = A;
+        lsqr_ws = std::max(lsqr_ws, lsqr_workspace_bytes(Pq));
+    }
     const size_t bkt_scr = build_buckets_scratch_ints(m, N * k) * sizeof(int);
     const size_t dht_ws = dht_scratch_bytes(N, o.precision);
     size_t work_bytes = std::max({qr_ws, inv_ws, lsqr_ws, bkt_scr, dht_ws});
@@ -1138,6 +1141,19 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
             info.prof_launches[q] += Rr.prof_launches[q];
         }
     };
+    auto solve = [&](const double* rhs, int64_t max_it) {
+        auto run = [&] {
+            return lsqr_run(P, rhs, o.it_tol, max_it, yv, work, C.dev_status, C.host_pinned, st, o.profile, C.stream);
+        };
+        LsqrResult R = run();
+        if (R.called_off) {   // on kernels that share the GPU, and their storage of A, from here on
+            split_dense(A, lda, n, d, A2, C.dev_status, st);
+            P.At = nullptr;
+            P.Ad = A2;
+            R = run();
+        }
+        return R;
+    };
     SKL_CUDA(cudaMemsetAsync(x_dev, 0, d * sizeof(double), st));
     info.it = 0;
     info.flag = 0;
@@ -1154,8 +1170,7 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
         // LSQR on A P1 M from r_s (CPQR path) or from b with y = 0 (noCPQR path)
         const double* rhs = b;
         if (cpqr_on) rhs = rs;
-        LsqrResult R = lsqr_run(P, rhs, o.it_tol, o.max_it, yv, work, C.dev_status, C.host_pinned,
-                                st, o.profile, C.stream);
+        LsqrResult R = solve(rhs, o.max_it);
         add_prof(R);
         int64_t total_it = R.it;
         int flag = R.flag;
@@ -1170,8 +1185,7 @@ static bool dense_pipeline(Context& C, cudaStream_t st, const double* A, int64_t
         while (o.backward_tol > 0.0 && be > o.backward_tol && restarts < o.max_refine &&
                total_it < o.max_it) {
             ++restarts;
-            R = lsqr_run(P, rs, o.it_tol, o.max_it - total_it, yv, work, C.dev_status,
-                         C.host_pinned, st, o.profile, C.stream);
+            R = solve(rs, o.max_it - total_it);
             add_prof(R);
             total_it += R.it;
             flag = R.flag;

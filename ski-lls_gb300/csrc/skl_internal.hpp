@@ -306,6 +306,8 @@ struct LsqrResult {
     int64_t it = 0;
     double prof_ms[4] = {0, 0, 0, 0};      // A*z, A^T*u, M*v, M^T*t (profile = 1)
     int64_t prof_launches[4] = {0, 0, 0, 0};
+    // one-pass dense kernel: another stream's kernel holds an SM, nothing was solved
+    bool called_off = false;
 };
 
 size_t lsqr_workspace_bytes(const LsqrProblem& P);
@@ -313,6 +315,7 @@ size_t lsqr_workspace_bytes(const LsqrProblem& P);
 LsqrResult lsqr_run(const LsqrProblem& P, const double* b, double tol, int64_t max_it, double* y,
                     void* work, unsigned* status, void* host_pinned, cudaStream_t st,
                     int profile = 0, cudaStream_t capture_stream = nullptr);
+void lsqr_load_dense_kernels();
 // The sparse iteration as one persistent kernel, or as phase kernels with the same
 // bits (k_lsqr_persist.cu), where the problem's vectors fit shared memory.
 bool lsqr_persist_fits(const LsqrProblem& P);
