@@ -310,6 +310,15 @@ struct SparseDev {
     const int64_t* Ap; const int64_t* Ai; const double* Ax; const double* b;
 };
 
+// Rows, entries and sketch rows are counted in 32 bits on the device, by loops that
+// step past their end by up to a grid's threads (at most 2^18): the last 2^20 below
+// 2^31 are refused with what lies beyond.
+constexpr int64_t kMaxIndex = 0x7fffffff - (1 << 20);
+static void check_index(int64_t v)
+{
+    if (v > kMaxIndex) fail(SKL_ERR_INVALID, "problem too large for 32-bit device indices");
+}
+
 // Workspace of the Gram route, the FP64 path's probe included.
 template <typename T>
 static size_t gram_bytes(int64_t m, int64_t d, int64_t ld, bool multi, bool drops)
@@ -328,8 +337,7 @@ static void sparse_pipeline(Context& C, cudaStream_t st, const SparseDev& in, do
     const int64_t k = o.k;
     const int64_t m = (int64_t)std::ceil((double)d * o.gamma);
     if (k > m) fail(SKL_ERR_INVALID, "k exceeds the sketch size m = ceil(gamma*d)");
-    if (m > 0x7fffffff || nnz > 0x7fffffff || n > 0x7fffffff)
-        fail(SKL_ERR_INVALID, "problem too large for 32-bit device indices");
+    for (int64_t v : {m, nnz, n}) check_index(v);
     const bool mixed = std::is_same<T, float>::value;
     const int64_t ld = round_up(m, 32);
     const int64_t mn = std::min(m, d);
@@ -729,6 +737,7 @@ static void validate_csc_header(const skl_csc* A)
     if (A->m < 0 || A->n < 0) fail(SKL_ERR_INVALID, "negative dimension");
     if (A->n > 0 && (!A->p)) fail(SKL_ERR_INVALID, "A->p is null");
     if (A->m < A->n) fail(SKL_ERR_NOT_OVERDETERMINED, "Matrix is not overdetermined.");
+    check_index(A->m);
 }
 
 // One sparse solve on context C and stream st.  The hash stream arrives
@@ -747,6 +756,7 @@ static void sparse_solve_core(Context& C, cudaStream_t st, const skl_csc* A, con
     if (host) {
         if (!A->p) fail(SKL_ERR_INVALID, "A->p is null");
         nnz = A->p[d];
+        check_index(nnz);
         if (nnz < 0) fail(SKL_ERR_INVALID, "negative nnz");
         if (nnz > 0 && (!A->i || !A->x)) fail(SKL_ERR_INVALID, "A->i or A->x is null");
         Sizer S;
@@ -800,6 +810,7 @@ static void sparse_solve_common(const skl_csc* A, const double* b, double* x, co
         if (info) *info = inf;
         return;
     }
+    if (host) check_index(A->p[d]);
     Context& C = context(o.device, 0);
     reset_launch_count();
     cudaStream_t st = o.stream ? (cudaStream_t)o.stream : C.stream;
@@ -1251,6 +1262,7 @@ static void dense_solve_common(const double* A, int64_t lda, int64_t n, int64_t 
     if (n < d) fail(SKL_ERR_NOT_OVERDETERMINED, "Matrix is not overdetermined.");
     if (!A || !b || !x) fail(SKL_ERR_INVALID, "A, b or x is null");
     if (lda < std::max<int64_t>(1, n)) fail(SKL_ERR_INVALID, "lda < n");
+    for (double v : {(double)n, std::ceil((double)d * o.gamma)}) check_index((int64_t)std::min(v, 1e18));
     skl_info inf;
     std::memset(&inf, 0, sizeof inf);
     if (d == 0) {
@@ -1261,9 +1273,9 @@ static void dense_solve_common(const double* A, int64_t lda, int64_t n, int64_t 
     reset_launch_count();
     cudaStream_t st = o.stream ? (cudaStream_t)o.stream : C.stream;
     const int64_t N = dht_length(n, o.wisdom);
+    check_index(N);
     const int64_t m = (int64_t)std::ceil((double)d * o.gamma);
     if (o.k > m) fail(SKL_ERR_INVALID, "k exceeds the sketch size m = ceil(gamma*d)");
-    if (N > 0x7fffffff || m > 0x7fffffff) fail(SKL_ERR_INVALID, "problem too large");
     if (sample_rows && m > N)
         fail(SKL_ERR_INVALID, "the sample has more rows (ceil(gamma*d)) than the transform");
     // signs then hash from one reseeded stream (srand(time(NULL)) in the
