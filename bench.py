@@ -593,6 +593,9 @@ def run_ours(args, rank, world):
                     "peak_kind": peak_kind, "alg_bytes_per_launch": kk["alg_bytes"]}
         if "note" in kk:
             roofline["note"] = kk["note"]
+        elif dom.startswith("lsqr_") and P.kind != "dense":
+            roofline["note"] = ("a phase of the LSQR kernel, timed as a kernel of its own; the timed solve runs "
+                                "the phases in one kernel")
 
     # ---- e2e through the host-pointer C ABI (pinned host buffers, copies timed)
     e2e = None

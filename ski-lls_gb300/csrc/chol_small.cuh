@@ -54,8 +54,8 @@ template <> SKL_DEV double t_rcp_chain<double>(double x) { return __drcp_rn(x); 
 
 // X = U^{-1} for the upper 16 x 16 block U (entries below its diagonal never
 // read): X's upper triangle, and zeros below it when zero_lower.  A zero
-// diagonal entry (a failed Cholesky pivot) leaves its row and column of X zero:
-// X is then the inverse of the rest.
+// diagonal entry leaves its row and column of X zero: X is then the inverse of
+// the rest.
 template <typename T>
 SKL_DEV void warp16_inv_upper(const T* U, int ldu, T* X, int ldx, bool zero_lower)
 {

@@ -26,9 +26,9 @@
 // same is done again on Q = S A M (at most twice): each pass takes the condition
 // number to about the root of what exceeds ~300.  40,000 x 4,000 (S A 6,800 x 4,000):
 // QR and inverse 20.2 + 1.4 ms, one pass ~3.3 ms, two (condition number 1e3 to
-// 1e5) 7.5 ms with LSQR's iterations, x and residual unchanged.  Beyond, by size
-// (12,007 x 1,201: from 1e7 on), attempts end early and the QR comes on top of a
-// pass's time.
+// 1e4) 7.4 ms, three (to 1e6) 11.4 with LSQR's iterations, x and residual unchanged.
+// From ~3e6 on at that size (12,007 x 1,201: 1e7) M is too large for the rank proof,
+// and the QR comes on top of the passes.
 // The sparse path takes the later passes where no pivot failed but the bound on M D
 // does, or where the dropped columns are all at least four thresholds away from
 // dependence (120,000 x 5,000, S A 8,500 x 5,000: 11.2 and 16 to 19 ms; the QR and
@@ -1515,9 +1515,10 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
         // Too ill-conditioned for its Gram matrix, or with boosted pivots: the same
         // on Q = S A M, whose condition number is about the root of the excess, at
         // most twice; M and R are the passes' products.  Boosted pivots can make a
-        // pass's inverse grow (at 1e5 and beyond, by size), which costs the product
-        // its digits and ends the attempt: eps ||S A|| ||M_1|| ||M_2|| was at most 30
-        // where LSQR took the QR's iterations.
+        // pass's inverse grow, which costs the product its digits: the limit of 64 on
+        // eps ||S A|| ||M_1|| ||M_2|| stands above what accepted attempts showed (1,500
+        // x 100 to 40,000 x 4,000, condition numbers to 3e7: at most 15; 30 to 257
+        // where the rank rule below refused) and keeps a runaway from a third pass.
         const double unit = (double)eps * std::sqrt(gmax);
         if (unit * std::sqrt(mf2 * (double)d) > 64.0) return false;
         for (int pass = 2;; ++pass) {

@@ -1,4 +1,8 @@
-// k_lsqr.cu -- preconditioned LSQR on the GPU.
+// k_lsqr.cu -- preconditioned LSQR on the GPU, as kernels of a few CTAs per SM, and
+// the FP64 residual checks and preconditioner products around it.  Most solves take
+// the resident kernels of k_lsqr_persist.cu; these serve FP64 and very wide dense
+// problems, sparse ones whose vectors do not fit shared memory, a dense solve beside
+// another stream's kernel that keeps an SM, and SKILLS_LSQR_PERSIST=0.
 //
 // Restates the Paige-Saunders recurrences of lsqr() (src/IterSolver.cpp:160-284)
 // for the operator Abar = A * P1 * D * M of LinOP_sparse_preconditioner /

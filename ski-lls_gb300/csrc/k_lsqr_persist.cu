@@ -33,7 +33,8 @@
 // an acquire poll by one thread; fences of its own around them cost 0.3 us more)
 // and ~2.5 to 4 us per phase.  What a phase reads that the previous one does not
 // write (first row and chunk, old u and v, column numbers) is on its way before
-// the staged vector arrives: 21.4 -> 19.1 us per iteration at 20,000 x 1,000.
+// the staged vector arrives; with the short barriers, 22.6 -> 19.1 us per iteration at
+// 20,000 x 1,000.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
