@@ -1571,7 +1571,7 @@ size_t gram_probe_bytes(int64_t m, int64_t d, int64_t ld)
 {
     if (d < kGramProbeCols) return 0;
     return up256((size_t)ld * d * sizeof(float)) + up256(kGramDropMax * sizeof(int)) +
-           gram_workspace_bytes<float>(m, d, false, true);
+           gram_workspace_bytes<float>(m, d, true, true);
 }
 
 bool gram_probe(const double* SA, int64_t m, int64_t d, int64_t ld, int* jpvt, double* Mc, double* Mr, void* work,
@@ -1583,11 +1583,16 @@ bool gram_probe(const double* SA, int64_t m, int64_t d, int64_t ld, int* jpvt, d
     void* rest = (char*)drop + up256(kGramDropMax * sizeof(int));
     launch_k(k_gc_narrow, dim3((unsigned)((m + 1023) / 1024), (unsigned)d), 256, 0, st, SA, ld, (int)m, SAf);
     SKL_LAUNCHED();
-    const double rel = 2.0 * std::sqrt((double)m) * 5.960464477539063e-08;
+    const double eps = 5.960464477539063e-08;
     GramResult res;
-    const bool found = gram_precond<float>(SAf, m, d, ld, nullptr, jpvt, (float*)Mc, (float*)Mr, (d + 3) / 4 * 4, 0.0,
-                                           rel, 0.0, res, drop, false, rest, status, host_pinned, st);
-    return !(found && res.dropped > 0);
+    auto attempt = [&](double rel, int* dropped) {
+        return gram_precond<float>(SAf, m, d, ld, nullptr, jpvt, (float*)Mc, (float*)Mr, (d + 3) / 4 * 4, 0.0, rel, 0.0,
+                                   res, dropped, true, rest, status, host_pinned, st);
+    };
+    if (attempt(2.0 * std::sqrt((double)m) * eps, drop)) return res.dropped == 0;
+    // too ill-conditioned for that: as far as FP32 passes resolve it (~1e6) the FP64
+    // Gram matrix (~1e7) does
+    return attempt(eps, nullptr);
 }
 
 void gram_unit_dropped(const int* drop, int64_t k, float* Mc, float* Mr, int64_t ldm, cudaStream_t st)

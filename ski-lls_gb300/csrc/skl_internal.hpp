@@ -249,11 +249,13 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
                   double abs_thresh, double rel_thresh, double rcond_min, GramResult& res, int* drop, bool multi, void* work,
                   unsigned* status, void* host_pinned, cudaStream_t st);
 // Whether gram_precond<double> is worth its attempt: false where the FP32 one finds
-// columns that depend on the others (the FP64 sweep then almost surely ends at one
-// of them, after the FP64 Gram matrix).  From kGramProbeCols columns on: 40,000 x
-// 2,000, 20 dependent columns: 128 ms with the FP64 attempt, 108 without, with the FP32 one
-// 112; 120,000 x 5,000 with 50: 831, 575 and 584; at 1,000 columns the FP64
-// attempt costs 4 of 48 ms, and the FP32 one would cost well-conditioned solves 8 %.
+// columns that depend on the others, or that its later passes cannot resolve (the
+// FP64 sweep then almost surely ends in a refusal, after the FP64 Gram matrix).  From
+// kGramProbeCols columns on.  Sparse 40,000 x 2,000, 20 dependent columns: 128 ms with
+// the FP64 attempt, 108 without, 112 with the FP32 one; 120,000 x 5,000 with 50: 831,
+// 575 and 584.  Dense 30,000 x 3,500, condition number 1e9: 423 and 331 with the FP32
+// one.  At 1,000 columns the FP64 attempt costs 4 of 48 ms, and the FP32 one would
+// cost well-conditioned solves 8 %.
 // Uses gram_probe_bytes of work, Mc and Mr as scratch.
 constexpr int64_t kGramProbeCols = 1500;
 size_t gram_probe_bytes(int64_t m, int64_t d, int64_t ld);
