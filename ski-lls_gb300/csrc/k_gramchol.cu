@@ -28,7 +28,7 @@
 // QR and inverse 20.2 + 1.4 ms, one pass ~3.3 ms, two (condition number 1e3 to
 // 1e4) 7.4 ms, three (to 1e6) 11.4 with LSQR's iterations, x and residual unchanged.
 // From ~3e6 on at that size (12,007 x 1,201: 1e7) M is too large for the rank proof,
-// and the QR comes on top of the passes.
+// and the QR comes on top of two passes.
 // The sparse path takes the later passes where no pivot failed but the bound on M D
 // does, or where the dropped columns are all at least four thresholds away from
 // dependence (120,000 x 5,000, S A 8,500 x 5,000: 11.2 and 16 to 19 ms; the QR and
@@ -1545,6 +1545,10 @@ bool gram_precond(const T* SA, int64_t m, int64_t d, int64_t ld, double* c, int*
             mf2 = hp[2];
             if (!std::isfinite(mf2) || !resolves()) return false;
             if (last) break;
+            // raised pivots understate M: with 0.28 and more of the FP32 resolution here,
+            // all of ten third passes ended beyond it (12,007 x 1,201 to 40,000 x 4,000);
+            // 12,000 x 4,500, condition number 1e7: a refusal costs 8.1 ms instead of 12
+            if (hp[7] != 0.0 && unit * std::sqrt(mf2) > 0.3) return false;
             if (pass == 3) return false;
         }
         R = B.Racc;
